@@ -319,291 +319,479 @@ li_bwd_apply_rev_kernel(const bf16* __restrict__ feat, const bf16* __restrict__ 
 
 // ------------------------------------------------------------------------------------ tiled kernels
 // The kernels above walk the sequence with 2-byte loads at a stride of a whole row: a warp moves 192 useful bytes per
-// step with 96 load instructions, and the time loop waits on them.  The tiled kernels below (D % 8 == 0) stage
-// [rows x 128 channels] tiles of the interleaved features in shared memory with 16-byte asynchronous copies that are all
-// in flight at once, run the recurrences out of shared memory, and store their outputs as 16-byte chunks.
-//   forward   local / apply: sub-tiles of LT_ROWS steps, double buffered, any chunk length that is a multiple of LT_ROWS
-//   backward  one kernel per chunk of LB_TC steps holds the chunk's features, dz and dx1 in shared memory: the forward
-//             sweep (state, sensitivity: y, dx1, filter-gradient partials) and the reverse sweep (adjoint: du) run back
-//             to back, so dx1 never goes through global memory and the chunk is read once.
-constexpr int LT_ROWS = 16, LT_CH = 128;
-constexpr int LB_TC = 64;
+// step with 96 load instructions, and the time loop waits on them.  The tiled kernels below (D % 8 == 0, 16-byte aligned
+// tensors) stage rows of the interleaved features in shared memory with 16-byte asynchronous copies and run the
+// recurrences out of it.
+//
+// One thread owns TWO neighbouring channels and carries every fp32 quantity as a (channel, channel + 1) pair in a 64-bit
+// register, so each recurrence step is one packed `fma.rn.f32x2`.  With one channel per thread these kernels were bound
+// by shared memory: the three 2-byte reads of an interleaved (x1, x2, v) triple hit 16 of the 32 banks twice.  The pair's
+// 12 bytes are three 32-bit words at a stride of three words between lanes - every bank once - and the word layout
+// (x1 x2 | v x1 | x2 v) unpacks with one shift or mask per value.
+//   forward   local / apply: a ring of LV_STAGES tiles of LV_ROWS steps, any chunk length; z leaves straight from
+//             registers (a warp stores 128 contiguous bytes per step)
+//   backward  chunks of LB_TC steps resident in shared memory.  `li_bwd_local`: two warps run the state forward, two the
+//             adjoint backward.  `li_bwd_apply`: three roles of two warps share the staged chunk: (1) y, dx1 and the dR
+//             partials, (2) the dlam partials, (3) the adjoint, dx2 and dv.
+// The backward carries the adjoint without the residues, ah[t] = dy[t] + lam ah[t+1] (a = R ah; one FMA less per mode and
+// step), and takes the pole gradient chunk by chunk from the sensitivity w[t] = ds[t]/dlam WITHIN the chunk (w = 0 at its
+// left edge):
+//     dlam = R ( sum_t dy[t] w[t] + lam ah(right edge) w(last step) ),
+// the second term being what the chunk's end state still does to the rest of the sequence.  So no sensitivity is passed
+// between chunks: the prefix pass carries two arrays instead of three.
+//
+// Measured at B = 1, L = 8192, D = 4096 on a B200 (us; in brackets the one-channel-per-thread kernels these replace):
+// forward 43 + 10 + 81 (55 + 29 + 95), backward 80 + 54 + 272 + 18 (143 + 156 + 319 and about ten tensor operations that
+// prepared the filter and summed the partials).  Forward and backward with their host side: 848 -> 567.  The recurrences
+// need 48 FMA per value forward and 144 backward, 54 and 163 us at the 30 TFMA/s that packed and plain FMA both reach here
+// (the packed form only halves the issue slots), so the sweeps sit between that bound and the copy time of their data.
+typedef unsigned long long f2;           // two packed fp32 values
+__device__ __forceinline__ f2 f2_pack(float a, float b) { f2 d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b)); return d; }
+__device__ __forceinline__ float2 f2_unpack(f2 v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) { f2 d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) { f2 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) { f2 d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ float lo_f(uint32_t w) { return __uint_as_float(w << 16); }
+__device__ __forceinline__ float hi_f(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
+__device__ __forceinline__ uint32_t pack_bf2(f2 v) {
+  const float2 t = f2_unpack(v);
+  __nv_bfloat162 r = __floats2bfloat162_rn(t.x, t.y);
+  return *reinterpret_cast<uint32_t*>(&r);
+}
 
-__device__ __forceinline__ void li_cp_async16(void* smem_dst, const void* src, int nbytes) {
-  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(nbytes) : "memory");
+constexpr int LV_CH = 128;               // channels per block
+constexpr int LV_PAIRS = LV_CH / 2;      // threads of one role
+constexpr int LV_ROWS = 16;              // steps per ring tile (forward)
+constexpr int LV_STAGES = 3;
+constexpr int LB_TC = 64;                // chunk length of the backward
+constexpr int LV_FW = 3 * LV_CH / 2;     // 32-bit words per staged feature row
+constexpr int LV_GW = LV_CH / 2;         // 32-bit words per staged row of a [.., D] tensor
+
+// The filter, prepared once per call by li_prep_kernel: log-poles -exp(p) exp(gamma), poles and residues, [D, 16] fp32
+// (modes beyond the order O: pole 0, residue 0).
+struct LiModal { const float* ll; const float* lam; const float* R; int O; };
+
+__global__ void li_prep_kernel(const float* __restrict__ gamma, const float* __restrict__ p, const float* __restrict__ R,
+                               float* __restrict__ out, int D, int O) {
+  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x, n = (size_t)D * LO;
+  if (i >= n) return;
+  const int o = (int)(i % LO);
+  const size_t j = i / LO * O + o;
+  const float ll = o < O ? -expf(p[j]) * expf(gamma[j]) : -1.0e30f;
+  out[i] = ll;
+  out[n + i] = o < O ? expf(ll) : 0.f;
+  out[2 * n + i] = o < O ? R[j] : 0.f;
+}
+
+// [.., D, 16] scratch: rows ch and ch + 1 are 32 consecutive floats
+__device__ __forceinline__ void load_pairs(const float* p, bool live, f2 (&r)[LO]) {
+  float a[LO], b[LO];
+#pragma unroll
+  for (int o = 0; o < LO; ++o) { a[o] = 0.f; b[o] = 0.f; }
+  if (live) { load_vec16(p, a); load_vec16(p + LO, b); }
+#pragma unroll
+  for (int o = 0; o < LO; ++o) r[o] = f2_pack(a[o], b[o]);
+}
+__device__ __forceinline__ void store_pairs(float* p, const f2 (&r)[LO]) {
+  float a[LO], b[LO];
+#pragma unroll
+  for (int o = 0; o < LO; ++o) { const float2 t = f2_unpack(r[o]); a[o] = t.x; b[o] = t.y; }
+  store_vec16(p, a);
+  store_vec16(p + LO, b);
+}
+
+__device__ __forceinline__ void li_cp_async16(uint32_t smem_dst, const void* src, int nbytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_dst), "l"(src), "r"(nbytes) : "memory");
 }
 __device__ __forceinline__ void li_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void li_cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// Stage `rows` feature rows starting at time t_lo (rows beyond t_hi are zero-filled) for channels [c0, c0 + 128) into
-// tile[rows][3 * 128]; chunks of 8 bf16.  `ncv` = number of valid 16-byte chunks per row (channels beyond D: zeros).
-__device__ __forceinline__ void li_stage_feat(bf16 (*tile)[3 * LT_CH], const bf16* feat_b, int t_lo, int t_hi, int rows, int c0,
-                                              int D, int tid, int nthreads) {
-  constexpr int CHK = 3 * LT_CH / 8;                        // 48 chunks per row
-  const int ncv = min(CHK, (3 * (D - c0)) / 8);
-  for (int idx = tid; idx < rows * CHK; idx += nthreads) {
-    const int r = idx / CHK, ch = idx - r * CHK, t = t_lo + r;
-    const bool ok = t < t_hi && ch < ncv;
-    const bf16* src = ok ? feat_b + (size_t)t * 3 * D + 3 * c0 + ch * 8 : feat_b;
-    li_cp_async16(&tile[r][ch * 8], src, ok ? 16 : 0);
-  }
-}
-__device__ __forceinline__ void li_stage_d(bf16 (*tile)[LT_CH], const bf16* g_b, int t_lo, int t_hi, int rows, int c0, int D,
-                                           int tid, int nthreads) {
-  constexpr int CHK = LT_CH / 8;                            // 16 chunks per row
-  const int ncv = min(CHK, (D - c0) / 8);
-  for (int idx = tid; idx < rows * CHK; idx += nthreads) {
-    const int r = idx / CHK, ch = idx - r * CHK, t = t_lo + r;
-    const bool ok = t < t_hi && ch < ncv;
-    const bf16* src = ok ? g_b + (size_t)t * D + c0 + ch * 8 : g_b;
-    li_cp_async16(&tile[r][ch * 8], src, ok ? 16 : 0);
-  }
-}
-
-// pass 1 (tiled): chunk-local end state from a zero state
-__global__ void __launch_bounds__(LT_CH)
-li_local_tiled_kernel(const bf16* __restrict__ feat, const float* __restrict__ loglam, float* __restrict__ Sloc, LiDims d) {
-  __shared__ __align__(16) bf16 fS[2][LT_ROWS][3 * LT_CH];
-  const int tid = threadIdx.x, c0 = blockIdx.x * LT_CH, ch = c0 + tid;
-  const int n = blockIdx.y, b = blockIdx.z;
-  const bool live = ch < d.D;
-  float lam[LO], s[LO];
-  if (live) load_vec16(loglam + (size_t)ch * LO, lam);
-#pragma unroll
-  for (int o = 0; o < LO; ++o) { lam[o] = live ? __expf(lam[o]) : 0.f; s[o] = 0.f; }
-  const int t0 = n * d.TC, t1 = min(t0 + d.TC, d.L);
-  const bf16* fb = feat + (size_t)b * d.L * 3 * d.D;
-  const int ntile = (t1 - t0 + LT_ROWS - 1) / LT_ROWS;
-  li_stage_feat(fS[0], fb, t0, t1, LT_ROWS, c0, d.D, tid, LT_CH);
-  li_cp_commit();
-  for (int k = 0; k < ntile; ++k) {
-    if (k + 1 < ntile) li_stage_feat(fS[(k + 1) & 1], fb, t0 + (k + 1) * LT_ROWS, t1, LT_ROWS, c0, d.D, tid, LT_CH);
-    li_cp_commit();
-    li_cp_wait<1>();
-    __syncthreads();
-    const bf16 (*T)[3 * LT_CH] = fS[k & 1];
-    const int rows = min(LT_ROWS, t1 - (t0 + k * LT_ROWS));
+// Stage ROWS rows of `src` (row r at src + r * ld elements; rows >= n_rows and 16-byte chunks >= ncv zero-filled) into
+// dst[ROWS][CHK chunks] with NT threads: a thread keeps its chunk column and walks down the rows.
+template <int ROWS, int CHK, int NT>
+__device__ __forceinline__ void li_stage(uint32_t dst, const bf16* src, size_t ld, int n_rows, int ncv, int tid) {
+  constexpr int STEP = NT / CHK;                         // rows staged side by side
+  const int r0 = tid / CHK, c = tid - r0 * CHK;
+  if (r0 >= STEP) return;
+  const bf16* p = src + (size_t)r0 * ld + c * 8;
+  uint32_t q = dst + (r0 * CHK + c) * 16;
 #pragma unroll 8
-    for (int r = 0; r < rows; ++r) {
-      const float u = b2f(T[r][3 * tid + 1]) * b2f(T[r][3 * tid + 2]);
-#pragma unroll
-      for (int o = 0; o < LO; ++o) s[o] = lam[o] * s[o] + u;
-    }
-    __syncthreads();                                        // the buffer is refilled two iterations from now
-  }
-  if (live) store_vec16(Sloc + (((size_t)b * d.NC + n) * d.D + ch) * LO, s);
-}
-
-// pass 3 (tiled): rerun each chunk from its entering state and emit z through a staged tile
-__global__ void __launch_bounds__(LT_CH)
-li_apply_tiled_kernel(const bf16* __restrict__ feat, const float* __restrict__ loglam, const float* __restrict__ R,
-                      const float* __restrict__ bias, const float* __restrict__ Sin, bf16* __restrict__ z, LiDims d) {
-  __shared__ __align__(16) bf16 fS[2][LT_ROWS][3 * LT_CH];
-  __shared__ __align__(16) bf16 zS[LT_ROWS][LT_CH];
-  const int tid = threadIdx.x, c0 = blockIdx.x * LT_CH, ch = c0 + tid;
-  const int n = blockIdx.y, b = blockIdx.z;
-  const bool live = ch < d.D;
-  float lam[LO], s[LO], rr[LO];
-  float be = 0.f;
-  if (live) {
-    load_vec16(loglam + (size_t)ch * LO, lam);
-    load_vec16(R + (size_t)ch * LO, rr);
-    load_vec16(Sin + (((size_t)b * d.NC + n) * d.D + ch) * LO, s);
-    be = bias[ch];
-  }
-#pragma unroll
-  for (int o = 0; o < LO; ++o) { lam[o] = live ? __expf(lam[o]) : 0.f; if (!live) { s[o] = 0.f; rr[o] = 0.f; } }
-  const int t0 = n * d.TC, t1 = min(t0 + d.TC, d.L);
-  const bf16* fb = feat + (size_t)b * d.L * 3 * d.D;
-  bf16* zb = z + (size_t)b * d.L * d.D;
-  const int ntile = (t1 - t0 + LT_ROWS - 1) / LT_ROWS;
-  const int zcv = min(LT_CH / 8, (d.D - c0) / 8);
-  li_stage_feat(fS[0], fb, t0, t1, LT_ROWS, c0, d.D, tid, LT_CH);
-  li_cp_commit();
-  for (int k = 0; k < ntile; ++k) {
-    if (k + 1 < ntile) li_stage_feat(fS[(k + 1) & 1], fb, t0 + (k + 1) * LT_ROWS, t1, LT_ROWS, c0, d.D, tid, LT_CH);
-    li_cp_commit();
-    li_cp_wait<1>();
-    __syncthreads();
-    const bf16 (*T)[3 * LT_CH] = fS[k & 1];
-    const int tt = t0 + k * LT_ROWS, rows = min(LT_ROWS, t1 - tt);
-#pragma unroll 8
-    for (int r = 0; r < rows; ++r) {
-      const float x1 = b2f(T[r][3 * tid]);
-      const float u = b2f(T[r][3 * tid + 1]) * b2f(T[r][3 * tid + 2]);
-      float y = be * u;
-#pragma unroll
-      for (int o = 0; o < LO; ++o) { s[o] = lam[o] * s[o] + u; y += rr[o] * s[o]; }
-      zS[r][tid] = __float2bfloat16_rn(x1 * y);
-    }
-    __syncthreads();
-    for (int idx = tid; idx < rows * (LT_CH / 8); idx += LT_CH) {
-      const int r = idx / (LT_CH / 8), cv = idx - r * (LT_CH / 8);
-      if (cv < zcv) *reinterpret_cast<uint4*>(zb + (size_t)(tt + r) * d.D + c0 + cv * 8) = *reinterpret_cast<const uint4*>(&zS[r][cv * 8]);
-    }
-    __syncthreads();
+  for (int r = r0; r < ROWS; r += STEP, p += STEP * ld, q += STEP * CHK * 16) {
+    const bool ok = r < n_rows && c < ncv;
+    li_cp_async16(q, ok ? p : src, ok ? 16 : 0);
   }
 }
 
-// backward pass B1 (tiled): Sloc, Wloc, Aloc of a chunk (see li_bwd_local_kernel)
-__global__ void __launch_bounds__(LT_CH)
-li_bwd_local_tiled_kernel(const bf16* __restrict__ feat, const bf16* __restrict__ dz, const float* __restrict__ loglam,
-                          const float* __restrict__ R, float* __restrict__ Sloc, float* __restrict__ Wloc,
-                          float* __restrict__ Aloc, LiDims d) {
-  __shared__ __align__(16) bf16 fS[2][LT_ROWS][3 * LT_CH];
-  __shared__ __align__(16) bf16 gS[2][LT_ROWS][LT_CH];
-  const int tid = threadIdx.x, c0 = blockIdx.x * LT_CH, ch = c0 + tid;
+struct FeatPair { f2 x1, x2, v; };
+__device__ __forceinline__ FeatPair li_feat(const uint32_t* row, int lane3) {
+  const uint32_t w0 = row[lane3], w1 = row[lane3 + 1], w2 = row[lane3 + 2];
+  return FeatPair{f2_pack(lo_f(w0), hi_f(w1)), f2_pack(hi_f(w0), lo_f(w2)), f2_pack(lo_f(w1), hi_f(w2))};
+}
+__device__ __forceinline__ f2 li_pair(const uint32_t* row, int i) { const uint32_t w = row[i]; return f2_pack(lo_f(w), hi_f(w)); }
+
+// forward pass 1 (APPLY = false): end state of each chunk from a zero state.
+// forward pass 3 (APPLY = true): rerun each chunk from its entering state S and emit z.
+template <bool APPLY>
+__global__ void __launch_bounds__(LV_PAIRS)
+li_fwd_tiled_kernel(const bf16* __restrict__ feat, const LiModal m, const float* __restrict__ bias, float* __restrict__ S,
+                    bf16* __restrict__ z, LiDims d) {
+  __shared__ __align__(16) uint32_t ring[LV_STAGES][LV_ROWS][LV_FW];
+  const int tid = threadIdx.x, c0 = blockIdx.x * LV_CH, ch = c0 + 2 * tid;
   const int n = blockIdx.y, b = blockIdx.z;
   const bool live = ch < d.D;
-  float lam[LO], s[LO], w[LO], pw[LO], a[LO];
-  if (live) load_vec16(loglam + (size_t)ch * LO, lam);
-#pragma unroll
-  for (int o = 0; o < LO; ++o) { lam[o] = live ? __expf(lam[o]) : 0.f; s[o] = 0.f; w[o] = 0.f; pw[o] = 1.f; a[o] = 0.f; }
   const int t0 = n * d.TC, t1 = min(t0 + d.TC, d.L);
-  const bf16* fb = feat + (size_t)b * d.L * 3 * d.D;
-  const bf16* gb = dz + (size_t)b * d.L * d.D;
-  const int ntile = (t1 - t0 + LT_ROWS - 1) / LT_ROWS;
-  li_stage_feat(fS[0], fb, t0, t1, LT_ROWS, c0, d.D, tid, LT_CH);
-  li_stage_d(gS[0], gb, t0, t1, LT_ROWS, c0, d.D, tid, LT_CH);
-  li_cp_commit();
-  for (int k = 0; k < ntile; ++k) {
-    if (k + 1 < ntile) {
-      li_stage_feat(fS[(k + 1) & 1], fb, t0 + (k + 1) * LT_ROWS, t1, LT_ROWS, c0, d.D, tid, LT_CH);
-      li_stage_d(gS[(k + 1) & 1], gb, t0 + (k + 1) * LT_ROWS, t1, LT_ROWS, c0, d.D, tid, LT_CH);
-    }
+  const size_t ld = (size_t)3 * d.D;
+  const bf16* src = feat + ((size_t)b * d.L + t0) * ld + 3 * c0;
+  const int ncv = min(3 * LV_CH / 8, 3 * (d.D - c0) / 8);
+  const int ntile = (t1 - t0 + LV_ROWS - 1) / LV_ROWS;
+  const uint32_t ring_a = static_cast<uint32_t>(__cvta_generic_to_shared(&ring[0][0][0]));
+  constexpr uint32_t TILE_B = LV_ROWS * LV_FW * 4;
+#pragma unroll
+  for (int k = 0; k < LV_STAGES - 1; ++k) {
+    if (k < ntile)
+      li_stage<LV_ROWS, 3 * LV_CH / 8, LV_PAIRS>(ring_a + k * TILE_B, src + (size_t)k * LV_ROWS * ld, ld, t1 - t0 - k * LV_ROWS, ncv, tid);
     li_cp_commit();
-    li_cp_wait<1>();
-    __syncthreads();
-    const bf16 (*T)[3 * LT_CH] = fS[k & 1];
-    const bf16 (*G)[LT_CH] = gS[k & 1];
-    const int rows = min(LT_ROWS, t1 - (t0 + k * LT_ROWS));
+  }
+  f2 lam[LO], s[LO], rr[APPLY ? LO : 1], be = 0;
+  load_pairs(m.lam + (size_t)ch * LO, live, lam);
+  float* Sp = S + (((size_t)b * d.NC + n) * d.D + ch) * LO;
+  if constexpr (APPLY) {
+    load_pairs(m.R + (size_t)ch * LO, live, rr);
+    load_pairs(Sp, live, s);
+    if (live) be = f2_pack(bias[ch], bias[ch + 1]);
+  } else {
+#pragma unroll
+    for (int o = 0; o < LO; ++o) s[o] = 0;
+  }
+  uint32_t* zo = APPLY ? reinterpret_cast<uint32_t*>(z + ((size_t)b * d.L + t0) * d.D + ch) : nullptr;
+  const size_t zld = d.D / 2;
+  for (int k = 0; k < ntile; ++k) {
+    li_cp_wait<LV_STAGES - 2>();
+    __syncthreads();                     // tile k has landed for everyone; everyone is done with tile k - 1's buffer
+    const int kn = k + LV_STAGES - 1;
+    if (kn < ntile)
+      li_stage<LV_ROWS, 3 * LV_CH / 8, LV_PAIRS>(ring_a + (kn % LV_STAGES) * TILE_B, src + (size_t)kn * LV_ROWS * ld, ld,
+                                                 t1 - t0 - kn * LV_ROWS, ncv, tid);
+    li_cp_commit();
+    const uint32_t (*T)[LV_FW] = ring[k % LV_STAGES];
+    const int rows = min(LV_ROWS, t1 - t0 - k * LV_ROWS);
+    auto step = [&](int r) {
+      const FeatPair f = li_feat(T[r], 3 * tid);
+      const f2 u = f2_mul(f.x2, f.v);
+      if constexpr (APPLY) {
+        f2 y0 = f2_mul(be, u), y1 = 0;
+#pragma unroll
+        for (int o = 0; o < LO; o += 2) {
+          s[o] = f2_fma(lam[o], s[o], u);
+          s[o + 1] = f2_fma(lam[o + 1], s[o + 1], u);
+          y0 = f2_fma(rr[o], s[o], y0);
+          y1 = f2_fma(rr[o + 1], s[o + 1], y1);
+        }
+        if (live) zo[0] = pack_bf2(f2_mul(f.x1, f2_add(y0, y1)));
+        zo += zld;
+      } else {
+#pragma unroll
+        for (int o = 0; o < LO; ++o) s[o] = f2_fma(lam[o], s[o], u);
+      }
+    };
+    if (rows == LV_ROWS) {
 #pragma unroll 4
-    for (int r = 0; r < rows; ++r) {
-      const float u = b2f(T[r][3 * tid + 1]) * b2f(T[r][3 * tid + 2]);
-      const float dy = b2f(G[r][tid]) * b2f(T[r][3 * tid]);
+      for (int r = 0; r < LV_ROWS; ++r) step(r);
+    } else {
+#pragma unroll 1
+      for (int r = 0; r < rows; ++r) step(r);
+    }
+  }
+  if constexpr (!APPLY) {
+    if (live) store_pairs(Sp, s);
+  }
+}
+
+// Exclusive prefix of the chunk states over the chunks, in place (see li_prefix_kernel): one thread per (b, ch, o), the
+// loads of 16 chunks in flight ahead of the serial carry.  REVERSE: exclusive suffix (the adjoint).  `scale`: factor on the
+// local terms; `carry`: what enters at the first chunk; `tail`: gradient of the returned state (REVERSE).
+constexpr int LP_AHEAD = 16;
+template <bool REVERSE>
+__device__ __forceinline__ float li_carry(float* __restrict__ p, size_t per_b, float ll, float scale, float carry, float tail,
+                                          const LiDims& d) {
+  const float step = expf(ll * d.TC);
+  for (int k0 = 0; k0 < d.NC; k0 += LP_AHEAD) {
+    float loc[LP_AHEAD];
 #pragma unroll
-      for (int o = 0; o < LO; ++o) {
-        w[o] = s[o] + lam[o] * w[o];
-        s[o] = lam[o] * s[o] + u;
-        a[o] += pw[o] * dy;
-        pw[o] *= lam[o];
+    for (int j = 0; j < LP_AHEAD; ++j) {
+      const int n = REVERSE ? d.NC - 1 - (k0 + j) : k0 + j;
+      loc[j] = k0 + j < d.NC ? p[(size_t)n * per_b] : 0.f;
+    }
+#pragma unroll
+    for (int j = 0; j < LP_AHEAD; ++j) {
+      if (k0 + j < d.NC) {
+        const int n = REVERSE ? d.NC - 1 - (k0 + j) : k0 + j;
+        p[(size_t)n * per_b] = carry;
+        const int len = min(d.TC, d.L - n * d.TC);
+        carry = fmaf(len == d.TC ? step : expf(ll * len), carry, scale * loc[j]);
+        // the gradient of the returned state enters at the last step without a factor lam (see li_bwd_prefix_kernel)
+        if (REVERSE && n == d.NC - 1 && tail != 0.f) carry += expf(ll * (len - 1)) * tail;
       }
     }
-    __syncthreads();
   }
-  if (!live) return;
-  float rr[LO];
-  load_vec16(R + (size_t)ch * LO, rr);
-#pragma unroll
-  for (int o = 0; o < LO; ++o) a[o] *= rr[o];
-  const size_t off = (((size_t)b * d.NC + n) * d.D + ch) * LO;
-  store_vec16(Sloc + off, s);
-  store_vec16(Wloc + off, w);
-  store_vec16(Aloc + off, a);
+  return carry;
+}
+__device__ __forceinline__ float state_at(const float* s, int b, int ch, int o, const LiModal& m, int D) {
+  return (s && o < m.O) ? s[((size_t)b * D + ch) * m.O + o] : 0.f;
 }
 
-// backward pass B3 + R3 in one kernel (chunk length LB_TC): the chunk's features and dz stay in shared memory between the
-// forward sweep (y, dx1 = dz y into shared memory, partial sums of dR / dlam / dbias) and the reverse sweep (adjoint scan,
-// du; the gradient tile overwrites the feature tile in place and leaves as 16-byte chunks).
-constexpr int LB_SMEM = LB_TC * (3 * LT_CH + LT_CH + LT_CH) * 2;     // features + dz + dx1
-__global__ void __launch_bounds__(LT_CH, 2)
-li_bwd_apply_tiled_kernel(const bf16* __restrict__ feat, const bf16* __restrict__ dz, const float* __restrict__ loglam,
-                          const float* __restrict__ R, const float* __restrict__ bias, const float* __restrict__ Sin,
-                          const float* __restrict__ Win, const float* __restrict__ Ain, bf16* __restrict__ dfeat,
-                          float* __restrict__ dRp, float* __restrict__ dLp, float* __restrict__ dBp,
-                          const float* __restrict__ dstate_out, LiDims d) {
-  extern __shared__ __align__(16) uint8_t li_smem[];
-  bf16 (*fS)[3 * LT_CH] = reinterpret_cast<bf16 (*)[3 * LT_CH]>(li_smem);
-  bf16 (*gS)[LT_CH] = reinterpret_cast<bf16 (*)[LT_CH]>(li_smem + LB_TC * 3 * LT_CH * 2);
-  bf16 (*xS)[LT_CH] = reinterpret_cast<bf16 (*)[LT_CH]>(li_smem + LB_TC * 4 * LT_CH * 2);
-  const int tid = threadIdx.x, c0 = blockIdx.x * LT_CH, ch = c0 + tid;
+__global__ void __launch_bounds__(128)
+li_prefix_tiled_kernel(float* __restrict__ S, const LiModal m, const float* __restrict__ state_in, float* __restrict__ state_out,
+                       LiDims d) {
+  const size_t per_b = (size_t)d.D * LO;
+  const size_t r = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  const int b = blockIdx.y;
+  if (r >= per_b) return;
+  const int ch = (int)(r / LO), o = (int)(r % LO);
+  const float ll = m.ll[r];
+  const float end = li_carry<false>(S + (size_t)b * d.NC * per_b + r, per_b, ll, 1.f, state_at(state_in, b, ch, o, m, d.D), 0.f, d);
+  if (state_out && o < m.O) state_out[((size_t)b * d.D + ch) * m.O + o] = end;
+}
+
+// Backward prefixes: blockIdx.z = 0 the states, 1 the adjoints (scaled by R when a state gradient has to ride along).
+__global__ void __launch_bounds__(128)
+li_bwd_prefix_tiled_kernel(float* __restrict__ S, float* __restrict__ A, const LiModal m, const float* __restrict__ state_in,
+                           const float* __restrict__ dstate_out, float* __restrict__ dstate_in, LiDims d) {
+  const size_t per_b = (size_t)d.D * LO;
+  const size_t r = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  const int b = blockIdx.y;
+  if (r >= per_b) return;
+  const int ch = (int)(r / LO), o = (int)(r % LO);
+  const bool real = o < m.O;
+  const float ll = m.ll[r];
+  const size_t base = (size_t)b * d.NC * per_b + r;
+  if (blockIdx.z == 0) {
+    li_carry<false>(S + base, per_b, ll, 1.f, state_at(state_in, b, ch, o, m, d.D), 0.f, d);
+  } else {
+    const float R = m.R[r];
+    const float end = li_carry<true>(A + base, per_b, ll, dstate_out ? R : 1.f, 0.f, state_at(dstate_out, b, ch, o, m, d.D), d);
+    if (dstate_in && real) dstate_in[((size_t)b * d.D + ch) * m.O + o] = expf(ll) * (dstate_out ? end : R * end);
+  }
+}
+
+// Shared-memory image of a backward chunk: features and dz as they are in memory.
+constexpr int LBL_SMEM = LB_TC * (LV_FW + LV_GW) * 4;            // 64 KB
+constexpr int LBA_SMEM = LBL_SMEM + LB_TC * LV_FW * 4;           // + the gradient tile: 112 KB, two blocks per SM
+
+// backward pass 1: end state (Sloc, warps 0-1) and adjoint leaving the left edge (Aloc, warps 2-3) of every chunk
+__global__ void __launch_bounds__(2 * LV_PAIRS)
+li_bwd_local_tiled_kernel(const bf16* __restrict__ feat, const bf16* __restrict__ dz, const LiModal m, float* __restrict__ S,
+                          float* __restrict__ A, LiDims d) {
+  extern __shared__ __align__(16) uint32_t li_sm[];
+  uint32_t (*fS)[LV_FW] = reinterpret_cast<uint32_t (*)[LV_FW]>(li_sm);
+  uint32_t (*gS)[LV_GW] = reinterpret_cast<uint32_t (*)[LV_GW]>(li_sm + LB_TC * LV_FW);
+  const int tid = threadIdx.x, c0 = blockIdx.x * LV_CH, pair = tid & (LV_PAIRS - 1), ch = c0 + 2 * pair;
   const int n = blockIdx.y, b = blockIdx.z;
   const bool live = ch < d.D;
-  const int t0 = n * LB_TC, t1 = min(t0 + LB_TC, d.L), rows = t1 - t0;
-  const bf16* fb = feat + (size_t)b * d.L * 3 * d.D;
-  const bf16* gb = dz + (size_t)b * d.L * d.D;
-  li_stage_feat(fS, fb, t0, t1, LB_TC, c0, d.D, tid, LT_CH);
-  li_stage_d(gS, gb, t0, t1, LB_TC, c0, d.D, tid, LT_CH);
+  const int t0 = n * LB_TC, rows = min(LB_TC, d.L - t0);
+  const uint32_t f_a = static_cast<uint32_t>(__cvta_generic_to_shared(fS)), g_a = static_cast<uint32_t>(__cvta_generic_to_shared(gS));
+  const int ncf = min(3 * LV_CH / 8, 3 * (d.D - c0) / 8), ncg = min(LV_CH / 8, (d.D - c0) / 8);
+  li_stage<LB_TC, 3 * LV_CH / 8, 2 * LV_PAIRS>(f_a, feat + ((size_t)b * d.L + t0) * 3 * d.D + 3 * c0, (size_t)3 * d.D, rows, ncf, tid);
+  li_stage<LB_TC, LV_CH / 8, 2 * LV_PAIRS>(g_a, dz + ((size_t)b * d.L + t0) * d.D + c0, d.D, rows, ncg, tid);
   li_cp_commit();
-  float lam[LO], rr[LO];
-  float be = 0.f;
-  const size_t off = (((size_t)b * d.NC + n) * d.D + ch) * LO;
-  if (live) { load_vec16(loglam + (size_t)ch * LO, lam); load_vec16(R + (size_t)ch * LO, rr); be = bias[ch]; }
+  f2 lam[LO], s[LO];
+  load_pairs(m.lam + (size_t)ch * LO, live, lam);
 #pragma unroll
-  for (int o = 0; o < LO; ++o) { lam[o] = live ? __expf(lam[o]) : 0.f; if (!live) rr[o] = 0.f; }
+  for (int o = 0; o < LO; ++o) s[o] = 0;
   li_cp_wait<0>();
   __syncthreads();
-  {
-    // ---- forward sweep
-    float s[LO], w[LO], dr[LO], dl[LO];
-    if (live) { load_vec16(Sin + off, s); load_vec16(Win + off, w); }
-#pragma unroll
-    for (int o = 0; o < LO; ++o) { dr[o] = 0.f; dl[o] = 0.f; if (!live) { s[o] = 0.f; w[o] = 0.f; } }
-    float db = 0.f;
+  float* out;
+  if (tid < LV_PAIRS) {
 #pragma unroll 4
     for (int r = 0; r < rows; ++r) {
-      const float x1 = b2f(fS[r][3 * tid]);
-      const float u = b2f(fS[r][3 * tid + 1]) * b2f(fS[r][3 * tid + 2]);
-      const float gz = b2f(gS[r][tid]);
-      const float dy = gz * x1;
-      float y = be * u;
+      const FeatPair f = li_feat(fS[r], 3 * pair);
+      const f2 u = f2_mul(f.x2, f.v);
 #pragma unroll
-      for (int o = 0; o < LO; ++o) {
-        w[o] = s[o] + lam[o] * w[o];
-        s[o] = lam[o] * s[o] + u;
-        y += rr[o] * s[o];
-        dr[o] += dy * s[o];
-        dl[o] += dy * w[o];
-      }
-      db += dy * u;
-      xS[r][tid] = __float2bfloat16_rn(gz * y);
+      for (int o = 0; o < LO; ++o) s[o] = f2_fma(lam[o], s[o], u);
     }
-    if (live) {
-#pragma unroll
-      for (int o = 0; o < LO; ++o) dl[o] *= rr[o];
-      store_vec16(dRp + off, dr);
-      store_vec16(dLp + off, dl);
-      dBp[((size_t)b * d.NC + n) * d.D + ch] = db;
-    }
-  }
-  {
-    // ---- reverse sweep (each thread touches only its own three tile entries: no barrier needed in between)
-    float a[LO], gs[LO];
-    if (live) load_vec16(Ain + off, a);
-    const bool tail = dstate_out != nullptr && n == d.NC - 1 && live;
-    if (tail) load_vec16(dstate_out + ((size_t)b * d.D + ch) * LO, gs);
-#pragma unroll
-    for (int o = 0; o < LO; ++o) { if (!live) a[o] = 0.f; if (!tail) gs[o] = 0.f; }
+    out = S;
+  } else {
 #pragma unroll 4
     for (int r = rows - 1; r >= 0; --r) {
-      const float x1 = b2f(fS[r][3 * tid]), x2 = b2f(fS[r][3 * tid + 1]), v = b2f(fS[r][3 * tid + 2]);
-      const float dy = b2f(gS[r][tid]) * x1;
-      float du = be * dy;
+      const f2 dy = f2_mul(li_pair(gS[r], pair), f2_pack(lo_f(fS[r][3 * pair]), hi_f(fS[r][3 * pair + 1])));
 #pragma unroll
-      for (int o = 0; o < LO; ++o) a[o] = rr[o] * dy + lam[o] * a[o];
-      if (tail && r == rows - 1) {
+      for (int o = 0; o < LO; ++o) s[o] = f2_fma(lam[o], s[o], dy);
+    }
+    out = A;
+  }
+  if (live) store_pairs(out + (((size_t)b * d.NC + n) * d.D + ch) * LO, s);
+}
+
+// backward pass 3: see the head of this section.  S and A hold the entering state / adjoint of every chunk and are
+// overwritten with the chunk's partial sums of dR and dlam (dlam without the factor R unless GOUT).  GOUT: the caller has a
+// gradient of the final state; the adjoint then carries R and that gradient (dstate_out, [B, D, O]).
+template <bool GOUT>
+__global__ void __launch_bounds__(3 * LV_PAIRS, 2)
+li_bwd_apply_tiled_kernel(const bf16* __restrict__ feat, const bf16* __restrict__ dz, const LiModal m, const float* __restrict__ bias,
+                          float* __restrict__ S, float* __restrict__ A, float* __restrict__ dBp, bf16* __restrict__ dfeat,
+                          const float* __restrict__ dstate_out, LiDims d) {
+  extern __shared__ __align__(16) uint32_t li_sm[];
+  uint32_t (*fS)[LV_FW] = reinterpret_cast<uint32_t (*)[LV_FW]>(li_sm);
+  uint32_t (*gS)[LV_GW] = reinterpret_cast<uint32_t (*)[LV_GW]>(li_sm + LB_TC * LV_FW);
+  uint32_t (*oS)[LV_FW] = reinterpret_cast<uint32_t (*)[LV_FW]>(li_sm + LB_TC * (LV_FW + LV_GW));
+  constexpr int NT = 3 * LV_PAIRS;
+  const int tid = threadIdx.x, c0 = blockIdx.x * LV_CH, role = tid / LV_PAIRS, pair = tid - role * LV_PAIRS, ch = c0 + 2 * pair;
+  const int n = blockIdx.y, b = blockIdx.z;
+  const bool live = ch < d.D;
+  const int t0 = n * LB_TC, rows = min(LB_TC, d.L - t0);
+  const uint32_t f_a = static_cast<uint32_t>(__cvta_generic_to_shared(fS)), g_a = static_cast<uint32_t>(__cvta_generic_to_shared(gS));
+  const int ncf = min(3 * LV_CH / 8, 3 * (d.D - c0) / 8), ncg = min(LV_CH / 8, (d.D - c0) / 8);
+  li_stage<LB_TC, 3 * LV_CH / 8, NT>(f_a, feat + ((size_t)b * d.L + t0) * 3 * d.D + 3 * c0, (size_t)3 * d.D, rows, ncf, tid);
+  li_stage<LB_TC, LV_CH / 8, NT>(g_a, dz + ((size_t)b * d.L + t0) * d.D + c0, d.D, rows, ncg, tid);
+  li_cp_commit();
+  const size_t off = (((size_t)b * d.NC + n) * d.D + ch) * LO;
+  f2 lam[LO], s[LO];                                     // s: state (roles 0, 1) or adjoint (role 2) entering the chunk
+  load_pairs(m.lam + (size_t)ch * LO, live, lam);
+  load_pairs((role == 2 ? A : S) + off, live, s);
+  li_cp_wait<0>();
+  __syncthreads();                                       // the chunk has landed; S and A of this block have been read
+  if (role == 0) {
+    f2 rr[LO], dr[LO], be = 0, db = 0;
+    load_pairs(m.R + (size_t)ch * LO, live, rr);
+    if (live) be = f2_pack(bias[ch], bias[ch + 1]);
 #pragma unroll
-        for (int o = 0; o < LO; ++o) a[o] += gs[o];
+    for (int o = 0; o < LO; ++o) dr[o] = 0;
+#pragma unroll 2
+    for (int r = 0; r < rows; ++r) {
+      const FeatPair f = li_feat(fS[r], 3 * pair);
+      const f2 u = f2_mul(f.x2, f.v), gz = li_pair(gS[r], pair), dy = f2_mul(gz, f.x1);
+      f2 y0 = f2_mul(be, u), y1 = 0;
+#pragma unroll
+      for (int o = 0; o < LO; o += 2) {
+        s[o] = f2_fma(lam[o], s[o], u);
+        s[o + 1] = f2_fma(lam[o + 1], s[o + 1], u);
+        y0 = f2_fma(rr[o], s[o], y0);
+        y1 = f2_fma(rr[o + 1], s[o + 1], y1);
+        dr[o] = f2_fma(dy, s[o], dr[o]);
+        dr[o + 1] = f2_fma(dy, s[o + 1], dr[o + 1]);
       }
+      db = f2_fma(dy, u, db);
+      const uint32_t w = pack_bf2(f2_mul(gz, f2_add(y0, y1)));
+      uint16_t* o16 = reinterpret_cast<uint16_t*>(&oS[r][3 * pair]);
+      o16[0] = (uint16_t)w;
+      o16[3] = (uint16_t)(w >> 16);
+    }
+    if (live) {
+      store_pairs(S + off, dr);
+      const float2 t = f2_unpack(db);
+      *reinterpret_cast<float2*>(dBp + ((size_t)b * d.NC + n) * d.D + ch) = t;
+    }
+  } else if (role == 1) {
+    f2 w[LO], dl[LO];
 #pragma unroll
-      for (int o = 0; o < LO; ++o) du += a[o];
-      fS[r][3 * tid] = xS[r][tid];
-      fS[r][3 * tid + 1] = __float2bfloat16_rn(du * v);
-      fS[r][3 * tid + 2] = __float2bfloat16_rn(du * x2);
+    for (int o = 0; o < LO; ++o) { w[o] = 0; dl[o] = 0; }
+#pragma unroll 2
+    for (int r = 0; r < rows; ++r) {
+      const FeatPair f = li_feat(fS[r], 3 * pair);
+      const f2 u = f2_mul(f.x2, f.v), dy = f2_mul(li_pair(gS[r], pair), f.x1);
+#pragma unroll
+      for (int o = 0; o < LO; ++o) {
+        w[o] = f2_fma(lam[o], w[o], s[o]);
+        s[o] = f2_fma(lam[o], s[o], u);
+        dl[o] = f2_fma(dy, w[o], dl[o]);
+      }
+    }
+    if (live) {
+      f2 a[LO];
+      load_pairs(A + off, true, a);
+#pragma unroll
+      for (int o = 0; o < LO; ++o) {
+        f2 e = f2_mul(lam[o], a[o]);
+        if constexpr (GOUT) {
+          if (n == d.NC - 1)
+            e = f2_add(e, f2_pack(state_at(dstate_out, b, ch, o, m, d.D), state_at(dstate_out, b, ch + 1, o, m, d.D)));
+          dl[o] = f2_mul(f2_pack(m.R[(size_t)ch * LO + o], m.R[(size_t)(ch + 1) * LO + o]), dl[o]);
+        }
+        dl[o] = f2_fma(e, w[o], dl[o]);
+      }
+      store_pairs(A + off, dl);
+    }
+  } else {
+    f2 rr[LO], be = 0;
+    load_pairs(m.R + (size_t)ch * LO, live, rr);
+    if (live) be = f2_pack(bias[ch], bias[ch + 1]);
+#pragma unroll 2
+    for (int r = rows - 1; r >= 0; --r) {
+      const FeatPair f = li_feat(fS[r], 3 * pair);
+      const f2 dy = f2_mul(li_pair(gS[r], pair), f.x1);
+      f2 d0 = f2_mul(be, dy), d1 = 0;
+      if constexpr (GOUT) {
+#pragma unroll
+        for (int o = 0; o < LO; ++o) s[o] = f2_fma(lam[o], s[o], f2_mul(rr[o], dy));
+        if (n == d.NC - 1 && r == rows - 1 && live) {
+#pragma unroll
+          for (int o = 0; o < LO; ++o)
+            s[o] = f2_add(s[o], f2_pack(state_at(dstate_out, b, ch, o, m, d.D), state_at(dstate_out, b, ch + 1, o, m, d.D)));
+        }
+#pragma unroll
+        for (int o = 0; o < LO; o += 2) { d0 = f2_add(d0, s[o]); d1 = f2_add(d1, s[o + 1]); }
+      } else {
+#pragma unroll
+        for (int o = 0; o < LO; o += 2) {
+          s[o] = f2_fma(lam[o], s[o], dy);
+          s[o + 1] = f2_fma(lam[o + 1], s[o + 1], dy);
+          d0 = f2_fma(rr[o], s[o], d0);
+          d1 = f2_fma(rr[o + 1], s[o + 1], d1);
+        }
+      }
+      const f2 du = f2_add(d0, d1);
+      const float2 dx2 = f2_unpack(f2_mul(du, f.v)), dv = f2_unpack(f2_mul(du, f.x2));
+      uint16_t* o16 = reinterpret_cast<uint16_t*>(&oS[r][3 * pair]);
+      o16[1] = __bfloat16_as_ushort(__float2bfloat16_rn(dx2.x));
+      o16[2] = __bfloat16_as_ushort(__float2bfloat16_rn(dv.x));
+      oS[r][3 * pair + 2] = pack_bf2(f2_pack(dx2.y, dv.y));
     }
   }
   __syncthreads();
-  constexpr int CHK = 3 * LT_CH / 8;
-  const int ncv = min(CHK, (3 * (d.D - c0)) / 8);
-  bf16* db_ = dfeat + (size_t)b * d.L * 3 * d.D;
-  for (int idx = tid; idx < rows * CHK; idx += LT_CH) {
-    const int r = idx / CHK, cv = idx - r * CHK;
-    if (cv < ncv) *reinterpret_cast<uint4*>(db_ + (size_t)(t0 + r) * 3 * d.D + 3 * c0 + cv * 8) = *reinterpret_cast<const uint4*>(&fS[r][cv * 8]);
+  bf16* dst = dfeat + ((size_t)b * d.L + t0) * 3 * d.D + 3 * c0;
+  constexpr int CHK = 3 * LV_CH / 8;
+  for (int idx = tid; idx < rows * CHK; idx += NT) {
+    const int r = idx / CHK, c = idx - r * CHK;
+    if (c < ncf) *reinterpret_cast<uint4*>(dst + (size_t)r * 3 * d.D + c * 8) = *reinterpret_cast<const uint4*>(&oS[r][c * 4]);
   }
 }
 
-static int g_li_tiled = 1;
+// Sums the per-chunk partials over batch and chunks (in a fixed order) and finishes the filter gradients:
+//   dR, dgamma = dp = dlam lam log(lam) ([D, O]) and dbias [D].  One thread per (channel, mode) column and row slice.
+constexpr int LR_COLS = 32, LR_SLICES = 8;
+__global__ void __launch_bounds__(LR_COLS * LR_SLICES)
+li_bwd_reduce_kernel(const float* __restrict__ dRp, const float* __restrict__ dLp, const float* __restrict__ dBp, const LiModal m,
+                     int scale_by_R, float* __restrict__ dR, float* __restrict__ dll, float* __restrict__ db, int n_rows, int D) {
+  __shared__ float red[2][LR_SLICES][LR_COLS];
+  const int cx = threadIdx.x % LR_COLS, sl = threadIdx.x / LR_COLS;
+  const int n_modal = (D * LO + LR_COLS - 1) / LR_COLS;              // blocks [0, n_modal): dR / dlam; the rest: dbias
+  const bool modal = (int)blockIdx.x < n_modal;
+  const size_t width = modal ? (size_t)D * LO : (size_t)D;
+  const size_t col = (size_t)(modal ? blockIdx.x : blockIdx.x - n_modal) * LR_COLS + cx;
+  float a0 = 0.f, a1 = 0.f;
+  if (col < width) {
+    if (modal) {
+#pragma unroll 4
+      for (int i = sl; i < n_rows; i += LR_SLICES) { a0 += dRp[(size_t)i * width + col]; a1 += dLp[(size_t)i * width + col]; }
+    } else {
+#pragma unroll 4
+      for (int i = sl; i < n_rows; i += LR_SLICES) a0 += dBp[(size_t)i * width + col];
+    }
+  }
+  red[0][sl][cx] = a0;
+  red[1][sl][cx] = a1;
+  __syncthreads();
+  if (sl || col >= width) return;
+#pragma unroll
+  for (int j = 1; j < LR_SLICES; ++j) { a0 += red[0][j][cx]; a1 += red[1][j][cx]; }
+  if (!modal) { db[col] = a0; return; }
+  const int ch = (int)(col / LO), o = (int)(col % LO);
+  if (o >= m.O) return;
+  const size_t i = (size_t)ch * m.O + o;
+  dR[i] = a0;
+  const float g = (scale_by_R ? m.R[col] * a1 : a1) * m.lam[col] * m.ll[col];
+  dll[i] = isfinite(g) ? g : 0.f;
+}
 
 // ------------------------------------------------------------------------------------ context parallel: all-to-all inside the scan
 // Sequence-sharded ranks (zigzag: rank r holds natural chunks r and 2cp-1-r of `chunk_len` rows, [B, l, Dtot] with
@@ -881,23 +1069,60 @@ extern "C" int sb_li_fwd(const void* feat, const float* loglam, const float* R, 
   LiDims d = li_dims(B, L, D, TC);
   dim3 grid((D + LI_THREADS - 1) / LI_THREADS, d.NC, B);
   const size_t n = (size_t)B * D * LO;
-  if (g_li_tiled && D % 8 == 0 && TC % LT_ROWS == 0) {
-    li_local_tiled_kernel<<<grid, LT_CH, 0, st>>>((const bf16*)feat, loglam, S_scratch, d);
-    li_prefix_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(S_scratch, loglam, state_in, state_out, d);
-    li_apply_tiled_kernel<<<grid, LT_CH, 0, st>>>((const bf16*)feat, loglam, R, bias, S_scratch, (bf16*)z, d);
-    return cudaGetLastError() == cudaSuccess ? 0 : -2;
-  }
   li_local_kernel<<<grid, LI_THREADS, 0, st>>>((const bf16*)feat, loglam, S_scratch, d);
   li_prefix_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(S_scratch, loglam, state_in, state_out, d);
   li_apply_kernel<<<grid, LI_THREADS, 0, st>>>((const bf16*)feat, loglam, R, bias, S_scratch, (bf16*)z, d);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-// 1 (default): shared-memory tiled scan kernels where the shape allows; 0: the per-thread streaming kernels
-extern "C" int sb_li_set_variant(int tiled) { sb::g_li_tiled = tiled ? 1 : 0; return 0; }
-// Chunk length the backward pass uses for a given forward choice: the tiled backward keeps a whole chunk in shared memory
-// and therefore fixes its own chunk length; callers size the scratch arrays with the value returned here.
-extern "C" int sb_li_bwd_chunk(int D, int TC) { return (sb::g_li_tiled && D % 8 == 0) ? sb::LB_TC : TC; }
+// Tiled forward: gamma, p, R [D, O] fp32 (O <= 16), state_in / state_out [B, D, O] or null.  Scratch: modal 3*D*16 floats
+// (the prepared filter, which the backward takes over), S B*NC*D*16 floats.  D % 8 == 0, feat and z 16-byte aligned.
+extern "C" int sb_li_fwd_tiled(const void* feat, const float* gamma, const float* p, const float* R, const float* bias,
+                               const float* state_in, float* state_out, float* modal, float* S, void* z, int B, int L, int D, int O,
+                               int TC, cudaStream_t st) {
+  if ((D % 8) || O < 1 || O > LO || TC < 1 || ((uintptr_t)feat % 16) || ((uintptr_t)z % 16)) return -1;
+  if ((long long)B * L * D == 0) return 0;
+  LiDims d = li_dims(B, L, D, TC);
+  const size_t n = (size_t)D * LO;
+  const LiModal m{modal, modal + n, modal + 2 * n, O};
+  dim3 grid((D + LV_CH - 1) / LV_CH, d.NC, B);
+  li_prep_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(gamma, p, R, modal, D, O);
+  li_fwd_tiled_kernel<false><<<grid, LV_PAIRS, 0, st>>>((const bf16*)feat, m, bias, S, nullptr, d);
+  li_prefix_tiled_kernel<<<dim3((unsigned)((n + 127) / 128), B), 128, 0, st>>>(S, m, state_in, state_out, d);
+  li_fwd_tiled_kernel<true><<<grid, LV_PAIRS, 0, st>>>((const bf16*)feat, m, bias, S, (bf16*)z, d);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+extern "C" int sb_li_bwd_tiled_chunk() { return LB_TC; }
+
+// Tiled backward, chunk length sb_li_bwd_tiled_chunk().  modal: as the forward left it.  Scratch: S, A B*NC*D*16 floats,
+// dBp B*NC*D floats.  Outputs: dfeat, dR and dll = dgamma = dp [D, O], db [D], dstate_in [B, D, O] or null.
+extern "C" int sb_li_bwd_tiled(const void* feat, const void* dz, const float* modal, const float* bias, const float* state_in,
+                               const float* dstate_out, float* S, float* A, float* dBp, void* dfeat, float* dR, float* dll,
+                               float* db, float* dstate_in, int B, int L, int D, int O, cudaStream_t st) {
+  if ((D % 8) || O < 1 || O > LO || ((uintptr_t)feat % 16) || ((uintptr_t)dz % 16) || ((uintptr_t)dfeat % 16)) return -1;
+  if ((long long)B * L * D == 0) return 0;
+  // function attributes belong to the current device's context: set on every call (they cost a lookup)
+  if (cudaFuncSetAttribute(li_bwd_local_tiled_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LBL_SMEM) != cudaSuccess ||
+      cudaFuncSetAttribute(li_bwd_apply_tiled_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, LBA_SMEM) != cudaSuccess ||
+      cudaFuncSetAttribute(li_bwd_apply_tiled_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, LBA_SMEM) != cudaSuccess)
+    return -5;
+  LiDims d = li_dims(B, L, D, LB_TC);
+  const size_t n = (size_t)D * LO;
+  const LiModal m{modal, modal + n, modal + 2 * n, O};
+  const dim3 grid((D + LV_CH - 1) / LV_CH, d.NC, B);
+  li_bwd_local_tiled_kernel<<<grid, 2 * LV_PAIRS, LBL_SMEM, st>>>((const bf16*)feat, (const bf16*)dz, m, S, A, d);
+  li_bwd_prefix_tiled_kernel<<<dim3((unsigned)((n + 127) / 128), B, 2), 128, 0, st>>>(S, A, m, state_in, dstate_out, dstate_in, d);
+  if (dstate_out)
+    li_bwd_apply_tiled_kernel<true><<<grid, 3 * LV_PAIRS, LBA_SMEM, st>>>((const bf16*)feat, (const bf16*)dz, m, bias, S, A, dBp,
+                                                                         (bf16*)dfeat, dstate_out, d);
+  else
+    li_bwd_apply_tiled_kernel<false><<<grid, 3 * LV_PAIRS, LBA_SMEM, st>>>((const bf16*)feat, (const bf16*)dz, m, bias, S, A, dBp,
+                                                                          (bf16*)dfeat, nullptr, d);
+  const unsigned blocks = (unsigned)((n + LR_COLS - 1) / LR_COLS + (D + LR_COLS - 1) / LR_COLS);
+  li_bwd_reduce_kernel<<<blocks, LR_COLS * LR_SLICES, 0, st>>>(S, A, dBp, m, dstate_out ? 0 : 1, dR, dll, db, B * d.NC, D);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
 
 // Scratch: S, W, A, dRp, dLp each B*NC*D*16 floats; dBp B*NC*D floats; dx1_tmp B*L*D bf16.
 // Outputs: dfeat; per-chunk partials dRp/dLp/dBp (the caller sums over B and NC); w_end, dstate_in optional.
@@ -909,18 +1134,6 @@ extern "C" int sb_li_bwd(const void* feat, const void* dz, const float* loglam, 
   LiDims d = li_dims(B, L, D, TC);
   dim3 grid((D + LI_THREADS - 1) / LI_THREADS, d.NC, B);
   const size_t n = (size_t)B * D * LO;
-  if (g_li_tiled && D % 8 == 0 && TC == LB_TC) {
-    static bool attr = false;
-    if (!attr) {
-      if (cudaFuncSetAttribute(li_bwd_apply_tiled_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LB_SMEM) != cudaSuccess) return -5;
-      attr = true;
-    }
-    li_bwd_local_tiled_kernel<<<grid, LT_CH, 0, st>>>((const bf16*)feat, (const bf16*)dz, loglam, R, S, W, A, d);
-    li_bwd_prefix_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(S, W, A, loglam, state_in, dstate_out, w_end, dstate_in, d);
-    li_bwd_apply_tiled_kernel<<<grid, LT_CH, LB_SMEM, st>>>((const bf16*)feat, (const bf16*)dz, loglam, R, bias, S, W, A,
-                                                           (bf16*)dfeat, dRp, dLp, dBp, dstate_out, d);
-    return cudaGetLastError() == cudaSuccess ? 0 : -2;
-  }
   li_bwd_local_kernel<<<grid, LI_THREADS, 0, st>>>((const bf16*)feat, (const bf16*)dz, loglam, R, S, W, A, d);
   li_bwd_prefix_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(S, W, A, loglam, state_in, dstate_out, w_end, dstate_in, d);
   li_bwd_apply_fwd_kernel<<<grid, LI_THREADS, 0, st>>>((const bf16*)feat, (const bf16*)dz, loglam, R, bias, S, W,

@@ -118,8 +118,9 @@ class _Sig:
     sb_conv_set_fwd_variant = [I]
     sb_mr_tc_bwd = [P, P, P, P, P, P, P, P, P, I, I, I, I, I, P]
     sb_li_fwd = [P, P, P, P, P, P, P, P, I, I, I, I, P]
-    sb_li_set_variant = [I]
-    sb_li_bwd_chunk = [I, I]
+    sb_li_fwd_tiled = [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, P]
+    sb_li_bwd_tiled_chunk = []
+    sb_li_bwd_tiled = [P, P, P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, P]
     sb_li_bwd = [P, P, P, P, P, P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, P]
 
 
@@ -1201,6 +1202,12 @@ def _f32c(t):
     return t.detach().float().contiguous()
 
 
+def _aligned(t):
+    """Contiguous and on a 16-byte boundary (a view into the middle of another tensor need not be)."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 class _DwConv(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, halo):
@@ -1361,7 +1368,6 @@ def set_li_variant(tiled: bool) -> None:
     """True (default): shared-memory tiled scan kernels; False: the per-thread streaming kernels (A/B measurements, tests)."""
     global LI_TILED
     LI_TILED = bool(tiled)
-    require().sb_li_set_variant(int(LI_TILED))
 
 
 def _li_chunk(B: int, L: int, D: int) -> int:
@@ -1376,6 +1382,17 @@ def _li_chunk(B: int, L: int, D: int) -> int:
     return tc
 
 
+def _li_tiled_chunk(B: int, L: int, D: int) -> int:
+    """As `_li_chunk` for the tiled kernels, whose blocks have two warps: small problems go down to chunks of 32 steps to
+    fill the chip (B = 2, L = 1237, D = 1024 forward: 69 us with 128-step chunks of the former kernels, 48 us)."""
+    if LI_CHUNK_OVERRIDE:
+        return int(LI_CHUNK_OVERRIDE)
+    tc = 1024
+    while tc > 32 and B * ((D + 127) // 128) * ((L + tc - 1) // tc) < 2048:
+        tc //= 2
+    return tc
+
+
 def _pad_order(t, fill):
     D, O = t.shape
     if O == LI_ORDER:
@@ -1385,7 +1402,60 @@ def _pad_order(t, fill):
     return out
 
 
+class _HyenaLITiled(torch.autograd.Function):
+    """The shared-memory tiled scan (csrc/li_scan.cu): D % 8 == 0.  The filter is prepared by the forward's first kernel and
+    handed to the backward; the filter gradients come finished out of the backward's last one."""
+
+    @staticmethod
+    def forward(ctx, feat, gamma, R, p, bias, state_in, want_state):
+        lib = require()
+        B, L, C3 = feat.shape
+        D, O = C3 // 3, gamma.shape[1]
+        dev = feat.device
+        fc, bf = _aligned(feat), _f32c(bias)
+        sin = _f32c(state_in) if state_in is not None else None
+        tc = _li_tiled_chunk(B, L, D)
+        modal = _alloc((3, D, LI_ORDER), dtype=torch.float32, device=dev)
+        S = _alloc((B, (L + tc - 1) // tc, D, LI_ORDER), dtype=torch.float32, device=dev)
+        sout = _alloc((B, D, O), dtype=torch.float32, device=dev) if want_state else None
+        z = _alloc((B, L, D), dtype=bf16, device=dev)
+        gf, pf, Rf = _f32c(gamma), _f32c(p), _f32c(R)
+        _check(lib.sb_li_fwd_tiled(fc.data_ptr(), gf.data_ptr(), pf.data_ptr(), Rf.data_ptr(), bf.data_ptr(), _ptr(sin), _ptr(sout),
+                                   modal.data_ptr(), S.data_ptr(), z.data_ptr(), B, L, D, O, tc, _stream()), "li_fwd_tiled")
+        _count(4)
+        ctx.save_for_backward(fc, modal, bf, sin)
+        ctx.meta = (O, gamma.dtype, R.dtype, p.dtype, bias.dtype, want_state)
+        return z, sout
+
+    @staticmethod
+    def backward(ctx, gz, gstate):
+        lib = require()
+        fc, modal, bf, sin = ctx.saved_tensors
+        O, gdt, rdt, pdt, bdt, want_state = ctx.meta
+        B, L, C3 = fc.shape
+        D = C3 // 3
+        dev = fc.device
+        tc = int(lib.sb_li_bwd_tiled_chunk())
+        NC = (L + tc - 1) // tc
+        g = _aligned(gz)
+        S, A = (_alloc((B, NC, D, LI_ORDER), dtype=torch.float32, device=dev) for _ in range(2))
+        dBp = _alloc((B, NC, D), dtype=torch.float32, device=dev)
+        df = _alloc_like(fc)
+        dso = _f32c(gstate) if (want_state and gstate is not None) else None
+        dR, dll = (_alloc((D, O), dtype=torch.float32, device=dev) for _ in range(2))
+        db = _alloc(D, dtype=torch.float32, device=dev)
+        dsi = _alloc((B, D, O), dtype=torch.float32, device=dev) if sin is not None else None
+        _check(lib.sb_li_bwd_tiled(fc.data_ptr(), g.data_ptr(), modal.data_ptr(), bf.data_ptr(), _ptr(sin), _ptr(dso), S.data_ptr(),
+                                   A.data_ptr(), dBp.data_ptr(), df.data_ptr(), dR.data_ptr(), dll.data_ptr(), db.data_ptr(),
+                                   _ptr(dsi), B, L, D, O, _stream()), "li_bwd_tiled")
+        _count(4)
+        dp = dll.to(pdt) if pdt != torch.float32 else dll.clone()          # gamma and p get gradients of their own storage
+        return df, dll.to(gdt), dR.to(rdt), dp, db.to(bdt), dsi, None
+
+
 class _HyenaLI(torch.autograd.Function):
+    """The per-thread streaming scan: any D."""
+
     @staticmethod
     def forward(ctx, feat, gamma, R, p, bias, state_in, want_state):
         lib = require()
@@ -1423,16 +1493,13 @@ class _HyenaLI(torch.autograd.Function):
         B, L, C3 = fc.shape
         D = C3 // 3
         dev = fc.device
-        # the shared-memory tiled backward keeps a whole chunk on chip and fixes the chunk length itself
-        tc_fwd = _li_chunk(B, L, D)
-        tc = int(lib.sb_li_bwd_chunk(D, tc_fwd))
+        tc = _li_chunk(B, L, D)
         NC = (L + tc - 1) // tc
         g = gz.contiguous()
         shape = (B, NC, D, LI_ORDER)
         S, W, A, dRp, dLp = (_alloc(shape, dtype=torch.float32, device=dev) for _ in range(5))
         dBp = _alloc((B, NC, D), dtype=torch.float32, device=dev)
-        tiled = tc != tc_fwd
-        tmp = None if tiled else _alloc((B, L, D), dtype=bf16, device=dev)     # dx1 round trip of the streaming kernels only
+        tmp = _alloc((B, L, D), dtype=bf16, device=dev)
         df = _alloc_like(fc)
         dso = None
         if want_state and gstate is not None:
@@ -1459,5 +1526,6 @@ class _HyenaLI(torch.autograd.Function):
 def hyena_li_modal(feat, gamma, R, p, bias, state_in=None, return_state=False):
     if not _is_bf16(feat) or gamma.shape[1] > LI_ORDER:
         return ref.hyena_li_modal(feat, gamma, R, p, bias, state_in, return_state)
-    z, s = _HyenaLI.apply(feat, gamma, R, p, bias, state_in, return_state)
+    fn = _HyenaLITiled if LI_TILED and feat.shape[-1] % 24 == 0 and feat.numel() > 0 else _HyenaLI
+    z, s = fn.apply(feat, gamma, R, p, bias, state_in, return_state)
     return (z, s) if return_state else z

@@ -1,0 +1,56 @@
+"""Tile edges of the sequence kernels: sizes around one tile, partial channel blocks, the shortest and longest filters,
+against the fp32 PyTorch statements (ops/reference.py)."""
+import math
+import os
+
+import pytest
+import torch
+
+from savanna_b200 import ops
+from savanna_b200.ops import reference as ref
+
+pytestmark = pytest.mark.gpu
+DEV, BF = "cuda", torch.bfloat16
+TINY = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "configs", "baseline", "tiny_sh2_gpu.yml")
+
+
+def _close(a, b, tol, what):
+    """Every element within tol of its value plus tol of the tensor's rms (bf16 results: half an ulp is 2^-9 = 0.2 %)."""
+    a, b = a.float(), b.float()
+    rms = b.pow(2).mean().sqrt().clamp(min=1e-12)
+    excess = ((a - b).abs() - tol * (rms + b.abs())).max().item()
+    assert excess <= 0, f"{what}: {excess:.4g} outside the bound (rms {rms.item():.4g})"
+
+
+@pytest.mark.parametrize("B,L,D,O", [(1, 1, 8, 16), (2, 15, 24, 1), (1, 16, 128, 16), (1, 63, 136, 5), (2, 64, 8, 16), (1, 65, 264, 16),
+                                     (3, 129, 120, 16), (1, 2049, 16, 8)])
+def test_li_scan(B, L, D, O):
+    torch.manual_seed(L * 31 + D)
+    args = [(torch.randn(B, L, 3 * D, device=DEV) * 0.7).to(BF), (torch.rand(D, O, device=DEV) * 0.09 + 0.01).log(),
+            torch.randn(D, O, device=DEV) / math.sqrt(O), -torch.ones(D, O, device=DEV), torch.randn(D, device=DEV)]
+    leaves = [t.clone().requires_grad_() for t in args]
+    z = ops.hyena_li_modal(*leaves)
+    g = torch.randn_like(z)
+    z.backward(g)
+    rl = [t.float().clone().requires_grad_() for t in args]
+    zr = ref.hyena_li_modal(*rl)
+    zr.backward(g.float())
+    # fp32 recurrence, one bf16 rounding of z / dfeat: 2^-9; 4x for the fp32 FFT of the oracle and cancelling sums
+    _close(z, zr, 8e-3, "z")
+    _close(leaves[0].grad, rl[0].grad, 8e-3, "dfeat")
+    if L > 1:                                            # at L = 1 the pole gradients are zero up to the oracle's FFT noise
+        for i, n in ((1, "dgamma"), (3, "dp")):
+            _close(leaves[i].grad, rl[i].grad, 2e-3, n)
+    _close(leaves[2].grad, rl[2].grad, 2e-3, "dR")
+    _close(leaves[4].grad, rl[4].grad, 2e-3, "dbias")
+
+
+def test_li_scan_unaligned_view():
+    """A contiguous view that starts off a 16-byte boundary."""
+    torch.manual_seed(5)
+    L, D, O = 40, 16, 16
+    buf = torch.randn(L * 3 * D + 1, device=DEV).to(BF)
+    feat = buf[1:].view(1, L, 3 * D)
+    a = [(torch.rand(D, O, device=DEV) * 0.09 + 0.01).log(), torch.randn(D, O, device=DEV) / 4, -torch.ones(D, O, device=DEV),
+         torch.randn(D, device=DEV)]
+    assert torch.equal(ops.hyena_li_modal(feat, *a), ops.hyena_li_modal(feat.clone(), *a))
