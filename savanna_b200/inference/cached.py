@@ -11,13 +11,15 @@ Every operator of a StripedHyena 2 block has a small recurrent form:
 from the layers' inputs (forward pre-hooks; the Hyena-LI state comes from the scan kernel's `return_state`);
 `CachedDecoder.step(token)` then advances all layers by one position.  Role of the reference's cached inference path
 (savanna/text_generation_utils.py:173-365 `stream_tokens` with `InferenceParams`, :672-774 the interactive driver; its
-recurrent Hyena inference lives in the separate vortex project).  Decode steps are matrix-vector work on one token and
-use plain PyTorch operations on the model's own parameters.  Supported: one device (no tensor / context / pipeline
+recurrent Hyena inference lives in the separate vortex project).  Decode steps are matrix-vector work on one token: on CUDA
+one native call per step runs five kernels per layer (csrc/decode.cu, see `_FusedStep` for what it covers); everything else
+uses plain PyTorch operations on the model's own parameters.  Supported: one device (no tensor / context / pipeline
 parallelism), pre-norm blocks with the gated MLP, rotary or no position embedding, implicit-modal Hyena-LI filters; any
 other configuration raises and the caller falls back to `stream_tokens` (recompute).
 """
 from __future__ import annotations
 
+import ctypes
 import math
 from typing import Dict, List, Optional
 
@@ -38,6 +40,170 @@ def _rms(x, norm):
 
 def _act(name: str):
     return {"silu": F.silu, "gelu": F.gelu, "relu": F.relu, "identity": lambda t: t}[name]
+
+
+class _DecLayer(ctypes.Structure):
+    """Mirrors sb::dec::Layer (csrc/decode.cu)."""
+    _fields_ = ([(n, ctypes.c_int) for n in ("kind", "H", "F", "kf", "K", "G", "O", "heads", "rd", "act", "pregate", "postgate",
+                                             "form1", "form2", "norm2", "cap")]
+                + [(n, ctypes.c_float) for n in ("eps1", "eps2", "pos_scale")]
+                + [(n, ctypes.c_void_p) for n in ("norm1_w", "w_in", "w_out", "b_out", "norm2_w", "w12", "w3", "b3", "conv_w", "taps",
+                                                  "bias", "lam", "R", "inv_freq", "proj_ring", "u_ring", "state", "kc", "vc")])
+
+
+def _ring(tail: torch.Tensor, pos: int) -> torch.Tensor:
+    """[B, n, C] rows of times pos - n .. pos - 1, oldest first -> the same rows with time t in slot t mod n."""
+    n = tail.shape[1]
+    return torch.roll(tail, pos % n, dims=1).contiguous() if n else tail.contiguous()
+
+
+class _FusedStep:
+    """The decode step of csrc/decode.cu: the layers' weights by address, their state in the layout of its kernels.  Built at
+    the end of a prefill; `build` returns None when something is not covered (CPU tensors, other dtypes than bf16, other norms
+    than RMSNorm, head sizes other than 128, more than 8 sequences, unaligned or non-contiguous weights), and the decoder then
+    steps operator by operator."""
+
+    @staticmethod
+    def build(dec: "CachedDecoder", batch: int):
+        from .. import ops
+        from ..models.norms import RMSNorm
+        model, cfg = dec.model, dec.cfg
+        w = model.embedding.word_embeddings.weight
+        if not ops._k(w) or cfg.params_dtype != torch.bfloat16:
+            return None
+        from ..ops import cuda_ops
+        lib = cuda_ops.require()
+        if not getattr(lib, "_sb_decode_ready", False):
+            P, I, F_ = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
+            lib.sb_decode_max_width.restype = lib.sb_decode_layer_bytes.restype = lib.sb_decode_step.restype = I
+            lib.sb_decode_max_width.argtypes = [I]
+            lib.sb_decode_layer_bytes.argtypes = []
+            lib.sb_decode_step.argtypes = [P, I, P, P, P, P, P, I, I, I, P, F_, I, P, I, P, P]
+            lib._sb_decode_ready = True
+        if lib.sb_decode_layer_bytes() != ctypes.sizeof(_DecLayer):
+            raise RuntimeError("decode layer descriptor does not match the native library (rebuild savanna_b200.csrc)")
+        D, wmax = cfg.hidden_size, lib.sb_decode_max_width(batch)
+
+        def weight(t, *shape):
+            return (t is not None and t.dtype == torch.bfloat16 and t.is_cuda and t.is_contiguous() and t.data_ptr() % 16 == 0
+                    and tuple(t.shape) == shape)
+
+        def norm(m):
+            return isinstance(m, RMSNorm) and weight(m.gain, D)
+
+        for blk in dec.blocks:
+            mixer, mlp = blk.mixer, blk.mlp
+            H, Fi = mixer.inner_size, mlp.ffn_local
+            if (D % 8 or H % 8 or Fi % 8 or max(D, H, Fi) > wmax or mlp.act not in cuda_ops._ACT or not norm(blk.input_layernorm)
+                    or (blk.pre_mlp_norm and not norm(blk.pre_mlp_layernorm)) or not weight(mixer.dense_projection.weight, 3 * H, D)
+                    or not weight(mixer.dense.weight, D, H) or not weight(mlp.w12, 2 * Fi, D) or not weight(mlp.w3.weight, D, Fi)
+                    or any(b is not None and not weight(b, D) for b in (mixer.dense.bias, mlp.w3.bias))):
+                return None
+            if isinstance(mixer.mixer, SelfAttention) and (mixer.mixer.hd != 128 or mixer.mixer.heads * 128 != H):
+                return None
+        return _FusedStep(dec, lib, batch)
+
+    def __init__(self, dec: "CachedDecoder", lib, batch: int):
+        from ..models.norms import RMSNorm
+        from ..ops import cuda_ops
+        model, cfg = dec.model, dec.cfg
+        self.lib, self.model, self.batch, self.D = lib, model, batch, cfg.hidden_size
+        dev = model.embedding.word_embeddings.weight.device
+        n = len(dec.blocks)
+        self.layers = (_DecLayer * n)()
+        self.keep = []                          # tensors the descriptors point into
+        self.attn = []                          # (layer index, key cache, value cache)
+
+        def own(t):
+            self.keep.append(t)
+            return t.data_ptr()
+
+        def f32(t):
+            return own(t.detach().float().contiguous())
+
+        wide = 0
+        for i, (blk, st) in enumerate(zip(dec.blocks, dec.states)):
+            L, mixer, inner, mlp = self.layers[i], blk.mixer, blk.mixer.mixer, blk.mlp
+            L.H, L.F, L.act = mixer.inner_size, mlp.ffn_local, cuda_ops._ACT[mlp.act]
+            L.norm1_w, L.eps1, L.form1 = own(blk.input_layernorm.gain), blk.input_layernorm.eps, int(blk.input_layernorm.form != "te")
+            L.norm2 = int(bool(blk.pre_mlp_norm))
+            if L.norm2:
+                m = blk.pre_mlp_layernorm
+                L.norm2_w, L.eps2, L.form2 = own(m.gain), m.eps, int(m.form != "te")
+            L.w_in, L.w_out, L.b_out = own(mixer.dense_projection.weight), own(mixer.dense.weight), \
+                own(mixer.dense.bias) if mixer.dense.bias is not None else None
+            L.w12, L.w3, L.b3 = own(mlp.w12), own(mlp.w3.weight), own(mlp.w3.bias) if mlp.w3.bias is not None else None
+            wide = max(wide, L.H, L.F)
+            if isinstance(inner, SelfAttention):
+                L.kind, L.heads, L.rd, L.pos_scale = 3, inner.heads, 0, 1.0
+                if inner._rotary:
+                    r = inner._rotary[0]
+                    L.rd, L.pos_scale = r.dim, r.scaling_factor
+                    L.inv_freq = f32(1.0 / (r.base ** (torch.arange(0, r.dim, 2, device=dev, dtype=torch.float32) / r.dim)))
+                self.attn.append([i, st["k"], st["v"]])
+            else:
+                conv = mixer.hyena_proj_conv
+                w = conv.taps()
+                L.kf = w.shape[1]
+                L.conv_w = f32(w.repeat_interleave(conv.group_dim, dim=0) if conv.group_dim > 1 else w)
+                L.proj_ring = own(_ring(st["proj_tail"].to(torch.bfloat16), dec.pos))
+                L.pregate = L.postgate = 1
+                if isinstance(inner, ShortHyenaOperator):
+                    taps = inner.short_conv.taps()
+                    L.kind, L.pregate, L.postgate = 0, int(bool(inner.pregate)), int(bool(inner.postgate))
+                    L.taps, L.K, L.G = f32(taps), taps.shape[1], taps.shape[0]
+                    L.u_ring = own(_ring(st["u_tail"].float(), dec.pos))
+                elif inner.is_mr:
+                    taps = inner.filter(st["u_tail"].shape[1] + 1).flip(-1)
+                    L.kind, L.taps, L.K, L.G, L.bias = 1, f32(taps), taps.shape[1], taps.shape[0], f32(inner.conv_bias)
+                    L.u_ring = own(_ring(st["u_tail"].float(), dec.pos))
+                else:
+                    g, R, p = inner._modal()
+                    L.kind, L.O, L.bias = 2, g.shape[1], f32(inner.conv_bias)
+                    L.lam, L.R = f32(torch.exp(-torch.exp(p.detach().float()) * torch.exp(g.detach().float()))), f32(R)
+                    L.state = own(st["s"].float().contiguous().clone())
+            st.clear()                           # this object owns the state from here on
+        self._reserve(dec.pos + 1)
+        bf = dict(dtype=torch.bfloat16, device=dev)
+        self.proj, self.z, self.ab = torch.empty(batch, 3 * wide, **bf), torch.empty(batch, wide, **bf), torch.empty(batch, 2 * wide, **bf)
+        self.a = torch.empty(batch, self.D, **bf)
+        fn = model.final_norm.norm if hasattr(model.final_norm, "norm") else None
+        head = model.embedding.word_embeddings.weight
+        self.head = None
+        if (not cfg.no_weight_tying and model.mup_output_mult == 1.0 and isinstance(fn, RMSNorm) and fn.gain.dtype == torch.bfloat16
+                and head.dtype == torch.bfloat16 and head.is_contiguous() and head.data_ptr() % 16 == 0):
+            self.head, self.norm = head, fn
+
+    def _reserve(self, n: int) -> None:
+        """Room for n tokens in every key / value cache (doubled when it runs out)."""
+        for e in self.attn:
+            i, k, v = e
+            L = self.layers[i]
+            if L.cap >= n:
+                continue
+            cap = max(2 * L.cap, n + 63)
+            for j, (name, old) in enumerate((("kc", k), ("vc", v))):
+                new = torch.empty((old.shape[0], cap) + tuple(old.shape[2:]), dtype=torch.bfloat16, device=old.device)
+                new[:, : old.shape[1]] = old
+                setattr(L, name, new.data_ptr())
+                e[1 + j] = new
+            L.cap = cap
+
+    def __call__(self, token: torch.Tensor, pos: int) -> torch.Tensor:
+        from ..ops.cuda_ops import _check, _count, _stream
+        if token.shape[0] != self.batch:
+            raise ValueError(f"decode step for {token.shape[0]} sequences, prefilled with {self.batch}")
+        self._reserve(pos + 1)
+        x = self.model.embedding(token[:, None], None)[:, 0].contiguous()
+        V = self.head.shape[0] if self.head is not None else 0
+        out = torch.empty(self.batch, V, dtype=torch.float32, device=x.device) if V else None
+        _check(self.lib.sb_decode_step(ctypes.addressof(self.layers), len(self.layers), x.data_ptr(), self.proj.data_ptr(),
+                                       self.z.data_ptr(), self.a.data_ptr(), self.ab.data_ptr(), self.batch, self.D, pos,
+                                       self.norm.gain.data_ptr() if V else None, self.norm.eps if V else 0.0,
+                                       int(self.norm.form != "te") if V else 0, self.head.data_ptr() if V else None, V,
+                                       out.data_ptr() if V else None, _stream()), "decode_step")
+        _count(5 * len(self.layers) + (1 if V else 0))
+        return out if V else self.model.logits(x[:, None])[:, 0].float()
 
 
 class CachedDecoder:
@@ -66,6 +232,7 @@ class CachedDecoder:
                 raise NotImplementedError("cached generation does not cover two-sided filters or outer-product heads")
         self.states: List[Dict] = []
         self.pos = 0
+        self._fused: Optional[_FusedStep] = None
 
     # ------------------------------------------------------------------ prefill
     @torch.no_grad()
@@ -74,6 +241,7 @@ class CachedDecoder:
         from .. import ops
         model = self.model
         B, T = tokens.shape
+        self._fused = None
         self.states = [dict() for _ in self.blocks]
         hooks = []
 
@@ -127,6 +295,7 @@ class CachedDecoder:
                 h.remove()
             model.train(was_training)
         self.pos = T
+        self._fused = _FusedStep.build(self, B)
         return logits
 
     # ------------------------------------------------------------------ one decode step
@@ -184,6 +353,17 @@ class CachedDecoder:
     def step(self, token: torch.Tensor) -> torch.Tensor:
         """token [B] -> logits of the next position [B, V]; advances every layer's state by one token."""
         model, cfg = self.model, self.cfg
+        if self._fused is not None:
+            was_training = model.training
+            if was_training:
+                model.eval()
+            try:
+                logits = self._fused(token, self.pos)
+            finally:
+                if was_training:
+                    model.train()
+            self.pos += 1
+            return logits
         dtype = cfg.params_dtype
         pos = torch.tensor([self.pos], device=token.device)
         was_training = model.training
