@@ -215,7 +215,9 @@ def _count(n: int = 1) -> None:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # the raw handle: building a Stream object per launch was a sixth of a small model's training step (tiny four-operator
+    # model, 2 x 1024 tokens: 5.1 -> 4.3 ms together with the status word's lookup below)
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _ptr(t: Optional[torch.Tensor]):
@@ -229,10 +231,11 @@ def _check(rc: int, what: str) -> None:
 
 def status_word(device) -> torch.Tensor:
     """Per-device uint32 word the bounded waits of the kernels write when they give up."""
-    key = torch.device(device).index or 0
-    if key not in _STATUS:
-        _STATUS[key] = _zeros(1, dtype=torch.int32, device=device)
-    return _STATUS[key]
+    key = (device if isinstance(device, torch.device) else torch.device(device)).index or 0
+    word = _STATUS.get(key)
+    if word is None:
+        word = _STATUS[key] = _zeros(1, dtype=torch.int32, device=device)
+    return word
 
 
 def check_status(device=None) -> int:
