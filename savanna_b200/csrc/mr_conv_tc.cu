@@ -8,10 +8,17 @@
 // the warp-level MMA path; the wide GEMMs and attention use tcgen05.)  fp32 accumulation; u and h are rounded to
 // bf16 for the product, like every other tensor-core operand in the model.
 //
-//   mr_tc_fwd : z = x1 * (h*u + bias*u)                                  tile 128 time x 64 channels
+//   mr_tc_fwd : z = x1 * (h*u + bias*u)
 //   mr_tc_bwd : dfeat = (dz*y, du*v, du*x2), du = h (*) g + bias*g (anticausal), g = dz*x1;
-//               dh[s] += sum g[t] u[t-s]  (as P_d = G_blk^T-contracted-over-channels MMAs), dbias += sum g*u
-//               tile 64 time x 64 channels, y recomputed instead of saved
+//               dh[s] += sum g[t] u[t-s]  (as P_d = G_blk^T-contracted-over-channels MMAs), dbias += sum g*u;
+//               y recomputed instead of saved
+// Both walk a segment of 32-row tiles of 64 channels.
+//
+// Measured at B = 1, L = 8192, D = 4096, K = 128 on a B200 (us; in brackets the kernels these replace, which staged 128-row
+// tiles with their halo, or rebuilt 72 fragment registers from global memory for every 64-row tile): forward 73 (108),
+// backward 260 (475), forward and backward with their host side 589 -> 333.  Copying the data takes 40 and 71 us.  What bounds
+// them now is issue slots and latency at four (two) blocks per SM: of the first streaming version (106 and 411 us) most of
+// the difference was address arithmetic of the copies, unpacking to fp32 for the gates, and spilled fragments.
 // Rows before the sequence start come from `halo` [B, K-1, 3D] (context-parallel shards) or are zero; the
 // backward kernel also produces the halo rows' gradient.  Requires dg % 16 == 0 (a warp's 16-channel slab shares
 // one filter); other group widths use the CUDA-core kernels in mr_conv.cu.
@@ -27,12 +34,16 @@ namespace sb {
 typedef __nv_bfloat16 bf16;
 
 constexpr int TC_CH = 64;                 // channels per tile (4 slabs of 16)
-constexpr int TC_LD = 72;                 // padded smem row (elements) -> 144 B, conflict-free ldmatrix
-constexpr int TC_HALO = 128;              // staged past/future rows
-constexpr int TC_THREADS = 256;
-constexpr int FWD_TT = 128;
-constexpr int BWD_TT = 64;
+constexpr int TC_LD = 72;                 // padded row of a u / g ring (elements) -> 144 B, conflict-free ldmatrix
+constexpr int TC_TT = 32;                 // rows per tile step
+constexpr int TC_HALO = 128;              // rows of u behind (g ahead of) the tile
+constexpr int TC_RING = TC_HALO + TC_TT;  // 160 rows: ten 16-row blocks, a block never wraps
+constexpr int RAW_LD = 200;               // padded row of a staged feature tile (elements): 400 B, so that the 8 rows x 4
+                                          // channel pairs of an MMA fragment fall into 32 different banks
+constexpr int FWD_THREADS = 128;          // one warp per 16-channel slab
+constexpr int BWD_THREADS = 256;          // two warps per slab
 constexpr int ND = 9;                     // Toeplitz block diagonals d = 0..8
+constexpr int NF = 2 * ND + 1;            // distinct fragment registers of all diagonals (see toeplitz_frags)
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], uint32_t addr) {
@@ -54,20 +65,23 @@ __device__ __forceinline__ float2 unpack2(uint32_t u) {
 }
 __device__ __forceinline__ float tap(const float* h, int K, int s) { return (s >= 0 && s < K) ? h[s] : 0.f; }
 
-// A fragments of the Toeplitz block diagonals for this thread.  transpose = false: A_d[r][c] = h[16d + r - c]
-// (causal);  transpose = true: A_d[r][c] = h[16d + c - r] (the anticausal product of the backward pass).
-__device__ __forceinline__ void toeplitz_frags(uint32_t (&a)[ND][4], const float* h, int K, int lane, bool transpose) {
-  const int g = lane >> 2, t = lane & 3;
+// A fragments of the Toeplitz block diagonals for this thread.  CAUSAL: A_d[r][c] = h[16d + r - c];  otherwise
+// A_d[r][c] = h[16d + c - r] (the anticausal product of the backward pass).  Register q of diagonal d holds the taps at
+// 16 d + base + {0, 8, -8, 0}[q] (signs swapped when anticausal): the off-diagonal 8 x 8 quarter of one diagonal is the
+// next one's, so the nine diagonals share 19 registers and stay resident over a whole segment.
+template <bool CAUSAL>
+__device__ __forceinline__ void toeplitz_frags(uint32_t (&f)[NF], const float* h, int K, int lane) {
+  const int g = lane >> 2, t = lane & 3, base = CAUSAL ? g - 2 * t : 2 * t - g;
 #pragma unroll
-  for (int d = 0; d < ND; ++d) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int r = g + ((q & 1) ? 8 : 0), c = 2 * t + ((q & 2) ? 8 : 0);
-      const int s0 = transpose ? 16 * d + c - r : 16 * d + r - c;
-      const int s1 = transpose ? s0 + 1 : s0 - 1;
-      a[d][q] = pack2(tap(h, K, s0), tap(h, K, s1));
-    }
+  for (int m = 0; m < NF; ++m) {
+    const int s = 8 * (m - 1) + base;
+    f[m] = pack2(tap(h, K, s), tap(h, K, CAUSAL ? s - 1 : s + 1));
   }
+}
+template <bool CAUSAL>
+__device__ __forceinline__ void toeplitz_mma(float (&d)[4], const uint32_t (&f)[NF], int diag, uint32_t b0, uint32_t b1) {
+  const uint32_t a[4] = {f[2 * diag + 1], f[2 * diag + (CAUSAL ? 2 : 0)], f[2 * diag + (CAUSAL ? 0 : 2)], f[2 * diag + 1]};
+  mma16816(d, a, b0, b1);
 }
 
 struct MrArgs {
@@ -77,542 +91,352 @@ struct MrArgs {
   int ahead_mode; HaloSrc ahead_f, ahead_g;
 };
 
-// Loads 8 channels (c0..c0+7) of feature row t (halo-aware): returns false (zeros) outside the sequence.
-__device__ __forceinline__ bool load_row8(const MrArgs& a, int b, int t, int c0, float (&x1)[8], float (&x2)[8], float (&v)[8]) {
-  const bf16* row = nullptr;
-  if (t >= 0 && t < a.L) row = a.feat + ((size_t)b * a.L + t) * 3 * a.D;
-  else if (t < 0 && t >= -(a.K - 1)) row = halo_row(a.halo, b, t + a.K - 1, a.K - 1, (size_t)3 * a.D);
-  if (!row || c0 >= a.D) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) { x1[i] = 0.f; x2[i] = 0.f; v[i] = 0.f; }
-    return false;
-  }
-  const uint4* p = reinterpret_cast<const uint4*>(row + 3 * c0);
-  uint4 q0 = p[0], q1 = p[1], q2 = p[2];
-  float all[24];
-  const uint32_t w[12] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w, q2.x, q2.y, q2.z, q2.w};
-#pragma unroll
-  for (int i = 0; i < 12; ++i) { float2 f = unpack2(w[i]); all[2 * i] = f.x; all[2 * i + 1] = f.y; }
-#pragma unroll
-  for (int i = 0; i < 8; ++i) { x1[i] = all[3 * i]; x2[i] = all[3 * i + 1]; v[i] = all[3 * i + 2]; }
-  return true;
+// Feature row t of batch row b: the sequence, the rows before it, or null (zeros).
+__device__ __forceinline__ const bf16* mr_row(const MrArgs& a, int b, int t) {
+  if (t >= 0) return t < a.L ? a.feat + ((size_t)b * a.L + t) * 3 * a.D : nullptr;
+  return t >= -(a.K - 1) ? halo_row(a.halo, b, t + a.K - 1, a.K - 1, (size_t)3 * a.D) : nullptr;
 }
-__device__ __forceinline__ void st8(bf16* dst, const float (&f)[8]) {
-  uint4 o = make_uint4(pack2(f[0], f[1]), pack2(f[2], f[3]), pack2(f[4], f[5]), pack2(f[6], f[7]));
-  *reinterpret_cast<uint4*>(dst) = o;
+// Three words of two channels' interleaved triples (x1 x2 | v x1 | x2 v) -> packed pairs.  bf16 products of bf16 values round
+// once, exactly as the fp32 product rounded to bf16 does.
+__device__ __forceinline__ uint32_t tri_x1(uint32_t w0, uint32_t w1) { return __byte_perm(w0, w1, 0x7610); }
+__device__ __forceinline__ uint32_t tri_x2(uint32_t w0, uint32_t w2) { return __byte_perm(w0, w2, 0x5432); }
+__device__ __forceinline__ uint32_t tri_v(uint32_t w1, uint32_t w2) { return __byte_perm(w1, w2, 0x7610); }
+__device__ __forceinline__ uint32_t mul_bf2(uint32_t a, uint32_t b) {
+  __nv_bfloat162 r = __hmul2(*reinterpret_cast<__nv_bfloat162*>(&a), *reinterpret_cast<__nv_bfloat162*>(&b));
+  return *reinterpret_cast<uint32_t*>(&r);
+}
+// u = x2 v of eight channels from their 48 staged bytes
+__device__ __forceinline__ uint4 gate_u(const uint4* p) {
+  const uint4 a = p[0], b = p[1], c = p[2];
+  return make_uint4(mul_bf2(tri_x2(a.x, a.z), tri_v(a.y, a.z)), mul_bf2(tri_x2(a.w, b.y), tri_v(b.x, b.y)),
+                    mul_bf2(tri_x2(b.z, c.x), tri_v(b.w, c.x)), mul_bf2(tri_x2(c.y, c.w), tri_v(c.z, c.w)));
+}
+// g = dz x1 of eight channels
+__device__ __forceinline__ uint4 gate_g(const uint4* p, const uint4 z) {
+  const uint4 a = p[0], b = p[1], c = p[2];
+  return make_uint4(mul_bf2(tri_x1(a.x, a.y), z.x), mul_bf2(tri_x1(a.w, b.x), z.y), mul_bf2(tri_x1(b.z, b.w), z.z),
+                    mul_bf2(tri_x1(c.y, c.z), z.w));
+}
+__device__ __forceinline__ void mr_cp_async16(void* dst, const void* src, int nbytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(nbytes) : "memory");
+}
+__device__ __forceinline__ void mr_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void mr_cp_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
+// Issue the asynchronous copies of feature rows t .. t + TC_TT - 1, channels [c_base, c_base + 64), into dst[TC_TT][RAW_LD]:
+// 96 threads, four rows of 24 chunks side by side.  Tiles inside the sequence walk one pointer.
+__device__ __forceinline__ void mr_stage_feat(bf16* dst, const MrArgs& a, int b, int t, int c_base, int tid) {
+  const int r0 = tid / 24, c = tid - r0 * 24;
+  if (r0 >= 4) return;
+  const bool live = 3 * c_base + c * 8 < 3 * a.D;
+  bf16* d = dst + r0 * RAW_LD + c * 8;
+  if (t >= 0 && t + TC_TT <= a.L) {
+    const size_t ld = (size_t)3 * a.D;
+    const bf16* p = live ? a.feat + ((size_t)b * a.L + t + r0) * ld + 3 * c_base + c * 8 : a.feat;
+    const size_t step = live ? 4 * ld : 0;
+    const int nb = live ? 16 : 0;
+#pragma unroll
+    for (int j = 0; j < TC_TT / 4; ++j, p += step, d += 4 * RAW_LD) mr_cp_async16(d, p, nb);
+  } else {
+    for (int j = 0; j < TC_TT / 4; ++j, d += 4 * RAW_LD) {
+      const bf16* row = mr_row(a, b, t + r0 + 4 * j);
+      const bool ok = row && live;
+      mr_cp_async16(d, ok ? row + 3 * c_base + c * 8 : a.feat, ok ? 16 : 0);
+    }
+  }
 }
 
 // ------------------------------------------------------------------------------------ forward
-// smem: U [(HALO + TT) x LD] bf16 (row r <-> local time r - HALO), X1 [TT x LD] (overwritten with z)
-constexpr int FWD_SMEM = ((TC_HALO + FWD_TT) + FWD_TT) * TC_LD * 2;
+// A block owns 64 channels and a segment of consecutive 32-row tiles.  The tile's features land in shared memory by
+// asynchronous copies one step ahead; u = x2*v goes into a bf16 ring of 160 rows (128 behind the tile), the Toeplitz MMAs
+// read it from there, and z = x1 (y + bias u) is formed in fp32 from the accumulators and the staged features.  Every
+// feature row is read once per segment plus the 128 rows behind its start.  48 KB of shared memory and 4 warps: four
+// blocks per SM.
+constexpr int FWD_SMEM = (2 * TC_TT * RAW_LD + TC_RING * TC_LD) * 2;
 
-__global__ void __launch_bounds__(TC_THREADS)
-mr_tc_fwd_kernel(MrArgs a, bf16* __restrict__ z) {
+template <bool FULL>       // FULL: all nine diagonals (K > 112), so that the loads and MMAs of the diagonals interleave
+__global__ void __launch_bounds__(FWD_THREADS, 4)
+mr_tc_fwd_kernel(MrArgs a, bf16* __restrict__ z, int n_tiles, int tiles_per_seg) {
   extern __shared__ __align__(16) uint8_t smraw[];
-  bf16* sU = reinterpret_cast<bf16*>(smraw);
-  bf16* sX = sU + (TC_HALO + FWD_TT) * TC_LD;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int c_base = blockIdx.x * TC_CH, t0 = blockIdx.y * FWD_TT, b = blockIdx.z;
-  // ---- stage u (and x1) : 8 threads per row, 8 channels each
-  for (int i = tid; i < (TC_HALO + FWD_TT) * 8; i += TC_THREADS) {
-    const int r = i >> 3, cv = i & 7;
-    const int t = t0 + r - TC_HALO;
-    float x1[8], x2[8], v[8], u[8];
-    load_row8(a, b, t, c_base + cv * 8, x1, x2, v);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) u[j] = x2[j] * v[j];
-    st8(sU + r * TC_LD + cv * 8, u);
-    if (r >= TC_HALO) st8(sX + (r - TC_HALO) * TC_LD + cv * 8, x1);
-  }
-  const int slab = warp & 3, half = warp >> 2;
+  bf16* sRaw = reinterpret_cast<bf16*>(smraw);                 // [2][TT][RAW_LD]
+  bf16* sU = sRaw + 2 * TC_TT * RAW_LD;                        // [RING][LD]
+  const int tid = threadIdx.x, lane = tid & 31, slab = tid >> 5;
+  const int c_base = blockIdx.x * TC_CH, b = blockIdx.z;
+  const int k0 = blockIdx.y * tiles_per_seg, k1 = min(k0 + tiles_per_seg, n_tiles);
+  if (k0 >= k1) return;
+  const int seg_t0 = k0 * TC_TT;
   const int ch0 = c_base + slab * 16;
-  uint32_t A[ND][4];
-  {
-    const int grp = min(ch0, a.D - 1) / a.dg;
-    toeplitz_frags(A, a.h + (size_t)grp * a.K, a.K, lane, false);
-  }
   const int nd = min(ND, (a.K - 1) / 16 + 2);
-  __syncthreads();
   const int g = lane >> 2, tq = lane & 3;
-  // ldmatrix.trans lane address: matrix m = lane/8 -> (time 8*(m&1), channel 8*(m>>1)), row lane%8
-  const int lm_row = (lane & 7) + ((lane >> 3) & 1) * 8, lm_col = (lane >> 4) * 8;
-  const float b_lo0 = ch0 + 2 * tq < a.D ? a.bias[ch0 + 2 * tq] : 0.f, b_lo1 = ch0 + 2 * tq + 1 < a.D ? a.bias[ch0 + 2 * tq + 1] : 0.f;
-  const float b_hi0 = ch0 + 8 + 2 * tq < a.D ? a.bias[ch0 + 8 + 2 * tq] : 0.f, b_hi1 = ch0 + 9 + 2 * tq < a.D ? a.bias[ch0 + 9 + 2 * tq] : 0.f;
-#pragma unroll 1
-  for (int blk = 0; blk < FWD_TT / 32; ++blk) {
-    const int i0 = half * (FWD_TT / 2) + blk * 16;            // local output time of the block
-    float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+  const int lm_row = (lane & 7) + ((lane >> 3) & 1) * 8, lm_col = slab * 16 + (lane >> 4) * 8;
+  // The 128 rows behind the segment run through the same pipeline as tiles that produce no output; diagonals beyond nd are
+  // never read, so filters shorter than 128 taps start closer to the segment.
+  const int lead = min(TC_HALO / TC_TT, (16 * (nd - 1) + TC_TT - 1) / TC_TT);
+  mr_stage_feat(sRaw, a, b, seg_t0 - lead * TC_TT, c_base, tid);
+  mr_cp_commit();
+  uint32_t F[NF];
+  toeplitz_frags<true>(F, a.h + (size_t)(min(ch0, a.D - 1) / a.dg) * a.K, a.K, lane);
+  float bias[2][2];
 #pragma unroll
-    for (int d = 0; d < ND; ++d) {
-      if (d < nd) {
-        const int jr = TC_HALO + i0 - 16 * d;                   // smem row of the input block
-        uint32_t bf[4];
-        ldsm_x4_t(bf, smem_addr(sU + (jr + lm_row) * TC_LD + slab * 16 + lm_col));
-        mma16816(acc[0], A[d], bf[0], bf[1]);
-        mma16816(acc[1], A[d], bf[2], bf[3]);
-      }
+  for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) { const int c = ch0 + nt * 8 + 2 * tq + e; bias[nt][e] = c < a.D ? a.bias[c] : 0.f; }
+  int rel = (TC_RING - lead * TC_TT) % TC_RING;                // ring row of the step's first row
+  for (int k = k0 - lead; k < k1; ++k) {
+    bf16* raw = sRaw + ((k - k0 + lead) & 1) * TC_TT * RAW_LD;
+    mr_cp_wait_all();
+    __syncthreads();                                           // tile k is here; all reads of tile k - 1 (raw, ring) are done
+    if (k + 1 < k1) mr_stage_feat(sRaw + ((k - k0 + lead + 1) & 1) * TC_TT * RAW_LD, a, b, (k + 1) * TC_TT, c_base, tid);
+    mr_cp_commit();
+#pragma unroll
+    for (int j = 0; j < TC_TT * 8 / FWD_THREADS; ++j) {
+      const int i = tid + j * FWD_THREADS, r = i >> 3, cv = i & 7;
+      *reinterpret_cast<uint4*>(sU + (rel + r) * TC_LD + cv * 8) = gate_u(reinterpret_cast<const uint4*>(raw + r * RAW_LD + cv * 24));
     }
-    // epilogue in place: z = x1 * (y + bias*u)
+    __syncthreads();
+    if (k >= k0) {
+      float acc[2][2][4];
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt) {
+      for (int i = 0; i < 16; ++i) acc[i >> 3][(i >> 2) & 1][i & 3] = 0.f;
+      // input block e (rows 16 e behind the tile's second output block) feeds diagonal e of block 1 and e - 1 of block 0
 #pragma unroll
-      for (int hh = 0; hh < 2; ++hh) {
-        const int row = i0 + g + hh * 8, col = slab * 16 + nt * 8 + 2 * tq;
-        const float2 u = unpack2(*reinterpret_cast<const uint32_t*>(sU + (TC_HALO + row) * TC_LD + col));
-        uint32_t* xp = reinterpret_cast<uint32_t*>(sX + row * TC_LD + col);
-        const float2 x = unpack2(*xp);
-        const float bi0 = nt ? b_hi0 : b_lo0, bi1 = nt ? b_hi1 : b_lo1;
-        *xp = pack2(x.x * (acc[nt][hh * 2] + bi0 * u.x), x.y * (acc[nt][hh * 2 + 1] + bi1 * u.y));
+      for (int e = 0; e <= ND; ++e) {
+        if (FULL || e <= nd) {
+          int row = rel + 16 - 16 * e;
+          if (row < 0) row += TC_RING;
+          uint32_t bf[4];
+          ldsm_x4_t(bf, smem_addr(sU + (row + lm_row) * TC_LD + lm_col));
+          if (e < ND && (FULL || e < nd)) {
+            toeplitz_mma<true>(acc[1][0], F, e < ND ? e : 0, bf[0], bf[1]);
+            toeplitz_mma<true>(acc[1][1], F, e < ND ? e : 0, bf[2], bf[3]);
+          }
+          if (e > 0) {
+            toeplitz_mma<true>(acc[0][0], F, e > 0 ? e - 1 : 0, bf[0], bf[1]);
+            toeplitz_mma<true>(acc[0][1], F, e > 0 ? e - 1 : 0, bf[2], bf[3]);
+          }
+        }
       }
+      // z = x1 (y + bias u) in fp32 at the fragment positions; the four lanes of a row store 16 consecutive bytes
+#pragma unroll
+      for (int blk = 0; blk < 2; ++blk)
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+          for (int hh = 0; hh < 2; ++hh) {
+            const int row = blk * 16 + g + hh * 8, c = slab * 16 + nt * 8 + 2 * tq;
+            uint32_t* w = reinterpret_cast<uint32_t*>(raw + row * RAW_LD + 3 * c);
+            const float2 p0 = unpack2(w[0]), p1 = unpack2(w[1]), p2 = unpack2(w[2]);      // (x1 x2) (v x1) (x2 v)
+            const float z0 = p0.x * (acc[blk][nt][hh * 2] + bias[nt][0] * (p0.y * p1.x));
+            const float z1 = p1.y * (acc[blk][nt][hh * 2 + 1] + bias[nt][1] * (p2.x * p2.y));
+            const int t = k * TC_TT + row, cg = c_base + c;
+            if (t < a.L && cg < a.D) *reinterpret_cast<uint32_t*>(z + ((size_t)b * a.L + t) * a.D + cg) = pack2(z0, z1);
+          }
     }
-  }
-  __syncthreads();
-  for (int i = tid; i < FWD_TT * 8; i += TC_THREADS) {
-    const int r = i >> 3, cv = i & 7;
-    const int t = t0 + r, c = c_base + cv * 8;
-    if (t < a.L && c < a.D)
-      *reinterpret_cast<uint4*>(z + ((size_t)b * a.L + t) * a.D + c) = *reinterpret_cast<const uint4*>(sX + r * TC_LD + cv * 8);
+    rel += TC_TT;
+    if (rel >= TC_RING) rel -= TC_RING;
   }
 }
 
 // ------------------------------------------------------------------------------------ backward
-// smem rows: U [HALO + TT] (past), G [TT + HALO] (future), tiles X2, V, DZ [TT]; staging for dfeat reuses G.
-constexpr int BWD_ROWS = TC_HALO + BWD_TT;
-constexpr int BWD_SMEM = (2 * BWD_ROWS + 3 * BWD_TT) * TC_LD * 2 + (4 * 128 + TC_CH) * 4;
+// A block owns 64 channels and a segment of consecutive 32-row tiles.  Two rings of 160 rows hold bf16 u = x2*v (the tile
+// and 128 rows behind it) and g = dz*x1 (the tile and 128 rows ahead).  A step stages two raw tiles by asynchronous copies
+// that are issued one step ahead: the front rows (t0 + 128 ..), from which g is formed, and the tile itself, from which u is
+// formed and which stays until the end of the step: y and du come out of the accumulators in fp32, are combined with the
+// tile's x2, v and dz at their fragment positions and replace the features in place, and the tile leaves as 16-byte
+// chunks.  The filter-gradient accumulators stay in registers over the segment (one flush per block).  Every input row is
+// read twice (the second time from L2).
+constexpr int RAWG_LD = 72;                                    // padded row of a staged dz tile
+constexpr int RAW_TILE = TC_TT * (RAW_LD + RAWG_LD);           // elements of a staged (features, dz) tile
+constexpr int BWD_SMEM = (3 * RAW_TILE + 2 * TC_RING * TC_LD) * 2 + (4 * 128 + TC_CH + 4 * NF * 32) * 4;
 
-__global__ void __launch_bounds__(TC_THREADS, 2)
-mr_tc_bwd_kernel(MrArgs a, const bf16* __restrict__ dz, bf16* __restrict__ dfeat, bf16* __restrict__ dhalo,
-                 float* __restrict__ dh, float* __restrict__ dbias, int n_halo_tiles) {
-  extern __shared__ __align__(16) uint8_t smraw[];
-  bf16* sU = reinterpret_cast<bf16*>(smraw);
-  bf16* sG = sU + BWD_ROWS * TC_LD;
-  bf16* sX2 = sG + BWD_ROWS * TC_LD;
-  bf16* sV = sX2 + BWD_TT * TC_LD;
-  bf16* sDZ = sV + BWD_TT * TC_LD;
-  float* sdh = reinterpret_cast<float*>(sDZ + BWD_TT * TC_LD);      // [4 slabs][128]
-  float* sdb = sdh + 4 * 128;                                        // [64]
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int c_base = blockIdx.x * TC_CH, b = blockIdx.z;
-  const int t0 = ((int)blockIdx.y - n_halo_tiles) * BWD_TT;          // halo tiles have negative t0
-  for (int i = tid; i < 4 * 128 + TC_CH; i += TC_THREADS) sdh[i] = 0.f;
-  // ---- stage U rows [t0-HALO, t0+TT) and G rows [t0, t0+TT+HALO); tile rows also keep x2, v, dz
-  float db_part[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) db_part[j] = 0.f;
-  for (int i = tid; i < (TC_HALO + BWD_TT + TC_HALO) * 8; i += TC_THREADS) {
-    const int r = i >> 3, cv = i & 7;                                // r: 0 .. HALO+TT+HALO-1  <->  t = t0 - HALO + r
-    const int t = t0 - TC_HALO + r, c0 = c_base + cv * 8;
-    float x1[8], x2[8], v[8], f[8];
-    load_row8(a, b, t, c0, x1, x2, v);
-    float gz[8];
-    const bool in_seq = t >= 0 && t < a.L && c0 < a.D;
-    if (in_seq) {
-      const uint4 q = *reinterpret_cast<const uint4*>(dz + ((size_t)b * a.L + t) * a.D + c0);
-      const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) { float2 p = unpack2(w[j]); gz[2 * j] = p.x; gz[2 * j + 1] = p.y; }
-    } else {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) gz[j] = 0.f;
+// dz row t, or null: the sequence, or (context-parallel look-ahead) the next chunk's first rows
+__device__ __forceinline__ void mr_rows_fg(const MrArgs& a, const bf16* dz, int b, int t, const bf16*& fr, const bf16*& gr) {
+  gr = nullptr;
+  if (t >= a.L) {
+    fr = nullptr;
+    if (a.ahead_mode && t < a.L + a.K - 1) {
+      fr = halo_row(a.ahead_f, b, t - a.L, a.K - 1, (size_t)3 * a.D);
+      gr = halo_row(a.ahead_g, b, t - a.L, a.K - 1, (size_t)a.D);
     }
-    if (r < BWD_ROWS) {                                              // U rows
-#pragma unroll
-      for (int j = 0; j < 8; ++j) f[j] = x2[j] * v[j];
-      st8(sU + r * TC_LD + cv * 8, f);
-    }
-    if (r >= TC_HALO) {                                              // G rows
-      float gg[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) gg[j] = gz[j] * x1[j];
-      st8(sG + (r - TC_HALO) * TC_LD + cv * 8, gg);
-      if (r < BWD_ROWS) {                                            // the tile itself
-        const int tr = r - TC_HALO;
-        st8(sX2 + tr * TC_LD + cv * 8, x2);
-        st8(sV + tr * TC_LD + cv * 8, v);
-        st8(sDZ + tr * TC_LD + cv * 8, gz);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) db_part[j] += gg[j] * x2[j] * v[j];
-      }
-    }
+    return;
   }
-  {
-    const int cv = tid & 7;                                          // fixed per thread over the loop above
+  fr = mr_row(a, b, t);
+  if (t >= 0) gr = dz + ((size_t)b * a.L + t) * a.D;
+}
+// Features and dz of rows t .. t + TC_TT - 1: threads 0-191 copy features (eight rows of 24 chunks side by side), the other 64
+// dz (eight rows of 8 chunks).
+__device__ __forceinline__ void mr_stage_fg(bf16* dst, const MrArgs& a, const bf16* dz, int b, int t, int c_base, int tid) {
+  const bool fe = tid < 192;
+  const int i = fe ? tid : tid - 192, per = fe ? 24 : 8, r0 = fe ? i / 24 : i >> 3, c = i - r0 * per;
+  const size_t ld = fe ? (size_t)3 * a.D : (size_t)a.D;
+  const int col = (fe ? 3 * c_base : c_base) + c * 8, dld = fe ? RAW_LD : RAWG_LD;
+  const bool live = col < (int)ld;
+  bf16* d = dst + (fe ? 0 : TC_TT * RAW_LD) + r0 * dld + c * 8;
+  if (t >= 0 && t + TC_TT <= a.L) {
+    const bf16* p = live ? (fe ? a.feat : dz) + ((size_t)b * a.L + t + r0) * ld + col : a.feat;
+    const size_t step = live ? 8 * ld : 0;
+    const int nb = live ? 16 : 0;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) atomicAdd(&sdb[cv * 8 + j], db_part[j]);
-  }
-  const int slab = warp & 3, half = warp >> 2;
-  const int ch0 = c_base + slab * 16;
-  const int grp = min(ch0, a.D - 1) / a.dg;
-  const float* hg = a.h + (size_t)grp * a.K;
-  const int nd = min(ND, (a.K - 1) / 16 + 2);
-  const int g = lane >> 2, tq = lane & 3;
-  const int lm_row = (lane & 7) + ((lane >> 3) & 1) * 8, lm_col = (lane >> 4) * 8;
-  __syncthreads();
-  // ---- pass 1: y (causal) and du (anticausal) for this warp's blocks; results parked in registers
-  float yacc[2][2][4], dacc[2][2][4];
-  {
-    uint32_t A[ND][4];
-    toeplitz_frags(A, hg, a.K, lane, false);
-#pragma unroll
-    for (int blk = 0; blk < 2; ++blk) {
-      const int i0 = half * 32 + blk * 16;
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) yacc[blk][nt][q] = 0.f;
-#pragma unroll
-      for (int d = 0; d < ND; ++d) {
-        if (d < nd) {
-          uint32_t bf[4];
-          ldsm_x4_t(bf, smem_addr(sU + (TC_HALO + i0 - 16 * d + lm_row) * TC_LD + slab * 16 + lm_col));
-          mma16816(yacc[blk][0], A[d], bf[0], bf[1]);
-          mma16816(yacc[blk][1], A[d], bf[2], bf[3]);
-        }
-      }
+    for (int j = 0; j < TC_TT / 8; ++j, p += step, d += 8 * dld) mr_cp_async16(d, p, nb);
+  } else {
+    for (int j = 0; j < TC_TT / 8; ++j, d += 8 * dld) {
+      const bf16 *fr, *gr;
+      mr_rows_fg(a, dz, b, t + r0 + 8 * j, fr, gr);
+      const bf16* row = fe ? fr : gr;
+      const bool ok = row && live;
+      mr_cp_async16(d, ok ? row + col : a.feat, ok ? 16 : 0);
     }
-    toeplitz_frags(A, hg, a.K, lane, true);
-#pragma unroll
-    for (int blk = 0; blk < 2; ++blk) {
-      const int i0 = half * 32 + blk * 16;
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) dacc[blk][nt][q] = 0.f;
-#pragma unroll
-      for (int d = 0; d < ND; ++d) {
-        if (d < nd) {
-          uint32_t bf[4];
-          ldsm_x4_t(bf, smem_addr(sG + (i0 + 16 * d + lm_row) * TC_LD + slab * 16 + lm_col));
-          mma16816(dacc[blk][0], A[d], bf[0], bf[1]);
-          mma16816(dacc[blk][1], A[d], bf[2], bf[3]);
-        }
-      }
-      // du += bias * g  (g is read now: its shared-memory rows are reused as output staging later)
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-          const int row = i0 + g + hh * 8, col = slab * 16 + nt * 8 + 2 * tq;
-          const float2 gg = unpack2(*reinterpret_cast<const uint32_t*>(sG + row * TC_LD + col));
-          const int ca = c_base + col;
-          dacc[blk][nt][hh * 2] += (ca < a.D ? a.bias[ca] : 0.f) * gg.x;
-          dacc[blk][nt][hh * 2 + 1] += (ca + 1 < a.D ? a.bias[ca + 1] : 0.f) * gg.y;
-        }
-    }
-  }
-  // ---- pass 2: filter gradient.  P_d[i][j] = sum_c G[i0+i][c] U[i0-16d+j][c]  ->  dh[16d + i - j]
-  if (t0 >= 0) {
-    float P[ND][2][4];
-#pragma unroll
-    for (int d = 0; d < ND; ++d)
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) P[d][nt][q] = 0.f;
-    // non-transposed ldmatrix lane addresses
-    const int a_row = (lane & 7) + ((lane >> 3) & 1) * 8, a_col = (lane >> 4) * 8;       // A: (rows 0-7|8-15, k 0-7|8-15)
-    const int b_row = (lane & 7) + (lane >> 4) * 8, b_col = ((lane >> 3) & 1) * 8;       // B: (time 0-7 k0-7, time 0-7 k8-15, time 8-15 ...)
-#pragma unroll
-    for (int blk = 0; blk < 2; ++blk) {
-      const int i0 = half * 32 + blk * 16;
-      uint32_t af[4];
-      ldsm_x4(af, smem_addr(sG + (i0 + a_row) * TC_LD + slab * 16 + a_col));
-#pragma unroll
-      for (int d = 0; d < ND; ++d) {
-        if (d < nd) {
-          uint32_t bf[4];
-          ldsm_x4(bf, smem_addr(sU + (TC_HALO + i0 - 16 * d + b_row) * TC_LD + slab * 16 + b_col));
-          mma16816(P[d][0], af, bf[0], bf[1]);
-          mma16816(P[d][1], af, bf[2], bf[3]);
-        }
-      }
-    }
-#pragma unroll
-    for (int d = 0; d < ND; ++d) {
-      if (d < nd) {
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int i = g + ((q & 2) ? 8 : 0), j = nt * 8 + 2 * tq + (q & 1);
-            const int s = 16 * d + i - j;
-            if (s >= 0 && s < a.K) atomicAdd(&sdh[slab * 128 + s], P[d][nt][q]);
-          }
-      }
-    }
-  }
-  __syncthreads();                                                    // all MMAs done: G rows can be reused as staging
-  bf16* sOut = sG;                                                    // [TT][3 * 64 (+pad 8)] -> row stride 200 elements
-  constexpr int OLD = 3 * TC_CH + 8;
-#pragma unroll
-  for (int blk = 0; blk < 2; ++blk) {
-    const int i0 = half * 32 + blk * 16;
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-      for (int hh = 0; hh < 2; ++hh) {
-        const int row = i0 + g + hh * 8, col = slab * 16 + nt * 8 + 2 * tq;
-        const float2 u = unpack2(*reinterpret_cast<const uint32_t*>(sU + (TC_HALO + row) * TC_LD + col));
-        const float2 x2 = unpack2(*reinterpret_cast<const uint32_t*>(sX2 + row * TC_LD + col));
-        const float2 v = unpack2(*reinterpret_cast<const uint32_t*>(sV + row * TC_LD + col));
-        const float2 gz = unpack2(*reinterpret_cast<const uint32_t*>(sDZ + row * TC_LD + col));
-        const int ca = c_base + col;
-        const float bi0 = ca < a.D ? a.bias[ca] : 0.f, bi1 = ca + 1 < a.D ? a.bias[ca + 1] : 0.f;
-        const float y0 = yacc[blk][nt][hh * 2] + bi0 * u.x, y1 = yacc[blk][nt][hh * 2 + 1] + bi1 * u.y;
-        const float du0 = dacc[blk][nt][hh * 2], du1 = dacc[blk][nt][hh * 2 + 1];
-        bf16* o = sOut + row * OLD + 3 * col;
-        o[0] = __float2bfloat16_rn(gz.x * y0); o[1] = __float2bfloat16_rn(du0 * v.x); o[2] = __float2bfloat16_rn(du0 * x2.x);
-        o[3] = __float2bfloat16_rn(gz.y * y1); o[4] = __float2bfloat16_rn(du1 * v.y); o[5] = __float2bfloat16_rn(du1 * x2.y);
-      }
-  }
-  __syncthreads();
-  // ---- coalesced write-out: 24 vectors of 16 B per row
-  for (int i = tid; i < BWD_TT * 24; i += TC_THREADS) {
-    const int r = i / 24, q = i - r * 24;
-    const int t = t0 + r, c3 = 3 * c_base + q * 8;
-    if (c3 >= 3 * a.D) continue;
-    const uint4 val = *reinterpret_cast<const uint4*>(sOut + r * OLD + q * 8);
-    if (t >= 0 && t < a.L) *reinterpret_cast<uint4*>(dfeat + ((size_t)b * a.L + t) * 3 * a.D + c3) = val;
-    else if (t < 0 && t >= -(a.K - 1) && dhalo) *reinterpret_cast<uint4*>(dhalo + ((size_t)b * (a.K - 1) + (t + a.K - 1)) * 3 * a.D + c3) = val;
-  }
-  if (t0 >= 0) {
-    for (int i = tid; i < 4 * 128; i += TC_THREADS) {
-      const int sl = i >> 7, s = i & 127;
-      const int c = c_base + sl * 16;
-      if (s < a.K && c < a.D) atomicAdd(dh + (size_t)(c / a.dg) * a.K + s, sdh[i]);
-    }
-    for (int i = tid; i < TC_CH; i += TC_THREADS)
-      if (c_base + i < a.D) atomicAdd(dbias + c_base + i, sdb[i]);
   }
 }
 
-// ------------------------------------------------------------------------------------ backward, streaming form
-// A CTA owns 64 channels and a segment of consecutive 64-row tiles.  The rows of u = x2*v and g = dz*x1 live in two
-// shared-memory rings of 320 rows (128 behind the current tile, the tile, 128 ahead); each tile step stages only the
-// 64 new rows at the front, so every input row is read once per CTA instead of five times, and the filter-gradient
-// accumulators stay in registers over the whole segment (one flush per CTA instead of one per tile).  Per tile: y and
-// du by Toeplitz MMAs into a bf16 staging tile, the filter-gradient MMAs (each warp keeps half of the nine block
-// diagonals for all 64 rows of its slab), then a coalesced pass that re-reads the tile's features and dz from global
-// memory (L2 hits), combines them with y and du and stores dfeat.
-constexpr int SB_TT = 64;                         // rows per tile step
-constexpr int SB_RING = TC_HALO + SB_TT + TC_HALO; // 320
-constexpr int SB_SMEM = (2 * SB_RING + 2 * SB_TT) * TC_LD * 2 + (4 * 128 + TC_CH) * 4;
-
-__device__ __forceinline__ int ring_pos(int p) { return p < 0 ? p + SB_RING : (p >= SB_RING ? p - SB_RING : p); }
-
-__global__ void __launch_bounds__(TC_THREADS, 2)
-mr_tc_bwd_stream_kernel(MrArgs a, const bf16* __restrict__ dz, bf16* __restrict__ dfeat, bf16* __restrict__ dhalo,
-                        float* __restrict__ dh, float* __restrict__ dbias, int n_halo_tiles, int n_tiles, int tiles_per_seg) {
+template <bool FULL>
+__global__ void __launch_bounds__(BWD_THREADS, 2)
+mr_tc_bwd_kernel(MrArgs a, const bf16* __restrict__ dz, bf16* __restrict__ dfeat, bf16* __restrict__ dhalo,
+                 float* __restrict__ dh, float* __restrict__ dbias, int n_halo_tiles, int n_tiles, int tiles_per_seg) {
   extern __shared__ __align__(16) uint8_t smraw[];
-  bf16* sU = reinterpret_cast<bf16*>(smraw);
-  bf16* sG = sU + SB_RING * TC_LD;
-  bf16* sY = sG + SB_RING * TC_LD;                 // [64][LD] y (with the bias term) of the current tile
-  bf16* sDU = sY + SB_TT * TC_LD;                  // [64][LD] du
-  float* sdh = reinterpret_cast<float*>(sDU + SB_TT * TC_LD);       // [4 slabs][128]
+  bf16* sT = reinterpret_cast<bf16*>(smraw);                   // the tile, double buffered
+  bf16* sF = sT + 2 * RAW_TILE;                                // the front rows
+  bf16* sU = sF + RAW_TILE;
+  bf16* sG = sU + TC_RING * TC_LD;
+  float* sdh = reinterpret_cast<float*>(sG + TC_RING * TC_LD);      // [4 slabs][128]
   float* sdb = sdh + 4 * 128;                                        // [64]
+  uint32_t* sFa = reinterpret_cast<uint32_t*>(sdb + TC_CH);          // [4 slabs][NF][32] anticausal fragments
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int c_base = blockIdx.x * TC_CH, b = blockIdx.z;
   const int k0 = blockIdx.y * tiles_per_seg, k1 = min(k0 + tiles_per_seg, n_tiles);
   if (k0 >= k1) return;
-  const int seg_t0 = (k0 - n_halo_tiles) * SB_TT, seg_t1 = (k1 - n_halo_tiles) * SB_TT;
-  const int base_t = seg_t0 - TC_HALO;             // time of ring row 0 (the ring wraps modulo SB_RING from there)
-  for (int i = tid; i < 4 * 128 + TC_CH; i += TC_THREADS) sdh[i] = 0.f;
-
-  float db_part[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) db_part[j] = 0.f;
-  // rows [t_first, t_first + count) -> ring; u for every row that exists (sequence or halo), g inside the sequence
-  auto stage = [&](int t_first, int count) {
-    for (int i = tid; i < count * 8; i += TC_THREADS) {
-      const int r = i >> 3, cv = i & 7;
-      const int t = t_first + r, c0 = c_base + cv * 8;
-      const int pos = (t - base_t) % SB_RING;
-      float x1[8], x2[8], v[8], f[8], gg[8];
-      load_row8(a, b, t, c0, x1, x2, v);
-      const bool in_seq = t >= 0 && t < a.L && c0 < a.D;
-      if (in_seq) {
-        const uint4 q = *reinterpret_cast<const uint4*>(dz + ((size_t)b * a.L + t) * a.D + c0);
-        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) { float2 pq = unpack2(w[j]); gg[2 * j] = pq.x * x1[2 * j]; gg[2 * j + 1] = pq.y * x1[2 * j + 1]; }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) gg[j] = 0.f;
-        if (a.ahead_mode && t >= a.L && t < a.L + a.K - 1 && c0 < a.D) {
-          // look-ahead of g = dz * x1 past the end of the chunk: the next chunk's first rows, staged by their owner
-          const bf16* fr = halo_row(a.ahead_f, b, t - a.L, a.K - 1, (size_t)3 * a.D);
-          const bf16* gr = halo_row(a.ahead_g, b, t - a.L, a.K - 1, (size_t)a.D);
-          if (fr && gr) {
-            const uint4* fp = reinterpret_cast<const uint4*>(fr + 3 * c0);
-            const uint4 q0 = fp[0], q1 = fp[1], q2 = fp[2];
-            const uint32_t fw[12] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w, q2.x, q2.y, q2.z, q2.w};
-            float all[24];
-#pragma unroll
-            for (int j = 0; j < 12; ++j) { float2 pq = unpack2(fw[j]); all[2 * j] = pq.x; all[2 * j + 1] = pq.y; }
-            const uint4 q = *reinterpret_cast<const uint4*>(gr + c0);
-            const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) { float2 pq = unpack2(w[j]); gg[2 * j] = pq.x * all[6 * j]; gg[2 * j + 1] = pq.y * all[6 * j + 3]; }
-          }
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) f[j] = x2[j] * v[j];
-      st8(sU + pos * TC_LD + cv * 8, f);
-      st8(sG + pos * TC_LD + cv * 8, gg);
-      if (in_seq && t >= seg_t0 && t < seg_t1) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) db_part[j] += gg[j] * f[j];
-      }
-    }
-  };
-  stage(base_t, SB_RING);
-
+  const int seg_t0 = (k0 - n_halo_tiles) * TC_TT;              // halo tiles have negative times
+  for (int i = tid; i < 4 * 128 + TC_CH; i += BWD_THREADS) sdh[i] = 0.f;
   const int slab = warp & 3, half = warp >> 2;
   const int ch0 = c_base + slab * 16;
-  const int grp = min(ch0, a.D - 1) / a.dg;
-  const float* hg = a.h + (size_t)grp * a.K;
   const int nd = min(ND, (a.K - 1) / 16 + 2);
   const int g = lane >> 2, tq = lane & 3;
-  const int lm_row = (lane & 7) + ((lane >> 3) & 1) * 8, lm_col = (lane >> 4) * 8;
-  const int a_row = (lane & 7) + ((lane >> 3) & 1) * 8, a_col = (lane >> 4) * 8;
-  const int b_row = (lane & 7) + (lane >> 4) * 8, b_col = ((lane >> 3) & 1) * 8;
-  // filter-gradient accumulators: this warp covers diagonals d = half, half + 2, ... for all four row blocks of the tile
+  const int lm_row = (lane & 7) + ((lane >> 3) & 1) * 8, lm_col = slab * 16 + (lane >> 4) * 8;
+  const int b_row = (lane & 7) + (lane >> 4) * 8, b_col = slab * 16 + ((lane >> 3) & 1) * 8;
+  // fill the rings: steps -4 .. -1 stage rows behind the segment (u) and the segment's first 128 rows ahead (g)
+  constexpr int LEAD = TC_HALO / TC_TT;
+  mr_stage_fg(sT, a, dz, b, seg_t0 - LEAD * TC_TT, c_base, tid);
+  mr_stage_fg(sF, a, dz, b, seg_t0, c_base, tid);
+  mr_cp_commit();
+  // causal fragments in registers, anticausal ones in shared memory: both in registers would spill
+  uint32_t Fc[NF];
+  const uint32_t* Fa = sFa + slab * NF * 32 + lane;
+  {
+    const float* hg = a.h + (size_t)(min(ch0, a.D - 1) / a.dg) * a.K;
+    if (half == 0) {
+      toeplitz_frags<false>(Fc, hg, a.K, lane);
+#pragma unroll
+      for (int m = 0; m < NF; ++m) sFa[(slab * NF + m) * 32 + lane] = Fc[m];
+    }
+    toeplitz_frags<true>(Fc, hg, a.K, lane);
+  }
+  // filter-gradient accumulators: this warp covers diagonals d = half, half + 2, ... for both row blocks of the tile
   constexpr int NDH = (ND + 1) / 2;
   float P[NDH][2][4];
 #pragma unroll
-  for (int dd = 0; dd < NDH; ++dd)
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) P[dd][nt][q] = 0.f;
-  __syncthreads();
+  for (int i = 0; i < NDH * 8; ++i) P[i >> 3][(i >> 2) & 1][i & 3] = 0.f;
+  float db[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
 
-  for (int k = k0; k < k1; ++k) {
-    const int t0 = (k - n_halo_tiles) * SB_TT;
-    const int rel0 = (t0 - base_t) % SB_RING;                 // ring row of the tile's first row
-    // ---- y (causal) and du (anticausal) for this warp's two row blocks -> staging tiles
+  int rel = TC_RING - LEAD * TC_TT;                            // ring row of the step's first row (row t <-> (t - seg_t0) mod RING)
+  for (int k = k0 - LEAD; k < k1; ++k) {
+    const int t0 = (k - n_halo_tiles) * TC_TT;
+    bf16* raw = sT + ((k - k0 + LEAD) & 1) * RAW_TILE;
+    bf16* rawg = raw + TC_TT * RAW_LD;
+    mr_cp_wait_all();
+    __syncthreads();                                           // staged rows are here; reads of step k - 1 (raw, rings) are done
     {
-      uint32_t A[ND][4];
-      toeplitz_frags(A, hg, a.K, lane, false);
-      float acc[2][2][4];
-#pragma unroll
-      for (int blk = 0; blk < 2; ++blk) {
-        const int i0 = half * 32 + blk * 16;
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) acc[blk][nt][q] = 0.f;
-#pragma unroll
-        for (int d = 0; d < ND; ++d) {
-          if (d < nd) {
-            uint32_t bf[4];
-            ldsm_x4_t(bf, smem_addr(sU + (ring_pos(rel0 + i0 - 16 * d) + lm_row) * TC_LD + slab * 16 + lm_col));
-            mma16816(acc[blk][0], A[d], bf[0], bf[1]);
-            mma16816(acc[blk][1], A[d], bf[2], bf[3]);
-          }
-        }
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-          for (int hh = 0; hh < 2; ++hh) {
-            const int row = i0 + g + hh * 8, col = slab * 16 + nt * 8 + 2 * tq;
-            const float2 u = unpack2(*reinterpret_cast<const uint32_t*>(sU + ring_pos(rel0 + row) * TC_LD + col));
-            const int ca = c_base + col;
-            const float b0 = ca < a.D ? a.bias[ca] : 0.f, b1 = ca + 1 < a.D ? a.bias[ca + 1] : 0.f;
-            *reinterpret_cast<uint32_t*>(sY + row * TC_LD + col) = pack2(acc[blk][nt][hh * 2] + b0 * u.x, acc[blk][nt][hh * 2 + 1] + b1 * u.y);
-          }
-      }
-      toeplitz_frags(A, hg, a.K, lane, true);
-#pragma unroll
-      for (int blk = 0; blk < 2; ++blk) {
-        const int i0 = half * 32 + blk * 16;
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) acc[blk][nt][q] = 0.f;
-#pragma unroll
-        for (int d = 0; d < ND; ++d) {
-          if (d < nd) {
-            uint32_t bf[4];
-            ldsm_x4_t(bf, smem_addr(sG + (ring_pos(rel0 + i0 + 16 * d) + lm_row) * TC_LD + slab * 16 + lm_col));
-            mma16816(acc[blk][0], A[d], bf[0], bf[1]);
-            mma16816(acc[blk][1], A[d], bf[2], bf[3]);
-          }
-        }
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-          for (int hh = 0; hh < 2; ++hh) {
-            const int row = i0 + g + hh * 8, col = slab * 16 + nt * 8 + 2 * tq;
-            const float2 gg = unpack2(*reinterpret_cast<const uint32_t*>(sG + ring_pos(rel0 + row) * TC_LD + col));
-            const int ca = c_base + col;
-            const float b0 = ca < a.D ? a.bias[ca] : 0.f, b1 = ca + 1 < a.D ? a.bias[ca + 1] : 0.f;
-            *reinterpret_cast<uint32_t*>(sDU + row * TC_LD + col) = pack2(acc[blk][nt][hh * 2] + b0 * gg.x, acc[blk][nt][hh * 2 + 1] + b1 * gg.y);
-          }
-      }
+      const int r = tid >> 3, cv = tid & 7;                    // 32 rows x 8 vectors of 8 channels
+      *reinterpret_cast<uint4*>(sU + (rel + r) * TC_LD + cv * 8) = gate_u(reinterpret_cast<const uint4*>(raw + r * RAW_LD + cv * 24));
+      int fr = rel + TC_HALO;
+      if (fr >= TC_RING) fr -= TC_RING;
+      *reinterpret_cast<uint4*>(sG + (fr + r) * TC_LD + cv * 8) =
+          gate_g(reinterpret_cast<const uint4*>(sF + r * RAW_LD + cv * 24),
+                 *reinterpret_cast<const uint4*>(sF + TC_TT * RAW_LD + r * RAWG_LD + cv * 8));
     }
-    // ---- filter gradient: P_d[i][j] += sum_c G[i0+i][c] U[i0-16d+j][c] over the four row blocks, d = half, half+2, ..
-    if (t0 >= 0) {
+    __syncthreads();                                           // rings complete; the front buffer is free
+    if (k + 1 < k1) {
+      mr_stage_fg(sT + ((k - k0 + LEAD + 1) & 1) * RAW_TILE, a, dz, b, t0 + TC_TT, c_base, tid);
+      mr_stage_fg(sF, a, dz, b, t0 + TC_TT + TC_HALO, c_base, tid);
+    }
+    mr_cp_commit();
+    if (k >= k0) {
+      const int i0 = rel + half * 16;                          // ring row of this warp's output block
+      float ya[2][4], da[2][4];
 #pragma unroll
-      for (int blk = 0; blk < 4; ++blk) {
-        const int i0 = blk * 16;
-        uint32_t af[4];
-        ldsm_x4(af, smem_addr(sG + (ring_pos(rel0 + i0) + a_row) * TC_LD + slab * 16 + a_col));
+      for (int i = 0; i < 8; ++i) { ya[i >> 2][i & 3] = 0.f; da[i >> 2][i & 3] = 0.f; }
 #pragma unroll
-        for (int dd = 0; dd < NDH; ++dd) {
-          const int d = 2 * dd + half;
-          if (d < nd) {
-            uint32_t bf[4];
-            ldsm_x4(bf, smem_addr(sU + (ring_pos(rel0 + i0 - 16 * d) + b_row) * TC_LD + slab * 16 + b_col));
-            mma16816(P[dd][0], af, bf[0], bf[1]);
-            mma16816(P[dd][1], af, bf[2], bf[3]);
+      for (int d = 0; d < ND; ++d) {
+        if (FULL || d < nd) {
+          int ru = i0 - 16 * d, rg = i0 + 16 * d;
+          if (ru < 0) ru += TC_RING;
+          if (rg >= TC_RING) rg -= TC_RING;
+          uint32_t bu[4], bg[4];
+          ldsm_x4_t(bu, smem_addr(sU + (ru + lm_row) * TC_LD + lm_col));
+          ldsm_x4_t(bg, smem_addr(sG + (rg + lm_row) * TC_LD + lm_col));
+          toeplitz_mma<true>(ya[0], Fc, d, bu[0], bu[1]);
+          toeplitz_mma<true>(ya[1], Fc, d, bu[2], bu[3]);
+          const uint32_t fm = Fa[(2 * d + 1) * 32], fa[4] = {fm, Fa[2 * d * 32], Fa[(2 * d + 2) * 32], fm};
+          mma16816(da[0], fa, bg[0], bg[1]);
+          mma16816(da[1], fa, bg[2], bg[3]);
+        }
+      }
+      // filter gradient: P_d[i][j] += sum_c G[i0+i][c] U[i0-16d+j][c] over the two row blocks, d = half, half+2, ..
+      if (t0 >= 0) {
+#pragma unroll
+        for (int blk = 0; blk < 2; ++blk) {
+          uint32_t af[4];
+          ldsm_x4(af, smem_addr(sG + (rel + blk * 16 + lm_row) * TC_LD + lm_col));
+#pragma unroll
+          for (int dd = 0; dd < NDH; ++dd) {
+            const int d = 2 * dd + half;
+            if (FULL ? d < ND : d < nd) {
+              int ru = rel + blk * 16 - 16 * d;
+              if (ru < 0) ru += TC_RING;
+              uint32_t bf[4];
+              ldsm_x4(bf, smem_addr(sU + (ru + b_row) * TC_LD + b_col));
+              mma16816(P[dd][0], af, bf[0], bf[1]);
+              mma16816(P[dd][1], af, bf[2], bf[3]);
+            }
           }
         }
       }
-    }
-    __syncthreads();                                           // y / du tiles complete, ring reads of this tile done
-    // ---- coalesced output pass: (row, 8 channels) per thread and step
-    for (int i = tid; i < SB_TT * 8; i += TC_THREADS) {
-      const int r = i >> 3, cv = i & 7;
-      const int t = t0 + r, c0 = c_base + cv * 8;
-      if (c0 >= a.D) continue;
-      bf16* dst = nullptr;
-      if (t >= 0 && t < a.L) dst = dfeat + ((size_t)b * a.L + t) * 3 * a.D + 3 * c0;
-      else if (t < 0 && t >= -(a.K - 1) && dhalo) dst = dhalo + ((size_t)b * (a.K - 1) + (t + a.K - 1)) * 3 * a.D + 3 * c0;
-      if (!dst) continue;
-      float x1[8], x2[8], v[8], gz[8];
-      load_row8(a, b, t, c0, x1, x2, v);
-      if (t >= 0) {
-        const uint4 q = *reinterpret_cast<const uint4*>(dz + ((size_t)b * a.L + t) * a.D + c0);
-        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+      // combine at the fragment positions; the gradient replaces the features in place (each thread its own words)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) { float2 pq = unpack2(w[j]); gz[2 * j] = pq.x; gz[2 * j + 1] = pq.y; }
-      } else {
+      for (int nt = 0; nt < 2; ++nt) {
+        const int c = slab * 16 + nt * 8 + 2 * tq;
+        const float b0 = c_base + c < a.D ? a.bias[c_base + c] : 0.f, b1 = c_base + c + 1 < a.D ? a.bias[c_base + c + 1] : 0.f;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) gz[j] = 0.f;
+        for (int hh = 0; hh < 2; ++hh) {
+          const int row = half * 16 + g + hh * 8;
+          uint32_t* w = reinterpret_cast<uint32_t*>(raw + row * RAW_LD + 3 * c);
+          const float2 p0 = unpack2(w[0]), p1 = unpack2(w[1]), p2 = unpack2(w[2]);        // (x1 x2) (v x1) (x2 v)
+          const float2 gz = unpack2(*reinterpret_cast<const uint32_t*>(rawg + row * RAWG_LD + c));
+          const float u0 = p0.y * p1.x, u1 = p2.x * p2.y, g0 = gz.x * p0.x, g1 = gz.y * p1.y;
+          const float y0 = ya[nt][hh * 2] + b0 * u0, y1 = ya[nt][hh * 2 + 1] + b1 * u1;
+          const float d0 = da[nt][hh * 2] + b0 * g0, d1 = da[nt][hh * 2 + 1] + b1 * g1;
+          db[nt][0] += g0 * u0;                                // rows outside the sequence carry dz = 0
+          db[nt][1] += g1 * u1;
+          w[0] = pack2(gz.x * y0, d0 * p1.x);
+          w[1] = pack2(d0 * p0.y, gz.y * y1);
+          w[2] = pack2(d1 * p2.y, d1 * p2.x);
+        }
       }
-      const uint4 yq = *reinterpret_cast<const uint4*>(sY + r * TC_LD + cv * 8);
-      const uint4 dq = *reinterpret_cast<const uint4*>(sDU + r * TC_LD + cv * 8);
-      const uint32_t yw[4] = {yq.x, yq.y, yq.z, yq.w}, dw[4] = {dq.x, dq.y, dq.z, dq.w};
-      float o[24];
+      __syncthreads();
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 y = unpack2(yw[j]), du = unpack2(dw[j]);
-        o[6 * j + 0] = gz[2 * j] * y.x;       o[6 * j + 1] = du.x * v[2 * j];       o[6 * j + 2] = du.x * x2[2 * j];
-        o[6 * j + 3] = gz[2 * j + 1] * y.y;   o[6 * j + 4] = du.y * v[2 * j + 1];   o[6 * j + 5] = du.y * x2[2 * j + 1];
+      for (int j = 0; j < TC_TT * 24 / BWD_THREADS; ++j) {
+        const int i = tid + j * BWD_THREADS, r = i / 24, q = i - r * 24;
+        const int t = t0 + r, c3 = 3 * c_base + q * 8;
+        if (c3 >= 3 * a.D) continue;
+        const uint4 val = *reinterpret_cast<const uint4*>(raw + r * RAW_LD + q * 8);
+        if (t >= 0 && t < a.L) *reinterpret_cast<uint4*>(dfeat + ((size_t)b * a.L + t) * 3 * a.D + c3) = val;
+        else if (t < 0 && t >= -(a.K - 1) && dhalo) *reinterpret_cast<uint4*>(dhalo + ((size_t)b * (a.K - 1) + (t + a.K - 1)) * 3 * a.D + c3) = val;
       }
-      uint4* d4 = reinterpret_cast<uint4*>(dst);
-      d4[0] = make_uint4(pack2(o[0], o[1]), pack2(o[2], o[3]), pack2(o[4], o[5]), pack2(o[6], o[7]));
-      d4[1] = make_uint4(pack2(o[8], o[9]), pack2(o[10], o[11]), pack2(o[12], o[13]), pack2(o[14], o[15]));
-      d4[2] = make_uint4(pack2(o[16], o[17]), pack2(o[18], o[19]), pack2(o[20], o[21]), pack2(o[22], o[23]));
     }
-    // ---- advance the rings: the 64 rows that fall out behind are replaced by the 64 rows ahead of the next tile
-    if (k + 1 < k1) stage(t0 + SB_TT + TC_HALO, SB_TT);
-    __syncthreads();
+    rel += TC_TT;
+    if (rel >= TC_RING) rel -= TC_RING;
   }
 
-  // ---- flush: filter gradient (once per CTA), bias gradient
+  // ---- flush: filter gradient (once per block), bias gradient
 #pragma unroll
   for (int dd = 0; dd < NDH; ++dd) {
     const int d = 2 * dd + half;
@@ -627,29 +451,49 @@ mr_tc_bwd_stream_kernel(MrArgs a, const bf16* __restrict__ dz, bf16* __restrict_
         }
     }
   }
-  {
-    const int cv = tid & 7;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) atomicAdd(&sdb[cv * 8 + j], db_part[j]);
-  }
+  for (int j = 0; j < 4; ++j) atomicAdd(&sdb[slab * 16 + (j >> 1) * 8 + 2 * tq + (j & 1)], db[j >> 1][j & 1]);
   __syncthreads();
-  for (int i = tid; i < 4 * 128; i += TC_THREADS) {
+  for (int i = tid; i < 4 * 128; i += BWD_THREADS) {
     const int sl = i >> 7, s = i & 127;
     const int c = c_base + sl * 16;
     if (s < a.K && c < a.D) atomicAdd(dh + (size_t)(c / a.dg) * a.K + s, sdh[i]);
   }
-  for (int i = tid; i < TC_CH; i += TC_THREADS)
+  for (int i = tid; i < TC_CH; i += BWD_THREADS)
     if (c_base + i < a.D) atomicAdd(dbias + c_base + i, sdb[i]);
 }
 
-static int g_mr_bwd_stream = 1;
+// Segments per (channel tile, batch row): as many as fit in one wave of `per_sm` blocks per SM (a partial second wave would
+// cost a whole segment time), but no shorter than 4 tiles (a segment's lead-in stages 4 tiles of rows).
+static inline int mr_tiles_per_seg(int n_tiles, int D, int B, int per_sm) {
+  int segs = (per_sm * num_sms()) / (((D + TC_CH - 1) / TC_CH) * B);
+  if (segs > (n_tiles + 3) / 4) segs = (n_tiles + 3) / 4;
+  if (segs < 1) segs = 1;
+  return (n_tiles + segs - 1) / segs;
+}
+
+static int mr_launch_fwd(const MrArgs& a, void* z, int B, cudaStream_t st) {
+  auto kern = a.K > 16 * (ND - 2) ? mr_tc_fwd_kernel<true> : mr_tc_fwd_kernel<false>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD_SMEM) != cudaSuccess) return -5;
+  const int n_tiles = (a.L + TC_TT - 1) / TC_TT, tps = mr_tiles_per_seg(n_tiles, a.D, B, 4);
+  const dim3 grid((a.D + TC_CH - 1) / TC_CH, (n_tiles + tps - 1) / tps, B);
+  kern<<<grid, FWD_THREADS, FWD_SMEM, st>>>(a, (bf16*)z, n_tiles, tps);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+static int mr_launch_bwd(const MrArgs& a, const void* dz, void* dfeat, void* dhalo, float* dh, float* dbias, int n_halo, int B,
+                         cudaStream_t st) {
+  auto kern = a.K > 16 * (ND - 2) ? mr_tc_bwd_kernel<true> : mr_tc_bwd_kernel<false>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM) != cudaSuccess) return -5;
+  const int n_tiles = (a.L + TC_TT - 1) / TC_TT + n_halo, tps = mr_tiles_per_seg(n_tiles, a.D, B, 2);
+  const dim3 grid((a.D + TC_CH - 1) / TC_CH, (n_tiles + tps - 1) / tps, B);
+  kern<<<grid, BWD_THREADS, BWD_SMEM, st>>>(a, (const bf16*)dz, (bf16*)dfeat, (bf16*)dhalo, dh, dbias, n_halo, n_tiles, tps);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
 
 }  // namespace sb
 
 using namespace sb;
-
-// 1 (default): streaming backward kernel; 0: one independent CTA per 64-row tile
-extern "C" int sb_mr_tc_set_bwd_variant(int streaming) { sb::g_mr_bwd_stream = streaming ? 1 : 0; return 0; }
 
 extern "C" int sb_mr_tc_supported(int D, int G, int K) {
   const int dg = D / G;
@@ -660,15 +504,8 @@ extern "C" int sb_mr_tc_fwd(const void* feat, const void* halo, const float* h, 
                             int D, int G, int K, cudaStream_t st) {
   if (!sb_mr_tc_supported(D, G, K)) return -1;
   if (B * L == 0) return 0;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(mr_tc_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD_SMEM) != cudaSuccess) return -5;
-    attr = true;
-  }
-  MrArgs a{(const bf16*)feat, halo_local(halo), h, bias, L, D, K, D / G, 0, halo_local(nullptr), halo_local(nullptr)};
-  dim3 grid((D + TC_CH - 1) / TC_CH, (L + FWD_TT - 1) / FWD_TT, B);
-  mr_tc_fwd_kernel<<<grid, TC_THREADS, FWD_SMEM, st>>>(a, (bf16*)z);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return mr_launch_fwd(MrArgs{(const bf16*)feat, halo_local(halo), h, bias, L, D, K, D / G, 0, halo_local(nullptr), halo_local(nullptr)},
+                       z, B, st);
 }
 
 // Context-parallel forward: feat [2B, L, 3D] (two zigzag chunks per sequence), rows before each chunk read in place
@@ -677,40 +514,20 @@ extern "C" int sb_mr_tc_fwd_cp(const void* feat, const HaloSrc* before, const fl
                                int L, int D, int G, int K, cudaStream_t st) {
   if (!sb_mr_tc_supported(D, G, K) || !before) return -9;
   if (B2 * L == 0) return 0;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(mr_tc_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD_SMEM) != cudaSuccess) return -5;
-    attr = true;
-  }
-  MrArgs a{(const bf16*)feat, *before, h, bias, L, D, K, D / G, 0, halo_local(nullptr), halo_local(nullptr)};
-  dim3 grid((D + TC_CH - 1) / TC_CH, (L + FWD_TT - 1) / FWD_TT, B2);
-  mr_tc_fwd_kernel<<<grid, TC_THREADS, FWD_SMEM, st>>>(a, (bf16*)z);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return mr_launch_fwd(MrArgs{(const bf16*)feat, *before, h, bias, L, D, K, D / G, 0, halo_local(nullptr), halo_local(nullptr)}, z, B2,
+                       st);
 }
 
-// Context-parallel backward (streaming kernel): the look-ahead of dz * x1 past each chunk's end comes from the next
-// chunk's staged head (`ahead_feat`, `ahead_dz`), so the gradients of the chunk's tail rows are complete and no halo
-// gradient is produced.  L must be a multiple of 64 (whole tiles: a look-ahead row never shares a tile with chunk rows).
+// Context-parallel backward: the look-ahead of dz * x1 past each chunk's end comes from the next chunk's staged head
+// (`ahead_feat`, `ahead_dz`), so the gradients of the chunk's tail rows are complete and no halo gradient is produced.
+// L must be a multiple of 64 (whole tiles: a look-ahead row never shares a tile with chunk rows).
 extern "C" int sb_mr_tc_bwd_cp(const void* feat, const HaloSrc* before, const float* h, const float* bias, const void* dz,
                                const HaloSrc* ahead_feat, const HaloSrc* ahead_dz, void* dfeat, float* dh, float* dbias, int B2,
                                int L, int D, int G, int K, cudaStream_t st) {
-  if (!sb_mr_tc_supported(D, G, K) || !before || !ahead_feat || !ahead_dz || (L % SB_TT)) return -9;
+  if (!sb_mr_tc_supported(D, G, K) || !before || !ahead_feat || !ahead_dz || (L % 64)) return -9;
   if (B2 * L == 0) return 0;
-  static bool attr2 = false;
-  if (!attr2) {
-    if (cudaFuncSetAttribute(mr_tc_bwd_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SB_SMEM) != cudaSuccess) return -5;
-    attr2 = true;
-  }
-  MrArgs a{(const bf16*)feat, *before, h, bias, L, D, K, D / G, 1, *ahead_feat, *ahead_dz};
-  const int n_tiles = L / SB_TT;
-  const int ctiles = (D + TC_CH - 1) / TC_CH;
-  int segs = (2 * sb::num_sms()) / (ctiles * B2);
-  if (segs > (n_tiles + 7) / 8) segs = (n_tiles + 7) / 8;
-  if (segs < 1) segs = 1;
-  const int tps = (n_tiles + segs - 1) / segs;
-  dim3 sgrid(ctiles, (n_tiles + tps - 1) / tps, B2);
-  mr_tc_bwd_stream_kernel<<<sgrid, TC_THREADS, SB_SMEM, st>>>(a, (const bf16*)dz, (bf16*)dfeat, nullptr, dh, dbias, 0, n_tiles, tps);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return mr_launch_bwd(MrArgs{(const bf16*)feat, *before, h, bias, L, D, K, D / G, 1, *ahead_feat, *ahead_dz}, dz, dfeat, nullptr, dh,
+                       dbias, 0, B2, st);
 }
 
 extern "C" int sb_mr_tc_bwd(const void* feat, const void* halo, const float* h, const float* bias, const void* dz,
@@ -718,33 +535,7 @@ extern "C" int sb_mr_tc_bwd(const void* feat, const void* halo, const float* h, 
                             cudaStream_t st) {
   if (!sb_mr_tc_supported(D, G, K)) return -1;
   if (B * L == 0) return 0;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(mr_tc_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM) != cudaSuccess) return -5;
-    attr = true;
-  }
-  MrArgs a{(const bf16*)feat, halo_local(halo), h, bias, L, D, K, D / G, 0, halo_local(nullptr), halo_local(nullptr)};
-  const int n_halo = (halo && dhalo) ? (K - 1 + BWD_TT - 1) / BWD_TT : 0;
-  if (g_mr_bwd_stream) {
-    static bool attr2 = false;
-    if (!attr2) {
-      if (cudaFuncSetAttribute(mr_tc_bwd_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SB_SMEM) != cudaSuccess) return -5;
-      attr2 = true;
-    }
-    const int n_tiles = (L + SB_TT - 1) / SB_TT + n_halo;
-    const int ctiles = (D + TC_CH - 1) / TC_CH;
-    // as many segments as fit in one wave of two CTAs per SM (a partial second wave would double the run time),
-    // but no shorter than 8 tiles (the ring prologue costs 4 tiles)
-    int segs = (2 * sb::num_sms()) / (ctiles * B);
-    if (segs > (n_tiles + 7) / 8) segs = (n_tiles + 7) / 8;
-    if (segs < 1) segs = 1;
-    const int tps = (n_tiles + segs - 1) / segs;
-    dim3 sgrid(ctiles, (n_tiles + tps - 1) / tps, B);
-    mr_tc_bwd_stream_kernel<<<sgrid, TC_THREADS, SB_SMEM, st>>>(a, (const bf16*)dz, (bf16*)dfeat, (bf16*)dhalo, dh, dbias, n_halo,
-                                                               n_tiles, tps);
-    return cudaGetLastError() == cudaSuccess ? 0 : -2;
-  }
-  dim3 grid((D + TC_CH - 1) / TC_CH, (L + BWD_TT - 1) / BWD_TT + n_halo, B);
-  mr_tc_bwd_kernel<<<grid, TC_THREADS, BWD_SMEM, st>>>(a, (const bf16*)dz, (bf16*)dfeat, (bf16*)dhalo, dh, dbias, n_halo);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  const int n_halo = (halo && dhalo) ? (K - 1 + TC_TT - 1) / TC_TT : 0;
+  return mr_launch_bwd(MrArgs{(const bf16*)feat, halo_local(halo), h, bias, L, D, K, D / G, 0, halo_local(nullptr), halo_local(nullptr)},
+                       dz, dfeat, dhalo, dh, dbias, n_halo, B, st);
 }

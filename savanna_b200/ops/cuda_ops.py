@@ -113,7 +113,6 @@ class _Sig:
     sb_mr_fwd = [P, P, P, P, P, P, I, I, I, I, I, P]
     sb_mr_bwd = [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, P]
     sb_mr_tc_fwd = [P, P, P, P, P, I, I, I, I, I, P]
-    sb_mr_tc_set_bwd_variant = [I]
     sb_se_set_bwd_variant = [I]
     sb_conv_set_fwd_variant = [I]
     sb_mr_tc_bwd = [P, P, P, P, P, P, P, P, P, I, I, I, I, I, P]
@@ -284,9 +283,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, a_mn: bool = False
 
 
 def set_mr_backward_variant(streaming: bool) -> None:
-    """Hyena-MR tensor-core backward: the streaming kernel (rings of u and g rows, one filter-gradient flush per CTA;
-    default) or one independent CTA per 64-row tile."""
-    require().sb_mr_tc_set_bwd_variant(int(bool(streaming)))
+    """Kept for callers of the former per-tile backward: the Hyena-MR tensor-core backward has one form, the streaming
+    kernel, and both values select it."""
 
 
 def set_se_backward_variant(tiled: bool) -> None:
@@ -1305,8 +1303,8 @@ class _HyenaMR(torch.autograd.Function):
         B, L, C3 = feat.shape
         D = C3 // 3
         G, K = h.shape
-        fc = feat.contiguous()
-        hc = halo.contiguous() if halo is not None else None
+        fc = _aligned(feat)
+        hc = _aligned(halo) if halo is not None else None
         hf, bf = _f32c(h), _f32c(bias)
         z = _alloc((B, L, D), dtype=bf16, device=feat.device)
         tc = (D // G) % 16 == 0 and D % 8 == 0
@@ -1332,7 +1330,7 @@ class _HyenaMR(torch.autograd.Function):
         B, L, C3 = fc.shape
         D = C3 // 3
         G, K = hf.shape
-        g = gz.contiguous()
+        g = _aligned(gz)
         df = _alloc_like(fc)
         dhalo = _zeros_like(hc) if has_halo else None
         dh = _zeros_like(hf)
@@ -1418,7 +1416,7 @@ class _HyenaLITiled(torch.autograd.Function):
         fc, bf = _aligned(feat), _f32c(bias)
         sin = _f32c(state_in) if state_in is not None else None
         tc = _li_tiled_chunk(B, L, D)
-        modal = _alloc((3, D, LI_ORDER), dtype=torch.float32, device=dev)
+        modal = _alloc((3 * D, LI_ORDER), dtype=torch.float32, device=dev)
         S = _alloc((B, (L + tc - 1) // tc, D, LI_ORDER), dtype=torch.float32, device=dev)
         sout = _alloc((B, D, O), dtype=torch.float32, device=dev) if want_state else None
         z = _alloc((B, L, D), dtype=bf16, device=dev)

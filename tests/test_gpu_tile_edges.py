@@ -56,6 +56,31 @@ def test_li_scan_unaligned_view():
     assert torch.equal(ops.hyena_li_modal(feat, *a), ops.hyena_li_modal(feat.clone(), *a))
 
 
+@pytest.mark.parametrize("B,L,D,G,K", [(1, 1, 16, 1, 128), (2, 31, 16, 1, 1), (1, 32, 80, 5, 16), (1, 33, 64, 1, 17), (2, 160, 48, 3, 113),
+                                       (1, 161, 144, 9, 128), (1, 700, 64, 4, 31)])
+@pytest.mark.parametrize("halo", [False, True])
+def test_mr_fir(B, L, D, G, K, halo):
+    torch.manual_seed(L * 7 + K)
+    f, h, b = torch.randn(B, L, 3 * D, device=DEV).to(BF), torch.randn(G, K, device=DEV) / math.sqrt(K), torch.randn(D, device=DEV)
+    hal = torch.randn(B, K - 1, 3 * D, device=DEV).to(BF) if halo and K > 1 else None
+    leaves = [t.clone().requires_grad_() for t in (f, h, b)] + ([hal.clone().requires_grad_()] if hal is not None else [])
+    z = ops.hyena_mr_inner(*leaves)
+    g = torch.randn_like(z)
+    z.backward(g)
+    rl = [t.float().clone().requires_grad_() for t in (f, h, b)] + ([hal.float().clone().requires_grad_()] if hal is not None else [])
+    zr = ref.hyena_mr_inner(*rl)
+    zr.backward(g.float())
+    # bf16 operands of the Toeplitz products (u, taps): two roundings of up to 2^-9 per term leave y and du an error of 0.2 %
+    # of their rms, 4 sigma over the elements, and z, dfeat multiply it by a factor of up to 4 times its rms: 3.2 %
+    _close(z, zr, 3.2e-2, "z")
+    _close(leaves[0].grad, rl[0].grad, 3.2e-2, "dfeat")
+    if hal is not None:
+        _close(leaves[3].grad, rl[3].grad, 3.2e-2, "dhalo")
+    # dh sums bf16-rounded products: relative to the norm of the whole gradient
+    assert (leaves[1].grad - rl[1].grad).norm() <= 1e-2 * rl[1].grad.norm()
+    assert (leaves[2].grad - rl[2].grad).norm() <= 1e-4 * rl[2].grad.norm()
+
+
 @pytest.mark.parametrize("B,T,steps", [(1, 1, 3), (2, 5, 70), (3, 130, 5), (8, 64, 4)])
 def test_decode_step(B, T, steps):
     """The native decode step against the operator-by-operator one: short prompts (rings that start zero-padded), key caches
