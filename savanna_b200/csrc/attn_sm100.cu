@@ -396,15 +396,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 //   dK  += dS^T Q           [keys x d]   A = dS^T (K-major),                    B = Q_i  (MN-major)
 //   dQ^T = K^T dS^T         [d x q]      A = K (MN-major),   B = dS^T (MN-major)   -> fp32 atomics into dq_acc
 // with P = exp(S * scale - lse) and dS = P (dP - delta) * scale computed by one thread per key row and 32 query columns
-// (two warpgroups split the 64 columns).  TMEM: S^T (2 x 64 columns, so the scores of the next tile are computed during
+// (two warpgroups split the 64 columns), and dQ^T read out by four warps of its own: with both in the same eight warps and
+// dP^T waiting for the previous tile's dS^T, three quarters of a tile's time was one chain (1574 us at L = 8192, 32 heads,
+// causal; 1475 now, the products' operand reads from shared memory being the next bound: about 2400 of 3200 cycles a tile).
+// Adding dQ straight from registers with red.global instead of through the staging tile took 2402.  TMEM: S^T (2 x 64 columns, so the scores of the next tile are computed during
 // this tile's softmax), dP^T (64), dQ^T (64), dV (128), dK (128).
 constexpr int BQ2 = 64;                          // query rows per backward tile
 constexpr int QTILE_BYTES = BQ2 * HD * 2;        // 16 KB: two boxes of 8 KB
 constexpr int QBOX_BYTES = BQ2 * 128;            // 8 KB
 constexpr int PT_BYTES = 128 * 128;              // P^T / dS^T tile: 128 key rows x 64 q columns bf16 = 16 KB
-constexpr int BWD_THREADS = 320;
+constexpr int BWD_THREADS = 448;                 // TMA, MMA, 8 softmax warps, 4 dQ read-out warps
+constexpr int STATS_BYTES = BQ2 * 8;             // (-lse, delta) of one query tile
 constexpr int STAGE_BYTES = BQ2 * HD * 4;          // dQ^T staging tile: 64 query rows x 128 fp32
-constexpr int BWD_SMEM = 2 * TILE_BYTES + 4 * QTILE_BYTES + 4 * PT_BYTES + STAGE_BYTES + 256 + 1024;
+constexpr int BWD_SMEM = 2 * TILE_BYTES + 4 * QTILE_BYTES + 4 * PT_BYTES + STAGE_BYTES + 256 + 3 * STATS_BYTES + 1024;
 
 struct BwdParams {
   const float* stats;        // [B, H, Lpad, 2]: (-lse * log2(e), scale * (rowsum(dO * O) - dlse)), Lpad = 64 * ceil(Lq / 64)
@@ -469,6 +473,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   auto pds_ready = [&](int s) { return bar_base + 80u + 8u * s; };
   const uint32_t dq_full = bar_base + 96u, dq_free = bar_base + 104u;
   const uint32_t stage_ready = bar_base + 112, stage_free = bar_base + 120;
+  const uint32_t dp_free = bar_base + 144;
+  auto pd_free = [&](int s) { return bar_base + 152u + 8u * s; };
+  auto sStats = [&](int s) { return bar_base + 256u + uint32_t(s) * STATS_BYTES; };
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + BAR_OFF + 128);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + BAR_OFF + 136);
 
@@ -482,8 +489,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     mbar_init(kv_full, 1); mbar_init(dkv_done, 1);
     for (int s = 0; s < NST; ++s) { mbar_init(qdo_full(s), 1); mbar_init(qdo_free(s), 1); }
     for (int s = 0; s < 2; ++s) { mbar_init(s_full(s), 1); mbar_init(pds_ready(s), 256); }
-    mbar_init(dq_full, 1); mbar_init(dq_free, 256);
-    mbar_init(stage_ready, 256); mbar_init(stage_free, 1);
+    mbar_init(dq_full, 1); mbar_init(dq_free, 128);
+    mbar_init(stage_ready, 128); mbar_init(stage_free, 1);
+    mbar_init(dp_free, 256); mbar_init(pd_free(0), 1); mbar_init(pd_free(1), 1);
     *abort_flag = 0;
     fence_barrier_init();
     prefetch_tmap(&tmQ); prefetch_tmap(&tmK); prefetch_tmap(&tmV); prefetch_tmap(&tmdO); prefetch_tmap(&tmDQ);
@@ -508,8 +516,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       for (int it = 0; it < n && ok; ++it) {
         const int s = it % NST;
         if (!mbar_wait(qdo_free(s), (uint32_t(it / NST) & 1u) ^ 1u, abort_flag, p.status, ST_ATTN + 17)) { ok = false; break; }
-        mbar_expect_tx(qdo_full(s), 2 * QTILE_BYTES);
+        mbar_expect_tx(qdo_full(s), 2 * QTILE_BYTES + STATS_BYTES);
         const int i0 = (i_start + it) * BQ2;
+        bulk_load(sStats(s), p.stats + (((long long)b * p.H + h) * (nq * BQ2) + i0) * 2, STATS_BYTES, qdo_full(s));
         load_qtile(sQ(s), &tmQ, i0, h, b, qdo_full(s));
         load_qtile(sdO(s), &tmdO, i0, h, b, qdo_full(s));
       }
@@ -535,7 +544,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           umma_bf16(tmem_base + T_S + s * 64, desc_kmajor(sK, kk), qdesc_kmajor(sQ(qs), kk), idesc_s, kk ? 1u : 0u);
         return true;
       };
-      // dP^T(it) goes into the single dP^T buffer: only after the softmax warps have read dP^T(it-1) (pds_ready(it-1))
+      // dP^T(it) goes into the single dP^T buffer: as soon as the softmax warps have read dP^T(it-1) into registers
+      // (dp_free(it-1)), so it runs during their exponentials instead of between two tiles
       auto issue_dp = [&](int it) {
         const int s = it & 1, qs = it % NST;
 #pragma unroll
@@ -550,9 +560,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const int s = it & 1, qs = it % NST;
         // the scores of the next tile run while the softmax warps work on this one
         if (it + 1 < n && !issue_s(it + 1)) { ok = false; break; }
+        if (it + 1 < n) {
+          if (!mbar_wait(dp_free, uint32_t(it) & 1u, abort_flag, p.status, ST_ATTN + 27)) { ok = false; break; }
+          tc_fence_after();
+          issue_dp(it + 1);
+        }
         if (!mbar_wait(pds_ready(s), (uint32_t(it) >> 1) & 1u, abort_flag, p.status, ST_ATTN + 21)) { ok = false; break; }
         tc_fence_after();
-        if (it + 1 < n) issue_dp(it + 1);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
           if (P_TMEM)   // 16 queries = 8 packed columns; each warpgroup wrote its 32 queries over its own S^T columns
@@ -565,76 +579,86 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         for (int kk = 0; kk < 4; ++kk)
           umma_bf16(tmem_base + T_DK, pdesc_kmajor(sdS(s), kk), qdesc_mnmajor(sQ(qs), kk), idesc_kv, (it | kk) ? 1u : 0u);
         umma_commit(qdo_free(qs));
-        // dQ^T(it) into its own buffer once dQ^T(it-1) has been read out (the softmax warps do that after P/dS of tile it)
+        // dQ^T(it) into its own buffer once the read-out warps have taken dQ^T(it-1)
         if (it >= 1 && !mbar_wait(dq_free, uint32_t(it - 1) & 1u, abort_flag, p.status, ST_ATTN + 19)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)
           umma_bf16(tmem_base + T_DQ, desc_mnmajor(sK, kk), pdesc_mnmajor(sdS(s), kk), idesc_dq, kk ? 1u : 0u);
         umma_commit(dq_full);
+        umma_commit(pd_free(s));             // P^T / dS^T of this parity may be overwritten
       }
       if (ok) umma_commit(dkv_done);
     }
-  } else {
-    // ------------------------------------------------------------------ P / dS, dQ read-out, dK / dV epilogue
-    const int wg = (warp - 2) >> 2;                  // which 32 query columns
-    const int quarter = warp & 3;
-    const int r = quarter * 32 + lane;               // key row of this thread; also head-dimension lane of dQ^T
-    const int key = k0 + r;
-    const uint32_t lane_off = uint32_t(quarter * 32) << 16;
-    const float sl2 = p.scale_log2;
-    const int tid_c = threadIdx.x - 64;              // 0..255 among the compute threads
-    const int lpad = nq * BQ2;
-    const float4* stats = reinterpret_cast<const float4*>(p.stats + (((long long)b * p.H + h) * lpad) * 2);
-    bool ok = n > 0;
-    // dQ^T of tile `it` leaves through shared memory: every thread holds 32 query rows of one head-dimension column,
-    // writes them into a [64 x 128] fp32 staging tile, and one thread hands the tile to a TMA reduce-add into dq_acc
-    // (rows beyond Lq are clipped by the tensor map).  `cnt` counts the read-outs of this CTA.
-    auto read_out_dq = [&](int it, int cnt) -> bool {
-      if (!mbar_wait(dq_full, uint32_t(it) & 1u, abort_flag, p.status, ST_ATTN + 22)) return false;
+  } else if (warp >= 10) {
+    // ------------------------------------------------------------------ dQ read-out
+    // dQ^T of a tile leaves through shared memory: a thread holds the 64 query rows of one head-dimension column, writes
+    // them into a [64 x 128] fp32 staging tile, and one thread hands the tile to a TMA reduce-add into dq_acc (rows beyond
+    // Lq are clipped by the tensor map).  These warps exist so that this chain (TMEM load, 32 KB of shared-memory stores,
+    // waiting for the previous reduce) overlaps the softmax warps' next tile instead of sitting between two of them.
+    const int r = (warp & 3) * 32 + lane;            // head-dimension lane of dQ^T
+    const uint32_t lane_off = uint32_t((warp & 3) * 32) << 16;
+    const bool first = threadIdx.x == 320;
+    for (int it = 0; it < n; ++it) {
+      if (!mbar_wait(dq_full, uint32_t(it) & 1u, abort_flag, p.status, ST_ATTN + 22)) break;
       tc_fence_after();
-      uint32_t v[32];
-      tmem_ld_32x32(tmem_base + lane_off + T_DQ + wg * 32, v);
+      uint32_t v0[32], v1[32];
+      tmem_ld_32x32(tmem_base + lane_off + T_DQ, v0);
+      tmem_ld_32x32(tmem_base + lane_off + T_DQ + 32, v1);
       tmem_wait_ld();
       tc_fence_before();
       mbar_arrive(dq_free);
-      if (cnt > 0) {
-        if (tid_c == 0) { bulk_wait_read<0>(); mbar_arrive(stage_free); }      // the previous reduce has read the tile
-        if (!mbar_wait(stage_free, uint32_t(cnt - 1) & 1u, abort_flag, p.status, ST_ATTN + 25)) return false;
+      if (it > 0) {
+        if (first) { bulk_wait_read<0>(); mbar_arrive(stage_free); }        // the previous reduce has read the tile
+        if (!mbar_wait(stage_free, uint32_t(it - 1) & 1u, abort_flag, p.status, ST_ATTN + 25)) break;
       }
-      const uint32_t dst = sStage + uint32_t(wg * 32) * 512u + uint32_t(r) * 4u;
+      const uint32_t dst = sStage + uint32_t(r) * 4u;
 #pragma unroll
-      for (int i = 0; i < 32; ++i)
-        asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst + uint32_t(i) * 512u), "r"(v[i]) : "memory");
+      for (int i = 0; i < 32; ++i) {
+        asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst + uint32_t(i) * 512u), "r"(v0[i]) : "memory");
+        asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst + uint32_t(i + 32) * 512u), "r"(v1[i]) : "memory");
+      }
       fence_proxy_async();
       mbar_arrive(stage_ready);
-      if (tid_c == 0) {
-        if (!mbar_wait(stage_ready, uint32_t(cnt) & 1u, abort_flag, p.status, ST_ATTN + 26)) return false;
+      if (first) {
+        if (!mbar_wait(stage_ready, uint32_t(it) & 1u, abort_flag, p.status, ST_ATTN + 26)) break;
         tma_reduce_add_4d(&tmDQ, sStage, 0, h, (i_start + it) * BQ2, b);
         bulk_commit();
       }
-      return true;
-    };
+    }
+    if (first) bulk_wait<0>();                       // the last reduce must have left shared memory
+  } else {
+    // ------------------------------------------------------------------ P / dS, dK / dV epilogue
+    const int wg = (warp - 2) >> 2;                  // which 32 query columns
+    const int quarter = warp & 3;
+    const int r = quarter * 32 + lane;               // key row of this thread
+    const int key = k0 + r;
+    const uint32_t lane_off = uint32_t(quarter * 32) << 16;
+    const float sl2 = p.scale_log2;
+    bool ok = n > 0;
     for (int it = 0; it < n && ok; ++it) {
       const int s = it & 1;
       const int qi = (i_start + it) * BQ2 + wg * 32;   // first query of this thread's 32 columns
-      // (-lse * log2(e), delta) pairs of the 32 queries: the same addresses in every lane (broadcast loads)
-      float4 st[16];
-#pragma unroll
-      for (int i = 0; i < 16; ++i) st[i] = __ldg(stats + (qi >> 1) + i);
+      const int qs = it % NST;
+      // (-lse * log2(e), delta) pairs of the 32 queries came with Q and dO: the same addresses in every lane (broadcasts)
+      if (!mbar_wait(qdo_full(qs), uint32_t(it / NST) & 1u, abort_flag, p.status, ST_ATTN + 24)) { ok = false; break; }
+      const float4* st = reinterpret_cast<const float4*>(smem_gen + BAR_OFF + 256 + qs * STATS_BYTES) + wg * 16;
       if (!mbar_wait(s_full(s), (uint32_t(it) >> 1) & 1u, abort_flag, p.status, ST_ATTN + 23)) { ok = false; break; }
       tc_fence_after();
       uint32_t sv[32], dp[32];
       tmem_ld_32x32(tmem_base + lane_off + T_S + s * 64 + wg * 32, sv);
       tmem_ld_32x32(tmem_base + lane_off + T_DP + wg * 32, dp);
       tmem_wait_ld();
+      tc_fence_before();
+      mbar_arrive(dp_free);
       uint32_t pw[16], dw[16];
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
-        const float pa = ex2(fmaf(__uint_as_float(sv[2 * i]), sl2, st[i].x));
-        const float pb = ex2(fmaf(__uint_as_float(sv[2 * i + 1]), sl2, st[i].z));
-        const float da = pa * fmaf(__uint_as_float(dp[2 * i]), p.scale, -st[i].y);
-        const float db = pb * fmaf(__uint_as_float(dp[2 * i + 1]), p.scale, -st[i].w);
+        const float4 sd = st[i];
+        const float pa = ex2(fmaf(__uint_as_float(sv[2 * i]), sl2, sd.x));
+        const float pb = ex2(fmaf(__uint_as_float(sv[2 * i + 1]), sl2, sd.z));
+        const float da = pa * fmaf(__uint_as_float(dp[2 * i]), p.scale, -sd.y);
+        const float db = pb * fmaf(__uint_as_float(dp[2 * i + 1]), p.scale, -sd.w);
         pw[i] = pack_bf16(pa, pb);
         dw[i] = pack_bf16(da, db);
       }
@@ -647,8 +671,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           else if (2 * i < vis) { pw[i] &= 0xffff0000u; dw[i] &= 0xffff0000u; }
         }
       }
-      // the P^T / dS^T buffers of this parity were last read by the products of tile it-2, which completed before
-      // dq_full of tile it-2, and this thread waited for that barrier in read_out_dq(it-2)
+      // the P^T / dS^T buffers of this parity were last read by the products of tile it-2
+      if (it >= 2) {
+        if (!mbar_wait(pd_free(s), (uint32_t(it - 2) >> 1) & 1u, abort_flag, p.status, ST_ATTN + 28)) { ok = false; break; }
+        tc_fence_after();
+      }
 #pragma unroll
       for (int g = 0; g < 4; ++g) {
         const uint32_t off = uint32_t(r) * 128u + (uint32_t((wg * 4 + g) ^ (r & 7)) << 4);
@@ -662,12 +689,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       fence_proxy_async();
       tc_fence_before();
       mbar_arrive(pds_ready(s));
-      // dQ^T of the previous tile: its product ran while this tile's P and dS were computed
-      if (it >= 1 && !read_out_dq(it - 1, it - 1)) { ok = false; break; }
     }
-    if (ok && !read_out_dq(n - 1, n - 1)) ok = false;
-    if (tid_c == 0) bulk_wait<0>();                     // the last reduce must have left shared memory
-    if (ok && mbar_wait(dkv_done, 0u, abort_flag, p.status, ST_ATTN + 24)) {
+    if (ok && mbar_wait(dkv_done, 0u, abort_flag, p.status, ST_ATTN + 29)) {
       tc_fence_after();
       // warpgroup 0 stores dV, warpgroup 1 stores dK: one key row (256 bytes) per thread
       const long long* ds = wg == 0 ? p.dv_str : p.dk_str;
