@@ -40,6 +40,7 @@ struct FwdParams {
   float scale_log2;          // softmax scale * log2(e)
   float scale;
   uint32_t* status;
+  int heads_fast;            // grid order (H, B, query blocks) instead of (query blocks, H, B)
   int pingpong;              // 1: the two softmax warpgroups take turns on the exponentials (see the kernel)
 };
 
@@ -115,8 +116,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   auto turn = [&](int t) { return bar_base + 136u + 8u * t; };
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int qblk = gridDim.x - 1 - blockIdx.x;          // longest rows first
-  const int h = blockIdx.y, b = blockIdx.z;
+  // longest rows first: within a head, or (heads_fast) over all heads, which packs the blocks of a short grid better
+  const int qblk = (p.heads_fast ? gridDim.z : gridDim.x) - 1 - (p.heads_fast ? blockIdx.z : blockIdx.x);
+  const int h = p.heads_fast ? blockIdx.x : blockIdx.y, b = p.heads_fast ? blockIdx.y : blockIdx.z;
   const int q0 = qblk * 2 * BQ;
   const int kv_blocks = (p.Lk + BK - 1) / BK;
   int nb[2];
@@ -843,8 +845,13 @@ extern "C" int sb_attn_fwd(const void* q, const void* k, const void* v, void* ou
     attr_set = true;
   }
   FwdParams p{reinterpret_cast<__nv_bfloat16*>(out), lse, o_str[0], o_str[1], o_str[2], B, H, Lq, Lk, causal,
-              scale * 1.4426950408889634f, scale, status, g_pingpong};
-  dim3 grid((Lq + 2 * BQ - 1) / (2 * BQ), H, B);
+              scale * 1.4426950408889634f, scale, status, 0, g_pingpong};
+  const int qblocks = (Lq + 2 * BQ - 1) / (2 * BQ);
+  // Causal rows differ in length.  While the keys and values of all heads together sit in the L2 cache, the longest blocks of
+  // all heads go first (B = 2, L = 1333, 16 heads: 192 blocks on 148 SMs, 44 -> 32 us); beyond that the blocks of one head
+  // stay together, so that its keys are read from memory once.
+  p.heads_fast = causal && (long long)B * H * Lk * HD * 4 <= (32LL << 20) && qblocks <= 65535 && B <= 65535;
+  const dim3 grid = p.heads_fast ? dim3(H, B, qblocks) : dim3(qblocks, H, B);
   if (g_fwd_p_tmem) attn_fwd_kernel<true><<<grid, FWD_THREADS, FWD_SMEM, stream>>>(tq, tk, tv, p);
   else attn_fwd_kernel<false><<<grid, FWD_THREADS, FWD_SMEM, stream>>>(tq, tk, tv, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -6;
