@@ -114,3 +114,42 @@ def test_decode_step(B, T, steps):
         assert (a - b).norm() <= 2.2e-2 * b.norm(), (i, ((a - b).norm() / b.norm()).item())
     with pytest.raises(ValueError):
         fast.step(toks[:1, 0].repeat(B + 1))
+
+
+@pytest.mark.parametrize("L", [1, 63, 64, 65, 127, 128, 129, 256, 300, 641])
+@pytest.mark.parametrize("causal", [True, False])
+def test_attention_tiles(L, causal):
+    """One tile more or less than the 64- and 128-row tiles of the kernels, forward and backward."""
+    torch.manual_seed(L)
+    q, k, v = (torch.randn(2, L, 3, 128, device=DEV).to(BF).requires_grad_() for _ in range(3))
+    o = ops.attention(q, k, v, causal)
+    g = torch.randn_like(o)
+    o.backward(g)
+    qr, kr, vr = (t.detach().float().requires_grad_() for t in (q, k, v))
+    orf = ref.attention(qr, kr, vr, causal)
+    orf.backward(g.float())
+    from savanna_b200.ops import cuda_ops
+    cuda_ops.check_status()
+    # bf16 probabilities and score gradients as MMA operands, one rounding (up to 2^-8) in each of three factors of a term and
+    # one of the result; the terms of dq and dk cancel to about half their size: 4 % of value plus rms
+    for got, want, n in ((o, orf, "o"), (q.grad, qr.grad, "dq"), (k.grad, kr.grad, "dk"), (v.grad, vr.grad, "dv")):
+        if L == 1 and n in ("dq", "dk"):                     # one key: the softmax is constant, the gradients are zero
+            assert got.abs().max() <= 1e-5, n
+        else:
+            _close(got, want, 4e-2, n)
+
+
+def test_packed_attention_rotary():
+    """Partial rotary dimensions and odd lengths of the packed projection, against the unpacked statement."""
+    for rd, L, H in ((16, 5, 1), (64, 70, 3), (128, 129, 33)):
+        torch.manual_seed(rd)
+        qkv = torch.randn(1, L, H, 384, device=DEV).to(BF).requires_grad_()
+        cos, sin = ref.rope_tables(torch.arange(L, device=DEV), rd)
+        o = ops.attention_packed(qkv, cos, sin, True)
+        g = torch.randn_like(o)
+        o.backward(g)
+        qr = qkv.detach().float().requires_grad_()
+        orf = ref.attention(ref.apply_rope(qr[..., :128], cos, sin), ref.apply_rope(qr[..., 128:256], cos, sin), qr[..., 256:], True)
+        orf.backward(g.float())
+        _close(o, orf, 2e-2, "o")                        # bf16 rotated q, k and probabilities: three roundings of up to 2^-8
+        _close(qkv.grad, qr.grad, 4e-2, "dqkv")          # as in test_attention_tiles, and the rounded q, k enter the scores
