@@ -15,9 +15,11 @@
 // Rings are indexed by position: the row of time t lives in slot t mod n.
 //
 // Measured on a B200: four layers (one of each operator), width 1024, two sequences, a prompt of 517 tokens and 16 steps:
-// 49.8 ms operator by operator (3 ms a step, all of it launches; the key / value cache was copied and converted to fp32 on
-// every step), 4.9 ms with these kernels, most of which is the prefill.  Two rows per warp keep 3072 outputs on 192 blocks
-// while every lane has eight 16-byte weight loads in flight.
+// 50.2 ms operator by operator (3 ms a step, all of it launches; the key / value cache was copied and converted to fp32 on
+// every step), 4.4 ms with these kernels, half of it the prefill.  Two rows per warp keep 3072 outputs on 192 blocks while
+// every lane has eight 16-byte weight loads in flight (6 us a matrix-vector kernel, 6.5 us a Hyena step, 9 us attention over
+// 525 keys).  Launching the kernels as programmatic dependents with the weight loads ahead of the wait changed nothing
+// (4476 against 4482 us): the host issues them no faster.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>

@@ -111,7 +111,8 @@ class _FusedStep:
         dev = model.embedding.word_embeddings.weight.device
         n = len(dec.blocks)
         self.layers = (_DecLayer * n)()
-        self.keep = []                          # tensors the descriptors point into
+        self.keep = []                          # buffers the descriptors point into
+        self.weights = []                       # (descriptor, field, parameter): followed when a parameter's storage moves
         self.attn = []                          # (layer index, key cache, value cache)
 
         def own(t):
@@ -121,18 +122,23 @@ class _FusedStep:
         def f32(t):
             return own(t.detach().float().contiguous())
 
+        def weight(L, **fields):
+            for name, p in fields.items():
+                if p is not None:
+                    self.weights.append((L, name, p))
+
         wide = 0
         for i, (blk, st) in enumerate(zip(dec.blocks, dec.states)):
             L, mixer, inner, mlp = self.layers[i], blk.mixer, blk.mixer.mixer, blk.mlp
             L.H, L.F, L.act = mixer.inner_size, mlp.ffn_local, cuda_ops._ACT[mlp.act]
-            L.norm1_w, L.eps1, L.form1 = own(blk.input_layernorm.gain), blk.input_layernorm.eps, int(blk.input_layernorm.form != "te")
+            L.eps1, L.form1 = blk.input_layernorm.eps, int(blk.input_layernorm.form != "te")
             L.norm2 = int(bool(blk.pre_mlp_norm))
             if L.norm2:
                 m = blk.pre_mlp_layernorm
-                L.norm2_w, L.eps2, L.form2 = own(m.gain), m.eps, int(m.form != "te")
-            L.w_in, L.w_out, L.b_out = own(mixer.dense_projection.weight), own(mixer.dense.weight), \
-                own(mixer.dense.bias) if mixer.dense.bias is not None else None
-            L.w12, L.w3, L.b3 = own(mlp.w12), own(mlp.w3.weight), own(mlp.w3.bias) if mlp.w3.bias is not None else None
+                L.eps2, L.form2 = m.eps, int(m.form != "te")
+                weight(L, norm2_w=m.gain)
+            weight(L, norm1_w=blk.input_layernorm.gain, w_in=mixer.dense_projection.weight, w_out=mixer.dense.weight,
+                   b_out=mixer.dense.bias, w12=mlp.w12, w3=mlp.w3.weight, b3=mlp.w3.bias)
             wide = max(wide, L.H, L.F)
             if isinstance(inner, SelfAttention):
                 L.kind, L.heads, L.rd, L.pos_scale = 3, inner.heads, 0, 1.0
@@ -194,6 +200,10 @@ class _FusedStep:
         if token.shape[0] != self.batch:
             raise ValueError(f"decode step for {token.shape[0]} sequences, prefilled with {self.batch}")
         self._reserve(pos + 1)
+        for L, name, p in self.weights:
+            ptr = p.data_ptr()
+            if getattr(L, name) != ptr:
+                setattr(L, name, ptr)
         x = self.model.embedding(token[:, None], None)[:, 0].contiguous()
         V = self.head.shape[0] if self.head is not None else 0
         out = torch.empty(self.batch, V, dtype=torch.float32, device=x.device) if V else None
@@ -287,13 +297,16 @@ class CachedDecoder:
                         st["s"] = s.float()
                 hooks.append(inner.register_forward_pre_hook(grab_feat))
         was_training = model.training
-        model.eval()
+        switch = any(m.training for m in model.modules())          # a model in eval mode is left alone
+        if switch:
+            model.eval()
         try:
             logits = model(tokens)[:, -1].float()
         finally:
             for h in hooks:
                 h.remove()
-            model.train(was_training)
+            if switch:
+                model.train(was_training)
         self.pos = T
         self._fused = _FusedStep.build(self, B)
         return logits
@@ -355,13 +368,14 @@ class CachedDecoder:
         model, cfg = self.model, self.cfg
         if self._fused is not None:
             was_training = model.training
-            if was_training:
+            switch = any(m.training for m in model.embedding.modules())       # the only module that runs here
+            if switch:
                 model.eval()
             try:
                 logits = self._fused(token, self.pos)
             finally:
-                if was_training:
-                    model.train()
+                if switch:
+                    model.train(was_training)
             self.pos += 1
             return logits
         dtype = cfg.params_dtype
