@@ -398,11 +398,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 //   dK  += dS^T Q           [keys x d]   A = dS^T (K-major),                    B = Q_i  (MN-major)
 //   dQ^T = K^T dS^T         [d x q]      A = K (MN-major),   B = dS^T (MN-major)   -> fp32 atomics into dq_acc
 // with P = exp(S * scale - lse) and dS = P (dP - delta) * scale computed by one thread per key row and 32 query columns
-// (two warpgroups split the 64 columns), and dQ^T read out by four warps of its own: with both in the same eight warps and
-// dP^T waiting for the previous tile's dS^T, three quarters of a tile's time was one chain (1574 us at L = 8192, 32 heads,
-// causal; 1475 now, the products' operand reads from shared memory being the next bound: about 2400 of 3200 cycles a tile).
-// Adding dQ straight from registers with red.global instead of through the staging tile took 2402.  TMEM: S^T (2 x 64 columns, so the scores of the next tile are computed during
-// this tile's softmax), dP^T (64), dQ^T (64), dV (128), dK (128).
+// (two warpgroups split the 64 columns); four more warps read dQ^T out.  TMEM: S^T (2 x 64 columns, so the scores of the
+// next tile are computed during this tile's softmax), dP^T (64; released as soon as it is in registers), dQ^T (64), dV (128),
+// dK (128).
+// Before, the eight softmax warps also read dQ^T out between two tiles, and dP^T waited for the previous tile's dS^T: 1574 us
+// at L = 8192, 32 heads, causal, 1475 now.  By count, the operand reads of the five products and the staging of a tile take
+// 2400 cycles of shared-memory bandwidth out of about 3200.  Adding dQ straight from registers with red.global instead of
+// through the staging tile took 2402 us.
 constexpr int BQ2 = 64;                          // query rows per backward tile
 constexpr int QTILE_BYTES = BQ2 * HD * 2;        // 16 KB: two boxes of 8 KB
 constexpr int QBOX_BYTES = BQ2 * 128;            // 8 KB
@@ -760,9 +762,10 @@ attn_stats_kernel(const __nv_bfloat16* __restrict__ go, const __nv_bfloat16* __r
 
 // Rotary embedding of up to two [B, L, H, 128] tensors in one pass (queries and keys; in the backward the fp32 query-gradient
 // accumulator and the key gradient, inverse).  A block takes one token; a thread keeps 8 channels and their partners half a
-// rotation away of ROPE_HEADS heads, so both halves are loaded once, the fp32 table row is read once for all of them (it is
-// as large as the data of four heads) and a bf16 destination may be its own source.  Channels beyond the rotary dimension are copied.  At L = 8192 with 32 heads: 89 us for
-// queries and keys (one launch each way), where the general kernel took 59 us a tensor and a cast of dq another 31.
+// rotation away of ROPE_HEADS heads, so both halves are loaded once, the fp32 table row is read once for all of them (it is as
+// large as the data of four heads) and a bf16 destination may be its own source.  Channels beyond the rotary dimension are
+// copied.  At L = 8192 with 32 heads: 89 us for queries and keys (one launch each way), where the general kernel took 59 us a
+// tensor and a cast of dq another 31.
 struct RopeSide {
   const void* src;
   __nv_bfloat16* dst;
