@@ -761,18 +761,19 @@ attn_stats_kernel(const __nv_bfloat16* __restrict__ go, const __nv_bfloat16* __r
 }
 
 // Rotary embedding of up to two [B, L, H, 128] tensors in one pass (queries and keys; in the backward the fp32 query-gradient
-// accumulator and the key gradient, inverse).  A block takes one token; a thread keeps 8 channels and their partners half a
-// rotation away of ROPE_HEADS heads, so both halves are loaded once, the fp32 table row is read once for all of them (it is as
-// large as the data of four heads) and a bf16 destination may be its own source.  Channels beyond the rotary dimension are
-// copied.  At L = 8192 with 32 heads: 89 us for queries and keys (one launch each way), where the general kernel took 59 us a
-// tensor and a cast of dq another 31.
+// accumulator and the key gradient, inverse).  A block takes one token of one tensor; a thread keeps 8 channels and their
+// partners half a rotation away of ROPE_HEADS heads, so both halves are loaded once, the fp32 table row is read once for all of
+// them (it is as large as the data of four heads) and a bf16 destination may be its own source.  Channels beyond the rotary
+// dimension are copied.  Bound by loads in flight: at L = 8192 with 32 heads 77 us for queries and keys (one launch each way;
+// 89 with both tensors in one block, two heads at a time), where the general kernel took 59 us a tensor and a cast of dq
+// another 31.
 struct RopeSide {
   const void* src;
   __nv_bfloat16* dst;
   long long s_sb, s_sl, s_sh, d_sb, d_sl, d_sh;       // element strides
   int f32;                                            // src is fp32
 };
-struct RopeArgs { RopeSide side[2]; const float* cs; const float* sn; int n, L, H, rd; float sign; };
+struct RopeArgs { RopeSide side[2]; const float* cs; const float* sn; int H, rd; float sign; };
 
 __device__ __forceinline__ void rope_ld8(const void* p, long long off, int f32, float (&f)[8]) {
   if (f32) {
@@ -797,6 +798,7 @@ constexpr int ROPE_HEADS = 4;
 __global__ void __launch_bounds__(256)
 attn_rope_kernel(const RopeArgs a) {
   const int l = blockIdx.x, b = blockIdx.y;
+  const RopeSide& d = a.side[blockIdx.z];
   const int half = a.rd / 2, nrot = half / 8, units = nrot + (HD - a.rd) / 8;
   for (int u = threadIdx.x & 7; u < units; u += 8) {
     const bool rot = u < nrot;
@@ -808,29 +810,24 @@ attn_rope_kernel(const RopeArgs a) {
       rope_ld8(cr, 0, 1, c1); rope_ld8(cr, half, 1, c2);
       rope_ld8(sr, 0, 1, s1); rope_ld8(sr, half, 1, s2);
     }
-#pragma unroll 2
+#pragma unroll 4
     for (int h = threadIdx.x >> 3; h < a.H; h += blockDim.x >> 3) {
+      const long long so = b * d.s_sb + l * d.s_sl + h * d.s_sh + c0;
+      __nv_bfloat16* dst = d.dst + b * d.d_sb + l * d.d_sl + h * d.d_sh + c0;
+      float lo[8];
+      rope_ld8(d.src, so, d.f32, lo);
+      if (rot) {
+        float hi[8], o1[8], o2[8];
+        rope_ld8(d.src, so + half, d.f32, hi);
 #pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        if (t >= a.n) break;
-        const RopeSide& d = a.side[t];
-        const long long so = b * d.s_sb + l * d.s_sl + h * d.s_sh + c0;
-        __nv_bfloat16* dst = d.dst + b * d.d_sb + l * d.d_sl + h * d.d_sh + c0;
-        float lo[8];
-        rope_ld8(d.src, so, d.f32, lo);
-        if (rot) {
-          float hi[8], o1[8], o2[8];
-          rope_ld8(d.src, so + half, d.f32, hi);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            o1[j] = lo[j] * c1[j] - hi[j] * (a.sign * s1[j]);
-            o2[j] = hi[j] * c2[j] + lo[j] * (a.sign * s2[j]);
-          }
-          rope_st8(dst, o1);
-          rope_st8(dst + half, o2);
-        } else {
-          rope_st8(dst, lo);
+        for (int j = 0; j < 8; ++j) {
+          o1[j] = lo[j] * c1[j] - hi[j] * (a.sign * s1[j]);
+          o2[j] = hi[j] * c2[j] + lo[j] * (a.sign * s2[j]);
         }
+        rope_st8(dst, o1);
+        rope_st8(dst + half, o2);
+      } else {
+        rope_st8(dst, lo);
       }
     }
   }
@@ -1016,9 +1013,9 @@ extern "C" int sb_attn_rope(const void* const* src, void* const* dst, const long
     a.side[i] = RopeSide{src[i], (__nv_bfloat16*)dst[i], src_str[3 * i], src_str[3 * i + 1], src_str[3 * i + 2],
                          dst_str[3 * i], dst_str[3 * i + 1], dst_str[3 * i + 2], src_f32[i]};
   }
-  a.cs = cs; a.sn = sn; a.n = n; a.L = L; a.H = H; a.rd = rd; a.sign = inverse ? -1.f : 1.f;
+  a.cs = cs; a.sn = sn; a.H = H; a.rd = rd; a.sign = inverse ? -1.f : 1.f;
   const int cols = (H + ROPE_HEADS - 1) / ROPE_HEADS;          // head columns of a block
-  attn_rope_kernel<<<dim3(L, B), cols < 4 ? 32 : (cols > 32 ? 256 : cols * 8), 0, stream>>>(a);
+  attn_rope_kernel<<<dim3(L, B, n), cols < 4 ? 32 : (cols > 32 ? 256 : cols * 8), 0, stream>>>(a);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
