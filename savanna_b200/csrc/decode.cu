@@ -8,7 +8,8 @@
 //                weights in 16-byte loads against the inputs of all batch rows, which every block prepares in shared
 //                memory (as they are, RMS-normalised, or gated); fp32 accumulation, one rounding of the result
 //   dec_hyena    featuriser taps, gate and the recurrent form of the operator: a ring of past u for the FIR filters, the
-//                modal states for the long filter
+//                modal states for the long filter.  Filters are read as their parameters are stored (decay window, poles
+//                from gamma and p), so a step never works from an older copy of them
 //   dec_attn     rotary embedding, append to the key / value cache, attention over the cache: the keys of one head are
 //                split over a cluster of eight blocks that merge their partial softmax through distributed shared memory
 //
@@ -41,12 +42,17 @@ constexpr int ATT_THREADS = 128;
 enum { IN_PLAIN = 0, IN_NORM = 1, IN_GATE = 2 };
 enum { OP_SE = 0, OP_MR = 1, OP_LI = 2, OP_ATTN = 3 };
 
+// Bits of Layer::f32: the filter parameters stored in fp32 (the others are bf16).
+enum { F_CONV = 1, F_TAPS = 2, F_DECAY = 4, F_BIAS = 8, F_GAMMA = 16, F_P = 32, F_R = 64 };
+
 // Mirrors `_DecLayer` of inference/cached.py.
 struct Layer {
   int kind, H, F, kf, K, G, O, heads, rd, act, pregate, postgate, form1, form2, norm2, cap;
+  int f32, conv_g, tap_ld, newest_first;   // conv_g: groups of the featuriser; taps [G, tap_ld], of which K are used
   float eps1, eps2, pos_scale;
   const bf16 *norm1_w, *w_in, *w_out, *b_out, *norm2_w, *w12, *w3, *b3;
-  const float *conv_w, *taps, *bias, *lam, *R, *inv_freq;
+  const void *conv_w, *taps, *decay, *bias, *gamma, *p, *R;    // [conv_g, kf], [G, tap_ld] x2, [H], [G, O] x3
+  const float* inv_freq;
   bf16* proj_ring;                     // [B, kf - 1, 3H]
   float* u_ring;                       // [B, K - 1, H]
   float* state;                        // [B, H, O]
@@ -69,6 +75,19 @@ __device__ __forceinline__ float activation(float x, int act) {
   if (act == 1) return 0.5f * x * (1.f + erff(x * 0.70710678118654752f));
   if (act == 2) return fmaxf(x, 0.f);
   return x;
+}
+
+__device__ __forceinline__ float param(const void* p, size_t i, bool f32) {
+  return f32 ? reinterpret_cast<const float*>(p)[i] : __bfloat162float(reinterpret_cast<const bf16*>(p)[i]);
+}
+// Tap j of filter group `grp`, j = 0 the one of the oldest value.  With a decay window the tap is their product, which is
+// rounded as the parameters' own type rounds it.
+__device__ __forceinline__ float fir_tap(const Layer& l, int grp, int j) {
+  const size_t i = (size_t)grp * l.tap_ld + (l.newest_first ? l.K - 1 - j : j);
+  const float t = param(l.taps, i, l.f32 & F_TAPS);
+  if (!l.decay) return t;
+  const float d = t * param(l.decay, i, l.f32 & F_DECAY);
+  return (l.f32 & (F_TAPS | F_DECAY)) ? d : rbf(d);
 }
 
 struct LinArgs {
@@ -199,39 +218,42 @@ dec_hyena_kernel(Layer l, const bf16* __restrict__ proj, bf16* __restrict__ z, i
 #pragma unroll
     for (int p = 0; p < 3; ++p) {
       const int c = 3 * ch + p;
-      const float* w = l.conv_w + (size_t)c * l.kf;
+      const size_t w = (size_t)(c / (3 * l.H / l.conv_g)) * l.kf;
+      const bool wf = l.f32 & F_CONV;
       const bf16 cur = proj[(size_t)b * 3 * l.H + c];
-      float acc = w[n] * __bfloat162float(cur);
+      float acc = param(l.conv_w, w + n, wf) * __bfloat162float(cur);
       bf16* ring = l.proj_ring + (size_t)b * n * 3 * l.H + c;
-      for (int j = 0; j < n; ++j) acc += w[j] * __bfloat162float(ring[(size_t)((pos + j) % n) * 3 * l.H]);
+      for (int j = 0; j < n; ++j) acc += param(l.conv_w, w + j, wf) * __bfloat162float(ring[(size_t)((pos + j) % n) * 3 * l.H]);
       if (n > 0) ring[(size_t)(pos % n) * 3 * l.H] = cur;
       f[p] = rbf(acc);                                     // the parallel path rounds the featuriser output
     }
     const float u = f[1] * f[2];
     sx1[cx] = f[0];
     su[cx] = (l.kind == OP_SE && !l.pregate) ? f[2] : u;
-    sb[cx] = l.kind == OP_SE ? 0.f : l.bias[ch] * u;
+    sb[cx] = l.kind == OP_SE ? 0.f : param(l.bias, ch, l.f32 & F_BIAS) * u;
   }
   __syncthreads();
   float y = 0.f;
+  const int grp = live ? ch / (l.H / l.G) : 0;
   if (live) {
     const float u = su[cx];
     if (l.kind == OP_LI) {
       const size_t base = ((size_t)b * l.H + ch) * l.O;
       for (int o = sl; o < l.O; o += HY_SLICES) {
-        const float s = l.lam[(size_t)ch * l.O + o] * l.state[base + o] + u;
+        const size_t i = (size_t)grp * l.O + o;
+        const float lam = expf(-expf(param(l.p, i, l.f32 & F_P)) * expf(param(l.gamma, i, l.f32 & F_GAMMA)));
+        const float s = lam * l.state[base + o] + u;
         l.state[base + o] = s;
-        y += l.R[(size_t)ch * l.O + o] * s;
+        y += param(l.R, i, l.f32 & F_R) * s;
       }
     } else {
       const int n = l.K - 1;
-      const float* taps = l.taps + (size_t)(ch / (l.H / l.G)) * l.K;      // oldest first
       const float* ring = l.u_ring + (size_t)b * n * l.H + ch;
 #pragma unroll 8
       for (int j = sl; j < n; j += HY_SLICES) {
         int slot = pos % n + j;
         if (slot >= n) slot -= n;
-        y += taps[j] * ring[(size_t)slot * l.H];
+        y += fir_tap(l, grp, j) * ring[(size_t)slot * l.H];
       }
     }
   }
@@ -242,7 +264,7 @@ dec_hyena_kernel(Layer l, const bf16* __restrict__ proj, bf16* __restrict__ z, i
   for (int j = 1; j < HY_SLICES; ++j) y += part[j][cx];
   if (l.kind != OP_LI) {
     const int n = l.K - 1;
-    y += l.taps[(size_t)(ch / (l.H / l.G)) * l.K + n] * su[cx];
+    y += fir_tap(l, grp, n) * su[cx];
     if (n > 0) l.u_ring[((size_t)b * n + pos % n) * l.H + ch] = su[cx];
   }
   y += sb[cx];

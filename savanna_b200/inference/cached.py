@@ -26,7 +26,7 @@ from typing import Dict, List, Optional
 import torch
 import torch.nn.functional as F
 
-from ..models.filters import ImplicitModalFilter
+from ..models.filters import ExplicitSingleDecayFilter, ImplicitModalFilter
 from ..models.hyena import HyenaOperator, ShortHyenaOperator
 from ..models.mixer import SelfAttention
 from ..models.mlp import ParallelGLU
@@ -45,10 +45,14 @@ def _act(name: str):
 class _DecLayer(ctypes.Structure):
     """Mirrors sb::dec::Layer (csrc/decode.cu)."""
     _fields_ = ([(n, ctypes.c_int) for n in ("kind", "H", "F", "kf", "K", "G", "O", "heads", "rd", "act", "pregate", "postgate",
-                                             "form1", "form2", "norm2", "cap")]
+                                             "form1", "form2", "norm2", "cap", "f32", "conv_g", "tap_ld", "newest_first")]
                 + [(n, ctypes.c_float) for n in ("eps1", "eps2", "pos_scale")]
                 + [(n, ctypes.c_void_p) for n in ("norm1_w", "w_in", "w_out", "b_out", "norm2_w", "w12", "w3", "b3", "conv_w", "taps",
-                                                  "bias", "lam", "R", "inv_freq", "proj_ring", "u_ring", "state", "kc", "vc")])
+                                                  "decay", "bias", "gamma", "p", "R", "inv_freq", "proj_ring", "u_ring", "state",
+                                                  "kc", "vc")])
+
+
+_F32 = {n: 1 << i for i, n in enumerate(("conv_w", "taps", "decay", "bias", "gamma", "p", "R"))}     # bits of _DecLayer.f32
 
 
 def _ring(tail: torch.Tensor, pos: int) -> torch.Tensor:
@@ -91,7 +95,26 @@ class _FusedStep:
         def norm(m):
             return isinstance(m, RMSNorm) and weight(m.gain, D)
 
-        for blk in dec.blocks:
+        def source(t, *shape):                  # a filter parameter, read as it is stored
+            return t.dtype in (torch.bfloat16, torch.float32) and t.is_cuda and t.is_contiguous() and tuple(t.shape) == shape
+
+        def filters(mixer, st):
+            conv, op, H = mixer.hyena_proj_conv, mixer.mixer, mixer.inner_size
+            if not source(conv.taps(), conv.num_groups, conv.kernel_size) or conv.num_groups * conv.group_dim != 3 * H \
+                    or st["proj_tail"].shape[1] != conv.kernel_size - 1:
+                return False
+            if isinstance(op, ShortHyenaOperator):
+                return source(op.short_conv.taps(), op.num_groups, op.kernel_size) and op.num_groups * op.group_dim == H
+            if not source(op.conv_bias, H) or op.num_groups * op.group_dim != H:
+                return False
+            if op.is_mr:
+                f, G, K = op.filter, op.num_groups, st["u_tail"].shape[1] + 1
+                if type(f) is not ExplicitSingleDecayFilter:
+                    return tuple(f(K).shape) == (G, K)
+                return f.h.dim() == 2 and f.h.shape[1] >= K and all(source(t, G, f.h.shape[1]) for t in (f.h, f.decay))
+            return all(source(t, op.num_groups, op.filter.gamma.shape[1]) for t in (op.filter.gamma, op.filter.p, op.filter.R))
+
+        for blk, st in zip(dec.blocks, dec.states):
             mixer, mlp = blk.mixer, blk.mlp
             H, Fi = mixer.inner_size, mlp.ffn_local
             if (D % 8 or H % 8 or Fi % 8 or max(D, H, Fi) > wmax or mlp.act not in cuda_ops._ACT or not norm(blk.input_layernorm)
@@ -99,7 +122,10 @@ class _FusedStep:
                     or not weight(mixer.dense.weight, D, H) or not weight(mlp.w12, 2 * Fi, D) or not weight(mlp.w3.weight, D, Fi)
                     or any(b is not None and not weight(b, D) for b in (mixer.dense.bias, mlp.w3.bias))):
                 return None
-            if isinstance(mixer.mixer, SelfAttention) and (mixer.mixer.hd != 128 or mixer.mixer.heads * 128 != H):
+            if isinstance(mixer.mixer, SelfAttention):
+                if mixer.mixer.hd != 128 or mixer.mixer.heads * 128 != H:
+                    return None
+            elif not filters(mixer, st):
                 return None
         return _FusedStep(dec, lib, batch)
 
@@ -113,19 +139,18 @@ class _FusedStep:
         self.layers = (_DecLayer * n)()
         self.keep = []                          # buffers the descriptors point into
         self.weights = []                       # (descriptor, field, parameter): followed when a parameter's storage moves
+        self.filters = []                       # (descriptor, module, taps): filters without a form of their own in the kernel
         self.attn = []                          # (layer index, key cache, value cache)
 
         def own(t):
             self.keep.append(t)
             return t.data_ptr()
 
-        def f32(t):
-            return own(t.detach().float().contiguous())
-
         def weight(L, **fields):
             for name, p in fields.items():
                 if p is not None:
                     self.weights.append((L, name, p))
+                    L.f32 |= _F32.get(name, 0) if p.dtype == torch.float32 else 0
 
         wide = 0
         for i, (blk, st) in enumerate(zip(dec.blocks, dec.states)):
@@ -145,28 +170,33 @@ class _FusedStep:
                 if inner._rotary:
                     r = inner._rotary[0]
                     L.rd, L.pos_scale = r.dim, r.scaling_factor
-                    L.inv_freq = f32(1.0 / (r.base ** (torch.arange(0, r.dim, 2, device=dev, dtype=torch.float32) / r.dim)))
+                    L.inv_freq = own(1.0 / (r.base ** (torch.arange(0, r.dim, 2, device=dev, dtype=torch.float32) / r.dim)))
                 self.attn.append([i, st["k"], st["v"]])
             else:
                 conv = mixer.hyena_proj_conv
-                w = conv.taps()
-                L.kf = w.shape[1]
-                L.conv_w = f32(w.repeat_interleave(conv.group_dim, dim=0) if conv.group_dim > 1 else w)
+                L.kf, L.conv_g = conv.kernel_size, conv.num_groups
+                weight(L, conv_w=conv.short_conv_weight)
                 L.proj_ring = own(_ring(st["proj_tail"].to(torch.bfloat16), dec.pos))
                 L.pregate = L.postgate = 1
+                L.G = inner.num_groups
                 if isinstance(inner, ShortHyenaOperator):
-                    taps = inner.short_conv.taps()
                     L.kind, L.pregate, L.postgate = 0, int(bool(inner.pregate)), int(bool(inner.postgate))
-                    L.taps, L.K, L.G = f32(taps), taps.shape[1], taps.shape[0]
+                    L.K = L.tap_ld = inner.kernel_size
+                    weight(L, taps=inner.short_conv.short_conv_weight)
                     L.u_ring = own(_ring(st["u_tail"].float(), dec.pos))
                 elif inner.is_mr:
-                    taps = inner.filter(st["u_tail"].shape[1] + 1).flip(-1)
-                    L.kind, L.taps, L.K, L.G, L.bias = 1, f32(taps), taps.shape[1], taps.shape[0], f32(inner.conv_bias)
+                    L.kind, L.newest_first, L.K = 1, 1, st["u_tail"].shape[1] + 1
+                    weight(L, bias=inner.conv_bias)
+                    if type(inner.filter) is ExplicitSingleDecayFilter:
+                        L.tap_ld = inner.filter.h.shape[1]
+                        weight(L, taps=inner.filter.h, decay=inner.filter.decay)
+                    else:
+                        L.tap_ld, L.f32 = L.K, L.f32 | _F32["taps"]
+                        self.filters.append([L, inner.filter, None])
                     L.u_ring = own(_ring(st["u_tail"].float(), dec.pos))
                 else:
-                    g, R, p = inner._modal()
-                    L.kind, L.O, L.bias = 2, g.shape[1], f32(inner.conv_bias)
-                    L.lam, L.R = f32(torch.exp(-torch.exp(p.detach().float()) * torch.exp(g.detach().float()))), f32(R)
+                    L.kind, L.O = 2, inner.filter.gamma.shape[1]
+                    weight(L, bias=inner.conv_bias, gamma=inner.filter.gamma, p=inner.filter.p, R=inner.filter.R)
                     L.state = own(st["s"].float().contiguous().clone())
             st.clear()                           # this object owns the state from here on
         self._reserve(dec.pos + 1)
@@ -204,6 +234,9 @@ class _FusedStep:
             ptr = p.data_ptr()
             if getattr(L, name) != ptr:
                 setattr(L, name, ptr)
+        for e in self.filters:
+            e[2] = e[1](e[0].K).float().contiguous()
+            e[0].taps = e[2].data_ptr()
         x = self.model.embedding(token[:, None], None)[:, 0].contiguous()
         V = self.head.shape[0] if self.head is not None else 0
         out = torch.empty(self.batch, V, dtype=torch.float32, device=x.device) if V else None

@@ -1,0 +1,86 @@
+"""The native decode step (csrc/decode.cu) against the operator-by-operator step of the same decoder: parameters that change
+between steps."""
+import os
+
+import pytest
+import torch
+
+from savanna_b200.config import GlobalConfig
+from savanna_b200.inference import cached
+from savanna_b200.inference.cached import CachedDecoder
+from savanna_b200.models import build_model
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+TINY = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "configs", "baseline", "tiny_sh2_gpu.yml")
+
+
+def _model(**over):
+    cfg = GlobalConfig.from_ymls([TINY], {"global_num_gpus": 1, **over})
+    cfg.build_tokenizer()
+    torch.manual_seed(0)
+    model = build_model(cfg, device=DEV)
+    with torch.no_grad():                                  # make the state-dependent terms matter
+        for n, p in model.named_parameters():
+            if n.endswith("filter.h"):
+                p.mul_(3e4)
+    return model.eval()
+
+
+def _slow(model, toks, monkeypatch):
+    """A decoder prefilled with `toks` that steps operator by operator."""
+    dec = CachedDecoder(model)
+    with monkeypatch.context() as m:
+        m.setattr(cached._FusedStep, "build", staticmethod(lambda *_: None))
+        dec.prefill(toks)
+    return dec
+
+
+def _toks(model, B, n):
+    return torch.randint(0, 256, (B, n), device=DEV, generator=torch.Generator(DEV).manual_seed(n))
+
+
+def _agree(fast, slow, toks):
+    """Both round activations to bf16, at different places: each step's logits within 2.2 % (2-norm), as derived in
+    test_gpu_tile_edges.py."""
+    for t in toks.unbind(1):
+        a, b = fast.step(t), slow.step(t)
+        assert (a - b).norm() <= 2.2e-2 * b.norm(), ((a - b).norm() / b.norm()).item()
+
+
+def _is_filter(n):
+    return any(k in n for k in ("short_conv", ".filter.", "conv_bias"))
+
+
+@pytest.mark.parametrize("which", ["filters", "projections"])
+@pytest.mark.parametrize("over", [{}, {"hyena_medium_filter_cls": "implicit_modal"}], ids=["explicit", "modal_mr"])
+def test_parameters_changed_in_place_between_steps(which, over, monkeypatch):
+    """A step reads every parameter as it is then, filters as well as projections."""
+    model = _model(**over)
+    toks = _toks(model, 2, 30)
+    fast, slow = CachedDecoder(model), _slow(model, toks[:, :20], monkeypatch)
+    fast.prefill(toks[:, :20])
+    assert fast._fused is not None
+    _agree(fast, slow, toks[:, 20:23])
+    before = slow.step(toks[:, 23])
+    fast.step(toks[:, 23])
+    g = torch.Generator(DEV).manual_seed(3)
+    with torch.no_grad():
+        for n, p in model.named_parameters():
+            if _is_filter(n) == (which == "filters") and "norm" not in n and "word_emb" not in n:
+                s = float(p.float().std()) or 0.1
+                p.data.add_(torch.randn(p.shape, device=DEV, generator=g) * s)
+    _agree(fast, slow, toks[:, 24:])
+    assert (slow.step(toks[:, 0]) - before).norm() > 0.1 * before.norm()          # the change reached the logits
+
+
+def test_filters_stored_in_bf16(monkeypatch):
+    model = _model()
+    for n, p in model.named_parameters():
+        if _is_filter(n):
+            p.data = p.data.bfloat16()
+    toks = _toks(model, 1, 30)
+    fast, slow = CachedDecoder(model), _slow(model, toks[:, :25], monkeypatch)
+    fast.prefill(toks[:, :25])
+    assert fast._fused is not None
+    _agree(fast, slow, toks[:, 25:])
