@@ -63,9 +63,10 @@ def _ring(tail: torch.Tensor, pos: int) -> torch.Tensor:
 
 class _FusedStep:
     """The decode step of csrc/decode.cu: the layers' weights by address, their state in the layout of its kernels.  Built at
-    the end of a prefill; `build` returns None when something is not covered (CPU tensors, other dtypes than bf16, other norms
-    than RMSNorm, head sizes other than 128, more than 8 sequences, unaligned or non-contiguous weights), and the decoder then
-    steps operator by operator."""
+    the end of a prefill and after the state was handed out (`CachedDecoder.states`); `build` returns None when something is not
+    covered (CPU tensors, other dtypes than bf16, other norms than RMSNorm, head sizes other than 128, more than 8 sequences, an
+    inner size above `sb_decode_max_width`: 102400 for one sequence, 12800 for eight; unaligned or non-contiguous weights), and the
+    decoder then steps operator by operator."""
 
     @staticmethod
     def build(dec: "CachedDecoder", batch: int):
@@ -87,6 +88,8 @@ class _FusedStep:
         if lib.sb_decode_layer_bytes() != ctypes.sizeof(_DecLayer):
             raise RuntimeError("decode layer descriptor does not match the native library (rebuild savanna_b200.csrc)")
         D, wmax = cfg.hidden_size, lib.sb_decode_max_width(batch)
+        if len(dec._states) != len(dec.blocks):
+            return None
 
         def weight(t, *shape):
             return (t is not None and t.dtype == torch.bfloat16 and t.is_cuda and t.is_contiguous() and t.data_ptr() % 16 == 0
@@ -98,23 +101,30 @@ class _FusedStep:
         def source(t, *shape):                  # a filter parameter, read as it is stored
             return t.dtype in (torch.bfloat16, torch.float32) and t.is_cuda and t.is_contiguous() and tuple(t.shape) == shape
 
+        def held(t, *shape):                    # a piece of state, whoever filled the dictionary
+            return t is not None and t.device == w.device and tuple(t.shape) == (batch,) + shape
+
         def filters(mixer, st):
             conv, op, H = mixer.hyena_proj_conv, mixer.mixer, mixer.inner_size
             if not source(conv.taps(), conv.num_groups, conv.kernel_size) or conv.num_groups * conv.group_dim != 3 * H \
-                    or st["proj_tail"].shape[1] != conv.kernel_size - 1:
+                    or not held(st.get("proj_tail"), conv.kernel_size - 1, 3 * H) or st["proj_tail"].dtype != torch.bfloat16:
                 return False
             if isinstance(op, ShortHyenaOperator):
-                return source(op.short_conv.taps(), op.num_groups, op.kernel_size) and op.num_groups * op.group_dim == H
+                return (source(op.short_conv.taps(), op.num_groups, op.kernel_size) and op.num_groups * op.group_dim == H
+                        and held(st.get("u_tail"), op.kernel_size - 1, H))
             if not source(op.conv_bias, H) or op.num_groups * op.group_dim != H:
                 return False
             if op.is_mr:
-                f, G, K = op.filter, op.num_groups, st["u_tail"].shape[1] + 1
+                f, G, K = op.filter, op.num_groups, op.hyena_mr_len
+                if not held(st.get("u_tail"), K - 1, H):
+                    return False
                 if type(f) is not ExplicitSingleDecayFilter:
                     return tuple(f(K).shape) == (G, K)
                 return f.h.dim() == 2 and f.h.shape[1] >= K and all(source(t, G, f.h.shape[1]) for t in (f.h, f.decay))
-            return all(source(t, op.num_groups, op.filter.gamma.shape[1]) for t in (op.filter.gamma, op.filter.p, op.filter.R))
+            O = op.filter.gamma.shape[1]
+            return held(st.get("s"), H, O) and all(source(t, op.num_groups, O) for t in (op.filter.gamma, op.filter.p, op.filter.R))
 
-        for blk, st in zip(dec.blocks, dec.states):
+        for blk, st in zip(dec.blocks, dec._states):
             mixer, mlp = blk.mixer, blk.mlp
             H, Fi = mixer.inner_size, mlp.ffn_local
             if (D % 8 or H % 8 or Fi % 8 or max(D, H, Fi) > wmax or mlp.act not in cuda_ops._ACT or not norm(blk.input_layernorm)
@@ -123,7 +133,9 @@ class _FusedStep:
                     or any(b is not None and not weight(b, D) for b in (mixer.dense.bias, mlp.w3.bias))):
                 return None
             if isinstance(mixer.mixer, SelfAttention):
-                if mixer.mixer.hd != 128 or mixer.mixer.heads * 128 != H:
+                heads = mixer.mixer.heads
+                if mixer.mixer.hd != 128 or heads * 128 != H or not all(
+                        held(st.get(n), dec.pos, heads, 128) and st[n].dtype == torch.bfloat16 for n in ("k", "v")):
                     return None
             elif not filters(mixer, st):
                 return None
@@ -141,9 +153,15 @@ class _FusedStep:
         self.weights = []                       # (descriptor, field, parameter): followed when a parameter's storage moves
         self.filters = []                       # (descriptor, module, taps): filters without a form of their own in the kernel
         self.attn = []                          # (layer index, key cache, value cache)
+        self.rings = []                         # (layer index, name of the state, buffer) of the Hyena layers
+        self.pos = dec.pos
 
         def own(t):
             self.keep.append(t)
+            return t.data_ptr()
+
+        def ring(i, name, t):
+            self.rings.append((i, name, t))
             return t.data_ptr()
 
         def weight(L, **fields):
@@ -153,7 +171,7 @@ class _FusedStep:
                     L.f32 |= _F32.get(name, 0) if p.dtype == torch.float32 else 0
 
         wide = 0
-        for i, (blk, st) in enumerate(zip(dec.blocks, dec.states)):
+        for i, (blk, st) in enumerate(zip(dec.blocks, dec._states)):
             L, mixer, inner, mlp = self.layers[i], blk.mixer, blk.mixer.mixer, blk.mlp
             L.H, L.F, L.act = mixer.inner_size, mlp.ffn_local, cuda_ops._ACT[mlp.act]
             L.eps1, L.form1 = blk.input_layernorm.eps, int(blk.input_layernorm.form != "te")
@@ -176,14 +194,14 @@ class _FusedStep:
                 conv = mixer.hyena_proj_conv
                 L.kf, L.conv_g = conv.kernel_size, conv.num_groups
                 weight(L, conv_w=conv.short_conv_weight)
-                L.proj_ring = own(_ring(st["proj_tail"].to(torch.bfloat16), dec.pos))
+                L.proj_ring = ring(i, "proj_tail", _ring(st["proj_tail"].to(torch.bfloat16), dec.pos))
                 L.pregate = L.postgate = 1
                 L.G = inner.num_groups
                 if isinstance(inner, ShortHyenaOperator):
                     L.kind, L.pregate, L.postgate = 0, int(bool(inner.pregate)), int(bool(inner.postgate))
                     L.K = L.tap_ld = inner.kernel_size
                     weight(L, taps=inner.short_conv.short_conv_weight)
-                    L.u_ring = own(_ring(st["u_tail"].float(), dec.pos))
+                    L.u_ring = ring(i, "u_tail", _ring(st["u_tail"].float(), dec.pos))
                 elif inner.is_mr:
                     L.kind, L.newest_first, L.K = 1, 1, st["u_tail"].shape[1] + 1
                     weight(L, bias=inner.conv_bias)
@@ -193,12 +211,11 @@ class _FusedStep:
                     else:
                         L.tap_ld, L.f32 = L.K, L.f32 | _F32["taps"]
                         self.filters.append([L, inner.filter, None])
-                    L.u_ring = own(_ring(st["u_tail"].float(), dec.pos))
+                    L.u_ring = ring(i, "u_tail", _ring(st["u_tail"].float(), dec.pos))
                 else:
                     L.kind, L.O = 2, inner.filter.gamma.shape[1]
                     weight(L, bias=inner.conv_bias, gamma=inner.filter.gamma, p=inner.filter.p, R=inner.filter.R)
-                    L.state = own(st["s"].float().contiguous().clone())
-            st.clear()                           # this object owns the state from here on
+                    L.state = ring(i, "s", st["s"].float().contiguous().clone())
         self._reserve(dec.pos + 1)
         bf = dict(dtype=torch.bfloat16, device=dev)
         self.proj, self.z, self.ab = torch.empty(batch, 3 * wide, **bf), torch.empty(batch, wide, **bf), torch.empty(batch, 2 * wide, **bf)
@@ -209,6 +226,7 @@ class _FusedStep:
         if (not cfg.no_weight_tying and model.mup_output_mult == 1.0 and isinstance(fn, RMSNorm) and fn.gain.dtype == torch.bfloat16
                 and head.dtype == torch.bfloat16 and head.is_contiguous() and head.data_ptr() % 16 == 0):
             self.head, self.norm = head, fn
+        dec._states = [dict() for _ in dec.blocks]          # this object holds the state from here on
 
     def _reserve(self, n: int) -> None:
         """Room for n tokens in every key / value cache (doubled when it runs out)."""
@@ -220,16 +238,27 @@ class _FusedStep:
             cap = max(2 * L.cap, n + 63)
             for j, (name, old) in enumerate((("kc", k), ("vc", v))):
                 new = torch.empty((old.shape[0], cap) + tuple(old.shape[2:]), dtype=torch.bfloat16, device=old.device)
-                new[:, : old.shape[1]] = old
+                new[:, : self.pos] = old[:, : self.pos]
                 setattr(L, name, new.data_ptr())
                 e[1 + j] = new
             L.cap = cap
 
-    def __call__(self, token: torch.Tensor, pos: int) -> torch.Tensor:
+    def export(self) -> List[Dict]:
+        """The state as the operator-by-operator step keeps it, in tensors that later steps leave alone (they only append to
+        the key / value caches)."""
+        out: List[Dict] = [dict() for _ in self.layers]
+        for i, name, t in self.rings:
+            n = t.shape[1]
+            out[i][name] = t.clone() if name == "s" or n == 0 else torch.roll(t, -(self.pos % n), dims=1)
+        for i, k, v in self.attn:
+            out[i]["k"], out[i]["v"] = k[:, : self.pos], v[:, : self.pos]
+        return out
+
+    def __call__(self, token: torch.Tensor) -> torch.Tensor:
         from ..ops.cuda_ops import _check, _count, _stream
         if token.shape[0] != self.batch:
             raise ValueError(f"decode step for {token.shape[0]} sequences, prefilled with {self.batch}")
-        self._reserve(pos + 1)
+        self._reserve(self.pos + 1)
         for L, name, p in self.weights:
             ptr = p.data_ptr()
             if getattr(L, name) != ptr:
@@ -241,11 +270,12 @@ class _FusedStep:
         V = self.head.shape[0] if self.head is not None else 0
         out = torch.empty(self.batch, V, dtype=torch.float32, device=x.device) if V else None
         _check(self.lib.sb_decode_step(ctypes.addressof(self.layers), len(self.layers), x.data_ptr(), self.proj.data_ptr(),
-                                       self.z.data_ptr(), self.a.data_ptr(), self.ab.data_ptr(), self.batch, self.D, pos,
+                                       self.z.data_ptr(), self.a.data_ptr(), self.ab.data_ptr(), self.batch, self.D, self.pos,
                                        self.norm.gain.data_ptr() if V else None, self.norm.eps if V else 0.0,
                                        int(self.norm.form != "te") if V else 0, self.head.data_ptr() if V else None, V,
                                        out.data_ptr() if V else None, _stream()), "decode_step")
         _count(5 * len(self.layers) + (1 if V else 0))
+        self.pos += 1
         return out if V else self.model.logits(x[:, None])[:, 0].float()
 
 
@@ -273,9 +303,33 @@ class CachedDecoder:
                 raise NotImplementedError("cached generation does not cover the block-sparse attention operators")
             if isinstance(m, HyenaOperator) and (m.bidirectional or m.slow_heads):
                 raise NotImplementedError("cached generation does not cover two-sided filters or outer-product heads")
-        self.states: List[Dict] = []
+        self._states: List[Dict] = []
         self.pos = 0
         self._fused: Optional[_FusedStep] = None
+        self._resume = False                     # the native step takes the state up again at the next token
+
+    @property
+    def states(self) -> List[Dict]:
+        """The state of every layer at position `pos`, a dictionary of tensors each.  A step replaces the entries and changes no
+        tensor, so a continuation is branched by copying the dictionaries (or the decoder) and resumed by assigning them
+        together with `pos`.  Taking the list out of a decoder that steps natively copies the state once: read it again after
+        further steps."""
+        self._hand_back()
+        return self._states
+
+    @states.setter
+    def states(self, value: List[Dict]) -> None:
+        self._states, self._fused, self._resume = value, None, True
+
+    def _hand_back(self) -> None:
+        if self._fused is not None:
+            self._states, self._fused, self._resume = self._fused.export(), None, True
+
+    def __getstate__(self):                      # copies: the native step's buffers stay with this decoder
+        d = dict(self.__dict__)
+        if self._fused is not None:
+            d["_states"], d["_fused"], d["_resume"] = self._fused.export(), None, True
+        return d
 
     # ------------------------------------------------------------------ prefill
     @torch.no_grad()
@@ -284,8 +338,8 @@ class CachedDecoder:
         from .. import ops
         model = self.model
         B, T = tokens.shape
-        self._fused = None
-        self.states = [dict() for _ in self.blocks]
+        self._fused, self._resume = None, False
+        self._states = [dict() for _ in self.blocks]
         hooks = []
 
         def tail(x, n):
@@ -296,7 +350,7 @@ class CachedDecoder:
                 return x[:, -n:].clone()
             return F.pad(x, (0, 0, n - x.shape[1], 0))
 
-        for st, blk in zip(self.states, self.blocks):
+        for st, blk in zip(self._states, self.blocks):
             mixer = blk.mixer
             inner = mixer.mixer
             if isinstance(inner, SelfAttention):
@@ -399,13 +453,17 @@ class CachedDecoder:
     def step(self, token: torch.Tensor) -> torch.Tensor:
         """token [B] -> logits of the next position [B, V]; advances every layer's state by one token."""
         model, cfg = self.model, self.cfg
+        if self._fused is not None and self._fused.pos != self.pos:
+            self._hand_back()                    # the caller moved to another position
+        if self._resume:
+            self._resume, self._fused = False, _FusedStep.build(self, token.shape[0])
         if self._fused is not None:
             was_training = model.training
             switch = any(m.training for m in model.embedding.modules())       # the only module that runs here
             if switch:
                 model.eval()
             try:
-                logits = self._fused(token, self.pos)
+                logits = self._fused(token)
             finally:
                 if switch:
                     model.train(was_training)
@@ -419,7 +477,7 @@ class CachedDecoder:
             x = model.embedding(token[:, None], pos)[:, 0]                                   # [B, D]
         finally:
             model.train(was_training)
-        for blk, st in zip(self.blocks, self.states):
+        for blk, st in zip(self.blocks, self._states):
             mixer = blk.mixer
             u = _rms(x.float(), blk.input_layernorm).to(dtype)
             proj = F.linear(u, mixer.dense_projection.weight)

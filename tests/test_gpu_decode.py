@@ -1,5 +1,6 @@
 """The native decode step (csrc/decode.cu) against the operator-by-operator step of the same decoder: parameters that change
-between steps."""
+between steps, state that is copied and put back."""
+import copy
 import os
 
 import pytest
@@ -84,3 +85,36 @@ def test_filters_stored_in_bf16(monkeypatch):
     fast.prefill(toks[:, :25])
     assert fast._fused is not None
     _agree(fast, slow, toks[:, 25:])
+
+
+@pytest.mark.parametrize("T", [1, 3, 20, 129, 260])
+def test_branched_continuations(T, monkeypatch):
+    """Two continuations of one prompt, branched by copying the state's dictionaries, the decoder, or a batch of rows."""
+    model = _model()
+    toks = _toks(model, 2, T + 20)
+    fast, slow = CachedDecoder(model), _slow(model, toks[:, :T], monkeypatch)
+    fast.prefill(toks[:, :T])
+    _agree(fast, slow, toks[:, T:T + 3])
+    saved = {d: ([dict(s) for s in d.states], d.pos) for d in (fast, slow)}
+    for a, b in zip(saved[fast][0], saved[slow][0]):
+        assert a.keys() == b.keys() and all(a[k].shape == b[k].shape for k in a)
+    twin, twin_slow = copy.deepcopy(fast), copy.deepcopy(slow)
+    first = fast.step(toks[:, T + 3])
+    assert fast._fused is not None                                   # the native step took the state up again
+    slow.step(toks[:, T + 3])
+    _agree(fast, slow, toks[:, T + 4:T + 8])
+    for d in (fast, slow):                                           # back to the branch
+        d.states, d.pos = [dict(s) for s in saved[d][0]], saved[d][1]
+    assert torch.equal(fast.step(toks[:, T + 3]), first)             # bit for bit: nothing of the first branch is left
+    slow.step(toks[:, T + 3])
+    _agree(fast, slow, toks[:, T + 8:T + 12])
+    assert twin._fused is None and torch.equal(twin.step(toks[:, T + 3]), first) and twin._fused is not None
+    twin_slow.step(toks[:, T + 3])
+    live = copy.deepcopy(twin)                                       # of a decoder in the middle of native steps
+    assert twin._fused is not None
+    _agree(twin, twin_slow, toks[:, T + 12:T + 16])
+    live.step(toks[:, T + 12])
+    for d in (fast, slow):                                           # another batch: rows picked by the caller
+        d.states, d.pos = [{k: v[[1, 0, 1]] for k, v in s.items()} for s in saved[d][0]], saved[d][1]
+    _agree(fast, slow, toks[[1, 0, 1], T + 3:T + 7])
+    assert fast._fused is not None and fast._fused.batch == 3
