@@ -18,13 +18,15 @@
 // Measured on a B200: four layers (one of each operator), width 1024, two sequences, a prompt of 517 tokens and 16 steps:
 // 50.2 ms operator by operator (3 ms a step, all of it launches; the key / value cache was copied and converted to fp32 on
 // every step), 4.4 ms with these kernels, half of it the prefill.  Two rows per warp keep 3072 outputs on 192 blocks while
-// every lane has eight 16-byte weight loads in flight (6 us a matrix-vector kernel, 6.5 us a Hyena step, 9 us attention over
-// 525 keys).  Launching the kernels as programmatic dependents with the weight loads ahead of the wait changed nothing
+// every lane has eight 16-byte weight loads in flight (6 us a matrix-vector kernel, 5 to 6 us a Hyena step, 9 us attention
+// over 525 keys).  Launching the kernels as programmatic dependents with the weight loads ahead of the wait changed nothing
 // (4476 against 4482 us): the host issues them no faster.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <type_traits>
 
 namespace sb {
 namespace dec {
@@ -77,18 +79,33 @@ __device__ __forceinline__ float activation(float x, int act) {
   return x;
 }
 
-__device__ __forceinline__ float param(const void* p, size_t i, bool f32) {
+// Type of a filter parameter: known at compile time (AS_BF16, AS_F32) or by its bit of Layer::f32 (AS_STORED).
+enum { AS_STORED = 0, AS_BF16 = 1, AS_F32 = 2 };
+template <int AS>
+__device__ __forceinline__ float param(const void* p, size_t i, int bit) {
+  const bool f32 = AS == AS_F32 || (AS == AS_STORED && bit);
   return f32 ? reinterpret_cast<const float*>(p)[i] : __bfloat162float(reinterpret_cast<const bf16*>(p)[i]);
 }
-// Tap j of filter group `grp`, j = 0 the one of the oldest value.  With a decay window the tap is their product, which is
-// rounded as the parameters' own type rounds it.
-__device__ __forceinline__ float fir_tap(const Layer& l, int grp, int j) {
-  const size_t i = (size_t)grp * l.tap_ld + (l.newest_first ? l.K - 1 - j : j);
-  const float t = param(l.taps, i, l.f32 & F_TAPS);
-  if (!l.decay) return t;
-  const float d = t * param(l.decay, i, l.f32 & F_DECAY);
-  return (l.f32 & (F_TAPS | F_DECAY)) ? d : rbf(d);
-}
+// The taps of one channel, j = 0 the one of the oldest value.  With a decay window a tap is their product, which is rounded as
+// the parameters' own type rounds it.
+template <int AS>
+struct Taps {
+  const void *t, *d;
+  size_t first;
+  ptrdiff_t step;
+  int f32;
+  __device__ __forceinline__ Taps(const Layer& l, int ch)
+      : t(l.taps), d(l.decay), first((size_t)(ch / (l.H / l.G)) * l.tap_ld + (l.newest_first ? l.K - 1 : 0)),
+        step(l.newest_first ? -1 : 1), f32(l.f32) {}
+  template <bool DECAY>
+  __device__ __forceinline__ float at(int j) const {
+    const size_t i = first + step * j;
+    const float v = param<AS>(t, i, f32 & F_TAPS);
+    if (!DECAY) return v;
+    const float w = v * param<AS>(d, i, f32 & F_DECAY);
+    return AS == AS_F32 || (f32 & (F_TAPS | F_DECAY)) ? w : rbf(w);
+  }
+};
 
 struct LinArgs {
   const bf16* x;          // [B, K] (IN_GATE: [B, 2K] = [a | b])
@@ -206,7 +223,12 @@ dec_linear_kernel(LinArgs a) {
 
 // ------------------------------------------------------------------------------------ Hyena operators
 // 32 channels of one batch row per block; eight slices share the filter taps (or modes) of a channel.
+// The types of the parameters as they usually are (featuriser bf16, filter all bf16 or all fp32) are compiled in, and what does
+// not need the new u comes before the first barrier, while one warp forms u: 6.1 us a launch for the medium and long filters at
+// width 1024, two sequences, against 8.3 (average of all three) with a test of Layer::f32 at every load, which keeps the loads
+// from being issued together, and everything after the barrier.
 constexpr int HY_SLICES = 8;
+template <int CONV, int FILT>
 __global__ void __launch_bounds__(32 * HY_SLICES)
 dec_hyena_kernel(Layer l, const bf16* __restrict__ proj, bf16* __restrict__ z, int pos) {
   __shared__ float su[32], sx1[32], sb[32], part[HY_SLICES][32];
@@ -219,42 +241,63 @@ dec_hyena_kernel(Layer l, const bf16* __restrict__ proj, bf16* __restrict__ z, i
     for (int p = 0; p < 3; ++p) {
       const int c = 3 * ch + p;
       const size_t w = (size_t)(c / (3 * l.H / l.conv_g)) * l.kf;
-      const bool wf = l.f32 & F_CONV;
+      const int wf = l.f32 & F_CONV;
       const bf16 cur = proj[(size_t)b * 3 * l.H + c];
-      float acc = param(l.conv_w, w + n, wf) * __bfloat162float(cur);
+      float acc = param<CONV>(l.conv_w, w + n, wf) * __bfloat162float(cur);
       bf16* ring = l.proj_ring + (size_t)b * n * 3 * l.H + c;
-      for (int j = 0; j < n; ++j) acc += param(l.conv_w, w + j, wf) * __bfloat162float(ring[(size_t)((pos + j) % n) * 3 * l.H]);
+      for (int j = 0; j < n; ++j) acc += param<CONV>(l.conv_w, w + j, wf) * __bfloat162float(ring[(size_t)((pos + j) % n) * 3 * l.H]);
       if (n > 0) ring[(size_t)(pos % n) * 3 * l.H] = cur;
       f[p] = rbf(acc);                                     // the parallel path rounds the featuriser output
     }
     const float u = f[1] * f[2];
     sx1[cx] = f[0];
     su[cx] = (l.kind == OP_SE && !l.pregate) ? f[2] : u;
-    sb[cx] = l.kind == OP_SE ? 0.f : param(l.bias, ch, l.f32 & F_BIAS) * u;
+    sb[cx] = l.kind == OP_SE ? 0.f : param<FILT>(l.bias, ch, l.f32 & F_BIAS) * u;
   }
-  __syncthreads();
+  // what does not need the new u: the past of the FIR filters, the parameters and states of the first modes
   float y = 0.f;
-  const int grp = live ? ch / (l.H / l.G) : 0;
-  if (live) {
-    const float u = su[cx];
-    if (l.kind == OP_LI) {
-      const size_t base = ((size_t)b * l.H + ch) * l.O;
-      for (int o = sl; o < l.O; o += HY_SLICES) {
-        const size_t i = (size_t)grp * l.O + o;
-        const float lam = expf(-expf(param(l.p, i, l.f32 & F_P)) * expf(param(l.gamma, i, l.f32 & F_GAMMA)));
-        const float s = lam * l.state[base + o] + u;
-        l.state[base + o] = s;
-        y += param(l.R, i, l.f32 & F_R) * s;
-      }
-    } else {
-      const int n = l.K - 1;
-      const float* ring = l.u_ring + (size_t)b * n * l.H + ch;
+  constexpr int MODES = 2;                                 // of this slice, held over the barrier: orders up to 16
+  float lam[MODES], st[MODES], R[MODES];
+  const size_t mode0 = live ? (size_t)(ch / (l.H / l.G)) * l.O : 0, st0 = ((size_t)b * l.H + ch) * l.O;
+  auto mode = [&](int o, float& lm, float& s, float& r) {
+    const size_t i = mode0 + o;
+    s = l.state[st0 + o];
+    r = param<FILT>(l.R, i, l.f32 & F_R);
+    lm = expf(-expf(param<FILT>(l.p, i, l.f32 & F_P)) * expf(param<FILT>(l.gamma, i, l.f32 & F_GAMMA)));
+  };
+  if (live && l.kind == OP_LI) {
+#pragma unroll
+    for (int k = 0; k < MODES; ++k)
+      if (sl + k * HY_SLICES < l.O) mode(sl + k * HY_SLICES, lam[k], st[k], R[k]);
+  } else if (live) {
+    const int n = l.K - 1, now = n > 0 ? pos % n : 0;
+    const Taps<FILT> taps(l, ch);
+    const float* ring = l.u_ring + (size_t)b * n * l.H + ch;
+    auto past = [&](auto decay) {
 #pragma unroll 8
       for (int j = sl; j < n; j += HY_SLICES) {
-        int slot = pos % n + j;
+        int slot = now + j;
         if (slot >= n) slot -= n;
-        y += fir_tap(l, grp, j) * ring[(size_t)slot * l.H];
+        y += taps.template at<decay.value>(j) * ring[(size_t)slot * l.H];
       }
+    };
+    if (l.decay) past(std::true_type{}); else past(std::false_type{});
+  }
+  __syncthreads();
+  if (live && l.kind == OP_LI) {
+    const float u = su[cx];
+    auto advance = [&](int o, float lm, float s, float r) {
+      s = lm * s + u;
+      l.state[st0 + o] = s;
+      y += r * s;
+    };
+#pragma unroll
+    for (int k = 0; k < MODES; ++k)
+      if (sl + k * HY_SLICES < l.O) advance(sl + k * HY_SLICES, lam[k], st[k], R[k]);
+    for (int o = sl + MODES * HY_SLICES; o < l.O; o += HY_SLICES) {
+      float lm, s, r;
+      mode(o, lm, s, r);
+      advance(o, lm, s, r);
     }
   }
   part[sl][cx] = y;
@@ -264,7 +307,8 @@ dec_hyena_kernel(Layer l, const bf16* __restrict__ proj, bf16* __restrict__ z, i
   for (int j = 1; j < HY_SLICES; ++j) y += part[j][cx];
   if (l.kind != OP_LI) {
     const int n = l.K - 1;
-    y += fir_tap(l, grp, n) * su[cx];
+    const Taps<FILT> taps(l, ch);
+    y += (l.decay ? taps.template at<true>(n) : taps.template at<false>(n)) * su[cx];
     if (n > 0) l.u_ring[((size_t)b * n + pos % n) * l.H + ch] = su[cx];
   }
   y += sb[cx];
@@ -377,6 +421,16 @@ dec_attn_kernel(Layer l, const bf16* __restrict__ proj, bf16* __restrict__ z, in
   cluster.sync();                                          // peers' shared memory stays until it has been read
 }
 
+static void launch_hyena(const Layer& l, const bf16* proj, bf16* z, int B, int pos, cudaStream_t st) {
+  const int used = l.kind == OP_SE ? F_TAPS : l.kind == OP_MR ? F_TAPS | F_BIAS | (l.decay ? F_DECAY : 0) : F_BIAS | F_GAMMA | F_P | F_R;
+  const dim3 grid((l.H + 31) / 32, B);
+  const int threads = 32 * HY_SLICES;
+  if (l.f32 & F_CONV) dec_hyena_kernel<AS_F32, AS_STORED><<<grid, threads, 0, st>>>(l, proj, z, pos);
+  else if ((l.f32 & used) == used) dec_hyena_kernel<AS_BF16, AS_F32><<<grid, threads, 0, st>>>(l, proj, z, pos);
+  else if (!(l.f32 & used)) dec_hyena_kernel<AS_BF16, AS_BF16><<<grid, threads, 0, st>>>(l, proj, z, pos);
+  else dec_hyena_kernel<AS_BF16, AS_STORED><<<grid, threads, 0, st>>>(l, proj, z, pos);
+}
+
 static int launch_linear(const LinArgs& a, cudaStream_t st) {
   const int blocks = (a.N + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK;
   const int bt = a.B <= 1 ? 1 : a.B <= 2 ? 2 : a.B <= 4 ? 4 : 8;
@@ -420,7 +474,7 @@ extern "C" int sb_decode_step(const Layer* layers, int n_layers, void* x, void* 
     rc = launch_linear(LinArgs{xb, l.norm1_w, l.w_in, nullptr, nullptr, pb, B, D, 3 * l.H, IN_NORM, 0, l.form1, 0, l.eps1}, st);
     if (rc) return rc;
     if (l.kind == OP_ATTN) dec_attn_kernel<<<dim3(l.heads * SPLIT, B), ATT_THREADS, 0, st>>>(l, pb, zb, pos);
-    else dec_hyena_kernel<<<dim3((l.H + 31) / 32, B), 32 * HY_SLICES, 0, st>>>(l, pb, zb, pos);
+    else launch_hyena(l, pb, zb, B, pos, st);
     rc = launch_linear(LinArgs{zb, nullptr, l.w_out, l.b_out, xb, abuf, B, l.H, D, IN_PLAIN, 0, 0, 0, 0.f}, st);
     if (rc) return rc;
     rc = launch_linear(LinArgs{abuf, l.norm2_w, l.w12, nullptr, nullptr, abb, B, D, 2 * l.F, l.norm2 ? IN_NORM : IN_PLAIN, 0, l.form2, 0,

@@ -21,6 +21,7 @@ from __future__ import annotations
 
 import ctypes
 import math
+import operator
 from typing import Dict, List, Optional
 
 import torch
@@ -30,6 +31,9 @@ from ..models.filters import ExplicitSingleDecayFilter, ImplicitModalFilter
 from ..models.hyena import HyenaOperator, ShortHyenaOperator
 from ..models.mixer import SelfAttention
 from ..models.mlp import ParallelGLU
+from ..models.norms import RMSNorm
+from .. import ops
+from ..ops import cuda_ops
 from ..ops import reference as ref
 from ..parallel import state
 
@@ -61,22 +65,125 @@ def _ring(tail: torch.Tensor, pos: int) -> torch.Tensor:
     return torch.roll(tail, pos % n, dims=1).contiguous() if n else tail.contiguous()
 
 
+class _Watch:
+    """Reads attributes and remembers where each was found, so that `same` can tell later, without reading the layers again,
+    whether any of them has been replaced."""
+
+    def __init__(self):
+        self.seen = []                           # (dictionary or list, key, value)
+
+    def __call__(self, obj, name):
+        d = obj.__dict__
+        for c in (d, d.get("_modules"), d.get("_parameters"), d.get("_buffers")):
+            if c is not None and name in c:
+                self.seen.append((c, name, c[name]))
+                return c[name]
+        raise AttributeError(f"{type(obj).__name__} has no attribute {name!r} of its own")
+
+    def same(self) -> bool:
+        try:
+            for c, k, v in self.seen:
+                if c[k] is not v:
+                    return False
+        except (KeyError, IndexError):
+            return False
+        return True
+
+
+def _short_taps(conv, at):
+    """(weight, the shape it must have) of a depthwise convolution: [groups, k] or [groups, 1, k], the same in memory."""
+    w, g, k = at(conv, "short_conv_weight"), conv.num_groups, conv.kernel_size
+    return w, ((g, 1, k) if w.dim() == 3 else (g, k))
+
+
+def _layer_form(blk, D, at):
+    """(what a layer computes, its weights) for csrc/decode.cu, or None where the kernels do not cover it; read through `at`, a
+    `_Watch`.  The form is a dictionary of descriptor fields; a weight is (field, tensor, shape it must have, whether it is a
+    filter parameter, read as it is stored)."""
+    mixer, mlp, n1 = at(blk, "mixer"), at(blk, "mlp"), at(blk, "input_layernorm")
+    n2 = at(blk, "pre_mlp_layernorm") if at(blk, "pre_mlp_norm") else None
+    if not isinstance(mlp, ParallelGLU) or not isinstance(n1, RMSNorm) or not (n2 is None or isinstance(n2, RMSNorm)) \
+            or at(mlp, "act") not in cuda_ops._ACT:
+        return None
+    op, H, Fi = at(mixer, "mixer"), at(mixer, "inner_size"), at(mlp, "ffn_local")
+    dense, w3 = at(mixer, "dense"), at(mlp, "w3")
+    form: Dict = {"H": H, "F": Fi, "act": cuda_ops._ACT[mlp.act], "norm2": int(n2 is not None)}
+    ws = [("w_in", at(at(mixer, "dense_projection"), "weight"), (3 * H, D), False), ("w_out", at(dense, "weight"), (D, H), False),
+          ("w12", at(mlp, "w12"), (2 * Fi, D), False), ("w3", at(w3, "weight"), (D, Fi), False),
+          ("b_out", at(dense, "bias"), (D,), False), ("b3", at(w3, "bias"), (D,), False)]
+    for n, i in ((n1, "1"), (n2, "2")):
+        if n is not None:
+            te = at(n, "form") == "te"
+            form["eps" + i], form["form" + i] = at(n, "eps"), int(not te)
+            ws.append((f"norm{i}_w", at(n, "weight" if te else "scale"), (D,), False))
+    if isinstance(op, SelfAttention):
+        if at(op, "hd") != 128 or at(op, "heads") * 128 != H:
+            return None
+        form.update(kind=3, heads=op.heads, rd=0, pos_scale=1.0, base=0.0)
+        if at(op, "_rotary"):
+            r = op._rotary[0]
+            at.seen.append((op._rotary, 0, r))
+            form.update(rd=at(r, "dim"), pos_scale=at(r, "scaling_factor"), base=at(r, "base"))
+        return form, ws
+    conv, G = at(mixer, "hyena_proj_conv"), at(op, "num_groups")
+    if at(conv, "num_groups") * at(conv, "group_dim") != 3 * H or G * at(op, "group_dim") != H:
+        return None
+    form.update(kf=at(conv, "kernel_size"), conv_g=conv.num_groups, G=G, pregate=1, postgate=1)
+    ws.append(("conv_w", *_short_taps(conv, at), True))
+    if isinstance(op, ShortHyenaOperator):
+        K, c = at(op, "kernel_size"), at(op, "short_conv")
+        form.update(kind=0, K=K, tap_ld=K, pregate=int(bool(at(op, "pregate"))), postgate=int(bool(at(op, "postgate"))))
+        if at(c, "num_groups") != G or at(c, "kernel_size") != K:
+            return None
+        ws.append(("taps", *_short_taps(c, at), True))
+        return form, ws
+    f = at(op, "filter")
+    ws.append(("bias", at(op, "conv_bias"), (H,), True))
+    if at(op, "is_mr"):
+        K = at(op, "hyena_mr_len")
+        if type(f) is ExplicitSingleDecayFilter:
+            h = at(f, "h")
+            if h.shape[1] < K:
+                return None
+            form["tap_ld"] = h.shape[1]
+            ws += [("taps", h, (G, h.shape[1]), True), ("decay", at(f, "decay"), (G, h.shape[1]), True)]
+        else:                                    # no form of its own in the kernel: the module evaluates it in every step
+            form["tap_ld"] = K
+            ws.append(("taps", f, (G, K), True))
+        form.update(kind=1, K=K, newest_first=1)
+        return form, ws
+    O = at(f, "gamma").shape[1]
+    form.update(kind=2, O=O)
+    return form, ws + [(n, at(f, n), (G, O), True) for n in ("gamma", "p", "R")]
+
+
+def _usable(t, shape, filt, device) -> bool:
+    """What the kernels assume of a weight: bf16 rows read 16 bytes at a time, or filter parameters read one by one."""
+    if t.shape != shape or t.device != device or not t.is_contiguous():
+        return False
+    return t.dtype in (torch.bfloat16, torch.float32) if filt else t.dtype == torch.bfloat16 and t.data_ptr() % 16 == 0
+
+
+_PTR, _NUMEL, _CONTIGUOUS = torch.Tensor.data_ptr, torch.Tensor.numel, torch.Tensor.is_contiguous
+_DTYPE = operator.attrgetter("dtype")
+
+
 class _FusedStep:
     """The decode step of csrc/decode.cu: the layers' weights by address, their state in the layout of its kernels.  Built at
     the end of a prefill and after the state was handed out (`CachedDecoder.states`); `build` returns None when something is not
     covered (CPU tensors, other dtypes than bf16, other norms than RMSNorm, head sizes other than 128, more than 8 sequences, an
     inner size above `sb_decode_max_width`: 102400 for one sequence, 12800 for eight; unaligned or non-contiguous weights), and the
-    decoder then steps operator by operator."""
+    decoder then steps operator by operator.
+
+    A step looks at the modules as they are then: `follow` refuses when a weight has changed its type, shape, device or alignment
+    into something that the kernels do not read, or a layer computes something else than it did.  It reads the layers again only
+    when an attribute or tensor that it read before is another one now, or lies elsewhere (four layers: 13 us of host time for
+    the comparison where the reading takes 130, of the 135 in which a step is issued)."""
 
     @staticmethod
     def build(dec: "CachedDecoder", batch: int):
-        from .. import ops
-        from ..models.norms import RMSNorm
-        model, cfg = dec.model, dec.cfg
-        w = model.embedding.word_embeddings.weight
-        if not ops._k(w) or cfg.params_dtype != torch.bfloat16:
+        if not ops._k(dec.model.embedding.word_embeddings.weight):
             return None
-        from ..ops import cuda_ops
         lib = cuda_ops.require()
         if not getattr(lib, "_sb_decode_ready", False):
             P, I, F_ = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
@@ -87,146 +194,142 @@ class _FusedStep:
             lib._sb_decode_ready = True
         if lib.sb_decode_layer_bytes() != ctypes.sizeof(_DecLayer):
             raise RuntimeError("decode layer descriptor does not match the native library (rebuild savanna_b200.csrc)")
-        D, wmax = cfg.hidden_size, lib.sb_decode_max_width(batch)
-        if len(dec._states) != len(dec.blocks):
-            return None
-
-        def weight(t, *shape):
-            return (t is not None and t.dtype == torch.bfloat16 and t.is_cuda and t.is_contiguous() and t.data_ptr() % 16 == 0
-                    and tuple(t.shape) == shape)
-
-        def norm(m):
-            return isinstance(m, RMSNorm) and weight(m.gain, D)
-
-        def source(t, *shape):                  # a filter parameter, read as it is stored
-            return t.dtype in (torch.bfloat16, torch.float32) and t.is_cuda and t.is_contiguous() and tuple(t.shape) == shape
-
-        def held(t, *shape):                    # a piece of state, whoever filled the dictionary
-            return t is not None and t.device == w.device and tuple(t.shape) == (batch,) + shape
-
-        def filters(mixer, st):
-            conv, op, H = mixer.hyena_proj_conv, mixer.mixer, mixer.inner_size
-            if not source(conv.taps(), conv.num_groups, conv.kernel_size) or conv.num_groups * conv.group_dim != 3 * H \
-                    or not held(st.get("proj_tail"), conv.kernel_size - 1, 3 * H) or st["proj_tail"].dtype != torch.bfloat16:
-                return False
-            if isinstance(op, ShortHyenaOperator):
-                return (source(op.short_conv.taps(), op.num_groups, op.kernel_size) and op.num_groups * op.group_dim == H
-                        and held(st.get("u_tail"), op.kernel_size - 1, H))
-            if not source(op.conv_bias, H) or op.num_groups * op.group_dim != H:
-                return False
-            if op.is_mr:
-                f, G, K = op.filter, op.num_groups, op.hyena_mr_len
-                if not held(st.get("u_tail"), K - 1, H):
-                    return False
-                if type(f) is not ExplicitSingleDecayFilter:
-                    return tuple(f(K).shape) == (G, K)
-                return f.h.dim() == 2 and f.h.shape[1] >= K and all(source(t, G, f.h.shape[1]) for t in (f.h, f.decay))
-            O = op.filter.gamma.shape[1]
-            return held(st.get("s"), H, O) and all(source(t, op.num_groups, O) for t in (op.filter.gamma, op.filter.p, op.filter.R))
-
-        for blk, st in zip(dec.blocks, dec._states):
-            mixer, mlp = blk.mixer, blk.mlp
-            H, Fi = mixer.inner_size, mlp.ffn_local
-            if (D % 8 or H % 8 or Fi % 8 or max(D, H, Fi) > wmax or mlp.act not in cuda_ops._ACT or not norm(blk.input_layernorm)
-                    or (blk.pre_mlp_norm and not norm(blk.pre_mlp_layernorm)) or not weight(mixer.dense_projection.weight, 3 * H, D)
-                    or not weight(mixer.dense.weight, D, H) or not weight(mlp.w12, 2 * Fi, D) or not weight(mlp.w3.weight, D, Fi)
-                    or any(b is not None and not weight(b, D) for b in (mixer.dense.bias, mlp.w3.bias))):
-                return None
-            if isinstance(mixer.mixer, SelfAttention):
-                heads = mixer.mixer.heads
-                if mixer.mixer.hd != 128 or heads * 128 != H or not all(
-                        held(st.get(n), dec.pos, heads, 128) and st[n].dtype == torch.bfloat16 for n in ("k", "v")):
-                    return None
-            elif not filters(mixer, st):
-                return None
-        return _FusedStep(dec, lib, batch)
+        self = _FusedStep(dec, lib, batch)
+        return self if self.follow() and self._adopt(dec) else None
 
     def __init__(self, dec: "CachedDecoder", lib, batch: int):
-        from ..models.norms import RMSNorm
-        from ..ops import cuda_ops
-        model, cfg = dec.model, dec.cfg
-        self.lib, self.model, self.batch, self.D = lib, model, batch, cfg.hidden_size
-        dev = model.embedding.word_embeddings.weight.device
-        n = len(dec.blocks)
-        self.layers = (_DecLayer * n)()
-        self.keep = []                          # buffers the descriptors point into
-        self.weights = []                       # (descriptor, field, parameter): followed when a parameter's storage moves
-        self.filters = []                       # (descriptor, module, taps): filters without a form of their own in the kernel
+        self.model, self.cfg, self.blocks = dec.model, dec.cfg, dec.blocks       # not `dec`, which holds this object
+        self.lib, self.batch, self.D, self.wmax = lib, batch, dec.cfg.hidden_size, lib.sb_decode_max_width(batch)
+        self.device = dec.model.embedding.word_embeddings.weight.device
+        self.layers = (_DecLayer * len(dec.blocks))()
+        self.forms: List[Dict] = []             # what each layer computes
+        self.watch = None                       # what `follow` read: attributes ...
+        self.tensors: List[torch.Tensor] = []   # ... and tensors, with their addresses, types and sizes in `seen`
+        self.seen, self.storage = None, []
+        self.modules = []                       # (descriptor, filter module): evaluated in every step
+        self.temps: List[torch.Tensor] = []     # the evaluated filters
+        self.freqs: List[torch.Tensor] = []     # rotary frequencies
         self.attn = []                          # (layer index, key cache, value cache)
         self.rings = []                         # (layer index, name of the state, buffer) of the Hyena layers
         self.pos = dec.pos
 
-        def own(t):
-            self.keep.append(t)
-            return t.data_ptr()
+    def follow(self) -> bool:
+        """Points the descriptors at the weights as they are now; False when the kernels must not read them."""
+        if self.watch is None or not self._unchanged():
+            if not self._read():
+                self.watch = None
+                return False
+        self.temps = [f(L.K).float().contiguous() for L, f in self.modules]
+        for (L, _), t in zip(self.modules, self.temps):
+            if t.shape != (L.G, L.K) or t.device != self.device:
+                return False
+            L.taps = t.data_ptr()
+        return True
+
+    def _signature(self):
+        ts = self.tensors
+        return list(map(_PTR, ts)), list(map(_DTYPE, ts)), list(map(_NUMEL, ts)), list(map(_CONTIGUOUS, ts))
+
+    def _unchanged(self) -> bool:
+        return self.watch.same() and self._signature() == self.seen
+
+    def _read(self) -> bool:
+        at = _Watch()
+        model, cfg = self.model, self.cfg
+        seq = at(model, "sequential")
+        emb = at(at(seq, "0"), "word_embeddings")
+        head = at(emb, "weight")
+        at.seen.append((ops.__dict__, "_BACKEND", ops._BACKEND))
+        at(cfg, "precision")
+        if cfg.params_dtype != torch.bfloat16 or not ops._k(head):
+            return False
+        self.tensors, self.modules = [], []
+        for i, (L, blk) in enumerate(zip(self.layers, self.blocks)):
+            lw = _layer_form(blk, self.D, at)
+            if lw is None:
+                return False
+            if i == len(self.forms):             # the first time
+                if any(n % 8 or n > self.wmax for n in (self.D, lw[0]["H"], lw[0]["F"])):
+                    return False
+                self.forms.append(lw[0])
+                for name, v in lw[0].items():
+                    if name != "base":
+                        setattr(L, name, v)
+            elif lw[0] != self.forms[i]:
+                return False
+            f32 = 0
+            for name, t, shape, filt in lw[1]:
+                if isinstance(t, torch.nn.Module):
+                    self.modules.append((L, t))
+                    f32 |= _F32[name]
+                elif t is None:                  # no bias
+                    setattr(L, name, None)
+                elif _usable(t, shape, filt, self.device):
+                    self.tensors.append(t)
+                    if filt and t.dtype == torch.float32:
+                        f32 |= _F32[name]
+                    setattr(L, name, t.data_ptr())
+                else:
+                    return False
+            L.f32 = f32
+        # the logits, where the kernels can form them: (final norm, head weight)
+        self.head = None
+        tail = at(seq, str(model.num_layers + 3))
+        fn = at(tail, "norm") if hasattr(tail, "norm") else None
+        if not at(cfg, "no_weight_tying") and at(model, "mup_output_mult") == 1.0 and isinstance(fn, RMSNorm):
+            gain = at(fn, "weight" if at(fn, "form") == "te" else "scale")
+            self.tensors += [gain, head]
+            if _usable(gain, (self.D,), False, self.device) and _usable(head, (head.shape[0], self.D), False, self.device):
+                self.head = (gain, at(fn, "eps"), int(fn.form != "te"), head)
+        self.watch, self.seen = at, self._signature()
+        self.storage = [t.detach() for t in self.tensors]      # held, so that an address seen again is the same memory
+        return True
+
+    def _adopt(self, dec: "CachedDecoder") -> bool:
+        """Takes over the decoder's state, whoever filled its dictionaries, if its tensors are what the kernels expect."""
+        bf = torch.bfloat16
+        if len(dec._states) != len(self.forms):
+            return False
+
+        def held(st, name, *shape, dtype=None):
+            t = st.get(name)
+            return (t is not None and t.device == self.device and tuple(t.shape) == (self.batch,) + shape
+                    and (dtype is None or t.dtype == dtype))
+
+        for f, st in zip(self.forms, dec._states):
+            if f["kind"] == 3:
+                ok = all(held(st, n, self.pos, f["heads"], 128, dtype=bf) for n in ("k", "v"))
+            else:
+                ok = (held(st, "proj_tail", f["kf"] - 1, 3 * f["H"], dtype=bf)
+                      and (held(st, "s", f["H"], f["O"]) if f["kind"] == 2 else held(st, "u_tail", f["K"] - 1, f["H"])))
+            if not ok:
+                return False
 
         def ring(i, name, t):
             self.rings.append((i, name, t))
             return t.data_ptr()
 
-        def weight(L, **fields):
-            for name, p in fields.items():
-                if p is not None:
-                    self.weights.append((L, name, p))
-                    L.f32 |= _F32.get(name, 0) if p.dtype == torch.float32 else 0
-
-        wide = 0
-        for i, (blk, st) in enumerate(zip(dec.blocks, dec._states)):
-            L, mixer, inner, mlp = self.layers[i], blk.mixer, blk.mixer.mixer, blk.mlp
-            L.H, L.F, L.act = mixer.inner_size, mlp.ffn_local, cuda_ops._ACT[mlp.act]
-            L.eps1, L.form1 = blk.input_layernorm.eps, int(blk.input_layernorm.form != "te")
-            L.norm2 = int(bool(blk.pre_mlp_norm))
-            if L.norm2:
-                m = blk.pre_mlp_layernorm
-                L.eps2, L.form2 = m.eps, int(m.form != "te")
-                weight(L, norm2_w=m.gain)
-            weight(L, norm1_w=blk.input_layernorm.gain, w_in=mixer.dense_projection.weight, w_out=mixer.dense.weight,
-                   b_out=mixer.dense.bias, w12=mlp.w12, w3=mlp.w3.weight, b3=mlp.w3.bias)
-            wide = max(wide, L.H, L.F)
-            if isinstance(inner, SelfAttention):
-                L.kind, L.heads, L.rd, L.pos_scale = 3, inner.heads, 0, 1.0
-                if inner._rotary:
-                    r = inner._rotary[0]
-                    L.rd, L.pos_scale = r.dim, r.scaling_factor
-                    L.inv_freq = own(1.0 / (r.base ** (torch.arange(0, r.dim, 2, device=dev, dtype=torch.float32) / r.dim)))
+        for i, (L, f, st) in enumerate(zip(self.layers, self.forms, dec._states)):
+            if f["kind"] == 3:
+                if f["rd"]:
+                    inv = 1.0 / (f["base"] ** (torch.arange(0, f["rd"], 2, device=self.device, dtype=torch.float32) / f["rd"]))
+                    self.freqs.append(inv)
+                    L.inv_freq = inv.data_ptr()
                 self.attn.append([i, st["k"], st["v"]])
+                continue
+            L.proj_ring = ring(i, "proj_tail", _ring(st["proj_tail"], self.pos))
+            if f["kind"] == 2:
+                L.state = ring(i, "s", st["s"].float().contiguous().clone())
             else:
-                conv = mixer.hyena_proj_conv
-                L.kf, L.conv_g = conv.kernel_size, conv.num_groups
-                weight(L, conv_w=conv.short_conv_weight)
-                L.proj_ring = ring(i, "proj_tail", _ring(st["proj_tail"].to(torch.bfloat16), dec.pos))
-                L.pregate = L.postgate = 1
-                L.G = inner.num_groups
-                if isinstance(inner, ShortHyenaOperator):
-                    L.kind, L.pregate, L.postgate = 0, int(bool(inner.pregate)), int(bool(inner.postgate))
-                    L.K = L.tap_ld = inner.kernel_size
-                    weight(L, taps=inner.short_conv.short_conv_weight)
-                    L.u_ring = ring(i, "u_tail", _ring(st["u_tail"].float(), dec.pos))
-                elif inner.is_mr:
-                    L.kind, L.newest_first, L.K = 1, 1, st["u_tail"].shape[1] + 1
-                    weight(L, bias=inner.conv_bias)
-                    if type(inner.filter) is ExplicitSingleDecayFilter:
-                        L.tap_ld = inner.filter.h.shape[1]
-                        weight(L, taps=inner.filter.h, decay=inner.filter.decay)
-                    else:
-                        L.tap_ld, L.f32 = L.K, L.f32 | _F32["taps"]
-                        self.filters.append([L, inner.filter, None])
-                    L.u_ring = ring(i, "u_tail", _ring(st["u_tail"].float(), dec.pos))
-                else:
-                    L.kind, L.O = 2, inner.filter.gamma.shape[1]
-                    weight(L, bias=inner.conv_bias, gamma=inner.filter.gamma, p=inner.filter.p, R=inner.filter.R)
-                    L.state = ring(i, "s", st["s"].float().contiguous().clone())
-        self._reserve(dec.pos + 1)
-        bf = dict(dtype=torch.bfloat16, device=dev)
-        self.proj, self.z, self.ab = torch.empty(batch, 3 * wide, **bf), torch.empty(batch, wide, **bf), torch.empty(batch, 2 * wide, **bf)
-        self.a = torch.empty(batch, self.D, **bf)
-        fn = model.final_norm.norm if hasattr(model.final_norm, "norm") else None
-        head = model.embedding.word_embeddings.weight
-        self.head = None
-        if (not cfg.no_weight_tying and model.mup_output_mult == 1.0 and isinstance(fn, RMSNorm) and fn.gain.dtype == torch.bfloat16
-                and head.dtype == torch.bfloat16 and head.is_contiguous() and head.data_ptr() % 16 == 0):
-            self.head, self.norm = head, fn
+                L.u_ring = ring(i, "u_tail", _ring(st["u_tail"].float(), self.pos))
+        self._reserve(self.pos + 1)
+        wide = max([self.D] + [max(f["H"], f["F"]) for f in self.forms])
+        # the in-projection, the operator's output, the stream after the mixer, the gate's two halves
+        self.scratch = [torch.empty(self.batch, n, dtype=bf, device=self.device) for n in (3 * wide, wide, self.D, 2 * wide)]
+        self.scratch_ptrs = [t.data_ptr() for t in self.scratch]
+        self.descr = ctypes.addressof(self.layers)
         dec._states = [dict() for _ in dec.blocks]          # this object holds the state from here on
+        return True
 
     def _reserve(self, n: int) -> None:
         """Room for n tokens in every key / value cache (doubled when it runs out)."""
@@ -254,29 +357,30 @@ class _FusedStep:
             out[i]["k"], out[i]["v"] = k[:, : self.pos], v[:, : self.pos]
         return out
 
-    def __call__(self, token: torch.Tensor) -> torch.Tensor:
-        from ..ops.cuda_ops import _check, _count, _stream
+    def __call__(self, token: torch.Tensor) -> Optional[torch.Tensor]:
+        """Logits of the next position, or None (and nothing changed) when the embedding left what the kernels read."""
         if token.shape[0] != self.batch:
             raise ValueError(f"decode step for {token.shape[0]} sequences, prefilled with {self.batch}")
+        model = self.model
+        x = model.embedding(token[:, None], None)
+        if x.dtype != torch.bfloat16 or x.shape != (self.batch, 1, self.D) or x.device != self.device:
+            return None
+        x = x.contiguous()
+        ptr = x.data_ptr()
+        if ptr % 16:
+            return None
         self._reserve(self.pos + 1)
-        for L, name, p in self.weights:
-            ptr = p.data_ptr()
-            if getattr(L, name) != ptr:
-                setattr(L, name, ptr)
-        for e in self.filters:
-            e[2] = e[1](e[0].K).float().contiguous()
-            e[0].taps = e[2].data_ptr()
-        x = self.model.embedding(token[:, None], None)[:, 0].contiguous()
-        V = self.head.shape[0] if self.head is not None else 0
-        out = torch.empty(self.batch, V, dtype=torch.float32, device=x.device) if V else None
-        _check(self.lib.sb_decode_step(ctypes.addressof(self.layers), len(self.layers), x.data_ptr(), self.proj.data_ptr(),
-                                       self.z.data_ptr(), self.a.data_ptr(), self.ab.data_ptr(), self.batch, self.D, self.pos,
-                                       self.norm.gain.data_ptr() if V else None, self.norm.eps if V else 0.0,
-                                       int(self.norm.form != "te") if V else 0, self.head.data_ptr() if V else None, V,
-                                       out.data_ptr() if V else None, _stream()), "decode_step")
-        _count(5 * len(self.layers) + (1 if V else 0))
+        norm, eps, form, head, V, out, logits = None, 0.0, 0, None, 0, None, None
+        if self.head is not None:
+            gain, eps, form, w = self.head
+            norm, head, V = gain.data_ptr(), w.data_ptr(), w.shape[0]
+            out = torch.empty(self.batch, V, dtype=torch.float32, device=self.device)
+            logits = out.data_ptr()
+        cuda_ops._check(self.lib.sb_decode_step(self.descr, len(self.layers), ptr, *self.scratch_ptrs, self.batch, self.D, self.pos,
+                                                norm, eps, form, head, V, logits, cuda_ops._stream()), "decode_step")
+        cuda_ops._count(5 * len(self.layers) + (1 if V else 0))
         self.pos += 1
-        return out if V else self.model.logits(x[:, None])[:, 0].float()
+        return out if V else model.logits(x)[:, 0].float()
 
 
 class CachedDecoder:
@@ -335,7 +439,6 @@ class CachedDecoder:
     @torch.no_grad()
     def prefill(self, tokens: torch.Tensor) -> torch.Tensor:
         """tokens [B, T] -> logits of the last position [B, V]; leaves every layer's state at position T."""
-        from .. import ops
         model = self.model
         B, T = tokens.shape
         self._fused, self._resume = None, False
@@ -453,8 +556,8 @@ class CachedDecoder:
     def step(self, token: torch.Tensor) -> torch.Tensor:
         """token [B] -> logits of the next position [B, V]; advances every layer's state by one token."""
         model, cfg = self.model, self.cfg
-        if self._fused is not None and self._fused.pos != self.pos:
-            self._hand_back()                    # the caller moved to another position
+        if self._fused is not None and (self._fused.pos != self.pos or not self._fused.follow()):
+            self._hand_back()                    # the caller moved to another position, or changed the model
         if self._resume:
             self._resume, self._fused = False, _FusedStep.build(self, token.shape[0])
         if self._fused is not None:
@@ -467,8 +570,10 @@ class CachedDecoder:
             finally:
                 if switch:
                     model.train(was_training)
-            self.pos += 1
-            return logits
+            if logits is not None:
+                self.pos += 1
+                return logits
+            self._hand_back()
         dtype = cfg.params_dtype
         pos = torch.tensor([self.pos], device=token.device)
         was_training = model.training

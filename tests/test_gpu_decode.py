@@ -53,9 +53,10 @@ def _is_filter(n):
     return any(k in n for k in ("short_conv", ".filter.", "conv_bias"))
 
 
+@pytest.mark.parametrize("moved", [False, True], ids=["in_place", "moved"])
 @pytest.mark.parametrize("which", ["filters", "projections"])
 @pytest.mark.parametrize("over", [{}, {"hyena_medium_filter_cls": "implicit_modal"}], ids=["explicit", "modal_mr"])
-def test_parameters_changed_in_place_between_steps(which, over, monkeypatch):
+def test_parameters_changed_between_steps(which, over, moved, monkeypatch):
     """A step reads every parameter as it is then, filters as well as projections."""
     model = _model(**over)
     toks = _toks(model, 2, 30)
@@ -70,7 +71,11 @@ def test_parameters_changed_in_place_between_steps(which, over, monkeypatch):
         for n, p in model.named_parameters():
             if _is_filter(n) == (which == "filters") and "norm" not in n and "word_emb" not in n:
                 s = float(p.float().std()) or 0.1
-                p.data.add_(torch.randn(p.shape, device=DEV, generator=g) * s)
+                new = p.data + (torch.randn(p.shape, device=DEV, generator=g) * s).to(p.dtype)
+                if moved:
+                    p.data = new
+                else:
+                    p.data.copy_(new)
     _agree(fast, slow, toks[:, 24:])
     assert (slow.step(toks[:, 0]) - before).norm() > 0.1 * before.norm()          # the change reached the logits
 
@@ -118,3 +123,77 @@ def test_branched_continuations(T, monkeypatch):
         d.states, d.pos = [{k: v[[1, 0, 1]] for k, v in s.items()} for s in saved[d][0]], saved[d][1]
     _agree(fast, slow, toks[[1, 0, 1], T + 3:T + 7])
     assert fast._fused is not None and fast._fused.batch == 3
+
+
+def _get(model, name):
+    mod, _, leaf = name.rpartition(".")
+    return model.get_submodule(mod), leaf
+
+
+@pytest.mark.parametrize("name", ["sequential.2.mixer.dense_projection.weight", "sequential.3.mixer.mixer.filter.h",
+                                  "sequential.4.mixer.mixer.filter.R", "sequential.4.mlp.w12", "sequential.5.input_layernorm.weight",
+                                  "sequential.7.norm.weight", "sequential.0.word_embeddings.weight"])
+def test_replaced_parameter_is_followed(name, monkeypatch):
+    model = _model()
+    toks = _toks(model, 2, 30)
+    fast, slow = CachedDecoder(model), _slow(model, toks[:, :20], monkeypatch)
+    fast.prefill(toks[:, :20])
+    _agree(fast, slow, toks[:, 20:22])
+    mod, leaf = _get(model, name)
+    old = getattr(mod, leaf)
+    setattr(mod, leaf, torch.nn.Parameter(old.detach() * (10 if _is_filter(name) else 1.5) + 0.25 * old.detach().roll(1, 0)))
+    _agree(fast, slow, toks[:, 22:26])
+    assert fast._fused is not None
+
+
+def test_replaced_module_and_settings_are_followed(monkeypatch):
+    model = _model()
+    toks = _toks(model, 2, 40)
+    fast, slow = CachedDecoder(model), _slow(model, toks[:, :20], monkeypatch)
+    fast.prefill(toks[:, :20])
+    other = _model(seed=5)
+    blocks = model.blocks()
+    blocks[1].mlp = other.blocks()[2].mlp
+    _agree(fast, slow, toks[:, 20:24])
+    blocks[2].mlp.act = "gelu"
+    blocks[0].input_layernorm.eps = 1e-2
+    _agree(fast, slow, toks[:, 24:28])
+    blocks[0].mixer.mixer.pregate = False                  # the FIR's past is then of another signal, in both steps alike
+    _agree(fast, slow, toks[:, 28:32])
+    assert fast._fused is not None
+
+
+def test_unusable_weights_are_refused(monkeypatch):
+    """A weight that the kernels cannot read sends the step down the operator-by-operator path, which computes with it or raises
+    as it always has; the state survives either."""
+    model = _model()
+    toks = _toks(model, 2, 40)
+    fast, slow = CachedDecoder(model), _slow(model, toks[:, :20], monkeypatch)
+    fast.prefill(toks[:, :20])
+    _agree(fast, slow, toks[:, 20:22])
+    p = model.blocks()[1].mixer.dense_projection.weight
+    keep = p.data
+    shifted = torch.empty(p.numel() + 1, device=DEV, dtype=p.dtype)[1:].view(p.shape)          # two bytes off a 16-byte boundary
+    shifted.copy_(keep)
+    p.data = shifted
+    _agree(fast, slow, toks[:, 22:24])
+    assert fast._fused is None
+    p.data = keep.t().contiguous().t()                     # not contiguous
+    _agree(fast, slow, toks[:, 24:26])
+    p.data = keep
+    fast.states = fast.states                              # takes the native step up again
+    _agree(fast, slow, toks[:, 26:28])
+    assert fast._fused is not None
+    model.float()
+    for dec in (fast, slow):
+        with pytest.raises(RuntimeError):
+            dec.step(toks[:, 28])
+    model.to(torch.bfloat16)                               # every parameter, the filters too
+    fast.states = fast.states
+    _agree(fast, slow, toks[:, 28:30])
+    assert fast._fused is not None
+    model.cpu()
+    for dec in (fast, slow):
+        with pytest.raises(RuntimeError):
+            dec.step(toks[:, 30].cpu())
+    assert fast._fused is None

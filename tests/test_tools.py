@@ -267,6 +267,18 @@ def test_cached_generation_matches_recompute():
     assert "".join(said) == generate(model, cfg.tokenizer, ["ACGTACGT"], maximum_tokens=5)[0]["text"]
 
 
+def test_decode_weights_the_kernels_may_read():
+    """The native decode step reads 16 bytes of bf16 at a time: what it accepts as a weight, and as a filter parameter."""
+    from savanna_b200.inference.cached import _usable
+    dev, buf = torch.device("cpu"), torch.zeros(8 * 16 + 8, dtype=torch.bfloat16)
+    buf = buf[(-buf.data_ptr() % 16) // 2:]                # starts on a 16-byte boundary
+    w = buf[:128].view(8, 16)
+    assert _usable(w, (8, 16), False, dev) and _usable(w, (8, 16), True, dev)
+    for bad, filt_ok in ((buf[1:129].view(8, 16), True), (w.float(), True), (w.half(), False), (w.t(), False), (w.view(16, 8), False),
+                         (w[:, ::2], False), (w.to("meta"), False)):
+        assert not _usable(bad, (8, 16), False, dev) and _usable(bad, (8, 16), True, dev) == filt_ok
+
+
 def test_checkpoint_stores_posix_and_s3(tmp_path):
     """Uploads to a posix store (with retention) and to an S3 store driven through a fake client: retries, markers, and
     a failed upload that leaves `.uploading` in place so that pruning keeps the directory."""
