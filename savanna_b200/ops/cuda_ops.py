@@ -1524,9 +1524,31 @@ class _HyenaLI(torch.autograd.Function):
         return (df, dll.to(gdt), dR.to(rdt), dll.to(pdt), db.to(bdt), dsi[..., :O].contiguous() if has_sin else None, None)
 
 
+def _spread(t, shape, device):
+    """t broadcast to `shape`, on `device` (the kernels index whole tensors; what cannot be broadcast raises).  Autograd sums the
+    gradient back."""
+    if t.device != device:
+        if t.dim() > 0:
+            raise RuntimeError(f"hyena_li_modal: features on {device}, an operand of shape {tuple(t.shape)} on {t.device}")
+        t = t.to(device)
+    return t if t.shape == shape else t.expand(shape)
+
+
 def hyena_li_modal(feat, gamma, R, p, bias, state_in=None, return_state=False):
-    if not _is_bf16(feat) or gamma.shape[1] > LI_ORDER:
+    """gamma, R, p: anything that broadcasts to [D, O]; bias to [D]; state_in to [B, D, O]."""
+    B, L, C3 = feat.shape
+    D, O, dev = C3 // 3, gamma.shape[1], feat.get_device()
+    if not ((D, O) == gamma.shape == R.shape == p.shape and bias.shape == (D,) and state_in is None
+            and dev == gamma.get_device() == R.get_device() == p.get_device() == bias.get_device()):
+        O = torch.broadcast_shapes(gamma.shape, R.shape, p.shape)[-1]
+        gamma, R, p = (_spread(t, (D, O), feat.device) for t in (gamma, R, p))
+        bias = _spread(bias, (D,), feat.device)
+        if state_in is not None:
+            while state_in.dim() > 3 and state_in.shape[0] == 1:
+                state_in = state_in[0]
+            state_in = _spread(state_in, (B, D, O), feat.device)
+    if feat.dtype != bf16 or O > LI_ORDER:
         return ref.hyena_li_modal(feat, gamma, R, p, bias, state_in, return_state)
-    fn = _HyenaLITiled if LI_TILED and feat.shape[-1] % 24 == 0 and feat.numel() > 0 else _HyenaLI
+    fn = _HyenaLITiled if LI_TILED and C3 % 24 == 0 and B * L > 0 else _HyenaLI
     z, s = fn.apply(feat, gamma, R, p, bias, state_in, return_state)
     return (z, s) if return_state else z

@@ -45,6 +45,49 @@ def test_li_scan(B, L, D, O):
     _close(leaves[4].grad, rl[4].grad, 2e-3, "dbias")
 
 
+@pytest.mark.parametrize("D", [24, 20])                  # the tiled scan, the per-thread one
+@pytest.mark.parametrize("gs,Rs,ps,bs,ss", [("DO", "DO", "D1", "D", None), ("DO", "DO", "11", "D", "1DO"), ("DO", "DO", "", "1", "DO"),
+                                            ("1O", "DO", "DO", "", "BD1"), ("D1", "1O", "O", "D", "1"), ("1O", "1O", "1O", "D", "11DO")])
+def test_li_scan_broadcast_operands(D, gs, Rs, ps, bs, ss):
+    """Operands that broadcast to [D, O], [D] and [B, D, O], with their gradients, against the same call with them spelled out."""
+    torch.manual_seed(7)
+    B, L, O = 3, 70, 5
+    n = {"D": D, "O": O, "B": B, "1": 1}
+
+    def rand(form, scale=1.0):
+        return (torch.randn([n[c] for c in form], device=DEV) * scale).requires_grad_() if form is not None else None
+    feat = (torch.randn(B, L, 3 * D, device=DEV) * 0.7).to(BF)
+    args = [rand(gs, 0.3), rand(Rs), rand(ps, 0.3), rand(bs), rand(ss)]
+    full = [t.detach().expand(s).clone().requires_grad_() if t is not None else None
+            for t, s in zip([*args[:4], args[4][0] if ss == "11DO" else args[4]], [(D, O)] * 3 + [(D,), (B, D, O)])]
+    gz, gs_ = torch.randn(B, L, D, device=DEV), torch.randn(B, D, O, device=DEV)
+    for a in (args, full):
+        z, s = ops.hyena_li_modal(feat, *a, True)
+        a.append((z, s))
+        ((z.float() * gz).sum() + (s * gs_).sum()).backward()
+    assert torch.equal(args[5][0], full[5][0]) and torch.equal(args[5][1], full[5][1])
+    for t, f in zip(args[:5], full[:5]):
+        if t is not None:
+            # the same gradient, summed over the broadcast dimensions (fp32 sums in another order)
+            want = f.grad.sum_to_size(t.shape[1:] if t.dim() == 4 else t.shape).view(t.shape)
+            assert (t.grad - want).norm() <= 1e-5 * want.norm().clamp(min=1e-3)
+    with torch.no_grad():                                # against the fp32 statement
+        zr = ref.hyena_li_modal(feat.float(), *[t.detach() if t is not None else None for t in full[:5]])
+    _close(full[5][0], zr, 8e-3, "z")
+
+
+def test_li_scan_host_operands():
+    """A host scalar for p is accepted, as PyTorch's operators accept it; a host tensor has no address for the kernels."""
+    D, O = 16, 4
+    feat, g, R, b = torch.randn(1, 9, 3 * D, device=DEV).to(BF), torch.randn(D, O, device=DEV), torch.randn(D, O, device=DEV), torch.randn(D, device=DEV)
+    assert torch.equal(ops.hyena_li_modal(feat, g, R, torch.tensor(-1.0), b), ops.hyena_li_modal(feat, g, R, -torch.ones(D, O, device=DEV), b))
+    for i in range(4):
+        args = [g, R, -torch.ones(D, O, device=DEV), b]
+        args[i] = args[i].cpu()
+        with pytest.raises(RuntimeError):
+            ops.hyena_li_modal(feat, *args)
+
+
 def test_li_scan_unaligned_view():
     """A contiguous view that starts off a 16-byte boundary."""
     torch.manual_seed(5)
