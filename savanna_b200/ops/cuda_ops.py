@@ -1415,6 +1415,8 @@ class _HyenaLITiled(torch.autograd.Function):
         dev = feat.device
         fc, bf = _aligned(feat), _f32c(bias)
         sin = _f32c(state_in) if state_in is not None else None
+        if sin is not None and sin.data_ptr() == state_in.data_ptr():
+            sin = sin.clone()                    # the backward reads it: the caller may go on with its own buffer
         tc = _li_tiled_chunk(B, L, D)
         modal = _alloc((3 * D, LI_ORDER), dtype=torch.float32, device=dev)
         S = _alloc((B, (L + tc - 1) // tc, D, LI_ORDER), dtype=torch.float32, device=dev)

@@ -88,6 +88,25 @@ def test_li_scan_host_operands():
             ops.hyena_li_modal(feat, *args)
 
 
+@pytest.mark.parametrize("D", [24, 20])
+def test_li_scan_state_buffer_reused(D):
+    """The caller's state buffer may be overwritten between forward and backward (a running state carried in place)."""
+    torch.manual_seed(9)
+    B, L, O = 2, 40, 16
+    feat = (torch.randn(B, L, 3 * D, device=DEV) * 0.7).to(BF)
+    a = [(torch.rand(D, O, device=DEV) * 0.09 + 0.01).log(), torch.randn(D, O, device=DEV) / 4, -torch.ones(D, O, device=DEV),
+         torch.randn(D, device=DEV)]
+    s0, grads = torch.randn(B, D, O, device=DEV), []
+    for overwrite in (False, True):
+        leaves, buf = [t.clone().requires_grad_() for t in a], s0.clone()
+        z = ops.hyena_li_modal(feat, *leaves, buf)
+        if overwrite:
+            buf.zero_()
+        z.float().sum().backward()
+        grads.append([t.grad for t in leaves])
+    assert all(torch.equal(x, y) for x, y in zip(*grads))
+
+
 def test_li_scan_unaligned_view():
     """A contiguous view that starts off a 16-byte boundary."""
     torch.manual_seed(5)
