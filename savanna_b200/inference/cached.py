@@ -15,7 +15,9 @@ recurrent Hyena inference lives in the separate vortex project).  Decode steps a
 one native call per step runs five kernels per layer (csrc/decode.cu, see `_FusedStep` for what it covers); everything else
 uses plain PyTorch operations on the model's own parameters.  Supported: one device (no tensor / context / pipeline
 parallelism), pre-norm blocks with the gated MLP, rotary or no position embedding, implicit-modal Hyena-LI filters; any
-other configuration raises and the caller falls back to `stream_tokens` (recompute).
+other configuration raises NotImplementedError and the caller falls back to `stream_tokens` (recompute).  So does a sequence
+longer than `rotary_emb_max_unscaled_seq_len` under `rotary_ntk_scaled`: from there on the rotary base of all positions changes
+with every token, and with it every key and everything computed from them.
 """
 from __future__ import annotations
 
@@ -407,6 +409,9 @@ class CachedDecoder:
                 raise NotImplementedError("cached generation does not cover the block-sparse attention operators")
             if isinstance(m, HyenaOperator) and (m.bidirectional or m.slow_heads):
                 raise NotImplementedError("cached generation does not cover two-sided filters or outer-product heads")
+        # the longest sequence whose keys stay what they are as it grows
+        self.limit = min((r.max_unscaled_len for b in self.blocks if isinstance(b.mixer.mixer, SelfAttention)
+                          for r in b.mixer.mixer._rotary if r.kind == "rotary_ntk_scaled"), default=None)
         self._states: List[Dict] = []
         self.pos = 0
         self._fused: Optional[_FusedStep] = None
@@ -425,6 +430,10 @@ class CachedDecoder:
     def states(self, value: List[Dict]) -> None:
         self._states, self._fused, self._resume = value, None, True
 
+    def check_length(self, n: int) -> None:
+        if self.limit is not None and n > self.limit:
+            raise NotImplementedError(f"cached generation of {n} tokens: rotary_ntk_scaled changes its base beyond {self.limit}")
+
     def _hand_back(self) -> None:
         if self._fused is not None:
             self._states, self._fused, self._resume = self._fused.export(), None, True
@@ -441,6 +450,7 @@ class CachedDecoder:
         """tokens [B, T] -> logits of the last position [B, V]; leaves every layer's state at position T."""
         model = self.model
         B, T = tokens.shape
+        self.check_length(T)
         self._fused, self._resume = None, False
         self._states = [dict() for _ in self.blocks]
         hooks = []
@@ -556,6 +566,7 @@ class CachedDecoder:
     def step(self, token: torch.Tensor) -> torch.Tensor:
         """token [B] -> logits of the next position [B, V]; advances every layer's state by one token."""
         model, cfg = self.model, self.cfg
+        self.check_length(self.pos + 1)
         if self._fused is not None and (self._fused.pos != self.pos or not self._fused.follow()):
             self._hand_back()                    # the caller moved to another position, or changed the model
         if self._resume:
@@ -603,18 +614,24 @@ class CachedDecoder:
         return model.logits(x[:, None])[:, 0].float()
 
 
-@torch.no_grad()
 def stream_tokens_cached(model, context_tokens: List[List[int]], eos_token_id: Optional[int] = None, maximum_tokens: int = 64,
                          temperature: float = 0.0, top_k: int = 0, top_p: float = 0.0, generator=None):
     """Cached counterpart of `generation.stream_tokens` for prompts of equal length: one prefill, then one `step` per
-    generated token.  Yields (tokens [B, T], logits of the step, finished mask)."""
-    from .generation import sample_tokens
+    generated token.  Yields (tokens [B, T], logits of the step, finished mask).  Raises before the first token when the model, or
+    a sequence of the full length, has no cached form."""
     lens = {len(c) for c in context_tokens}
     if len(lens) != 1:
         raise ValueError("cached generation takes prompts of equal length (pad or group them by length)")
-    device = next(model.parameters()).device
-    toks = torch.tensor(context_tokens, dtype=torch.long, device=device)
     dec = CachedDecoder(model)
+    dec.check_length(lens.pop() + maximum_tokens)
+    return _stream(dec, context_tokens, eos_token_id, maximum_tokens, temperature, top_k, top_p, generator)
+
+
+@torch.no_grad()
+def _stream(dec, context_tokens, eos_token_id, maximum_tokens, temperature, top_k, top_p, generator):
+    from .generation import sample_tokens
+    device = next(dec.model.parameters()).device
+    toks = torch.tensor(context_tokens, dtype=torch.long, device=device)
     logits = dec.prefill(toks)
     done = torch.zeros(toks.shape[0], dtype=torch.bool, device=device)
     for _ in range(maximum_tokens):

@@ -267,6 +267,44 @@ def test_cached_generation_matches_recompute():
     assert "".join(said) == generate(model, cfg.tokenizer, ["ACGTACGT"], maximum_tokens=5)[0]["text"]
 
 
+def test_cached_generation_with_a_growing_rotary_base():
+    """`rotary_ntk_scaled` enlarges the base once the sequence exceeds `rotary_emb_max_unscaled_seq_len`: the cached decoder
+    agrees with the full forward up to that length, refuses longer sequences, and its callers recompute instead."""
+    from savanna_b200.inference.cached import CachedDecoder, stream_tokens_cached
+    from savanna_b200.inference.generation import generate, generate_samples_interactive
+    from savanna_b200.models import build_model
+    cfg = GlobalConfig.from_ymls([TINY], {"global_num_gpus": 1, "hidden_dropout": 0.0, "pos_emb": "rotary_ntk_scaled",
+                                          "rotary_emb_max_unscaled_seq_len": 20, "rotary_emb_scaling_factor": 4.0})
+    cfg.build_tokenizer()
+    torch.manual_seed(0)
+    model = build_model(cfg)
+    with torch.no_grad():                                  # attention that depends on the positions
+        for n, p in model.named_parameters():
+            if "dense_projection" in n:
+                p.mul_(20)
+    toks = torch.randint(65, 90, (2, 24))
+    full = [model(toks[:, :n])[:, -1].float() for n in range(1, 25)]
+    dec = CachedDecoder(model)
+    assert torch.allclose(dec.prefill(toks[:, :16]), full[15], atol=1e-4)
+    for n in range(17, 21):
+        assert torch.allclose(dec.step(toks[:, n - 1]), full[n - 1], atol=2e-3, rtol=2e-3), n
+    for _ in range(2):
+        with pytest.raises(NotImplementedError):
+            dec.step(toks[:, 20])
+    with pytest.raises(NotImplementedError):
+        dec.prefill(toks[:, :21])
+    with pytest.raises(NotImplementedError):
+        stream_tokens_cached(model, toks[:, :16].tolist(), maximum_tokens=5)
+    assert len(list(stream_tokens_cached(model, toks[:, :16].tolist(), maximum_tokens=4))) == 4
+    prompt = cfg.tokenizer.detokenize(toks[0, :16].tolist())
+    want = generate(model, cfg.tokenizer, [prompt], maximum_tokens=8, use_cache=False)[0]
+    assert generate(model, cfg.tokenizer, [prompt], maximum_tokens=8, use_cache=True)[0]["text"] == want["text"]
+    said, prompts = [], iter([prompt, ""])
+    generate_samples_interactive(model, cfg, input_fn=lambda _: next(prompts), print_fn=lambda *x, **k: said.append(x[0]),
+                                 maximum_tokens=8)
+    assert "".join(said) == want["text"]
+
+
 def test_decode_weights_the_kernels_may_read():
     """The native decode step reads 16 bytes of bf16 at a time: what it accepts as a weight, and as a filter parameter."""
     from savanna_b200.inference.cached import _usable
