@@ -368,8 +368,10 @@ constexpr int LV_FW = 3 * LV_CH / 2;     // 32-bit words per staged feature row
 constexpr int LV_GW = LV_CH / 2;         // 32-bit words per staged row of a [.., D] tensor
 
 // The filter, prepared once per call by li_prep_kernel: log-poles -exp(p) exp(gamma), poles and residues, [D, 16] fp32
-// (modes beyond the order O: pole 0, residue 0).
+// (modes beyond the order O: pole 0, residue 0).  The C entries that are handed log-poles (sb_li_fwd, sb_li_bwd) have no poles:
+// lam is null there and the kernels form them.
 struct LiModal { const float* ll; const float* lam; const float* R; int O; };
+static int g_li_tiled = 1;               // sb_li_set_variant
 
 __global__ void li_prep_kernel(const float* __restrict__ gamma, const float* __restrict__ p, const float* __restrict__ R,
                                float* __restrict__ out, int D, int O) {
@@ -422,6 +424,13 @@ __device__ __forceinline__ void li_stage(uint32_t dst, const bf16* src, size_t l
   }
 }
 
+__device__ __forceinline__ void load_poles(const LiModal& m, size_t off, bool live, f2 (&lam)[LO]) {
+  load_pairs((m.lam ? m.lam : m.ll) + off, live, lam);
+  if (m.lam) return;
+#pragma unroll
+  for (int o = 0; o < LO; ++o) { const float2 t = f2_unpack(lam[o]); lam[o] = f2_pack(expf(t.x), expf(t.y)); }
+}
+
 struct FeatPair { f2 x1, x2, v; };
 __device__ __forceinline__ FeatPair li_feat(const uint32_t* row, int lane3) {
   const uint32_t w0 = row[lane3], w1 = row[lane3 + 1], w2 = row[lane3 + 2];
@@ -453,7 +462,7 @@ li_fwd_tiled_kernel(const bf16* __restrict__ feat, const LiModal m, const float*
     li_cp_commit();
   }
   f2 lam[LO], s[LO], rr[APPLY ? LO : 1], be = 0;
-  load_pairs(m.lam + (size_t)ch * LO, live, lam);
+  load_poles(m, (size_t)ch * LO, live, lam);
   float* Sp = S + (((size_t)b * d.NC + n) * d.D + ch) * LO;
   if constexpr (APPLY) {
     load_pairs(m.R + (size_t)ch * LO, live, rr);
@@ -556,10 +565,11 @@ li_prefix_tiled_kernel(float* __restrict__ S, const LiModal m, const float* __re
   if (state_out && o < m.O) state_out[((size_t)b * d.D + ch) * m.O + o] = end;
 }
 
-// Backward prefixes: blockIdx.z = 0 the states, 1 the adjoints (scaled by R when a state gradient has to ride along).
+// Backward prefixes: blockIdx.z = 0 the states, 1 the adjoints (carrying R, `with_R`, when a state gradient has to ride along or
+// the caller wants finished partial sums).
 __global__ void __launch_bounds__(128)
 li_bwd_prefix_tiled_kernel(float* __restrict__ S, float* __restrict__ A, const LiModal m, const float* __restrict__ state_in,
-                           const float* __restrict__ dstate_out, float* __restrict__ dstate_in, LiDims d) {
+                           const float* __restrict__ dstate_out, float* __restrict__ dstate_in, int with_R, LiDims d) {
   const size_t per_b = (size_t)d.D * LO;
   const size_t r = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   const int b = blockIdx.y;
@@ -572,9 +582,9 @@ li_bwd_prefix_tiled_kernel(float* __restrict__ S, float* __restrict__ A, const L
     li_carry<false, LP_AHEAD_BWD>(S + base, per_b, ll, 1.f, state_at(state_in, b, ch, o, m, d.D), 0.f, d);
   } else {
     const float R = m.R[r];
-    const float end = li_carry<true, LP_AHEAD_BWD>(A + base, per_b, ll, dstate_out ? R : 1.f, 0.f,
+    const float end = li_carry<true, LP_AHEAD_BWD>(A + base, per_b, ll, with_R ? R : 1.f, 0.f,
                                                    state_at(dstate_out, b, ch, o, m, d.D), d);
-    if (dstate_in && real) dstate_in[((size_t)b * d.D + ch) * m.O + o] = expf(ll) * (dstate_out ? end : R * end);
+    if (dstate_in && real) dstate_in[((size_t)b * d.D + ch) * m.O + o] = expf(ll) * (with_R ? end : R * end);
   }
 }
 
@@ -599,7 +609,7 @@ li_bwd_local_tiled_kernel(const bf16* __restrict__ feat, const bf16* __restrict_
   li_stage<LB_TC, LV_CH / 8, 2 * LV_PAIRS>(g_a, dz + ((size_t)b * d.L + t0) * d.D + c0, d.D, rows, ncg, tid);
   li_cp_commit();
   f2 lam[LO], s[LO];
-  load_pairs(m.lam + (size_t)ch * LO, live, lam);
+  load_poles(m, (size_t)ch * LO, live, lam);
 #pragma unroll
   for (int o = 0; o < LO; ++o) s[o] = 0;
   li_cp_wait<0>();
@@ -626,13 +636,13 @@ li_bwd_local_tiled_kernel(const bf16* __restrict__ feat, const bf16* __restrict_
   if (live) store_pairs(out + (((size_t)b * d.NC + n) * d.D + ch) * LO, s);
 }
 
-// backward pass 3: see the head of this section.  S and A hold the entering state / adjoint of every chunk and are
-// overwritten with the chunk's partial sums of dR and dlam (dlam without the factor R unless GOUT).  GOUT: the caller has a
-// gradient of the final state; the adjoint then carries R and that gradient (dstate_out, [B, D, O]).
+// backward pass 3: see the head of this section.  S and A hold the entering state / adjoint of every chunk; dRp and dLp (which
+// may be S and A) receive the chunk's partial sums of dR and dlam (dlam without the factor R unless GOUT).  GOUT: the adjoint
+// carries R, and the gradient of the final state (dstate_out, [B, D, O]) if there is one.
 template <bool GOUT>
 __global__ void __launch_bounds__(3 * LV_PAIRS, 2)
 li_bwd_apply_tiled_kernel(const bf16* __restrict__ feat, const bf16* __restrict__ dz, const LiModal m, const float* __restrict__ bias,
-                          float* __restrict__ S, float* __restrict__ A, float* __restrict__ dBp, bf16* __restrict__ dfeat,
+                          const float* S, const float* A, float* dRp, float* dLp, float* __restrict__ dBp, bf16* __restrict__ dfeat,
                           const float* __restrict__ dstate_out, LiDims d) {
   extern __shared__ __align__(16) uint32_t li_sm[];
   uint32_t (*fS)[LV_FW] = reinterpret_cast<uint32_t (*)[LV_FW]>(li_sm);
@@ -650,7 +660,7 @@ li_bwd_apply_tiled_kernel(const bf16* __restrict__ feat, const bf16* __restrict_
   li_cp_commit();
   const size_t off = (((size_t)b * d.NC + n) * d.D + ch) * LO;
   f2 lam[LO], s[LO];                                     // s: state (roles 0, 1) or adjoint (role 2) entering the chunk
-  load_pairs(m.lam + (size_t)ch * LO, live, lam);
+  load_poles(m, (size_t)ch * LO, live, lam);
   load_pairs((role == 2 ? A : S) + off, live, s);
   li_cp_wait<0>();
   __syncthreads();                                       // the chunk has landed; S and A of this block have been read
@@ -681,7 +691,7 @@ li_bwd_apply_tiled_kernel(const bf16* __restrict__ feat, const bf16* __restrict_
       o16[3] = (uint16_t)(w >> 16);
     }
     if (live) {
-      store_pairs(S + off, dr);
+      store_pairs(dRp + off, dr);
       const float2 t = f2_unpack(db);
       *reinterpret_cast<float2*>(dBp + ((size_t)b * d.NC + n) * d.D + ch) = t;
     }
@@ -713,7 +723,7 @@ li_bwd_apply_tiled_kernel(const bf16* __restrict__ feat, const bf16* __restrict_
         }
         dl[o] = f2_fma(e, w[o], dl[o]);
       }
-      store_pairs(A + off, dl);
+      store_pairs(dLp + off, dl);
     }
   } else {
     f2 rr[LO], be = 0;
@@ -1067,17 +1077,41 @@ static inline LiDims li_dims(int B, int L, int D, int TC) { return LiDims{B, L, 
 // Scratch sizes (floats): S = B*NC*D*16.  Callers allocate and pass them.
 extern "C" int sb_li_num_chunks(int L, int TC) { return (L + TC - 1) / TC; }
 
+static inline bool aligned16(const void* a, const void* b, const void* c = nullptr) {
+  return (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) & 15) == 0;
+}
+
+// The forward scan on prepared log-poles and residues ([D, 16]): the tiled kernels for D % 8 == 0 and 16-byte aligned features and
+// output, else the per-thread ones (L = 8192, D = 4096: 0.14 and 0.28 ms).
+static int li_forward(const void* feat, const float* loglam, const float* R, const float* bias, const float* state_in,
+                      float* state_out, float* S, void* z, const LiDims& d, cudaStream_t st) {
+  const size_t n = (size_t)d.D * LO;
+  if (g_li_tiled && d.D % 8 == 0 && aligned16(feat, z)) {
+    const LiModal m{loglam, nullptr, R, LO};
+    const dim3 grid((d.D + LV_CH - 1) / LV_CH, d.NC, d.B);
+    li_fwd_tiled_kernel<false><<<grid, LV_PAIRS, 0, st>>>((const bf16*)feat, m, bias, S, nullptr, d);
+    li_prefix_tiled_kernel<<<dim3((unsigned)((n + 127) / 128), d.B), 128, 0, st>>>(S, m, state_in, state_out, d);
+    li_fwd_tiled_kernel<true><<<grid, LV_PAIRS, 0, st>>>((const bf16*)feat, m, bias, S, (bf16*)z, d);
+  } else {
+    const dim3 grid((d.D + LI_THREADS - 1) / LI_THREADS, d.NC, d.B);
+    li_local_kernel<<<grid, LI_THREADS, 0, st>>>((const bf16*)feat, loglam, S, d);
+    li_prefix_kernel<<<(unsigned)((d.B * n + 255) / 256), 256, 0, st>>>(S, loglam, state_in, state_out, d);
+    li_apply_kernel<<<grid, LI_THREADS, 0, st>>>((const bf16*)feat, loglam, R, bias, S, (bf16*)z, d);
+  }
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
 extern "C" int sb_li_fwd(const void* feat, const float* loglam, const float* R, const float* bias, const float* state_in,
                          float* state_out, float* S_scratch, void* z, int B, int L, int D, int TC, cudaStream_t st) {
   if (B * L == 0) return 0;
-  LiDims d = li_dims(B, L, D, TC);
-  dim3 grid((D + LI_THREADS - 1) / LI_THREADS, d.NC, B);
-  const size_t n = (size_t)B * D * LO;
-  li_local_kernel<<<grid, LI_THREADS, 0, st>>>((const bf16*)feat, loglam, S_scratch, d);
-  li_prefix_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(S_scratch, loglam, state_in, state_out, d);
-  li_apply_kernel<<<grid, LI_THREADS, 0, st>>>((const bf16*)feat, loglam, R, bias, S_scratch, (bf16*)z, d);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return li_forward(feat, loglam, R, bias, state_in, state_out, S_scratch, z, li_dims(B, L, D, TC), st);
 }
+
+// 1 (default): shared-memory tiled scan kernels where the shape allows; 0: the per-thread streaming kernels
+extern "C" int sb_li_set_variant(int tiled) { sb::g_li_tiled = tiled ? 1 : 0; return 0; }
+// Chunk length with which sb_li_bwd takes the tiled kernels, which keep a whole chunk in shared memory, for a given choice of
+// the caller; the scratch arrays are sized with the value returned here.
+extern "C" int sb_li_bwd_chunk(int D, int TC) { return (sb::g_li_tiled && D % 8 == 0) ? sb::LB_TC : TC; }
 
 // Tiled forward: gamma, p, R [D, O] fp32 (O <= 16), state_in / state_out [B, D, O] or null.  Scratch: modal 3*D*16 floats
 // (the prepared filter, which the backward takes over), S B*NC*D*16 floats.  D % 8 == 0, feat and z 16-byte aligned.
@@ -1099,6 +1133,13 @@ extern "C" int sb_li_fwd_tiled(const void* feat, const float* gamma, const float
 
 extern "C" int sb_li_bwd_tiled_chunk() { return LB_TC; }
 
+// function attributes belong to the current device's context: set on every call (they cost a lookup)
+static bool li_bwd_tiled_ready() {
+  return cudaFuncSetAttribute(li_bwd_local_tiled_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LBL_SMEM) == cudaSuccess &&
+         cudaFuncSetAttribute(li_bwd_apply_tiled_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, LBA_SMEM) == cudaSuccess &&
+         cudaFuncSetAttribute(li_bwd_apply_tiled_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, LBA_SMEM) == cudaSuccess;
+}
+
 // Tiled backward, chunk length sb_li_bwd_tiled_chunk().  modal: as the forward left it.  Scratch: S, A B*NC*D*16 floats,
 // dBp B*NC*D floats.  Outputs: dfeat, dR and dll = dgamma = dp [D, O], db [D], dstate_in [B, D, O] or null.
 extern "C" int sb_li_bwd_tiled(const void* feat, const void* dz, const float* modal, const float* bias, const float* state_in,
@@ -1106,22 +1147,19 @@ extern "C" int sb_li_bwd_tiled(const void* feat, const void* dz, const float* mo
                                float* db, float* dstate_in, int B, int L, int D, int O, cudaStream_t st) {
   if ((D % 8) || O < 1 || O > LO || ((uintptr_t)feat % 16) || ((uintptr_t)dz % 16) || ((uintptr_t)dfeat % 16)) return -1;
   if ((long long)B * L * D == 0) return 0;
-  // function attributes belong to the current device's context: set on every call (they cost a lookup)
-  if (cudaFuncSetAttribute(li_bwd_local_tiled_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LBL_SMEM) != cudaSuccess ||
-      cudaFuncSetAttribute(li_bwd_apply_tiled_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, LBA_SMEM) != cudaSuccess ||
-      cudaFuncSetAttribute(li_bwd_apply_tiled_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, LBA_SMEM) != cudaSuccess)
-    return -5;
+  if (!li_bwd_tiled_ready()) return -5;
   LiDims d = li_dims(B, L, D, LB_TC);
   const size_t n = (size_t)D * LO;
   const LiModal m{modal, modal + n, modal + 2 * n, O};
   const dim3 grid((D + LV_CH - 1) / LV_CH, d.NC, B);
   li_bwd_local_tiled_kernel<<<grid, 2 * LV_PAIRS, LBL_SMEM, st>>>((const bf16*)feat, (const bf16*)dz, m, S, A, d);
-  li_bwd_prefix_tiled_kernel<<<dim3((unsigned)((n + 127) / 128), B, 2), 128, 0, st>>>(S, A, m, state_in, dstate_out, dstate_in, d);
+  li_bwd_prefix_tiled_kernel<<<dim3((unsigned)((n + 127) / 128), B, 2), 128, 0, st>>>(S, A, m, state_in, dstate_out, dstate_in,
+                                                                                              dstate_out != nullptr, d);
   if (dstate_out)
-    li_bwd_apply_tiled_kernel<true><<<grid, 3 * LV_PAIRS, LBA_SMEM, st>>>((const bf16*)feat, (const bf16*)dz, m, bias, S, A, dBp,
+    li_bwd_apply_tiled_kernel<true><<<grid, 3 * LV_PAIRS, LBA_SMEM, st>>>((const bf16*)feat, (const bf16*)dz, m, bias, S, A, S, A, dBp,
                                                                          (bf16*)dfeat, dstate_out, d);
   else
-    li_bwd_apply_tiled_kernel<false><<<grid, 3 * LV_PAIRS, LBA_SMEM, st>>>((const bf16*)feat, (const bf16*)dz, m, bias, S, A, dBp,
+    li_bwd_apply_tiled_kernel<false><<<grid, 3 * LV_PAIRS, LBA_SMEM, st>>>((const bf16*)feat, (const bf16*)dz, m, bias, S, A, S, A, dBp,
                                                                           (bf16*)dfeat, nullptr, d);
   const unsigned blocks = (unsigned)((n + LR_COLS - 1) / LR_COLS + (D + LR_COLS - 1) / LR_COLS);
   li_bwd_reduce_kernel<<<blocks, LR_COLS * LR_SLICES, 0, st>>>(S, A, dBp, m, dstate_out ? 0 : 1, dR, dll, db, B * d.NC, D);
@@ -1129,13 +1167,27 @@ extern "C" int sb_li_bwd_tiled(const void* feat, const void* dz, const float* mo
 }
 
 // Scratch: S, W, A, dRp, dLp each B*NC*D*16 floats; dBp B*NC*D floats; dx1_tmp B*L*D bf16.
-// Outputs: dfeat; per-chunk partials dRp/dLp/dBp (the caller sums over B and NC); w_end, dstate_in optional.
+// Outputs: dfeat; per-chunk partials dRp/dLp/dBp (the caller sums over B and NC); w_end, dstate_in optional.  The tiled kernels
+// run for chunks of sb_li_bwd_chunk(D, TC) steps; with a gradient of the final state, whose share of dlam the caller forms from
+// w_end, the per-thread ones do.
 extern "C" int sb_li_bwd(const void* feat, const void* dz, const float* loglam, const float* R, const float* bias,
                          const float* state_in, const float* dstate_out, float* S, float* W, float* A, float* dRp,
                          float* dLp, float* dBp, void* dx1_tmp, void* dfeat, float* w_end, float* dstate_in, int B, int L,
                          int D, int TC, cudaStream_t st) {
   if (B * L == 0) return 0;
   LiDims d = li_dims(B, L, D, TC);
+  if (g_li_tiled && D % 8 == 0 && TC == LB_TC && !dstate_out && !w_end && aligned16(feat, dz, dfeat)) {
+    if (!li_bwd_tiled_ready()) return -5;
+    const LiModal m{loglam, nullptr, R, LO};
+    const dim3 tiles((D + LV_CH - 1) / LV_CH, d.NC, B);
+    li_bwd_local_tiled_kernel<<<tiles, 2 * LV_PAIRS, LBL_SMEM, st>>>((const bf16*)feat, (const bf16*)dz, m, S, A, d);
+    li_bwd_prefix_tiled_kernel<<<dim3((unsigned)(((size_t)D * LO + 127) / 128), B, 2), 128, 0, st>>>(S, A, m, state_in, nullptr,
+                                                                                                     dstate_in, 1, d);
+    li_bwd_apply_tiled_kernel<true><<<tiles, 3 * LV_PAIRS, LBA_SMEM, st>>>((const bf16*)feat, (const bf16*)dz, m, bias, S, A, dRp, dLp,
+                                                                          dBp, (bf16*)dfeat, nullptr, d);
+    return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  }
+  if (!dx1_tmp || !W) return -1;
   dim3 grid((D + LI_THREADS - 1) / LI_THREADS, d.NC, B);
   const size_t n = (size_t)B * D * LO;
   li_bwd_local_kernel<<<grid, LI_THREADS, 0, st>>>((const bf16*)feat, (const bf16*)dz, loglam, R, S, W, A, d);
@@ -1245,11 +1297,5 @@ extern "C" int sb_li_fwd_noalloc(const void* feat, const float* loglam, const fl
     }
     g_li_noalloc_ptr[dev] = p;
   }
-  float* S = g_li_noalloc_ptr[dev];
-  dim3 grid((D + LI_THREADS - 1) / LI_THREADS, d.NC, B);
-  li_local_kernel<<<grid, LI_THREADS, 0, st>>>((const bf16*)feat, loglam, S, d);
-  const size_t n = (size_t)B * D * LO;
-  li_prefix_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(S, loglam, state_in, state_out, d);
-  li_apply_kernel<<<grid, LI_THREADS, 0, st>>>((const bf16*)feat, loglam, R, bias, S, (bf16*)z, d);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return li_forward(feat, loglam, R, bias, state_in, state_out, g_li_noalloc_ptr[dev], z, d, st);
 }

@@ -117,6 +117,8 @@ class _Sig:
     sb_conv_set_fwd_variant = [I]
     sb_mr_tc_bwd = [P, P, P, P, P, P, P, P, P, I, I, I, I, I, P]
     sb_li_fwd = [P, P, P, P, P, P, P, P, I, I, I, I, P]
+    sb_li_set_variant = [I]
+    sb_li_bwd_chunk = [I, I]
     sb_li_fwd_tiled = [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, P]
     sb_li_bwd_tiled_chunk = []
     sb_li_bwd_tiled = [P, P, P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, P]
@@ -1369,6 +1371,7 @@ def set_li_variant(tiled: bool) -> None:
     """True (default): shared-memory tiled scan kernels; False: the per-thread streaming kernels (A/B measurements, tests)."""
     global LI_TILED
     LI_TILED = bool(tiled)
+    require().sb_li_set_variant(int(LI_TILED))
 
 
 def _li_chunk(B: int, L: int, D: int) -> int:

@@ -118,6 +118,60 @@ def test_li_scan_unaligned_view():
     assert torch.equal(ops.hyena_li_modal(feat, *a), ops.hyena_li_modal(feat.clone(), *a))
 
 
+@pytest.mark.parametrize("D,offset,tiled", [(24, 0, True), (136, 0, True), (20, 0, False), (24, 1, False)])
+@pytest.mark.parametrize("state", [False, True])
+def test_li_c_entries(D, offset, tiled, state):
+    """`sb_li_fwd` / `sb_li_bwd` on prepared log-poles: the tiled kernels where the shape and the alignment allow, the per-thread
+    ones elsewhere, the same numbers from both."""
+    from savanna_b200.ops import cuda_ops
+    lib = cuda_ops.require()
+    torch.manual_seed(D + offset)
+    B, L, O, st = 2, 200, 16, torch.cuda.current_stream().cuda_stream
+
+    def buf(*shape, dtype=torch.float32):
+        n = math.prod(shape)
+        t = torch.zeros(n + offset, device=DEV, dtype=dtype)[offset:].view(shape) if dtype == BF else torch.zeros(shape, device=DEV)
+        return t
+    feat, dz, z = buf(B, L, 3 * D, dtype=BF), buf(B, L, D, dtype=BF), buf(B, L, D, dtype=BF)
+    feat.copy_(torch.randn(B, L, 3 * D, device=DEV) * 0.7), dz.copy_(torch.randn(B, L, D, device=DEV))
+    g, R, p, bias = (torch.rand(D, O, device=DEV) * 0.09 + 0.01).log(), torch.randn(D, O, device=DEV) / 4, -torch.ones(D, O, device=DEV), \
+        torch.randn(D, device=DEV)
+    s_in = torch.randn(B, D, O, device=DEV) if state else None
+    ll = -torch.exp(p) * torch.exp(g)
+
+    def ptr(t):
+        return t.data_ptr() if t is not None else None
+    tc = lib.sb_li_bwd_chunk(D, 128)
+    assert tc == (64 if D % 8 == 0 else 128)
+    nf, nb = -(-L // 96), -(-L // tc)
+    S, sout = buf(B, nf, D, 16), buf(B, D, 16)
+    Sb, W, A, dRp, dLp = (buf(B, nb, D, 16) for _ in range(5))
+    dBp, tmp, df, dsi = buf(B, nb, D), buf(B, L, D, dtype=BF), buf(B, L, 3 * D, dtype=BF), buf(B, D, 16)
+    torch.cuda.synchronize()
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        assert lib.sb_li_fwd(ptr(feat), ptr(ll), ptr(R), ptr(bias), ptr(s_in), ptr(sout), ptr(S), ptr(z), B, L, D, 96, st) == 0
+        assert lib.sb_li_bwd(ptr(feat), ptr(dz), ptr(ll), ptr(R), ptr(bias), ptr(s_in), None, ptr(Sb), ptr(W), ptr(A), ptr(dRp), ptr(dLp),
+                             ptr(dBp), ptr(tmp), ptr(df), None, ptr(dsi) if state else None, B, L, D, tc, st) == 0
+        torch.cuda.synchronize()
+    names = [e.key for e in prof.key_averages()]
+    if any("li_" in n for n in names):                   # (no kernel names where the profiler has no access to the device)
+        assert all(("tiled" in n) == tiled for n in names if "li_" in n), names
+    leaves = [t.float().clone().requires_grad_() for t in (feat, g, R, p, bias)]
+    sr = s_in.clone().requires_grad_() if state else None
+    zr, sor = ref.hyena_li_modal(*leaves, sr, True)
+    zr.backward(dz.float())
+    lam = torch.exp(ll)
+    _close(z, zr, 8e-3, "z")                             # as in test_li_scan
+    _close(df, leaves[0].grad, 8e-3, "dfeat")
+    _close(sout, sor, 2e-3, "state_out")
+    _close(dRp.sum((0, 1)), leaves[2].grad, 2e-3, "dR")
+    _close(dLp.sum((0, 1)) * lam * ll, leaves[1].grad, 2e-3, "dgamma")
+    _close(dBp.sum((0, 1)), leaves[4].grad, 2e-3, "dbias")
+    if state:
+        _close(dsi, sr.grad, 2e-3, "dstate_in")
+
+
 @pytest.mark.parametrize("B,L,D,G,K", [(1, 1, 16, 1, 128), (2, 31, 16, 1, 1), (1, 32, 80, 5, 16), (1, 33, 64, 1, 17), (2, 160, 48, 3, 113),
                                        (1, 161, 144, 9, 128), (1, 700, 64, 4, 31)])
 @pytest.mark.parametrize("halo", [False, True])
