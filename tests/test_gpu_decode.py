@@ -1,5 +1,5 @@
-"""The native decode step (csrc/decode.cu) against the operator-by-operator step of the same decoder: parameters that change
-between steps, state that is copied and put back."""
+"""The native decode step (csrc/decode.cu) against the operator-by-operator step of the same decoder: the layers' forms,
+parameters that change between steps, state that is copied and put back."""
 import copy
 import os
 
@@ -47,6 +47,42 @@ def _agree(fast, slow, toks):
     for t in toks.unbind(1):
         a, b = fast.step(t), slow.step(t)
         assert (a - b).norm() <= 2.2e-2 * b.norm(), ((a - b).norm() / b.norm()).item()
+
+
+_FORMS = {
+    "gelu": {"mlp_activation": "gelu"}, "relu": {"mlp_activation": "relu"}, "identity": {"mlp_activation": "identity"},
+    "classic_norm": {"rmsnorm_form": "classic", "rms_norm_epsilon": 1e-2}, "no_second_norm": {"pre_mlp_norm": False},
+    "no_pregate": {"hyena_se_pregate": False}, "no_postgate": {"hyena_se_postgate": False},
+    "partial_rotary": {"rotary_pct": 0.25}, "linear_rotary": {"pos_emb": "rotary_linear_scaled", "rotary_emb_scaling_factor": 4.0},
+    "no_rotary": {"pos_emb": "none"}, "untied_head": {"no_weight_tying": True},
+    "scaled_head": {"use_mup": True, "mup_width_scale": 2, "mup_output_temp": 0.5, "mup_embedding_mult": 3.0},
+    "order_5": {"hyena_filter_order": 5}, "order_40": {"hyena_filter_order": 40}, "grouped_long_filter": {"num_groups_hyena": 64},
+    "short_taps": {"hyena_se_len": 4, "short-conv-L": 2, "hyena_mr_len": 17}, "one_tap": {"hyena_se_len": 1, "hyena_mr_len": 1},
+}
+
+
+@pytest.mark.parametrize("B,T", [(1, 7), (3, 150)])
+@pytest.mark.parametrize("form", _FORMS)
+def test_forms(form, B, T, monkeypatch):
+    """Every branch of the kernels: gates, norms, position embeddings, filter lengths and orders, heads that the step leaves to the
+    model."""
+    model = _model(**_FORMS[form])
+    toks = _toks(model, B, T + 12)
+    fast, slow = CachedDecoder(model), _slow(model, toks[:, :T], monkeypatch)
+    fast.prefill(toks[:, :T])
+    assert fast._fused is not None and (fast._fused.head is None) == (form in ("untied_head", "scaled_head"))
+    _agree(fast, slow, toks[:, T:])
+
+
+@pytest.mark.parametrize("B,ffn,native", [(8, 12800, True), (8, 12816, False), (4, 12816, True), (9, 512, False)])
+def test_limits(B, ffn, native, monkeypatch):
+    """The widest gate whose inputs fit in shared memory, one step wider, and more sequences than a launch takes."""
+    model = _model(ffn_hidden_size=ffn)
+    toks = _toks(model, B, 12)
+    fast, slow = CachedDecoder(model), _slow(model, toks[:, :9], monkeypatch)
+    fast.prefill(toks[:, :9])
+    assert (fast._fused is not None) == native
+    _agree(fast, slow, toks[:, 9:])
 
 
 def _is_filter(n):
