@@ -118,6 +118,63 @@ def test_li_scan_unaligned_view():
     assert torch.equal(ops.hyena_li_modal(feat, *a), ops.hyena_li_modal(feat.clone(), *a))
 
 
+def _same(a, b, what):
+    assert torch.equal(torch.nan_to_num(a.float()), torch.nan_to_num(b.float())), what
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_li_scan_non_finite_values_stay_where_they_belong(bad):
+    """A non-finite input reaches the outputs of its own channel from its own step on (the adjoint: up to it), and nothing else:
+    not the channel that shares its registers, not earlier chunks."""
+    torch.manual_seed(11)
+    B, L, D, O, t0, c = 2, 300, 24, 16, 133, 5
+    feat, dz = (torch.randn(B, L, n * D, device=DEV).to(BF) for n in (3, 1))
+    a = [(torch.rand(D, O, device=DEV) * 0.09 + 0.01).log(), torch.randn(D, O, device=DEV) / 4, -torch.ones(D, O, device=DEV),
+         torch.randn(D, device=DEV)]
+
+    def run(f, g):
+        leaves = [t.clone().requires_grad_() for t in (f, *a)]
+        z = ops.hyena_li_modal(*leaves)
+        z.backward(g)
+        return [z.detach()] + [t.grad for t in leaves]
+    clean = run(feat, dz)
+    f = feat.clone()
+    f[1, t0, 3 * c + 1] = bad
+    z, df, dg, dR, dp, db = run(f, dz)
+    others = [i for i in range(D) if i != c]
+    _same(z[0], clean[0][0], "other sequence"), _same(z[1][:, others], clean[0][1][:, others], "other channels")
+    _same(z[1, :t0, c], clean[0][1, :t0, c], "earlier steps")
+    assert not z[1, t0:, c].isfinite().any()
+    d, dc = df.view(B, L, D, 3), clean[1].view(B, L, D, 3)
+    _same(d[:, :, others], dc[:, :, others], "dfeat, other channels"), _same(d[1, :t0, c], dc[1, :t0, c], "dfeat, earlier steps")
+    for got, want in zip((dg, dR, dp, db), clean[2:]):
+        _same(got[others], want[others], "parameter gradients, other channels")
+    assert (dg[c] == 0).all() and (dp[c] == 0).all()               # non-finite pole gradients are dropped
+    g = dz.clone()
+    g[1, t0, c] = bad
+    z, df, *_ = run(feat, g)
+    d = df.view(B, L, D, 3)
+    _same(z, clean[0], "z"), _same(d[:, :, others], dc[:, :, others], "adjoint, other channels")
+    _same(d[1, t0 + 1:, c], dc[1, t0 + 1:, c], "adjoint, later steps")
+    assert not d[1, :t0, c, 1:].isfinite().any()
+
+
+def test_mr_fir_non_finite_values_stay_in_their_column():
+    """The Toeplitz products take sixteen steps at a time, zero taps included: a non-finite value reaches its own channel, from the
+    start of its sixteen steps to the end of the last sixteen that its taps touch."""
+    torch.manual_seed(12)
+    B, L, D, G, K, t0, c = 1, 500, 64, 4, 128, 203, 9
+    feat, h, b = torch.randn(B, L, 3 * D, device=DEV).to(BF), torch.randn(G, K, device=DEV) / 11, torch.randn(D, device=DEV)
+    clean = ops.hyena_mr_inner(feat, h, b)
+    feat[0, t0, 3 * c + 2] = float("nan")
+    z = ops.hyena_mr_inner(feat, h, b)
+    others = [i for i in range(D) if i != c]
+    lo, hi = t0 // 16 * 16, t0 // 16 * 16 + 16 + 128
+    _same(z[..., others], clean[..., others], "other channels"), _same(z[:, :lo, c], clean[:, :lo, c], "earlier steps")
+    _same(z[:, hi:, c], clean[:, hi:, c], "beyond the taps")
+    assert z[0, t0:t0 + K, c].isnan().all()
+
+
 @pytest.mark.parametrize("D,offset,tiled", [(24, 0, True), (136, 0, True), (20, 0, False), (24, 1, False)])
 @pytest.mark.parametrize("state", [False, True])
 def test_li_c_entries(D, offset, tiled, state):
