@@ -121,7 +121,7 @@ class _Sig:
     sb_li_bwd_chunk = [I, I]
     sb_li_fwd_tiled = [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, P]
     sb_li_bwd_tiled_chunk = []
-    sb_li_bwd_tiled = [P, P, P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, P]
+    sb_li_bwd_tiled = [P, P, P, P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, P]
     sb_li_bwd = [P, P, P, P, P, P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, P]
 
 
@@ -1410,7 +1410,7 @@ class _HyenaLITiled(torch.autograd.Function):
         if sin is not None and sin.data_ptr() == state_in.data_ptr():
             sin = sin.clone()                    # the backward reads it: the caller may go on with its own buffer
         tc = _li_tiled_chunk(B, L, D)
-        modal = _alloc((3 * D, LI_ORDER), dtype=torch.float32, device=dev)
+        modal = _alloc((4 * D, LI_ORDER), dtype=torch.float32, device=dev)
         S = _alloc((B, (L + tc - 1) // tc, D, LI_ORDER), dtype=torch.float32, device=dev)
         sout = _alloc((B, D, O), dtype=torch.float32, device=dev) if want_state else None
         z = _alloc((B, L, D), dtype=bf16, device=dev)
@@ -1433,7 +1433,7 @@ class _HyenaLITiled(torch.autograd.Function):
         tc = int(lib.sb_li_bwd_tiled_chunk())
         NC = (L + tc - 1) // tc
         g = _aligned(gz)
-        S, A = (_alloc((B, NC, D, LI_ORDER), dtype=torch.float32, device=dev) for _ in range(2))
+        S, A, dRp = (_alloc((B, NC, D, LI_ORDER), dtype=torch.float32, device=dev) for _ in range(3))
         dBp = _alloc((B, NC, D), dtype=torch.float32, device=dev)
         df = _alloc_like(fc)
         dso = _f32c(gstate) if (want_state and gstate is not None) else None
@@ -1441,7 +1441,7 @@ class _HyenaLITiled(torch.autograd.Function):
         db = _alloc(D, dtype=torch.float32, device=dev)
         dsi = _alloc((B, D, O), dtype=torch.float32, device=dev) if sin is not None else None
         _check(lib.sb_li_bwd_tiled(fc.data_ptr(), g.data_ptr(), modal.data_ptr(), bf.data_ptr(), _ptr(sin), _ptr(dso), S.data_ptr(),
-                                   A.data_ptr(), dBp.data_ptr(), df.data_ptr(), dR.data_ptr(), dll.data_ptr(), db.data_ptr(),
+                                   A.data_ptr(), dRp.data_ptr(), dBp.data_ptr(), df.data_ptr(), dR.data_ptr(), dll.data_ptr(), db.data_ptr(),
                                    _ptr(dsi), B, L, D, O, _stream()), "li_bwd_tiled")
         _count(4)
         dp = dll.to(pdt) if pdt != torch.float32 else dll.clone()          # gamma and p get gradients of their own storage

@@ -45,6 +45,39 @@ def test_li_scan(B, L, D, O):
     _close(leaves[4].grad, rl[4].grad, 2e-3, "dbias")
 
 
+@pytest.mark.parametrize("state", [False, True])
+def test_li_scan_pole_gradient_precision(state):
+    """Long memories over many chunks, against 64 bits.  In fp32 the poles themselves are rounded: 2^-25 on average, times the length
+    of the memory (1 / 0.0037 = 270 steps for the slowest of these poles), is 8e-6 for that mode and 4e-6 over all of them if the
+    recurrences use them throughout.  The scan uses exp(T log(pole)) between chunks and corrects what is left of the rounding
+    within one: 1.1e-6 by simulation with correctly rounded poles, where the uncorrected sum has 1.5e-6.  The device's expf is
+    documented to 2 ulp, so a pole may be off by twice as much and more: 2.2e-6 and 3.0e-6."""
+    torch.manual_seed(21)
+    B, L, D, O = 1, 4096, 64, 16
+    feat, dz = (torch.randn(B, L, 3 * D, device=DEV) * 0.7).to(BF), torch.randn(B, L, D, device=DEV).to(BF)
+    g, R, p, b = (torch.rand(D, O, device=DEV) * 0.09 + 0.01).log(), 0.1 * torch.randn(D, O, device=DEV) / 4, -torch.ones(D, O, device=DEV), \
+        torch.randn(D, device=DEV)
+    gs = torch.randn(B, D, O, device=DEV) if state else None
+    leaves = [t.clone().requires_grad_() for t in (g, R, p)]
+    z, s = ops.hyena_li_modal(feat, *leaves, b, None, True)
+    (z.float() * dz.float()).sum().backward() if gs is None else torch.autograd.backward([z, s], [dz, gs])
+    l64 = [t.double().requires_grad_() for t in (g, R, p)]
+    x1, x2, v = (feat[..., i::3].double() for i in range(3))
+    ll = -torch.exp(l64[2]) * torch.exp(l64[0])
+    u = (x2 * v).transpose(1, 2)                                       # [B, D, L]
+    t = torch.arange(L, device=DEV, dtype=torch.float64)
+    pw = torch.exp(ll[..., None] * t)                                  # [D, O, L]
+    h = (l64[1][..., None] * pw).sum(1)
+    y = torch.fft.irfft(torch.fft.rfft(u, n=2 * L) * torch.fft.rfft(h, n=2 * L), n=2 * L)[..., :L].transpose(1, 2)
+    loss = (x1 * (y + b.double() * u.transpose(1, 2)) * dz.double()).sum()
+    if state:
+        loss = loss + (torch.einsum("dol,bdl->bdo", pw.flip(-1), u) * gs.double()).sum()
+    loss.backward()
+    for got, want in ((leaves[0], l64[0]), (leaves[2], l64[2])):
+        err = ((got.grad.double() - want.grad).norm() / want.grad.norm()).item()
+        assert err <= 2.25e-6, err
+
+
 @pytest.mark.parametrize("D", [24, 20])                  # the tiled scan, the per-thread one
 @pytest.mark.parametrize("gs,Rs,ps,bs,ss", [("DO", "DO", "D1", "D", None), ("DO", "DO", "11", "D", "1DO"), ("DO", "DO", "", "1", "DO"),
                                             ("1O", "DO", "DO", "", "BD1"), ("D1", "1O", "O", "D", "1"), ("1O", "1O", "1O", "D", "11DO")])
