@@ -8,13 +8,14 @@
 //   2. prefix  : per (b, d, o) a serial pass over the NC chunk states turns them into the state ENTERING each chunk
 //   3. apply   : every chunk reruns from its entering state and writes z
 // so the cost is two streaming reads of the features and one write of z, instead of the size-2L fp32 FFTs the
-// filter's materialised form needs.  The backward pass uses the same structure twice: a forward scan that
-// carries the state s and its sensitivity w = ds/dlam (gradients of R, lam, bias and dx1), and a reverse scan of
-// the adjoint a[t] = R dy[t] + lam a[t+1] (gradients of x2 and v).  `state_in` / `state_out` expose the recurrence
-// state at the shard boundaries, which is all context parallelism needs to hand over.
+// filter's materialised form needs.  The backward pass uses the same structure twice: a forward scan of the state s and its
+// sensitivity w = ds/dlam (gradients of R, lam, bias and dx1), and a reverse scan of the adjoint a[t] = R dy[t] + lam a[t+1]
+// (gradients of x2 and v).  `state_in` / `state_out` expose the recurrence state at the shard boundaries, which is all context
+// parallelism needs to hand over.  O is padded to 16 (lam = 0, R = 0 beyond the real order).
 //
-// One thread owns one channel (its O states live in registers); a warp reads 32 channels x 3 features = 192
-// contiguous bytes per time step.  O is padded to 16 (lam = 0, R = 0 beyond the real order).
+// Two sets of kernels: first the per-thread ones (any D, any alignment; also the context-parallel scan at the end of the file), in
+// which one thread owns one channel, its O states in registers, and a warp reads 32 channels x 3 features = 192 contiguous bytes
+// per time step; then the tiled ones (D % 8 == 0, 16-byte aligned tensors), which are the ones that normally run.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -341,8 +342,8 @@ li_bwd_apply_rev_kernel(const bf16* __restrict__ feat, const bf16* __restrict__ 
 // between chunks: the prefix pass carries two arrays instead of three.
 //
 // Measured at B = 1, L = 8192, D = 4096 on a B200 (us; in brackets the one-channel-per-thread kernels these replace):
-// forward 43 + 10 + 81 (55 + 29 + 95), backward 80 + 54 + 272 + 18 (143 + 156 + 319 and about ten tensor operations that
-// prepared the filter and summed the partials).  Forward and backward with their host side: 848 -> 567.  The recurrences
+// forward 43 + 10 + 81 (55 + 29 + 95), backward 80 + 36 + 272 + 18 (143 + 156 + 319 and about ten tensor operations that
+// prepared the filter and summed the partials).  Forward and backward with their host side: 849 -> 552.  The recurrences
 // need 48 FMA per value forward and 144 backward, 54 and 163 us at the 30 TFMA/s that packed and plain FMA both reach here
 // (the packed form only halves the issue slots), so the sweeps sit between that bound and the copy time of their data.
 typedef unsigned long long f2;           // two packed fp32 values

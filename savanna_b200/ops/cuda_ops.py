@@ -1377,7 +1377,15 @@ def _li_chunk(B: int, L: int, D: int) -> int:
 
 def _li_tiled_chunk(B: int, L: int, D: int) -> int:
     """As `_li_chunk` for the tiled kernels, whose blocks have two warps: small problems go down to chunks of 32 steps to
-    fill the chip (B = 2, L = 1237, D = 1024 forward: 69 us with 128-step chunks of the former kernels, 48 us)."""
+    fill the chip.  Forward, us, by chunk length (* the one chosen here):
+        B, L, D         32     64    128    256    512   1024
+        1, 200, 4096   *28     30     36     46
+        2, 1237, 1024  *38     38     40     52     87    153
+        1, 2048, 4096  *69     58     58     56     87    153
+        1, 8192, 1024  *77     62     58     58     87    153
+        1, 8192, 4096  222    165   *148    152    142    163
+        1, 32768, 4096 849    601    484    443   *427    472
+    The 2048 blocks are those of the per-thread kernels; in between, 512 blocks would choose better."""
     if LI_CHUNK_OVERRIDE:
         return int(LI_CHUNK_OVERRIDE)
     tc = 1024
