@@ -73,6 +73,7 @@ class _Watch:
 
     def __init__(self):
         self.seen = []                           # (dictionary or list, key, value)
+        self.computed = False                    # something came out of a property: it can be another one at any time
 
     def __call__(self, obj, name):
         d = obj.__dict__
@@ -80,9 +81,12 @@ class _Watch:
             if c is not None and name in c:
                 self.seen.append((c, name, c[name]))
                 return c[name]
-        raise AttributeError(f"{type(obj).__name__} has no attribute {name!r} of its own")
+        self.computed = True
+        return getattr(obj, name)
 
     def same(self) -> bool:
+        if self.computed:
+            return False
         try:
             for c, k, v in self.seen:
                 if c[k] is not v:
@@ -585,6 +589,7 @@ class CachedDecoder:
                 self.pos += 1
                 return logits
             self._hand_back()
+            self._resume = False                 # not at every token again
         dtype = cfg.params_dtype
         pos = torch.tensor([self.pos], device=token.device)
         was_training = model.training

@@ -116,11 +116,14 @@ def test_parameters_changed_between_steps(which, over, moved, monkeypatch):
     assert (slow.step(toks[:, 0]) - before).norm() > 0.1 * before.norm()          # the change reached the logits
 
 
-def test_filters_stored_in_bf16(monkeypatch):
+@pytest.mark.parametrize("bf16", ["", "short_conv", "short_conv filter conv_bias", ".R .h", "conv_bias gamma"],
+                         ids=lambda s: s.replace(" ", "+") or "none")
+def test_types_of_stored_filters(bf16, monkeypatch):
+    """Filter parameters named here are bf16, the others fp32: each mixture has its kernel."""
     model = _model()
     for n, p in model.named_parameters():
         if _is_filter(n):
-            p.data = p.data.bfloat16()
+            p.data = p.data.bfloat16() if any(k in n for k in bf16.split()) else p.data.float()
     toks = _toks(model, 1, 30)
     fast, slow = CachedDecoder(model), _slow(model, toks[:, :25], monkeypatch)
     fast.prefill(toks[:, :25])
@@ -233,3 +236,51 @@ def test_unusable_weights_are_refused(monkeypatch):
         with pytest.raises(RuntimeError):
             dec.step(toks[:, 30].cpu())
     assert fast._fused is None
+
+
+def test_weight_behind_a_property(monkeypatch):
+    """A projection whose weight is computed when it is read, as adapters do it: read again in every step."""
+    class Adapted(torch.nn.Module):
+        def __init__(self, base):
+            super().__init__()
+            self.base, self.factor = base, 1.0
+            self.bias = base.bias
+
+        @property
+        def weight(self):
+            return self.base.weight * self.factor
+
+        def forward(self, x, *a):
+            return self.base(x * self.factor, *a)
+
+        def forward_normed(self, x, norm):
+            y, b, r = self.base.forward_normed(x, norm)
+            return y * self.factor, b, r
+    model = _model()
+    mixer = model.blocks()[1].mixer
+    mixer.dense_projection = Adapted(mixer.dense_projection)
+    toks = _toks(model, 2, 30)
+    fast, slow = CachedDecoder(model), _slow(model, toks[:, :20], monkeypatch)
+    fast.prefill(toks[:, :20])
+    assert fast._fused is not None
+    _agree(fast, slow, toks[:, 20:23])
+    mixer.dense_projection.factor = 3.0
+    _agree(fast, slow, toks[:, 23:27])
+    assert fast._fused is not None
+
+
+def test_embedding_of_another_type(monkeypatch):
+    """What the embedding returns is looked at too: fp32 activations go operator by operator."""
+    model = _model()
+    toks = _toks(model, 2, 30)
+    fast, slow = CachedDecoder(model), _slow(model, toks[:, :20], monkeypatch)
+    fast.prefill(toks[:, :20])
+    h = model.embedding.register_forward_hook(lambda m, a, out: out.float())
+    for i in (20, 21):
+        a, b = fast.step(toks[:, i]), slow.step(toks[:, i])
+        assert torch.equal(a, b) or (a - b).norm() <= 2.2e-2 * b.norm()
+        assert fast._fused is None and not fast._resume
+    h.remove()
+    fast.states = fast.states
+    _agree(fast, slow, toks[:, 22:26])
+    assert fast._fused is not None
