@@ -923,13 +923,13 @@ extern "C" int sb_attn_fwd(const void* q, const void* k, const void* v, void* ou
   FwdParams p{reinterpret_cast<__nv_bfloat16*>(out), lse, o_str[0], o_str[1], o_str[2], B, H, Lq, Lk, causal,
               scale * 1.4426950408889634f, scale, status, 0, g_pingpong};
   const int qblocks = (Lq + 2 * BQ - 1) / (2 * BQ);
-  // Causal rows differ in length.  While the keys and values of all heads together sit in the L2 cache, the longest blocks of
-  // all heads go first, which packs the last wave better; far beyond it the blocks of one head stay together, so that its keys
+  // Causal rows differ in length.  While the keys and values of all heads together fit the L2 cache, the longest blocks of
+  // all heads go first, which packs the last wave better; beyond it the blocks of one head stay together, so that its keys
   // are read from memory once.  Longest first against head by head, us with a cold L2: 21 MB (B = 2, L = 1333, 16 heads) 37 / 50,
   // 32 MB (L = 4096, 16 heads) 84 / 125, 64 MB (L = 8192, 16 heads) 279 / 350, 128 MB (L = 8192, 32 heads) 539 / 610, 256 MB
-  // (L = 32768, 16 heads) 4010 / 4014, 512 MB (L = 32768, 32 heads) 9090 / 8760.  The line is a quarter of the cache, well on the
-  // safe side of where the two meet.
-  p.heads_fast = causal && (long long)B * H * Lk * HD * 4 <= (32LL << 20) && qblocks <= 65535 && B <= 65535;
+  // (L = 32768, 16 heads) 4010 / 4014, 512 MB (L = 32768, 32 heads) 9090 / 8760.  The line is the size of the cache: its
+  // measured gain at 128 MB, and nothing to gain at 256 MB.
+  p.heads_fast = causal && (long long)B * H * Lk * HD * 4 <= (128LL << 20) && qblocks <= 65535 && B <= 65535;
   const dim3 grid = p.heads_fast ? dim3(H, B, qblocks) : dim3(qblocks, H, B);
   if (g_fwd_p_tmem) attn_fwd_kernel<true><<<grid, FWD_THREADS, FWD_SMEM, stream>>>(tq, tk, tv, p);
   else attn_fwd_kernel<false><<<grid, FWD_THREADS, FWD_SMEM, stream>>>(tq, tk, tv, p);
