@@ -1376,20 +1376,21 @@ def _li_chunk(B: int, L: int, D: int) -> int:
 
 
 def _li_tiled_chunk(B: int, L: int, D: int) -> int:
-    """As `_li_chunk` for the tiled kernels, whose blocks have two warps: small problems go down to chunks of 32 steps to
-    fill the chip.  Forward, us, by chunk length (* the one chosen here):
+    """Chunk length of the tiled forward: the longest of 32 .. 512 steps that leaves 512 blocks of 128 channels (two warps
+    each: seven warps per SM when they are dealt out evenly).  Longer chunks mean a shorter serial pass over the chunk states,
+    more blocks hide the latency of a chunk's own recurrence, and beyond 512 steps that recurrence is what the last wave waits
+    for.  Forward, us, by chunk length (* the one chosen here, + the one that 2048 blocks and up to 1024 steps chose):
         B, L, D         32     64    128    256    512   1024
-        1, 200, 4096   *28     30     36     46
-        2, 1237, 1024  *38     38     40     52     87    153
-        1, 2048, 4096  *69     58     58     56     87    153
-        1, 8192, 1024  *77     62     58     58     87    153
-        1, 8192, 4096  222    165   *148    152    142    163
-        1, 32768, 4096 849    601    484    443   *427    472
-    The 2048 blocks are those of the per-thread kernels; in between, 512 blocks would choose better."""
+        1, 200, 4096  *+28     30     36     46
+        2, 1237, 1024 *+38     38     40     52     87    153
+        1, 2048, 4096  +69     58    *58     56     87    153
+        1, 8192, 1024  +77     62    *58     58     87    153
+        1, 8192, 4096  222    165   +148    152   *142    163
+        1, 32768, 4096 849    601    484    443  *+427    472"""
     if LI_CHUNK_OVERRIDE:
         return int(LI_CHUNK_OVERRIDE)
-    tc = 1024
-    while tc > 32 and B * ((D + 127) // 128) * ((L + tc - 1) // tc) < 2048:
+    tc = 512
+    while tc > 32 and B * ((D + 127) // 128) * ((L + tc - 1) // tc) < 512:
         tc //= 2
     return tc
 
