@@ -1,7 +1,8 @@
 // Short causal depthwise convolutions, channel-last bf16, fp32 math:
 //   dwconv_*   : y[b,t,c] = sum_j w[c,j] x[b, t-(K-1)+j, c]           (featuriser, K = short_conv_L)
 //   se_*       : z = x1 * conv_K(x2 * v) on interleaved (x1,x2,v) features (Hyena-SE and hyena_mlp)
-// A thread owns CH consecutive channels and walks TL consecutive time steps with the filter window in
+// Three sets of kernels: streaming (conv_stream.cuh), tiled and per thread; the rule that chooses stands before the entry points.
+// In the per-thread ones a thread owns CH consecutive channels and walks TL consecutive time steps with the filter window in
 // registers, so every input element is read once (plus a K-1 overlap per run).  Optional `halo` tensors
 // hold the K-1 rows preceding the sequence (context-parallel shards); their gradients are produced too.
 // Filter-gradient partial sums stay in registers over the run and are flushed with fp32 atomics.
@@ -9,6 +10,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "conv_stream.cuh"
 #include "device_info.h"
 #include "halo_src.cuh"
 
@@ -178,7 +180,7 @@ constexpr int DW_CT_F = 64, DW_SEG_F = 32, DW_NSEG_F = 4;
 // asynchronous 16-byte copies, a thread then produces DW_SEG steps of two adjacent channels from shared memory.
 template <int K>
 __global__ void __launch_bounds__(DW_CT_F / 2 * DW_NSEG_F)
-dwconv_fwd_tiled_kernel(const bf16* __restrict__ x, const HaloSrc halo, const float* __restrict__ w,
+dwconv_fwd_tiled_kernel(const bf16* __restrict__ x, const HaloSrc halo, const CsTaps w, float* __restrict__ wf,
                         bf16* __restrict__ y, int L, int C) {
   constexpr int H = K - 1, T = DW_SEG_F * DW_NSEG_F, ROWS = T + H, NT = DW_CT_F / 2 * DW_NSEG_F, CHK = DW_CT_F / 8;
   __shared__ __align__(16) bf16 xS[ROWS][DW_CT_F];          // x_ext of times t0-H .. t0+T-1
@@ -199,7 +201,13 @@ dwconv_fwd_tiled_kernel(const bf16* __restrict__ x, const HaloSrc halo, const fl
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int j = 0; j < K; ++j) wr[i][j] = w[(size_t)(c0 + 2 * cp + i) * K + j];
+    for (int j = 0; j < K; ++j) wr[i][j] = cs_tap(w, (size_t)(c0 + 2 * cp + i) * K + j);
+  if (wf && blockIdx.y == 0 && b == 0 && seg == 0) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < K; ++j) wf[(size_t)(c0 + 2 * cp + i) * K + j] = wr[i][j];
+  }
   cp_async_wait_all();
   __syncthreads();
   auto ld2 = [&](int row, float (&f)[2]) {
@@ -467,7 +475,7 @@ constexpr int SE_CT = 32, SE_SEG = 32, SE_NSEG = 4, SE_T = SE_SEG * SE_NSEG;
 // 16-byte chunks.
 template <int K>
 __global__ void __launch_bounds__(SE_CT * SE_NSEG)
-se_fwd_tiled_kernel(const bf16* __restrict__ feat, const HaloSrc halo, const float* __restrict__ w,
+se_fwd_tiled_kernel(const bf16* __restrict__ feat, const HaloSrc halo, const CsTaps w, float* __restrict__ wf,
                     bf16* __restrict__ z, int L, int D, int dg, int pregate, int postgate) {
   constexpr int H = K - 1, ROWS = SE_T + H, NT = SE_CT * SE_NSEG, FCH = 3 * SE_CT / 8, ZCH = SE_CT / 8;
   __shared__ __align__(16) bf16 fS[ROWS][3 * SE_CT];        // features of times t0-H .. t0+SE_T-1
@@ -487,7 +495,11 @@ se_fwd_tiled_kernel(const bf16* __restrict__ feat, const HaloSrc halo, const flo
   const int c = tid % SE_CT, seg = tid / SE_CT, r0 = seg * SE_SEG;
   float wr[K], win[K];
 #pragma unroll
-  for (int j = 0; j < K; ++j) wr[j] = w[(size_t)((c0 + c) / dg) * K + j];
+  for (int j = 0; j < K; ++j) wr[j] = cs_tap(w, (size_t)((c0 + c) / dg) * K + j);
+  if (wf && blockIdx.y == 0 && b == 0 && seg == 0 && (c0 + c) % dg == 0) {
+#pragma unroll
+    for (int j = 0; j < K; ++j) wf[(size_t)((c0 + c) / dg) * K + j] = wr[j];
+  }
   cp_async_wait_all();
   __syncthreads();
   auto u_row = [&](int row) -> float {
@@ -638,8 +650,24 @@ se_bwd_tiled_kernel(const bf16* __restrict__ feat, const HaloSrc halo, const int
   }
 }
 
-static int g_se_bwd_tiled = 1;
-static int g_conv_fwd_tiled = 1;   // depthwise-conv forward through shared-memory tiles
+// Which kernels run (16-byte aligned tensors; the switches below pick the run-per-thread ones for A/B measurements):
+//   streaming   channels % 8 == 0 and at least CS_FULL rows of 128 channels per SM: one wave of runs keeps every SM busy
+//   tiled       fewer rows and whole tiles of channels: a block's 128 steps in parallel beat a warp's run (its edge rows and the
+//               latency of its first copies are the run's whole time)
+//   per thread  the rest
+// us, streaming / tiled, taps 3 (featuriser forward, backward) and 7 (Hyena-SE forward, backward):
+//   B, L, D             rows of 128 channels per SM (featuriser, Hyena-SE)
+//   1, 8192, 4096       5314, 1771     69 /  75     97 / 128     49 /  62     88 / 129
+//   1, 3000, 2048        973,  324     17 /  20     25 /  32     14 /  17     23 /  31
+//   2, 1237, 1024        401,  134    8.4 / 10.4    15 /  19   10.4 / 8.4     22 /  17
+//   3,  777,  512        189,   63    6.4 /  6.8    11 /  11    8.3 / 6.4     13 /  11     (4 taps)
+//   1,   64,  256          3,    1    6.3 /  5.3   6.5 / 6.3    8.4 / 4.7     13 / 8.4
+static int g_bwd_fast = 1;
+static int g_fwd_fast = 1;
+constexpr int CS_FULL = 200;
+static bool cs_full(int B, int L, int channels) {
+  return (long long)B * L * ((channels + 127) / 128) >= (long long)CS_FULL * sb::num_sms();
+}
 
 static inline int pick_tl(int L, int B, int cvecs) {
   // enough CTAs to fill 148 SMs a few times over, runs long enough to amortise the K-1 overlap
@@ -664,17 +692,112 @@ using namespace sb;
     default: return -7;                     \
   }
 
+// wf: when not null receives the taps in fp32 ([C, K]); w_bf16: w points at bf16 taps.
+static int dwconv_fwd_fast(const void* x, const HaloSrc& halo, const void* w, int w_bf16, float* wf, void* y, int B, int L, int C,
+                             int K, cudaStream_t st) {
+  const CsTaps taps{w_bf16 ? nullptr : (const float*)w, w_bf16 ? (const bf16*)w : nullptr};
+  if (C % DW_CT_F == 0 && !cs_full(B, L, C)) {
+    constexpr int T = DW_SEG_F * DW_NSEG_F;
+    const dim3 grid(C / DW_CT_F, (L + T - 1) / T, B);
+    K_SWITCH(K, (dwconv_fwd_tiled_kernel<KK><<<grid, DW_CT_F / 2 * DW_NSEG_F, 0, st>>>((const bf16*)x, halo, taps, wf, (bf16*)y, L, C)));
+    return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  }
+  int nchunk;
+  const int cols = (C + 255) / 256, R = cs_rows(B, L, cols, 9, nchunk);
+  const dim3 grid(cols, (nchunk * B + CS_WPB - 1) / CS_WPB);
+  K_SWITCH(K, (dwconv_fwd_stream_kernel<KK><<<grid, 32 * CS_WPB, CS_WPB * CS_RING<KK> * 512, st>>>((const bf16*)x, halo, taps, wf, (bf16*)y,
+                                                                                               B, L, C, R, nchunk)));
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+static int dwconv_bwd_fast(const void* x, const HaloSrc& halo, int has_halo, const float* w, const void* dy, void* dx, void* dhalo,
+                             float* dw, int B, int L, int C, int K, int ahead_mode, const HaloSrc& ahead, cudaStream_t st) {
+  if (C % DW_CT == 0 && !cs_full(B, L, C)) {
+    const dim3 grid(C / DW_CT, (L + (ahead_mode ? 0 : K - 1) + DW_T - 1) / DW_T, B);
+    K_SWITCH(K, (dwconv_bwd_tiled_kernel<KK><<<grid, DW_CT / 2 * DW_NSEG, 0, st>>>((const bf16*)x, halo, w, (const bf16*)dy, (bf16*)dx,
+                                                                                 (bf16*)dhalo, dw, L, C, ahead_mode, ahead)));
+    return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  }
+  int nchunk;
+  const int cols = (C + 127) / 128, R = cs_rows(B, L + (has_halo && !ahead_mode ? K - 1 : 0), cols, 2, nchunk);
+  const dim3 grid(cols, (nchunk * B + CS_WPB - 1) / CS_WPB);
+  K_SWITCH(K, (dwconv_bwd_stream_kernel<KK><<<grid, 32 * CS_WPB, CS_WPB * CS_RING<KK> * 512, st>>>(
+                  (const bf16*)x, halo, has_halo, w, (const bf16*)dy, (bf16*)dx, (bf16*)dhalo, dw, B, L, C, R, nchunk, ahead_mode, ahead)));
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+template <int K, bool SHARED>
+static int se_fwd_launch(dim3 grid, const void* feat, const HaloSrc& halo, const CsTaps& taps, float* wf, int G, void* z, int B, int L,
+                         int D, int R, int nchunk, int pre, int post, cudaStream_t st) {
+  constexpr int SMEM = CS_WPB * CS_RING<K> * CE_FROW;
+  if (SMEM > 49152 && cudaFuncSetAttribute(se_fwd_stream_kernel<K, SHARED>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
+    return -2;
+  se_fwd_stream_kernel<K, SHARED><<<grid, 32 * CS_WPB, SMEM, st>>>((const bf16*)feat, halo, taps, wf, G, (bf16*)z, B, L,
+                                                                                    D, D / G, R, nchunk, pre, post);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+static int se_fwd_fast(const void* feat, const HaloSrc& halo, const void* w, int w_bf16, float* wf, void* z, int B, int L, int D, int G,
+                         int K, int pre, int post, cudaStream_t st) {
+  const CsTaps taps{w_bf16 ? nullptr : (const float*)w, w_bf16 ? (const bf16*)w : nullptr};
+  if (D % SE_CT == 0 && !cs_full(B, L, D)) {
+    const dim3 grid(D / SE_CT, (L + SE_T - 1) / SE_T, B);
+    K_SWITCH(K, (se_fwd_tiled_kernel<KK><<<grid, SE_CT * SE_NSEG, 0, st>>>((const bf16*)feat, halo, taps, wf, (bf16*)z, L, D, D / G, pre,
+                                                                         post)));
+    return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  }
+  int nchunk, rc = -2;
+  const int cols = (D + 127) / 128, R = cs_rows(B, L, cols, 3, nchunk);
+  const dim3 grid(cols, (nchunk * B + CS_WPB - 1) / CS_WPB);
+  const bool shared = (D / G) % 4 == 0;                  // the four channels of a lane lie in one filter group
+  K_SWITCH(K, (rc = shared ? se_fwd_launch<KK, true>(grid, feat, halo, taps, wf, G, z, B, L, D, R, nchunk, pre, post, st)
+                           : se_fwd_launch<KK, false>(grid, feat, halo, taps, wf, G, z, B, L, D, R, nchunk, pre, post, st)));
+  return rc;
+}
+
+template <int K, bool SHARED>
+static int se_bwd_launch(dim3 grid, const void* feat, const HaloSrc& halo, int has_halo, const float* w, const void* dz, void* dfeat,
+                         void* dhalo, float* dw, int B, int L, int D, int G, int R, int nchunk, int pre, int post, int ahead_mode,
+                         const HaloSrc& af, const HaloSrc& ag, cudaStream_t st) {
+  constexpr int SMEM = CS_WPB * 2 * CE_U<K> * CE_BROW;
+  if (cudaFuncSetAttribute(se_bwd_stream_kernel<K, SHARED>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess) return -2;
+  se_bwd_stream_kernel<K, SHARED><<<grid, 32 * CS_WPB, SMEM, st>>>((const bf16*)feat, halo, has_halo, w, (const bf16*)dz, (bf16*)dfeat,
+                                                                   (bf16*)dhalo, dw, B, L, D, D / G, R, nchunk, pre, post, ahead_mode,
+                                                                   af, ag);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+static int se_bwd_fast(const void* feat, const HaloSrc& halo, int has_halo, const float* w, const void* dz, void* dfeat, void* dhalo,
+                         float* dw, int B, int L, int D, int G, int K, int pre, int post, int ahead_mode, const HaloSrc& af,
+                         const HaloSrc& ag, cudaStream_t st) {
+  if (D % SE_CT == 0 && !cs_full(B, L, D)) {
+    const dim3 grid(D / SE_CT, (L + (has_halo && !ahead_mode ? K - 1 : 0) + SE_T - 1) / SE_T, B);
+    K_SWITCH(K, (se_bwd_tiled_kernel<KK><<<grid, SE_CT * SE_NSEG, 0, st>>>((const bf16*)feat, halo, has_halo, w, (const bf16*)dz,
+                                                                         (bf16*)dfeat, (bf16*)dhalo, dw, L, D, D / G, pre, post,
+                                                                         ahead_mode, af, ag)));
+    return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  }
+  int nchunk, rc = -2;
+  const int cols = (D + 127) / 128, R = cs_rows(B, L + (has_halo && !ahead_mode ? K - 1 : 0), cols, 2, nchunk);
+  const dim3 grid(cols, (nchunk * B + CS_WPB - 1) / CS_WPB);
+  const bool shared = (D / G) % 4 == 0;
+  K_SWITCH(K, (rc = shared ? se_bwd_launch<KK, true>(grid, feat, halo, has_halo, w, dz, dfeat, dhalo, dw, B, L, D, G, R, nchunk, pre, post,
+                                                     ahead_mode, af, ag, st)
+                           : se_bwd_launch<KK, false>(grid, feat, halo, has_halo, w, dz, dfeat, dhalo, dw, B, L, D, G, R, nchunk, pre,
+                                                      post, ahead_mode, af, ag, st)));
+  return rc;
+}
+
+// As sb_dwconv_fwd with the taps as the parameter holds them (w_bf16: bf16, else fp32); wf (or null) receives them in fp32.
+extern "C" int sb_dwconv_fwd_taps(const void* x, const void* halo, const void* w, int w_bf16, float* wf, void* y, int B, int L, int C,
+                                  int K, cudaStream_t st) {
+  if (C % 8) return -1;
+  if (B * L == 0) return 0;
+  return dwconv_fwd_fast(x, halo_local(halo), w, w_bf16, wf, y, B, L, C, K, st);
+}
 extern "C" int sb_dwconv_fwd(const void* x, const void* halo, const float* w, void* y, int B, int L, int C, int K,
                              cudaStream_t st) {
   if (C % 8) return -1;
   if (B * L == 0) return 0;
-  if (g_conv_fwd_tiled && C % DW_CT_F == 0) {
-    constexpr int T = DW_SEG_F * DW_NSEG_F;
-    dim3 grid(C / DW_CT_F, (L + T - 1) / T, B);
-    K_SWITCH(K, (dwconv_fwd_tiled_kernel<KK><<<grid, DW_CT_F / 2 * DW_NSEG_F, 0, st>>>((const bf16*)x, halo_local(halo), w,
-                                                                                     (bf16*)y, L, C)));
-    return cudaGetLastError() == cudaSuccess ? 0 : -2;
-  }
+  if (g_fwd_fast) return dwconv_fwd_fast(x, halo_local(halo), w, 0, nullptr, y, B, L, C, K, st);
   const int cvecs = C / 8, threads = 128, tl = pick_tl(L, B, cvecs);
   dim3 grid((cvecs + threads - 1) / threads, (L + tl - 1) / tl, B);
   K_SWITCH(K, (dwconv_fwd_kernel<KK, 8><<<grid, threads, 0, st>>>((const bf16*)x, (const bf16*)halo, w, (bf16*)y, L, C, tl)));
@@ -685,13 +808,8 @@ extern "C" int sb_dwconv_bwd(const void* x, const void* halo, const float* w, co
                              float* dw, int B, int L, int C, int K, cudaStream_t st) {
   if (C % 4) return -1;
   if (B * L == 0) return 0;
-  if (g_se_bwd_tiled && C % DW_CT == 0) {
-    dim3 grid(C / DW_CT, (L + K - 1 + DW_T - 1) / DW_T, B);
-    K_SWITCH(K, (dwconv_bwd_tiled_kernel<KK><<<grid, DW_CT / 2 * DW_NSEG, 0, st>>>((const bf16*)x, halo_local(halo), w,
-                                                                                 (const bf16*)dy, (bf16*)dx, (bf16*)dhalo, dw, L, C,
-                                                                                 0, halo_local(nullptr))));
-    return cudaGetLastError() == cudaSuccess ? 0 : -2;
-  }
+  if (g_bwd_fast && C % 8 == 0)
+    return dwconv_bwd_fast(x, halo_local(halo), halo ? 1 : 0, w, dy, dx, dhalo, dw, B, L, C, K, 0, halo_local(nullptr), st);
   const int cvecs = C / 4, threads = 128, tl = pick_tl(L, B, cvecs);
   dim3 grid((cvecs + threads - 1) / threads, (L + tl - 1) / tl, B);
   K_SWITCH(K, (dwconv_bwd_kernel<KK, 4><<<grid, threads, 0, st>>>((const bf16*)x, (const bf16*)halo, w, (const bf16*)dy,
@@ -699,20 +817,22 @@ extern "C" int sb_dwconv_bwd(const void* x, const void* halo, const float* w, co
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-// 1: Hyena-SE and depthwise-conv backward through shared-memory tiles; 0: one run per thread straight from global memory.
-extern "C" int sb_se_set_bwd_variant(int tiled) { sb::g_se_bwd_tiled = tiled ? 1 : 0; return 0; }
-extern "C" int sb_conv_set_fwd_variant(int tiled) { sb::g_conv_fwd_tiled = tiled ? 1 : 0; return 0; }
+// 1: streaming or tiled kernels by size; 0: one run per thread straight from global memory (A/B measurements).
+extern "C" int sb_se_set_bwd_variant(int fast) { sb::g_bwd_fast = fast ? 1 : 0; return 0; }
+extern "C" int sb_conv_set_fwd_variant(int fast) { sb::g_fwd_fast = fast ? 1 : 0; return 0; }
 
+// As sb_se_fwd with the taps as the parameter holds them (w_bf16: bf16, else fp32); wf (or null) receives them in fp32.
+extern "C" int sb_se_fwd_taps(const void* feat, const void* halo, const void* w, int w_bf16, float* wf, void* z, int B, int L, int D,
+                              int G, int K, int pregate, int postgate, cudaStream_t st) {
+  if ((D % 8) || (D % G)) return -1;
+  if (B * L == 0) return 0;
+  return se_fwd_fast(feat, halo_local(halo), w, w_bf16, wf, z, B, L, D, G, K, pregate, postgate, st);
+}
 extern "C" int sb_se_fwd(const void* feat, const void* halo, const float* w, void* z, int B, int L, int D, int G, int K,
                          int pregate, int postgate, cudaStream_t st) {
   if ((D % 8) || (D % G)) return -1;
   if (B * L == 0) return 0;
-  if (g_conv_fwd_tiled && D % SE_CT == 0) {
-    dim3 grid(D / SE_CT, (L + SE_T - 1) / SE_T, B);
-    K_SWITCH(K, (se_fwd_tiled_kernel<KK><<<grid, SE_CT * SE_NSEG, 0, st>>>((const bf16*)feat, halo_local(halo), w, (bf16*)z, L, D,
-                                                                         D / G, pregate, postgate)));
-    return cudaGetLastError() == cudaSuccess ? 0 : -2;
-  }
+  if (g_fwd_fast) return se_fwd_fast(feat, halo_local(halo), w, 0, nullptr, z, B, L, D, G, K, pregate, postgate, st);
   const int cvecs = D / 8, threads = 128, tl = pick_tl(L, B, cvecs);
   dim3 grid((cvecs + threads - 1) / threads, (L + tl - 1) / tl, B);
   K_SWITCH(K, (se_fwd_kernel<KK, 8><<<grid, threads, 0, st>>>((const bf16*)feat, (const bf16*)halo, w, (bf16*)z, L, D, D / G, tl,
@@ -724,14 +844,9 @@ extern "C" int sb_se_bwd(const void* feat, const void* halo, const float* w, con
                          float* dw, int B, int L, int D, int G, int K, int pregate, int postgate, cudaStream_t st) {
   if ((D % 4) || (D % G)) return -1;
   if (B * L == 0) return 0;
-  if (g_se_bwd_tiled && D % SE_CT == 0) {
-    const int H = K - 1, steps = L + (halo ? H : 0);
-    dim3 grid(D / SE_CT, (steps + SE_T - 1) / SE_T, B);
-    K_SWITCH(K, (se_bwd_tiled_kernel<KK><<<grid, SE_CT * SE_NSEG, 0, st>>>((const bf16*)feat, halo_local(halo), halo ? 1 : 0, w,
-                                                                         (const bf16*)dz, (bf16*)dfeat, (bf16*)dhalo, dw, L, D, D / G,
-                                                                         pregate, postgate, 0, halo_local(nullptr), halo_local(nullptr))));
-    return cudaGetLastError() == cudaSuccess ? 0 : -2;
-  }
+  if (g_bwd_fast && D % 8 == 0)
+    return se_bwd_fast(feat, halo_local(halo), halo ? 1 : 0, w, dz, dfeat, dhalo, dw, B, L, D, G, K, pregate, postgate, 0,
+                         halo_local(nullptr), halo_local(nullptr), st);
   const int cvecs = D / 4, threads = 128, tl = pick_tl(L, B, cvecs);
   dim3 grid((cvecs + threads - 1) / threads, (L + tl - 1) / tl, B);
   K_SWITCH(K, (se_bwd_kernel<KK, 4><<<grid, threads, 0, st>>>((const bf16*)feat, (const bf16*)halo, w, (const bf16*)dz,
@@ -741,48 +856,36 @@ extern "C" int sb_se_bwd(const void* feat, const void* halo, const float* w, con
 
 
 // ------------------------------------------------------------------------------------ context-parallel entry points
-// The same tiled kernels with the edge rows read in place from the neighbours' staged chunk edges (peer memory, see
+// The same streaming / tiled kernels with the edge rows read in place from the neighbours' staged chunk edges (peer memory, see
 // halo_src.cuh): x / feat are [2B, L, .] (two zigzag chunks per sequence as consecutive batch rows), `before` describes
 // the staged tails (rows preceding each chunk), `ahead*` the staged heads of the tensors whose look-ahead the backward
-// needs.  No halo tensor and no halo gradient exist on this path.  Return -9 when the shape has no tiled kernel.
+// needs.  No halo tensor and no halo gradient exist on this path.  Return -9 when the channel count is not a multiple of 64
+// (featuriser) or 32 (Hyena-SE): the callers then pull the halos with separate kernels.
 extern "C" int sb_dwconv_fwd_cp(const void* x, const HaloSrc* before, const float* w, void* y, int B2, int L, int C, int K,
                                 cudaStream_t st) {
-  if (C % DW_CT_F || !before) return -9;
+  if (C % 64 || !before) return -9;
   if (B2 * L == 0) return 0;
-  constexpr int T = DW_SEG_F * DW_NSEG_F;
-  dim3 grid(C / DW_CT_F, (L + T - 1) / T, B2);
-  K_SWITCH(K, (dwconv_fwd_tiled_kernel<KK><<<grid, DW_CT_F / 2 * DW_NSEG_F, 0, st>>>((const bf16*)x, *before, w, (bf16*)y, L, C)));
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return dwconv_fwd_fast(x, *before, w, 0, nullptr, y, B2, L, C, K, st);
 }
 
 extern "C" int sb_dwconv_bwd_cp(const void* x, const HaloSrc* before, const float* w, const void* dy, const HaloSrc* ahead_dy,
                                 void* dx, float* dw, int B2, int L, int C, int K, cudaStream_t st) {
-  if (C % DW_CT || !before || !ahead_dy) return -9;
+  if (C % 64 || !before || !ahead_dy) return -9;
   if (B2 * L == 0) return 0;
-  dim3 grid(C / DW_CT, (L + DW_T - 1) / DW_T, B2);
-  K_SWITCH(K, (dwconv_bwd_tiled_kernel<KK><<<grid, DW_CT / 2 * DW_NSEG, 0, st>>>((const bf16*)x, *before, w, (const bf16*)dy,
-                                                                               (bf16*)dx, nullptr, dw, L, C, 1, *ahead_dy)));
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return dwconv_bwd_fast(x, *before, 1, w, dy, dx, nullptr, dw, B2, L, C, K, 1, *ahead_dy, st);
 }
 
 extern "C" int sb_se_fwd_cp(const void* feat, const HaloSrc* before, const float* w, void* z, int B2, int L, int D, int G, int K,
                             int pregate, int postgate, cudaStream_t st) {
-  if ((D % SE_CT) || (D % G) || !before) return -9;
+  if ((D % 32) || (D % G) || !before) return -9;
   if (B2 * L == 0) return 0;
-  dim3 grid(D / SE_CT, (L + SE_T - 1) / SE_T, B2);
-  K_SWITCH(K, (se_fwd_tiled_kernel<KK><<<grid, SE_CT * SE_NSEG, 0, st>>>((const bf16*)feat, *before, w, (bf16*)z, L, D, D / G,
-                                                                       pregate, postgate)));
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return se_fwd_fast(feat, *before, w, 0, nullptr, z, B2, L, D, G, K, pregate, postgate, st);
 }
 
 extern "C" int sb_se_bwd_cp(const void* feat, const HaloSrc* before, const float* w, const void* dz, const HaloSrc* ahead_feat,
                             const HaloSrc* ahead_dz, void* dfeat, float* dw, int B2, int L, int D, int G, int K, int pregate,
                             int postgate, cudaStream_t st) {
-  if ((D % SE_CT) || (D % G) || !before || !ahead_feat || !ahead_dz) return -9;
+  if ((D % 32) || (D % G) || !before || !ahead_feat || !ahead_dz) return -9;
   if (B2 * L == 0) return 0;
-  dim3 grid(D / SE_CT, (L + SE_T - 1) / SE_T, B2);
-  K_SWITCH(K, (se_bwd_tiled_kernel<KK><<<grid, SE_CT * SE_NSEG, 0, st>>>((const bf16*)feat, *before, 1, w, (const bf16*)dz,
-                                                                       (bf16*)dfeat, nullptr, dw, L, D, D / G, pregate, postgate,
-                                                                       1, *ahead_feat, *ahead_dz)));
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return se_bwd_fast(feat, *before, 1, w, dz, dfeat, nullptr, dw, B2, L, D, G, K, pregate, postgate, 1, *ahead_feat, *ahead_dz, st);
 }

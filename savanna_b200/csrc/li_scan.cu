@@ -20,6 +20,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "f32x2.cuh"
+
 namespace sb {
 typedef __nv_bfloat16 bf16;
 constexpr int LO = 16;            // padded filter order
@@ -346,20 +348,6 @@ li_bwd_apply_rev_kernel(const bf16* __restrict__ feat, const bf16* __restrict__ 
 // prepared the filter and summed the partials).  Forward and backward with their host side: 849 -> 552.  The recurrences
 // need 48 FMA per value forward and 144 backward, 54 and 163 us at the 30 TFMA/s that packed and plain FMA both reach here
 // (the packed form only halves the issue slots), so the sweeps sit between that bound and the copy time of their data.
-typedef unsigned long long f2;           // two packed fp32 values
-__device__ __forceinline__ f2 f2_pack(float a, float b) { f2 d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b)); return d; }
-__device__ __forceinline__ float2 f2_unpack(f2 v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
-__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) { f2 d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
-__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) { f2 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-__device__ __forceinline__ f2 f2_add(f2 a, f2 b) { f2 d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-__device__ __forceinline__ float lo_f(uint32_t w) { return __uint_as_float(w << 16); }
-__device__ __forceinline__ float hi_f(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
-__device__ __forceinline__ uint32_t pack_bf2(f2 v) {
-  const float2 t = f2_unpack(v);
-  __nv_bfloat162 r = __floats2bfloat162_rn(t.x, t.y);
-  return *reinterpret_cast<uint32_t*>(&r);
-}
-
 constexpr int LV_CH = 128;               // channels per block
 constexpr int LV_PAIRS = LV_CH / 2;      // threads of one role
 constexpr int LV_ROWS = 16;              // steps per ring tile (forward)
@@ -454,12 +442,8 @@ __device__ __forceinline__ void load_corr(const LiModal& m, size_t off, f2 (&c)[
   }
 }
 
-struct FeatPair { f2 x1, x2, v; };
-__device__ __forceinline__ FeatPair li_feat(const uint32_t* row, int lane3) {
-  const uint32_t w0 = row[lane3], w1 = row[lane3 + 1], w2 = row[lane3 + 2];
-  return FeatPair{f2_pack(lo_f(w0), hi_f(w1)), f2_pack(hi_f(w0), lo_f(w2)), f2_pack(lo_f(w1), hi_f(w2))};
-}
-__device__ __forceinline__ f2 li_pair(const uint32_t* row, int i) { const uint32_t w = row[i]; return f2_pack(lo_f(w), hi_f(w)); }
+__device__ __forceinline__ FeatPair li_feat(const uint32_t* row, int lane3) { return feat_pair(row[lane3], row[lane3 + 1], row[lane3 + 2]); }
+__device__ __forceinline__ f2 li_pair(const uint32_t* row, int i) { return f2_bf(row[i]); }
 
 // forward pass 1 (APPLY = false): end state of each chunk from a zero state.
 // forward pass 3 (APPLY = true): rerun each chunk from its entering state S and emit z.

@@ -109,6 +109,8 @@ class _Sig:
     sb_dwconv_fwd = [P, P, P, P, I, I, I, I, P]
     sb_dwconv_bwd = [P, P, P, P, P, P, P, I, I, I, I, P]
     sb_se_fwd = [P, P, P, P, I, I, I, I, I, I, I, P]
+    sb_dwconv_fwd_taps = [P, P, P, I, P, P, I, I, I, I, P]
+    sb_se_fwd_taps = [P, P, P, I, P, P, I, I, I, I, I, I, I, P]
     sb_se_bwd = [P, P, P, P, P, P, P, I, I, I, I, I, I, I, P]
     sb_mr_fwd = [P, P, P, P, P, P, I, I, I, I, I, P]
     sb_mr_bwd = [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, P]
@@ -289,14 +291,19 @@ def set_mr_backward_variant(streaming: bool) -> None:
     kernel, and both values select it."""
 
 
+CONV_FWD_FAST = True
+
+
 def set_se_backward_variant(tiled: bool) -> None:
-    """Hyena-SE backward: tiles staged through shared memory (default), or one run per thread reading global memory."""
+    """Hyena-SE and featuriser backward: streaming or tiled kernels by size (default), or one run per thread reading global memory."""
     require().sb_se_set_bwd_variant(int(bool(tiled)))
 
 
 def set_conv_forward_variant(tiled: bool) -> None:
-    """Depthwise (featuriser) convolution forward: tiles staged through shared memory, or one run per thread."""
-    require().sb_conv_set_fwd_variant(int(bool(tiled)))
+    """Hyena-SE and featuriser forward: streaming or tiled kernels by size (default), or one run per thread."""
+    global CONV_FWD_FAST
+    CONV_FWD_FAST = bool(tiled)
+    require().sb_conv_set_fwd_variant(int(CONV_FWD_FAST))
 
 
 _PAIR_MODE = 2
@@ -1200,17 +1207,31 @@ def _aligned(t):
     return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
+def _taps(w):
+    """(taps as the forward kernel reads them, whether they are bf16, the fp32 copy that it writes for the backward or None).  A bf16
+    parameter is converted by the kernel that reads it, not by a launch of its own."""
+    if w.dtype != bf16:
+        return _f32c(w), 0, None
+    return w.detach().contiguous(), 1, _alloc(w.shape, dtype=torch.float32, device=w.device)
+
+
 class _DwConv(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, halo):
         lib = require()
         B, L, C = x.shape
         K = w.shape[-1]
-        xc = x.contiguous()
-        hc = halo.contiguous() if halo is not None else None
-        wf = _f32c(w)
+        xc = _aligned(x)
+        hc = _aligned(halo) if halo is not None else None
+        wc, w_bf16, wf = _taps(w)
         y = _alloc_like(xc)
-        _check(lib.sb_dwconv_fwd(xc.data_ptr(), _ptr(hc), wf.data_ptr(), y.data_ptr(), B, L, C, K, _stream()), "dwconv_fwd")
+        if CONV_FWD_FAST:
+            _check(lib.sb_dwconv_fwd_taps(xc.data_ptr(), _ptr(hc), wc.data_ptr(), w_bf16, _ptr(wf), y.data_ptr(), B, L, C, K, _stream()),
+                   "dwconv_fwd")
+            wf = wc if wf is None else wf
+        else:
+            wf = _f32c(w)
+            _check(lib.sb_dwconv_fwd(xc.data_ptr(), _ptr(hc), wf.data_ptr(), y.data_ptr(), B, L, C, K, _stream()), "dwconv_fwd")
         _count()
         ctx.save_for_backward(xc, wf, hc if hc is not None else _alloc(0, device=x.device))
         ctx.meta = (halo is not None, w.dtype)
@@ -1223,7 +1244,7 @@ class _DwConv(torch.autograd.Function):
         has_halo, wdtype = ctx.meta
         B, L, C = xc.shape
         K = wf.shape[-1]
-        g = gy.contiguous()
+        g = _aligned(gy)
         dx = _alloc_like(xc)
         dh = _alloc_like(hc) if has_halo else None
         dw = _zeros_like(wf)
@@ -1247,12 +1268,18 @@ class _HyenaSE(torch.autograd.Function):
         B, L, C3 = feat.shape
         D = C3 // 3
         G, K = w.shape
-        fc = feat.contiguous()
-        hc = halo.contiguous() if halo is not None else None
-        wf = _f32c(w)
+        fc = _aligned(feat)
+        hc = _aligned(halo) if halo is not None else None
+        wc, w_bf16, wf = _taps(w)
         z = _alloc((B, L, D), dtype=bf16, device=feat.device)
-        _check(lib.sb_se_fwd(fc.data_ptr(), _ptr(hc), wf.data_ptr(), z.data_ptr(), B, L, D, G, K, int(pregate),
-                             int(postgate), _stream()), "se_fwd")
+        if CONV_FWD_FAST:
+            _check(lib.sb_se_fwd_taps(fc.data_ptr(), _ptr(hc), wc.data_ptr(), w_bf16, _ptr(wf), z.data_ptr(), B, L, D, G, K, int(pregate),
+                                      int(postgate), _stream()), "se_fwd")
+            wf = wc if wf is None else wf
+        else:
+            wf = _f32c(w)
+            _check(lib.sb_se_fwd(fc.data_ptr(), _ptr(hc), wf.data_ptr(), z.data_ptr(), B, L, D, G, K, int(pregate),
+                                 int(postgate), _stream()), "se_fwd")
         _count()
         ctx.save_for_backward(fc, wf, hc if hc is not None else _alloc(0, device=feat.device))
         ctx.meta = (halo is not None, w.dtype, pregate, postgate)
@@ -1266,7 +1293,7 @@ class _HyenaSE(torch.autograd.Function):
         B, L, C3 = fc.shape
         D = C3 // 3
         G, K = wf.shape
-        g = gz.contiguous()
+        g = _aligned(gz)
         df = _alloc_like(fc)
         dh = _alloc_like(hc) if has_halo else None
         dw = _zeros_like(wf)

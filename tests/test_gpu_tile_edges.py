@@ -359,3 +359,92 @@ def test_packed_attention_rotary():
         orf.backward(g.float())
         _close(o, orf, 2e-2, "o")                        # bf16 rotated q, k and probabilities: three roundings of up to 2^-8
         _close(qkv.grad, qr.grad, 4e-2, "dqkv")          # as in test_attention_tiles, and the rounded q, k enter the scores
+
+
+def _conv_grads(B, L, D, G, K, halo, pre=True, post=True, bf16_taps=False):
+    torch.manual_seed(L + K)
+    feat, w = torch.randn(B, L, 3 * D, device=DEV).to(BF), torch.randn(G, K, device=DEV) * 0.4
+    if bf16_taps:
+        w = w.to(BF)
+    h = torch.randn(B, K - 1, 3 * D, device=DEV).to(BF) if halo else None
+    g = torch.randn(B, L, D, device=DEV).to(BF)
+    out = []
+    for f32 in (False, True):
+        a = [None if t is None else (t.float() if f32 else t.clone()).requires_grad_() for t in (feat, w, h)]
+        z = (ref if f32 else ops).hyena_se_inner(a[0], a[1], a[2], pre, post)
+        z.backward(g.float() if f32 else g)
+        out.append([z.detach()] + [t.grad for t in a if t is not None])
+    return out
+
+
+# rows of 128 channels per SM: at least 200 on a chip of 148 SMs, where the streaming kernels start; runs that end on an odd row, strips
+# of 128 channels that are not full, groups of fewer than four channels (their taps differ within a lane), every filter length
+@pytest.mark.parametrize("B,L,D,G,K", [(1, 3703, 1024, 64, 7), (2, 1901, 1016, 127, 2), (3, 1301, 1000, 500, 3), (1, 1, 8, 1, 7),
+                                       (1, 3801, 1016, 254, 4), (2, 1999, 904, 452, 5), (1, 4001, 1024, 8, 6), (5, 797, 1024, 1024, 8)])
+@pytest.mark.parametrize("halo", [False, True])
+def test_se_streaming(B, L, D, G, K, halo):
+    got, want = _conv_grads(B, L, D, G, K, halo, bf16_taps=K == 7)
+    # fp32 sums, one bf16 rounding of the result: 2^-9; bf16 taps round their gradient once more
+    for a, b, n in zip(got, want, ("z", "dfeat", "dtaps", "dhalo")):
+        _close(a, b, 4e-3, n)
+
+
+@pytest.mark.parametrize("pre,post", [(False, True), (True, False), (False, False)])
+def test_se_streaming_gates(pre, post):
+    for a, b in zip(*_conv_grads(1, 3701, 1024, 64, 7, True, pre, post)):
+        _close(a, b, 4e-3, (pre, post))
+
+
+@pytest.mark.parametrize("B,L,C,K", [(1, 1301, 3072, 3), (2, 1901, 1016, 2), (3, 1301, 1000, 4), (1, 3801, 1016, 8), (2, 1999, 904, 5), (1, 2, 8, 3)])
+@pytest.mark.parametrize("halo", [False, True])
+def test_featuriser_streaming(B, L, C, K, halo):
+    torch.manual_seed(L + K)
+    x, w = torch.randn(B, L, C, device=DEV).to(BF), torch.randn(C, K, device=DEV).to(BF)
+    h, g = torch.randn(B, K - 1, C, device=DEV).to(BF) if halo else None, torch.randn(B, L, C, device=DEV).to(BF)
+    out = []
+    for f32 in (False, True):
+        a = [None if t is None else (t.float() if f32 else t.clone()).requires_grad_() for t in (x, w, h)]
+        y = (ref if f32 else ops).causal_conv1d(*a)
+        y.backward(g.float() if f32 else g)
+        out.append([y.detach()] + [t.grad for t in a if t is not None])
+    for a, b, n in zip(*out, ("y", "dx", "dtaps", "dhalo")):
+        _close(a, b, 4e-3, n)
+
+
+@pytest.mark.parametrize("L,D,K", [(3702, 1024, 7), (3710, 1088, 4)])
+def test_conv_streaming_chunks(L, D, K):
+    """Two chunks of one sequence as batch rows, their edge rows handed over as the context-parallel entry points take them: rows before
+    each chunk, and rows after it for the backward; the pieces together are the whole sequence's results."""
+    from savanna_b200.ops import cuda_ops
+    from savanna_b200.parallel import halo_fused
+    import ctypes
+    torch.manual_seed(L)
+    lib, c, H, G, C, st = cuda_ops.require(), L // 2, K - 1, D // 16, 3 * D, torch.cuda.current_stream().cuda_stream
+    P, I, S = ctypes.c_void_p, ctypes.c_int, ctypes.POINTER(halo_fused.HaloSrc)
+    lib.sb_dwconv_bwd_cp.argtypes = [P, S, P, P, S, P, P, I, I, I, I, P]
+    lib.sb_se_fwd_cp.argtypes = [P, S, P, P, I, I, I, I, I, I, I, P]
+    lib.sb_se_bwd_cp.argtypes = [P, S, P, P, S, S, P, P, I, I, I, I, I, I, I, P]
+    f, g, gx = (torch.randn(1, L, n, device=DEV).to(BF) for n in (C, D, C))
+    w, wc = torch.randn(G, K, device=DEV) * 0.4, torch.randn(C, K, device=DEV)
+
+    def edges(t, after):
+        zero = torch.zeros(1, H, t.shape[2], device=DEV, dtype=BF)
+        e = torch.cat([t[:, c:c + H], zero] if after else [zero, t[:, c - H:c]]).contiguous()
+        return e, halo_fused.HaloSrc(e.data_ptr(), e.data_ptr(), 0, 0, 0)
+
+    (k0, bf_), (k1, af), (k2, ag), (k3, agx) = edges(f, False), edges(f, True), edges(g, True), edges(gx, True)
+    z, df, dx = torch.empty_like(g), torch.empty_like(f), torch.empty_like(f)
+    dw, dwc = torch.zeros_like(w), torch.zeros_like(wc)
+    assert lib.sb_se_fwd_cp(f.data_ptr(), ctypes.byref(bf_), w.data_ptr(), z.data_ptr(), 2, c, D, G, K, 1, 1, st) == 0
+    assert lib.sb_se_bwd_cp(f.data_ptr(), ctypes.byref(bf_), w.data_ptr(), g.data_ptr(), ctypes.byref(af), ctypes.byref(ag), df.data_ptr(),
+                            dw.data_ptr(), 2, c, D, G, K, 1, 1, st) == 0
+    assert lib.sb_dwconv_bwd_cp(f.data_ptr(), ctypes.byref(bf_), wc.data_ptr(), gx.data_ptr(), ctypes.byref(agx), dx.data_ptr(), dwc.data_ptr(),
+                                2, c, C, K, st) == 0
+    torch.cuda.synchronize()
+    a, b = f.float().requires_grad_(), w.clone().requires_grad_()
+    zr = ref.hyena_se_inner(a, b)
+    zr.backward(g.float())
+    x, v = f.float().requires_grad_(), wc.clone().requires_grad_()
+    ref.causal_conv1d(x, v).backward(gx.float())
+    for got, want, n in ((z, zr, "z"), (df, a.grad, "dfeat"), (dw, b.grad, "dtaps"), (dx, x.grad, "dx"), (dwc, v.grad, "dconv")):
+        _close(got.view(want.shape), want, 4e-3, n)
