@@ -8,6 +8,7 @@
 #include <stdint.h>
 
 #include "device_info.h"
+#include "f32x2.cuh"
 
 namespace sb {
 
@@ -142,6 +143,7 @@ rmsnorm_bwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const
   }
   uint4 xn[VPT], gn[VPT], rn[VPT];                      // next row: x, dy and (optional) the gradient to add
   size_t row = blockIdx.x;
+  float an = row < (size_t)T ? a_in[row] : 0.f;         // its 1 / rms: as far away as they are
   if (row < (size_t)T) {
 #pragma unroll
     for (int v = 0; v < VPT; ++v) {
@@ -158,7 +160,9 @@ rmsnorm_bwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const
 #pragma unroll
     for (int v = 0; v < VPT; ++v) { xc[v] = xn[v]; gc[v] = gn[v]; rc[v] = rn[v]; }
     const size_t nxt = row + gridDim.x;
+    const float a = an;
     if (nxt < (size_t)T) {
+      an = a_in[nxt];
 #pragma unroll
       for (int v = 0; v < VPT; ++v) {
         const int i = threadIdx.x + v * blockDim.x;
@@ -168,7 +172,6 @@ rmsnorm_bwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const
         }
       }
     }
-    const float a = a_in[row];
     float dot = 0.f;
 #pragma unroll
     for (int v = 0; v < VPT; ++v) {
@@ -222,25 +225,159 @@ rmsnorm_bwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const
     }
   }
 }
-// dw[col] = sum_b partial[b, col] as bf16: a block covers 32 groups of four columns, its 8 thread rows split the partial
-// rows and are combined through shared memory (no atomics, no zero-initialised output)
-__global__ void __launch_bounds__(256)
+// The same for D <= 4096 (one vector per thread), two rows at a time.  A thread copies the 16 bytes of each row that it owns into a
+// ring in shared memory, two pairs of rows deep; nobody else reads them, so there is no barrier for them, only the thread's own wait.
+// Bound by the latency between a pair's arrival and its stores (two block-wide sums behind one barrier) and, with one row at a time,
+// by issue slots; hence pairs of rows and packed fp32.  T = 8192, D = 4096, us with the reduction of the partial rows: 64 with
+// one row ahead in registers, 51 with the ring alone, 39 like this (a three-tensor copy of that size takes 33); D = 1024: 41 -> 22.
+__device__ __forceinline__ void nr_copy(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ uint4 nr_take(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void unpack8(const uint4& v, f2 (&f)[4]) { f[0] = f2_bf(v.x); f[1] = f2_bf(v.y); f[2] = f2_bf(v.z); f[3] = f2_bf(v.w); }
+
+template <bool RES>
+__global__ void __launch_bounds__(512, 2)
+rmsnorm_bwd_pair_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const bf16* __restrict__ dy,
+                        const float* __restrict__ a_in, const bf16* __restrict__ gres, bf16* __restrict__ dx,
+                        float* __restrict__ partial, int T, int D, float eps, int form) {
+  constexpr int NT = RES ? 3 : 2;                        // tensors in a row's slot
+  __shared__ float2 red[2][32];
+  extern __shared__ __align__(16) uint4 nr_smem[];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const bool mine = (int)threadIdx.x < D >> 3;
+  const uint32_t part = blockDim.x * 16, ring = (uint32_t)__cvta_generic_to_shared(nr_smem) + threadIdx.x * 16;
+  const int col = threadIdx.x * 8, pairs = (T + 1) >> 1;
+  auto slot = [&](int s, int r) { return ring + (s * 2 + r) * NT * part; };
+  auto fetch = [&](int pr, int s) {
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int row = 2 * pr + r;
+      if (mine && row < T) {
+        const size_t o = (size_t)row * D + col;
+        nr_copy(slot(s, r), x + o);
+        nr_copy(slot(s, r) + part, dy + o);
+        if (RES) nr_copy(slot(s, r) + 2 * part, gres + o);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  auto inv_rms = [&](int pr) {
+    return make_float2(2 * pr < T ? a_in[2 * pr] : 0.f, 2 * pr + 1 < T ? a_in[2 * pr + 1] : 0.f);
+  };
+  int pr = blockIdx.x;
+  fetch(pr, 0);
+  float2 an = inv_rms(pr);                               // 1 / rms of the next rows: as far away as they are
+  f2 wv[4], acc[4];
+  unpack8(mine ? *reinterpret_cast<const uint4*>(w + col) : make_uint4(0, 0, 0, 0), wv);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) acc[j] = 0;
+  for (int it = 0; pr < pairs; pr += gridDim.x, ++it) {
+    fetch(pr + gridDim.x, (it + 1) & 1);
+    const float2 a = an;
+    an = inv_rms(pr + gridDim.x);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    const bool two = 2 * pr + 1 < T;
+    uint4 xc[2], gc[2];
+    float dot[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const bool have = mine && (r == 0 || two);
+      xc[r] = have ? nr_take(slot(it & 1, r)) : make_uint4(0, 0, 0, 0);
+      gc[r] = have ? nr_take(slot(it & 1, r) + part) : make_uint4(0, 0, 0, 0);
+      f2 xf[4], gf[4], d2 = 0;
+      unpack8(xc[r], xf); unpack8(gc[r], gf);
+      const f2 ar = r ? f2_pack(a.y, a.y) : f2_pack(a.x, a.x);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const f2 gx = f2_mul(gf[j], xf[j]);
+        acc[j] = f2_fma(gx, ar, acc[j]);
+        d2 = f2_fma(gx, wv[j], d2);
+      }
+      const float2 d = f2_unpack(d2);
+      dot[r] = d.x + d.y;
+    }
+    // both rows' block sums with one barrier (two alternating scratch rows)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      dot[0] += __shfl_xor_sync(0xffffffffu, dot[0], o);
+      dot[1] += __shfl_xor_sync(0xffffffffu, dot[1], o);
+    }
+    float2* rr = red[it & 1];
+    if (lane == 0) rr[wid] = make_float2(dot[0], dot[1]);
+    __syncthreads();
+    float2 tot = lane < nw ? rr[lane] : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {                    // 16 warps at most
+      tot.x += __shfl_xor_sync(0xffffffffu, tot.x, o);
+      tot.y += __shfl_xor_sync(0xffffffffu, tot.y, o);
+    }
+    tot.x = __shfl_sync(0xffffffffu, tot.x, 0);
+    tot.y = __shfl_sync(0xffffffffu, tot.y, 0);
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      if (r == 1 && !two) break;
+      const float ar = r ? a.y : a.x;
+      float c;
+      if (form == 0) c = ar * ar * ar;
+      else { const float rms = 1.f / ar - eps; c = ar * ar / fmaxf(rms, 1e-30f); }
+      const float k = c * (r ? tot.y : tot.x) / D;
+      const f2 a2 = f2_pack(ar, ar), k2 = f2_pack(-k, -k);
+      f2 xf[4], gf[4], o[4];
+      unpack8(xc[r], xf); unpack8(gc[r], gf);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) o[j] = f2_fma(xf[j], k2, f2_mul(f2_mul(a2, gf[j]), wv[j]));
+      if (mine) {
+        if (RES) {
+          f2 rf[4];
+          unpack8(nr_take(slot(it & 1, r) + 2 * part), rf);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) o[j] = f2_add(o[j], rf[j]);
+        }
+        *reinterpret_cast<uint4*>(dx + (size_t)(2 * pr + r) * D + col) =
+            make_uint4(pack_bf2(o[0]), pack_bf2(o[1]), pack_bf2(o[2]), pack_bf2(o[3]));
+      }
+    }
+  }
+  if (mine) {
+    float4* dst = reinterpret_cast<float4*>(partial + (size_t)blockIdx.x * D + col);
+    const float2 s0 = f2_unpack(acc[0]), s1 = f2_unpack(acc[1]), s2 = f2_unpack(acc[2]), s3 = f2_unpack(acc[3]);
+    dst[0] = make_float4(s0.x, s0.y, s1.x, s1.y);
+    dst[1] = make_float4(s2.x, s2.y, s3.x, s3.y);
+  }
+}
+
+// dw[col] = sum_b partial[b, col] as bf16: a block covers 32 groups of four columns, its 32 thread rows split the partial
+// rows and are combined through shared memory (no atomics, no zero-initialised output).  Latency bound: 296 partial rows are
+// ten loads per thread here and were 37 with eight thread rows (9.0 us, now 4.3).
+constexpr int DWR_ROWS = 32;
+__global__ void __launch_bounds__(32 * DWR_ROWS)
 rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, bf16* __restrict__ dw, int nblk, int D) {
-  __shared__ float4 part[8][32];
+  __shared__ float4 part[DWR_ROWS][32];
   const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
   const int c4 = blockIdx.x * 32 + cx;
   float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
   if (c4 * 4 < D) {
-    for (int b = ry; b < nblk; b += 8) {
+#pragma unroll 4
+    for (int b = ry; b < nblk; b += DWR_ROWS) {
       const float4 p = *reinterpret_cast<const float4*>(partial + (size_t)b * D + (size_t)c4 * 4);
       s.x += p.x; s.y += p.y; s.z += p.z; s.w += p.w;
     }
   }
   part[ry][cx] = s;
-  __syncthreads();
+  for (int h = DWR_ROWS / 2; h > 0; h >>= 1) {
+    __syncthreads();
+    if (ry < h) {
+      const float4 p = part[ry + h][cx];
+      s.x += p.x; s.y += p.y; s.z += p.z; s.w += p.w;
+      part[ry][cx] = s;
+    }
+  }
   if (ry == 0 && c4 * 4 < D) {
-#pragma unroll
-    for (int j = 1; j < 8; ++j) { const float4 p = part[j][cx]; s.x += p.x; s.y += p.y; s.z += p.z; s.w += p.w; }
     __nv_bfloat162 lo = __floats2bfloat162_rn(s.x, s.y), hi = __floats2bfloat162_rn(s.z, s.w);
     uint2 o;
     o.x = *reinterpret_cast<uint32_t*>(&lo); o.y = *reinterpret_cast<uint32_t*>(&hi);
@@ -825,14 +962,22 @@ static inline int grid_for(size_t work, int threads, int cap = sb::num_sms() * 1
 
 using namespace sb;
 
+// Threads of a norm block for rows of nv 16-byte vectors, and blocks for T rows: `warps` of them per SM at most, at most 16 blocks.
+// (Forward, T = 8192, us: D = 1024 12.4 -> 10.3, D = 256 10.3 -> 6.2 against four blocks per SM whatever their size.)
+static int norm_threads(int nv) { return nv >= 512 ? 512 : nv <= 64 ? 64 : (nv + 31) / 32 * 32; }
+static int norm_grid(int T, int threads, int warps) {
+  const int per_sm = warps * 32 / threads < 16 ? warps * 32 / threads : 16, cap = sb::num_sms() * per_sm;
+  return T < cap ? T : cap;
+}
+
 extern "C" int sb_rmsnorm_fwd(const void* x, const void* w, void* y, float* a_out, int T, int D, float eps, int form,
                               cudaStream_t st) {
   if (D % 8) return -1;
   if (T == 0) return 0;
   const int nv = D / 8;
-  const int threads = nv >= 512 ? 512 : (nv >= 256 ? 256 : (nv >= 128 ? 128 : 64));
+  const int threads = norm_threads(nv);
   const int vpt = (nv + threads - 1) / threads;
-  const int grid = T < sb::num_sms() * 4 ? T : sb::num_sms() * 4;
+  const int grid = norm_grid(T, threads, vpt == 1 ? 64 : 4 * threads / 32);
 #define LAUNCH(V) rmsnorm_fwd_kernel<V><<<grid, threads, 0, st>>>((const bf16*)x, (const bf16*)w, (bf16*)y, a_out, T, D, eps, form)
   if (vpt <= 1) LAUNCH(1);
   else if (vpt <= 2) LAUNCH(2);
@@ -842,25 +987,41 @@ extern "C" int sb_rmsnorm_fwd(const void* x, const void* w, void* y, float* a_ou
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-// Blocks of the backward kernel for T rows (also the number of rows of the `partial` scratch).
-extern "C" int sb_rmsnorm_bwd_blocks(int T) { return T < sb::num_sms() * 2 ? (T < 1 ? 1 : T) : sb::num_sms() * 2; }
+// Blocks of the backward kernel for T rows of D (also the number of rows of the `partial` scratch).  One vector per thread: 32 warps per
+// SM, but then at least two pairs of rows per block, and no fewer than two blocks per SM while there are pairs.
+extern "C" int sb_rmsnorm_bwd_blocks(int T, int D) {
+  const int nv = D / 8, threads = norm_threads(nv), sms = sb::num_sms();
+  const int rows = T < 1 ? 1 : T, pairs = (rows + 1) / 2, most = 2 * sms;
+  if (nv > threads) return rows < most ? rows : most;    // one row ahead in registers
+  const int full = norm_grid((rows + 3) / 4, threads, 32), two = pairs < most ? pairs : most;
+  return full > two ? full : two;
+}
 
-// dw: bf16 [D], written (not accumulated); partial is scratch of sb_rmsnorm_bwd_blocks(T) * D floats.  Two launches.
+// dw: bf16 [D], written (not accumulated); partial is scratch of sb_rmsnorm_bwd_blocks(T, D) * D floats.  Two launches.
 extern "C" int sb_rmsnorm_bwd(const void* x, const void* w, const void* dy, const float* a_in, const void* gres, void* dx,
                               void* dw, float* partial, int T, int D, float eps, int form, cudaStream_t st) {
   if (D % 8) return -1;
   if (T == 0) return 0;
   const int nv = D / 8;
-  int threads = nv >= 512 ? 512 : (nv >= 256 ? 256 : (nv >= 128 ? 128 : 64));
+  const int threads = norm_threads(nv);
   const int vpt = (nv + threads - 1) / threads;
-  const int grid = sb_rmsnorm_bwd_blocks(T);
+  const int grid = sb_rmsnorm_bwd_blocks(T, D);
 #define LAUNCH(V) rmsnorm_bwd_kernel<V><<<grid, threads, 0, st>>>((const bf16*)x, (const bf16*)w, (const bf16*)dy, a_in, (const bf16*)gres, (bf16*)dx, partial, T, D, eps, form)
-  if (vpt <= 1) LAUNCH(1);
+#define PAIR(R) rmsnorm_bwd_pair_kernel<R><<<grid, threads, ring, st>>>((const bf16*)x, (const bf16*)w, (const bf16*)dy, a_in, (const bf16*)gres, (bf16*)dx, partial, T, D, eps, form)
+  if (vpt <= 1) {
+    const int ring = 4 * threads * 16 * (gres ? 3 : 2);
+    if (ring > 49152 && (cudaFuncSetAttribute(rmsnorm_bwd_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 512 * 16 * 3) != cudaSuccess ||
+                         cudaFuncSetAttribute(rmsnorm_bwd_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 512 * 16 * 2) != cudaSuccess))
+      return -2;
+    if (gres) PAIR(true);
+    else PAIR(false);
+  }
   else if (vpt <= 2) LAUNCH(2);
   else if (vpt <= 4) LAUNCH(4);
   else return -3;
 #undef LAUNCH
-  rmsnorm_dw_reduce_kernel<<<(D / 4 + 31) / 32, 256, 0, st>>>(partial, (bf16*)dw, grid, D);
+#undef PAIR
+  rmsnorm_dw_reduce_kernel<<<(D / 4 + 31) / 32, 32 * DWR_ROWS, 0, st>>>(partial, (bf16*)dw, grid, D);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -1007,9 +1168,9 @@ extern "C" int sb_rmsnorm_fwd_fp8(const void* x, const void* w, void* q, float* 
   if ((D % 8) || slots < 3 || cur < 0 || cur >= slots) return -1;
   if (T == 0) return 0;
   const int nv = D / 8;
-  const int threads = nv >= 512 ? 512 : (nv >= 256 ? 256 : (nv >= 128 ? 128 : 64));
+  const int threads = norm_threads(nv);
   const int vpt = (nv + threads - 1) / threads;
-  const int grid = T < sb::num_sms() * 4 ? T : sb::num_sms() * 4;
+  const int grid = norm_grid(T, threads, vpt == 1 ? 64 : 4 * threads / 32);
 #define LAUNCH(V) rmsnorm_fwd_fp8_kernel<V><<<grid, threads, 0, st>>>((const bf16*)x, (const bf16*)w, (uint8_t*)q, a_out, T, D, eps, form, hist, slots, cur, scale_inv)
   if (vpt <= 1) LAUNCH(1);
   else if (vpt <= 2) LAUNCH(2);

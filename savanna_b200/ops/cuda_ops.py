@@ -98,7 +98,7 @@ class _Sig:
     sb_glu_fwd_fp8 = [P, P, LL, I, I, P, I, I, P, P]
     sb_glu_bwd_fp8 = [P, P, P, LL, I, I, P, I, I, P, P]
     sb_rmsnorm_bwd = [P, P, P, P, P, P, P, P, I, I, F, I, P]
-    sb_rmsnorm_bwd_blocks = [I]
+    sb_rmsnorm_bwd_blocks = [I, I]
     sb_glu_fwd = [P, P, LL, I, I, P]
     sb_glu_bwd = [P, P, P, LL, I, I, P]
     sb_rope = [P, P, P, P, I, I, I, I, I, LL, LL, I, P]
@@ -732,7 +732,7 @@ def _rmsnorm_bwd(x2, w, a, gy, gres, eps, form):
     r2 = gres.reshape(T, D).contiguous() if gres is not None else None
     dx = _alloc_like(x2)
     dw = _alloc(D, dtype=bf16, device=x2.device)
-    partial = _alloc(lib.sb_rmsnorm_bwd_blocks(T) * D, dtype=torch.float32, device=x2.device)
+    partial = _alloc(lib.sb_rmsnorm_bwd_blocks(T, D) * D, dtype=torch.float32, device=x2.device)
     _check(lib.sb_rmsnorm_bwd(x2.data_ptr(), w.data_ptr(), g2.data_ptr(), a.data_ptr(), _ptr(r2), dx.data_ptr(),
                               dw.data_ptr(), partial.data_ptr(), T, D, eps, form, _stream()), "rmsnorm_bwd")
     _count(2)

@@ -448,3 +448,21 @@ def test_conv_streaming_chunks(L, D, K):
     ref.causal_conv1d(x, v).backward(gx.float())
     for got, want, n in ((z, zr, "z"), (df, a.grad, "dfeat"), (dw, b.grad, "dtaps"), (dx, x.grad, "dx"), (dwc, v.grad, "dconv")):
         _close(got.view(want.shape), want, 4e-3, n)
+
+
+# rows in pairs: one row, odd counts, more and fewer pairs than blocks; widths of one vector per thread (not a multiple of a warp among them,
+# the widest 4096) and beyond
+@pytest.mark.parametrize("T,D", [(1, 64), (3, 72), (2, 4096), (597, 2816), (1185, 256), (37, 4104), (2371, 1024)])
+@pytest.mark.parametrize("form", ["te", "classic"])
+def test_rmsnorm_rows_in_pairs(T, D, form):
+    torch.manual_seed(T)
+    x, w, g, gr = (torch.randn(*s, device=DEV).to(BF) for s in ((T, D), (D,), (T, D), (T, D)))
+    a, b = x.clone().requires_grad_(), w.clone().requires_grad_()
+    y, res = ops.rmsnorm_residual(a, b, 1e-6, form)
+    torch.autograd.backward([y, res], [g, gr])
+    ar, br = x.float().requires_grad_(), w.float().requires_grad_()
+    yr = ref.rmsnorm(ar, br, 1e-6, form)
+    torch.autograd.backward([yr, ar * 1], [g.float(), gr.float()])
+    # fp32 sums, one bf16 rounding of each result: 2^-9
+    for got, want, n in ((y, yr, "y"), (a.grad, ar.grad, "dx"), (b.grad, br.grad, "dw")):
+        _close(got, want, 4e-3, n)
