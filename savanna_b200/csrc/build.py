@@ -5,10 +5,10 @@
   savanna_b200/libsavanna_b200.so    every CUDA kernel, compiled for sm_100a only
                                      (nvcc -gencode arch=compute_100a,code=sm_100a -lineinfo), C ABI
   savanna_b200/libsavanna_data.so    C++ dataset index builders, C ABI
+  savanna_b200/_native.so            C++ autograd functions that call the CUDA library's entry points (PyTorch extension module)
 
-The libraries expose plain C symbols and are loaded with ctypes (ops/cuda_ops.py, data/helpers.py), so
-no PyTorch headers are compiled and a rebuild takes seconds.  A content hash of the sources is stored
-next to each library; an up-to-date library is not rebuilt.
+The first two expose plain C symbols and are loaded with ctypes (ops/cuda_ops.py, data/helpers.py): the kernels include
+no PyTorch header.  A content hash of the sources is stored next to each library; an up-to-date library is not rebuilt.
 """
 from __future__ import annotations
 
@@ -25,6 +25,8 @@ PKG = os.path.dirname(HERE)
 BUILD = os.path.join(HERE, "build")
 CUDA_LIB = os.path.join(PKG, "libsavanna_b200.so")
 DATA_LIB = os.path.join(PKG, "libsavanna_data.so")
+NATIVE_MODULE = os.path.join(PKG, "_native.so")
+NATIVE_SOURCES = ("autograd_native.cpp",)
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-Xptxas", "-v"]
@@ -93,7 +95,7 @@ def build_cuda(force=False, verbose=False):
 
 
 def build_data(force=False):
-    cpps = _sources(".cpp")
+    cpps = [c for c in _sources(".cpp") if os.path.basename(c) not in NATIVE_SOURCES]
     digest = _digest(cpps)
     if not force and _fresh(DATA_LIB, digest):
         return DATA_LIB
@@ -105,8 +107,30 @@ def build_data(force=False):
     return DATA_LIB
 
 
+def build_native(force=False):
+    import sysconfig
+    import torch
+    from torch.utils import cpp_extension
+    cpps = [os.path.join(HERE, c) for c in NATIVE_SOURCES]
+    digest = _digest(cpps, f"{torch.__version__} {sys.version}")
+    if not force and _fresh(NATIVE_MODULE, digest):
+        return NATIVE_MODULE
+    cxx = shutil.which("g++") or "g++"
+    inc = cpp_extension.include_paths(device_type="cuda") + [sysconfig.get_paths()["include"]]
+    log = []
+    _run([cxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_native", "-DTORCH_API_INCLUDE_EXTENSION_H",
+          f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"] + ["-I" + i for i in inc] + cpps
+         + ["-o", NATIVE_MODULE] + ["-L" + d for d in cpp_extension.library_paths()]
+         + ["-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10", "-lc10_cuda", "-ltorch_cuda", "-ldl"], log)
+    with open(_stamp(NATIVE_MODULE), "w") as fh:
+        fh.write(digest)
+    return NATIVE_MODULE
+
+
 def build_all(force=False, verbose=False):
-    return build_cuda(force, verbose), build_data(force)
+    with cf.ThreadPoolExecutor(max_workers=3) as ex:
+        futs = [ex.submit(build_cuda, force, verbose), ex.submit(build_data, force), ex.submit(build_native, force)]
+        return tuple(f.result() for f in futs)
 
 
 if __name__ == "__main__":

@@ -37,17 +37,26 @@ def kernel_launch_count() -> int:
     return cuda_ops.launch_count()
 
 
+_CO = None               # cuda_ops, imported with the first CUDA tensor
+
+
 def _k(x: torch.Tensor) -> bool:
     if not x.is_cuda or _BACKEND == "torch":
         return False
-    from . import cuda_ops  # raises with a clear message when the extension is not built
-    cuda_ops.require()
+    if _CO is None:
+        _load()
     return True
 
 
+def _load() -> None:
+    global _CO
+    from . import cuda_ops  # raises with a clear message when the extension is not built
+    cuda_ops.require()
+    _CO = cuda_ops
+
+
 def _co():
-    from . import cuda_ops
-    return cuda_ops
+    return _CO
 
 
 # ----------------------------------------------------------------------------- dense

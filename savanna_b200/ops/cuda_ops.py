@@ -1,7 +1,8 @@
-"""CUDA operator implementations: autograd Functions over the in-tree sm_100a library.
+"""CUDA operator implementations: autograd functions over the in-tree sm_100a library.
 
 The library (`savanna_b200/libsavanna_b200.so`, built by `python -m savanna_b200.csrc.build`) exposes C
-symbols; they are called through ctypes with raw device pointers and the current CUDA stream, so the
+symbols; they are called with raw device pointers and the current CUDA stream, from C++ autograd functions
+(csrc/autograd_native.cpp, the bf16 operators) or through ctypes (fp8 projections, optimizer, the rest), so the
 kernels run in PyTorch's stream order and under its caching allocator.  All kernels take bf16
 activations and accumulate in fp32.  Tensors of another dtype run the PyTorch statement of the op
 (reference.py) — a debugging configuration, not a performance path.
@@ -12,7 +13,9 @@ number of kernels the C entry point launches).
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
+import sys
 from typing import Optional
 
 import torch
@@ -20,7 +23,9 @@ import torch
 from . import reference as ref
 
 _LIB = None
+_N = None                # the C++ autograd functions, loaded with the library
 _LIB_PATH = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "libsavanna_b200.so")
+_NATIVE_PATH = os.path.join(os.path.dirname(_LIB_PATH), "_native.so")
 _LAUNCHES = 0
 _STATUS = {}
 
@@ -32,7 +37,7 @@ c_void_p, c_int, c_float, c_ll = ctypes.c_void_p, ctypes.c_int, ctypes.c_float, 
 
 def require():
     """Load the native library; raise if it is missing (never fall back silently on a GPU)."""
-    global _LIB
+    global _LIB, _N
     if _LIB is not None:
         return _LIB
     if not os.path.exists(_LIB_PATH):
@@ -45,8 +50,51 @@ def require():
             fn = getattr(raw, name)
             fn.restype = c_int
             fn.argtypes = getattr(_Sig, name)
+    _N = _load_native()
     _LIB = _Library(raw)
     return _LIB
+
+
+def _load_native():
+    """The C++ autograd functions (csrc/autograd_native.cpp), bound to the library's entry points."""
+    if not os.path.exists(_NATIVE_PATH):
+        raise RuntimeError(f"{_NATIVE_PATH} is missing: build it with `python -m savanna_b200.csrc.build`")
+    spec = importlib.util.spec_from_file_location("savanna_b200._native", _NATIVE_PATH)
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    mod.load(_LIB_PATH, sys.modules[__name__])
+    mod.set_nvtx(NVTX)
+    mod.set_guarded(_GUARDED is not None)
+    return mod
+
+
+class _Traced(torch.autograd.Function):
+    """`torch.jit.trace` records a Python function as one node of its graph, where the C++ functions would leave nothing behind:
+    while it runs, they are called from here, on a graph of their own that the backward goes through."""
+
+    @staticmethod
+    def forward(ctx, name, *args):
+        ins = [a.detach().requires_grad_(a.requires_grad) if isinstance(a, torch.Tensor) else a for a in args]
+        with torch.enable_grad():
+            out = getattr(_N, name)(*ins)
+        ctx.graph = ins, out
+        many = isinstance(out, tuple)
+        got = tuple(None if o is None else o.detach() for o in (out if many else (out,)))
+        return got if many else got[0]
+
+    @staticmethod
+    def backward(ctx, *grads):
+        ins, out = ctx.graph
+        outs = [(o, g) for o, g in zip(out if isinstance(out, tuple) else (out,), grads) if o is not None and o.requires_grad]
+        want = [a for a in ins if isinstance(a, torch.Tensor) and a.requires_grad]
+        got = iter(torch.autograd.grad([o for o, _ in outs], want, [g for _, g in outs], retain_graph=True, allow_unused=True))
+        return (None,) + tuple(next(got) if isinstance(a, torch.Tensor) and a.requires_grad else None for a in ins)
+
+
+def _native(name, *args):
+    if torch._C._get_tracing_state() is not None:
+        return _Traced.apply(name, *args)
+    return getattr(_N, name)(*args)
 
 
 NVTX = False        # one NVTX range per native entry point (named after it) while True; the capture-range profiler turns it on
@@ -55,6 +103,8 @@ NVTX = False        # one NVTX range per native entry point (named after it) whi
 def set_nvtx(on: bool) -> None:
     global NVTX
     NVTX = bool(on)
+    if _N is not None:
+        _N.set_nvtx(NVTX)
 
 
 class _Library:
@@ -128,7 +178,7 @@ class _Sig:
 
 
 def launch_count() -> int:
-    return _LAUNCHES
+    return _LAUNCHES + (_N.launches() if _N is not None else 0)
 
 
 # ----------------------------------------------------------------------------- guarded allocation (debug aid)
@@ -188,11 +238,15 @@ class guarded_allocations:
     def __enter__(self):
         global _GUARDED
         self.prev, _GUARDED = _GUARDED, []
+        if _N is not None:
+            _N.set_guarded(True)
         return self
 
     def __exit__(self, *exc):
         global _GUARDED
         _GUARDED = self.prev
+        if _N is not None:
+            _N.set_guarded(_GUARDED is not None)
         return False
 
 
@@ -331,47 +385,6 @@ def _rows(x):
     if x2.stride(1) != 1 or (x2.stride(0) % 8) or (x2.data_ptr() % 16):
         x2 = x2.contiguous()
     return x2
-
-
-class _Linear(torch.autograd.Function):
-    """y = x w^T (+ bias) (+ residual).  The weight gradient is accumulated by the GEMM epilogue directly into
-    `w.grad` when the parameter lives in a persistent flat gradient buffer (marked `_fuse_grad_accum` by the
-    ZeRO optimizer): no temporary gradient, no separate accumulation pass."""
-
-    @staticmethod
-    def forward(ctx, x, w, bias, residual):
-        x2 = _rows(x)
-        out = _alloc((x2.shape[0], w.shape[0]), dtype=bf16, device=x.device)
-        r2 = _rows(residual) if residual is not None else None
-        gemm(x2, w, out, bias=bias, residual=r2)
-        ctx.save_for_backward(x2, w)
-        ctx.has_bias = bias is not None
-        ctx.has_res = residual is not None
-        ctx.xshape = x.shape
-        ctx.wref = w
-        return out.view(*x.shape[:-1], w.shape[0])
-
-    @staticmethod
-    def backward(ctx, gy):
-        x2, w = ctx.saved_tensors
-        g2 = _rows(gy)
-        gx = gw = gb = None
-        if ctx.needs_input_grad[0]:
-            gx = _alloc_like(x2)
-            gemm(g2, w, gx, a_mn=False, b_mn=True)                 # dX[T,K] = dY[T,N] . W[N,K]
-            gx = gx.view(ctx.xshape)
-        if ctx.needs_input_grad[1]:
-            wp = ctx.wref
-            tgt = wp.grad if getattr(wp, "_fuse_grad_accum", False) else None
-            if tgt is not None and tgt.dtype == bf16 and tgt.is_contiguous() and tgt.shape == w.shape:
-                gemm(g2, x2, tgt, a_mn=True, b_mn=True, accumulate=True)   # dW += dY^T X, straight into the flat buffer
-            else:
-                gw = _alloc_like(w)
-                gemm(g2, x2, gw, a_mn=True, b_mn=True)             # dW[N,K] = dY^T[N,T] . X[T,K]
-        if ctx.has_bias and ctx.needs_input_grad[2]:
-            gb = colsum(g2).to(gy.dtype) if g2.shape[1] % 8 == 0 else g2.float().sum(0).to(gy.dtype)
-        gr = gy if (ctx.has_res and ctx.needs_input_grad[3]) else None
-        return gx, gw, gb, gr
 
 
 # ----------------------------------------------------------------------------- fp8 projections (per-tensor scaling)
@@ -692,7 +705,7 @@ def linear(x, w, bias=None, fp8: bool = False, residual=None):
     if not _is_bf16(x, w, bias, residual) or (w.shape[0] % 8) or (w.shape[1] % 8):
         y = ref.linear(x, w, bias)
         return y if residual is None else y + residual
-    return _Linear.apply(x, w, bias, residual)
+    return _native("linear", x, w, bias, residual)
 
 
 def linear_allgather(x, w, bias, seq_dim, fp8):
@@ -737,44 +750,6 @@ def _rmsnorm_bwd(x2, w, a, gy, gres, eps, form):
                               dw.data_ptr(), partial.data_ptr(), T, D, eps, form, _stream()), "rmsnorm_bwd")
     _count(2)
     return dx, dw
-
-
-class _RMSNorm(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, w, eps, form):
-        x2, wc, a, y = _rmsnorm_fwd(x, w, eps, form)
-        ctx.save_for_backward(x2, wc, a)
-        ctx.meta = (eps, form, x.shape)
-        return y.view(x.shape)
-
-    @staticmethod
-    def backward(ctx, gy):
-        x2, w, a = ctx.saved_tensors
-        eps, form, shape = ctx.meta
-        dx, dw = _rmsnorm_bwd(x2, w, a, gy, None, eps, form)
-        return dx.view(shape), dw, None, None
-
-
-class _RMSNormResidual(torch.autograd.Function):
-    """(norm(x), x): the second output carries x down the residual branch; the gradient arriving there is added inside
-    the norm's backward kernel instead of by a separate accumulation kernel."""
-
-    @staticmethod
-    def forward(ctx, x, w, eps, form):
-        x2, wc, a, y = _rmsnorm_fwd(x, w, eps, form)
-        ctx.save_for_backward(x2, wc, a)
-        ctx.meta = (eps, form, x.shape)
-        ctx.set_materialize_grads(False)
-        return y.view(x.shape), x.view_as(x)
-
-    @staticmethod
-    def backward(ctx, gy, gres):
-        x2, w, a = ctx.saved_tensors
-        eps, form, shape = ctx.meta
-        if gy is None:
-            return gres, None, None, None
-        dx, dw = _rmsnorm_bwd(x2, w, a, gy, gres, eps, form)
-        return dx.view(shape), dw, None, None
 
 
 def _fp8_backward_gemms(ctx_w, gy2, xq, sx, wq, sw, need_gx, need_gw, quantised=None):
@@ -1002,8 +977,19 @@ def mlp_gated(x, norm_weight, eps, form, w12, w3, b3, act, fp8):
     if (fp8 and act in _ACT and _fp8_fusable(x, w12, norm_weight, b3) and _is_bf16(w3) and 64 <= x.shape[-1] <= 16384
             and w3.shape[0] % 16 == 0 and w3.shape[1] % 16 == 0 and (w12.shape[0] // 2) % 16 == 0):
         return _MlpFP8.apply(x, norm_weight, float(eps), 0 if form == "te" else 1, w12, w3, b3, _ACT[act])
+    if not fp8 and act in _ACT and _norm_covers(x, norm_weight) and _is_bf16(w12, w3, b3) and _gemm_covers(w12) and _gemm_covers(w3) \
+            and (w12.shape[0] // 2) % 8 == 0 and w3.shape[0] == x.shape[-1] and w12.shape[0] == 2 * w3.shape[1]:
+        return _native("mlp_gated", x, norm_weight, float(eps), 0 if form == "te" else 1, w12, w3, b3, _ACT[act])
     ab, res = norm_linear(x, norm_weight, eps, form, w12, None, fp8)
     return glu_linear(ab, act, w3, b3, res, fp8)
+
+
+def _gemm_covers(w) -> bool:
+    return w.dim() == 2 and w.shape[0] % 8 == 0 and w.shape[1] % 8 == 0
+
+
+def _norm_covers(x, weight) -> bool:
+    return _is_bf16(x, weight) and x.shape[-1] % 8 == 0 and 64 <= x.shape[-1] <= 16384
 
 
 def _fp8_fusable(x, w, *others) -> bool:
@@ -1016,6 +1002,8 @@ def norm_linear(x, norm_weight, eps, form, w, bias, fp8):
     """(linear(rmsnorm(x)), x).  With fp8 projections and delayed scaling the norm emits the fp8 operand itself."""
     if fp8 and _fp8_fusable(x, w, norm_weight, bias) and 64 <= x.shape[-1] <= 16384:
         return _NormLinearFP8.apply(x, norm_weight, float(eps), 0 if form == "te" else 1, w, bias)
+    if not fp8 and _norm_covers(x, norm_weight) and _is_bf16(w, bias) and _gemm_covers(w):
+        return _native("norm_linear", x, norm_weight, float(eps), 0 if form == "te" else 1, w, bias)
     y, res = rmsnorm_residual(x, norm_weight, eps, form)
     return linear(y, w, bias, fp8), res
 
@@ -1029,52 +1017,25 @@ def glu_linear(ab, act, w, bias, residual, fp8):
 
 def rmsnorm_residual(x, weight, eps, form="te"):
     """(rmsnorm(x), x) with the two gradients combined in one backward kernel."""
-    if not _is_bf16(x, weight) or x.shape[-1] % 8 or x.shape[-1] > 16384 or x.shape[-1] < 64:
+    if not _norm_covers(x, weight):
         return ref.rmsnorm(x, weight, eps, form), x
-    return _RMSNormResidual.apply(x, weight, float(eps), 0 if form == "te" else 1)
+    return _native("rmsnorm_residual", x, weight, float(eps), 0 if form == "te" else 1)
 
 
 def rmsnorm(x, weight, eps, form="te"):
-    if not _is_bf16(x, weight) or x.shape[-1] % 8 or x.shape[-1] > 16384 or x.shape[-1] < 64:
+    if not _norm_covers(x, weight):
         return ref.rmsnorm(x, weight, eps, form)
-    return _RMSNorm.apply(x, weight, float(eps), 0 if form == "te" else 1)
+    return _native("rmsnorm", x, weight, float(eps), 0 if form == "te" else 1)
 
 
 # ----------------------------------------------------------------------------- gated activation
-
-
-class _GluPacked(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, ab, act):
-        lib = require()
-        ab2 = ab.reshape(-1, ab.shape[-1]).contiguous()
-        T, F2 = ab2.shape
-        Fh = F2 // 2
-        h = _alloc((T, Fh), dtype=bf16, device=ab.device)
-        _check(lib.sb_glu_fwd(ab2.data_ptr(), h.data_ptr(), T, Fh, act, _stream()), "glu_fwd")
-        _count()
-        ctx.save_for_backward(ab2)
-        ctx.meta = (act, ab.shape)
-        return h.view(*ab.shape[:-1], Fh)
-
-    @staticmethod
-    def backward(ctx, gh):
-        lib = require()
-        (ab2,) = ctx.saved_tensors
-        act, shape = ctx.meta
-        T, F2 = ab2.shape
-        g2 = gh.reshape(T, F2 // 2).contiguous()
-        dab = _alloc_like(ab2)
-        _check(lib.sb_glu_bwd(ab2.data_ptr(), g2.data_ptr(), dab.data_ptr(), T, F2 // 2, act, _stream()), "glu_bwd")
-        _count()
-        return dab.view(shape), None
 
 
 def glu_act_packed(ab, act="silu"):
     if not _is_bf16(ab) or (ab.shape[-1] // 2) % 8 or act not in _ACT:
         a, b = ab.chunk(2, dim=-1)
         return ref.glu_act(a, b, act)
-    return _GluPacked.apply(ab, _ACT[act])
+    return _native("glu", ab, _ACT[act])
 
 
 def glu_act(a, b, act="silu"):
@@ -1126,39 +1087,10 @@ def apply_rope(x, cos, sin):
 # ----------------------------------------------------------------------------- cross entropy
 
 
-class _CrossEntropy(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, logits, labels):
-        lib = require()
-        V = logits.shape[-1]
-        l2 = logits.reshape(-1, V).contiguous()
-        lab = labels.reshape(-1).contiguous()
-        T = l2.shape[0]
-        loss = _alloc(T, dtype=torch.float32, device=logits.device)
-        lse = _alloc(T, dtype=torch.float32, device=logits.device)
-        _check(lib.sb_ce_fwd(l2.data_ptr(), lab.data_ptr(), loss.data_ptr(), lse.data_ptr(), T, V, _stream()), "ce_fwd")
-        _count()
-        ctx.save_for_backward(l2, lab, lse)
-        ctx.shape = logits.shape
-        return loss.view(labels.shape)
-
-    @staticmethod
-    def backward(ctx, g):
-        lib = require()
-        l2, lab, lse = ctx.saved_tensors
-        T, V = l2.shape
-        gc = g.reshape(-1).float().contiguous()
-        dl = _alloc_like(l2)
-        _check(lib.sb_ce_bwd(l2.data_ptr(), lab.data_ptr(), lse.data_ptr(), gc.data_ptr(), dl.data_ptr(), T, V, _stream()),
-               "ce_bwd")
-        _count()
-        return dl.view(ctx.shape), None
-
-
 def cross_entropy(logits, labels):
     if not _is_bf16(logits) or logits.shape[-1] % 8 or labels.dtype != torch.int64:
         return ref.cross_entropy(logits, labels)
-    return _CrossEntropy.apply(logits, labels)
+    return _native("cross_entropy", logits, labels)
 
 
 # ----------------------------------------------------------------------------- optimizer pieces
@@ -1207,100 +1139,11 @@ def _aligned(t):
     return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
-def _taps(w):
-    """(taps as the forward kernel reads them, whether they are bf16, the fp32 copy that it writes for the backward or None).  A bf16
-    parameter is converted by the kernel that reads it, not by a launch of its own."""
-    if w.dtype != bf16:
-        return _f32c(w), 0, None
-    return w.detach().contiguous(), 1, _alloc(w.shape, dtype=torch.float32, device=w.device)
-
-
-class _DwConv(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, w, halo):
-        lib = require()
-        B, L, C = x.shape
-        K = w.shape[-1]
-        xc = _aligned(x)
-        hc = _aligned(halo) if halo is not None else None
-        wc, w_bf16, wf = _taps(w)
-        y = _alloc_like(xc)
-        if CONV_FWD_FAST:
-            _check(lib.sb_dwconv_fwd_taps(xc.data_ptr(), _ptr(hc), wc.data_ptr(), w_bf16, _ptr(wf), y.data_ptr(), B, L, C, K, _stream()),
-                   "dwconv_fwd")
-            wf = wc if wf is None else wf
-        else:
-            wf = _f32c(w)
-            _check(lib.sb_dwconv_fwd(xc.data_ptr(), _ptr(hc), wf.data_ptr(), y.data_ptr(), B, L, C, K, _stream()), "dwconv_fwd")
-        _count()
-        ctx.save_for_backward(xc, wf, hc if hc is not None else _alloc(0, device=x.device))
-        ctx.meta = (halo is not None, w.dtype)
-        return y
-
-    @staticmethod
-    def backward(ctx, gy):
-        lib = require()
-        xc, wf, hc = ctx.saved_tensors
-        has_halo, wdtype = ctx.meta
-        B, L, C = xc.shape
-        K = wf.shape[-1]
-        g = _aligned(gy)
-        dx = _alloc_like(xc)
-        dh = _alloc_like(hc) if has_halo else None
-        dw = _zeros_like(wf)
-        _check(lib.sb_dwconv_bwd(xc.data_ptr(), hc.data_ptr() if has_halo else None, wf.data_ptr(), g.data_ptr(),
-                                 dx.data_ptr(), _ptr(dh), dw.data_ptr(), B, L, C, K, _stream()), "dwconv_bwd")
-        _count()
-        return dx, dw.to(wdtype), dh
-
-
 def causal_conv1d(x, w, halo=None):
     K = w.shape[-1]
     if not _is_bf16(x, halo) or x.shape[-1] % 8 or not 2 <= K <= 8:
         return ref.causal_conv1d(x, w, halo)
-    return _DwConv.apply(x, w, halo)
-
-
-class _HyenaSE(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, feat, w, halo, pregate, postgate):
-        lib = require()
-        B, L, C3 = feat.shape
-        D = C3 // 3
-        G, K = w.shape
-        fc = _aligned(feat)
-        hc = _aligned(halo) if halo is not None else None
-        wc, w_bf16, wf = _taps(w)
-        z = _alloc((B, L, D), dtype=bf16, device=feat.device)
-        if CONV_FWD_FAST:
-            _check(lib.sb_se_fwd_taps(fc.data_ptr(), _ptr(hc), wc.data_ptr(), w_bf16, _ptr(wf), z.data_ptr(), B, L, D, G, K, int(pregate),
-                                      int(postgate), _stream()), "se_fwd")
-            wf = wc if wf is None else wf
-        else:
-            wf = _f32c(w)
-            _check(lib.sb_se_fwd(fc.data_ptr(), _ptr(hc), wf.data_ptr(), z.data_ptr(), B, L, D, G, K, int(pregate),
-                                 int(postgate), _stream()), "se_fwd")
-        _count()
-        ctx.save_for_backward(fc, wf, hc if hc is not None else _alloc(0, device=feat.device))
-        ctx.meta = (halo is not None, w.dtype, pregate, postgate)
-        return z
-
-    @staticmethod
-    def backward(ctx, gz):
-        lib = require()
-        fc, wf, hc = ctx.saved_tensors
-        has_halo, wdtype, pregate, postgate = ctx.meta
-        B, L, C3 = fc.shape
-        D = C3 // 3
-        G, K = wf.shape
-        g = _aligned(gz)
-        df = _alloc_like(fc)
-        dh = _alloc_like(hc) if has_halo else None
-        dw = _zeros_like(wf)
-        _check(lib.sb_se_bwd(fc.data_ptr(), hc.data_ptr() if has_halo else None, wf.data_ptr(), g.data_ptr(), df.data_ptr(),
-                             _ptr(dh), dw.data_ptr(), B, L, D, G, K, int(pregate), int(postgate), _stream()), "se_bwd")
-        _count()
-        return df, dw.to(wdtype), dh, None, None
+    return _native("dwconv", x, w, halo, CONV_FWD_FAST)
 
 
 def hyena_se_inner(feat, w, halo=None, pregate=True, postgate=True):
@@ -1308,61 +1151,7 @@ def hyena_se_inner(feat, w, halo=None, pregate=True, postgate=True):
     D = feat.shape[-1] // 3
     if not _is_bf16(feat, halo) or D % 8 or not 2 <= K <= 8:
         return ref.hyena_se_inner(feat, w, halo, pregate, postgate)
-    return _HyenaSE.apply(feat, w, halo, pregate, postgate)
-
-
-class _HyenaMR(torch.autograd.Function):
-    """Tensor-core kernels (csrc/mr_conv_tc.cu) when a 16-channel slab shares one filter (dg % 16 == 0), else the
-    CUDA-core kernels (csrc/mr_conv.cu)."""
-
-    @staticmethod
-    def forward(ctx, feat, h, bias, halo):
-        lib = require()
-        B, L, C3 = feat.shape
-        D = C3 // 3
-        G, K = h.shape
-        fc = _aligned(feat)
-        hc = _aligned(halo) if halo is not None else None
-        hf, bf = _f32c(h), _f32c(bias)
-        z = _alloc((B, L, D), dtype=bf16, device=feat.device)
-        tc = (D // G) % 16 == 0 and D % 8 == 0
-        y = None
-        if tc:
-            _check(lib.sb_mr_tc_fwd(fc.data_ptr(), _ptr(hc), hf.data_ptr(), bf.data_ptr(), z.data_ptr(), B, L, D, G, K,
-                                    _stream()), "mr_tc_fwd")
-        else:
-            y = _alloc_like(z) if any(ctx.needs_input_grad) else None
-            _check(lib.sb_mr_fwd(fc.data_ptr(), _ptr(hc), hf.data_ptr(), bf.data_ptr(), z.data_ptr(), _ptr(y), B, L, D, G, K,
-                                 _stream()), "mr_fwd")
-        _count()
-        empty = _alloc(0, device=feat.device)
-        ctx.save_for_backward(fc, hf, bf, y if y is not None else empty, hc if hc is not None else empty)
-        ctx.meta = (halo is not None, h.dtype, bias.dtype, tc)
-        return z
-
-    @staticmethod
-    def backward(ctx, gz):
-        lib = require()
-        fc, hf, bf, y, hc = ctx.saved_tensors
-        has_halo, hdtype, bdtype, tc = ctx.meta
-        B, L, C3 = fc.shape
-        D = C3 // 3
-        G, K = hf.shape
-        g = _aligned(gz)
-        df = _alloc_like(fc)
-        dhalo = _zeros_like(hc) if has_halo else None
-        dh = _zeros_like(hf)
-        db = _zeros_like(bf)
-        hp = hc.data_ptr() if has_halo else None
-        if tc:
-            _check(lib.sb_mr_tc_bwd(fc.data_ptr(), hp, hf.data_ptr(), bf.data_ptr(), g.data_ptr(), df.data_ptr(), _ptr(dhalo),
-                                    dh.data_ptr(), db.data_ptr(), B, L, D, G, K, _stream()), "mr_tc_bwd")
-            _count()
-        else:
-            _check(lib.sb_mr_bwd(fc.data_ptr(), hp, hf.data_ptr(), bf.data_ptr(), g.data_ptr(), y.data_ptr(), df.data_ptr(),
-                                 _ptr(dhalo), dh.data_ptr(), db.data_ptr(), B, L, D, G, K, _stream()), "mr_bwd")
-            _count(2)
-        return df, dh.to(hdtype), db.to(bdtype), dhalo
+    return _native("hyena_se", feat, w, halo, bool(pregate), bool(postgate), CONV_FWD_FAST)
 
 
 def hyena_mr_inner(feat, h, bias, halo=None):
@@ -1371,7 +1160,7 @@ def hyena_mr_inner(feat, h, bias, halo=None):
     dg = D // G
     if not _is_bf16(feat, halo) or K > 128 or D % G or ((64 % dg) and (dg % 64)):
         return ref.hyena_mr_inner(feat, h, bias, halo)
-    return _HyenaMR.apply(feat, h, bias, halo)
+    return _native("hyena_mr", feat, h, bias, halo)
 
 
 # ----------------------------------------------------------------------------- Hyena-LI (modal scan)
@@ -1433,7 +1222,9 @@ def _pad_order(t, fill):
 
 class _HyenaLITiled(torch.autograd.Function):
     """The shared-memory tiled scan (csrc/li_scan.cu): D % 8 == 0.  The filter is prepared by the forward's first kernel and
-    handed to the backward; the filter gradients come finished out of the backward's last one."""
+    handed to the backward; the filter gradients come finished out of the backward's last one.  CUDA tensors take the same
+    steps in C++ (HyenaLI in csrc/autograd_native.cpp); this form calls whatever library `require` returns, which lets a stand-in
+    for it see without a GPU what the kernels are handed."""
 
     @staticmethod
     def forward(ctx, feat, gamma, R, p, bias, state_in, want_state):
@@ -1579,6 +1370,11 @@ def hyena_li_modal(feat, gamma, R, p, bias, state_in=None, return_state=False):
             state_in = _spread(state_in, (B, D, O), feat.device)
     if feat.dtype != bf16 or O > LI_ORDER:
         return ref.hyena_li_modal(feat, gamma, R, p, bias, state_in, return_state)
-    fn = _HyenaLITiled if LI_TILED and C3 % 24 == 0 and B * L > 0 else _HyenaLI
-    z, s = fn.apply(feat, gamma, R, p, bias, state_in, return_state)
+    if LI_TILED and C3 % 24 == 0 and B * L > 0:
+        if feat.is_cuda:
+            z, s = _native("hyena_li", feat, gamma, R, p, bias, state_in, bool(return_state), _li_tiled_chunk(B, L, D))
+        else:
+            z, s = _HyenaLITiled.apply(feat, gamma, R, p, bias, state_in, return_state)
+    else:
+        z, s = _HyenaLI.apply(feat, gamma, R, p, bias, state_in, return_state)
     return (z, s) if return_state else z

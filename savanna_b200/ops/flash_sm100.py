@@ -37,8 +37,6 @@ def _lib():
         lib.sb_attn_set_fwd_variant.argtypes = [I]
         lib.sb_attn_set_fwd_p_tmem.restype = I
         lib.sb_attn_set_fwd_p_tmem.argtypes = [I]
-        lib.sb_attn_rope.restype = I
-        lib.sb_attn_rope.argtypes = [P, P, P, P, P, I, P, P, I, I, I, I, I, P]
         lib.sb_attn_merge_fwd.restype = I
         lib.sb_attn_merge_fwd.argtypes = [P, P, P, P, I, I, I, I, P, P, P]
         lib.sb_attn_merge_bwd.restype = I
@@ -157,59 +155,6 @@ class _Flash(torch.autograd.Function):
         return dq, dk, dv, None
 
 
-def _rope(pairs, cos, sin, inverse):
-    """Rotary embedding of one or two tensors in one launch: pairs of (source [B, L, H, 128] bf16 or fp32, bf16 destination,
-    which may be the source)."""
-    n = len(pairs)
-    B, L, H, _ = pairs[0][0].shape
-    P, LL = ctypes.c_void_p * n, ctypes.c_longlong * (3 * n)
-    rc = _lib().sb_attn_rope(P(*[s.data_ptr() for s, _ in pairs]), P(*[d.data_ptr() for _, d in pairs]),
-                             LL(*[v for s, _ in pairs for v in s.stride()[:3]]), LL(*[v for _, d in pairs for v in d.stride()[:3]]),
-                             (ctypes.c_int * n)(*[int(s.dtype == torch.float32) for s, _ in pairs]), n, cos.data_ptr(), sin.data_ptr(),
-                             B, L, H, cos.shape[-1], int(inverse), cuda_ops._stream())
-    if rc != 0:
-        raise RuntimeError(f"rotary embedding failed (code {rc}): {[(tuple(s.shape), s.stride(), d.stride()) for s, d in pairs]}")
-    cuda_ops._count()
-
-
-class _FlashPacked(torch.autograd.Function):
-    """Attention on the packed projection qkv [B, L, H, 3*128] (per head: q, k, v) with rotary embedding of q and k inside
-    the function.  The backward writes dq, dk, dv straight into one packed gradient buffer: the slice / concatenate
-    bookkeeping of autograd (a zero fill, a strided copy and an add per slice) does not run."""
-
-    @staticmethod
-    def forward(ctx, qkv, cos, sin, causal):
-        B, L, H, _ = qkv.shape
-        q, k, v = qkv[..., :128], qkv[..., 128:256], qkv[..., 256:]
-        if cos is not None:
-            qr, kr = (_alloc((B, L, H, 128), dtype=torch.bfloat16, device=qkv.device) for _ in range(2))
-            _rope([(q, qr), (k, kr)], cos, sin, False)
-            q, k = qr, kr
-        scale = 1.0 / math.sqrt(128)
-        out, lse = forward(q, k, v, causal, scale)
-        ctx.save_for_backward(qkv, q if cos is not None else None, k if cos is not None else None, out, lse, cos, sin)
-        ctx.causal, ctx.scale = causal, scale
-        return out
-
-    @staticmethod
-    def backward(ctx, go):
-        qkv, q, k, out, lse, cos, sin = ctx.saved_tensors
-        rot = cos is not None
-        if not rot:
-            q, k = qkv[..., :128], qkv[..., 128:256]
-        v = qkv[..., 256:]
-        dqkv = _alloc(tuple(qkv.shape), dtype=torch.bfloat16, device=qkv.device)
-        dq_dst, dk_dst, dv_dst = dqkv[..., :128], dqkv[..., 128:256], dqkv[..., 256:]
-        if rot:
-            # the query gradient is rotated back out of its fp32 accumulator, the key gradient in place
-            dq_acc = _zeros(tuple(q.shape), dtype=torch.float32, device=qkv.device)
-            backward(go, q, k, v, out, lse, ctx.causal, ctx.scale, dq_acc=dq_acc, dk=dk_dst, dv=dv_dst)
-            _rope([(dq_acc, dq_dst), (dk_dst, dk_dst)], cos, sin, True)
-        else:
-            backward(go, q, k, v, out, lse, ctx.causal, ctx.scale, dq=dq_dst, dk=dk_dst, dv=dv_dst)
-        return dqkv, None, None, None
-
-
 def packed_supported(qkv) -> bool:
     return (qkv.dim() == 4 and qkv.dtype == torch.bfloat16 and qkv.is_cuda and qkv.shape[-1] == 384 and qkv.is_contiguous()
             and qkv.data_ptr() % 16 == 0)
@@ -217,9 +162,7 @@ def packed_supported(qkv) -> bool:
 
 def attention_packed(qkv, cos, sin, causal):
     """qkv [B, L, H, 384] bf16 contiguous; cos / sin [L, rd] fp32 (or None for no rotary embedding) -> [B, L, H, 128]."""
-    if cos is not None:
-        cos, sin = cuda_ops._aligned(cos.float()), cuda_ops._aligned(sin.float())
-    return _FlashPacked.apply(qkv, cos, sin, causal)
+    return cuda_ops._native("attention_packed", qkv, cos, sin, bool(causal))
 
 
 def attention(q, k, v, causal, return_lse=False):

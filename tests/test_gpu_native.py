@@ -1,0 +1,125 @@
+"""The C++ autograd functions (csrc/autograd_native.cpp): the nodes that join several operators against the operators one by one, which
+inputs get gradients, tracing, saved-tensor hooks, and what autograd refuses."""
+import itertools
+
+import pytest
+import torch
+
+from savanna_b200 import ops
+
+pytestmark = pytest.mark.gpu
+DEV, BF = "cuda", torch.bfloat16
+
+
+def _rand(*shape, std=1.0):
+    return (torch.randn(*shape, device=DEV) * std).to(BF)
+
+
+def _grads(fn, tensors, needs, gout):
+    leaves = [None if t is None else t.clone().requires_grad_(n) for t, n in zip(tensors, needs)]
+    out = fn(*leaves)
+    out.backward(gout)
+    return [out.detach()] + [None if t is None else t.grad for t in leaves]
+
+
+@pytest.mark.parametrize("T,D,F,bias", [(1, 64, 8, False), (37, 256, 704, True), (999, 1024, 2816, False)])
+@pytest.mark.parametrize("act", ["silu", "gelu"])
+def test_mlp_is_its_parts(T, D, F, bias, act):
+    torch.manual_seed(T)
+    ts = [_rand(1, T, D), _rand(D), _rand(2 * F, D, std=D ** -0.5), _rand(D, F, std=F ** -0.5), _rand(D) if bias else None]
+    g = _rand(1, T, D)
+
+    def parts(x, wn, w12, w3, b3):
+        y, res = ops.rmsnorm_residual(x, wn, 1e-6)
+        return ops.linear(ops.glu_act_packed(ops.linear(y, w12), act), w3, b3, residual=res)
+
+    def whole(x, wn, w12, w3, b3):
+        return ops.mlp_gated(x, wn, 1e-6, "te", w12, w3, b3, act)
+
+    for needs in ([True] * 5, [False, False, True, False, False], [False, True, False, False, False], [False, False, False, True, bias]):
+        for a, b in zip(_grads(whole, ts, needs, g), _grads(parts, ts, needs, g)):
+            assert (a is None) == (b is None)
+            # the same kernels on the same values; only the bias gradient is summed with atomics: fp32 sums, rounded once to bf16
+            assert a is None or torch.equal(a, b) or (a.float() - b.float()).norm() <= 2 ** -9 * b.float().norm()
+
+
+@pytest.mark.parametrize("bias", [False, True])
+def test_norm_and_projection_are_their_parts(bias):
+    torch.manual_seed(3)
+    ts = [_rand(2, 77, 512), _rand(512), _rand(1536, 512, std=0.05), _rand(1536) if bias else None]
+    for needs in itertools.product([False, True], repeat=3):
+        if not any(needs):
+            continue
+        got = []
+        for one in (True, False):
+            leaves = [None if t is None else t.clone().requires_grad_(n) for t, n in zip(ts, needs + (needs[2] and bias,))]
+            x, wn, w, b = leaves
+            if one:
+                y, res = ops.norm_linear(x, wn, 1e-6, "te", w, b)
+            else:
+                u, res = ops.rmsnorm_residual(x, wn, 1e-6)
+                y = ops.linear(u, w, b)
+            (y.float().square().mean() + (res * 0.5).float().square().sum()).backward()
+            got.append([y.detach(), res.detach()] + [None if t is None else t.grad for t in leaves])
+        for a, b in zip(*got):
+            assert (a is None) == (b is None)
+            assert a is None or torch.equal(a, b) or (a.float() - b.float()).norm() <= 2 ** -9 * b.float().norm()
+
+
+def test_only_the_residual_branch_is_used():
+    x = _rand(2, 8, 128).requires_grad_()
+    _, res = ops.norm_linear(x, _rand(128), 1e-6, "te", _rand(64, 128))
+    res.float().sum().backward()
+    assert torch.equal(x.grad, torch.ones_like(x))
+
+
+def _block(x, wn, w):
+    return ops.linear(ops.rmsnorm(x, wn, 1e-6), w).float().square().sum()
+
+
+def test_traced_graph_runs_the_kernels_on_new_inputs():
+    wn, w = _rand(256), _rand(512, 256, std=0.05)
+    f = torch.jit.trace(lambda t: _block(t, wn, w), (_rand(4, 256).requires_grad_(),), check_trace=False)
+    x = _rand(4, 256)
+    a, b = x.clone().requires_grad_(), x.clone().requires_grad_()
+    ya, yb = f(a), _block(b, wn, w)
+    ya.backward()
+    yb.backward()
+    assert torch.equal(ya, yb) and torch.equal(a.grad, b.grad)
+
+
+def test_saved_tensor_hooks_see_every_saved_tensor():
+    n = [0, 0]
+
+    def pack(t):
+        n[0] += 1
+        return t.cpu()
+
+    def unpack(t):
+        n[1] += 1
+        return t.cuda()
+    wn, w, x = _rand(256), _rand(512, 256, std=0.05), _rand(4, 256)
+    a, b = x.clone().requires_grad_(), x.clone().requires_grad_()
+    with torch.autograd.graph.saved_tensors_hooks(pack, unpack):
+        y, _ = ops.norm_linear(a, wn, 1e-6, "te", w)
+    y.float().sum().backward()
+    ops.norm_linear(b, wn, 1e-6, "te", w)[0].float().sum().backward()
+    assert n == [5, 5] and torch.equal(a.grad, b.grad)
+
+
+def test_refusals():
+    x, wn, w = _rand(4, 256), _rand(256), _rand(512, 256)
+    with pytest.raises(RuntimeError):
+        torch.vmap(lambda t: ops.rmsnorm(t, wn, 1e-6))(torch.stack([x, x]))
+    with pytest.raises(RuntimeError):
+        torch.func.grad(lambda t: _block(t, wn, w))(x)
+    a, v = x.clone().requires_grad_(), w.clone().requires_grad_()
+    y = ops.linear(a, v)
+    with torch.no_grad():
+        v.mul_(2)
+    with pytest.raises(RuntimeError):
+        y.sum().backward()                           # a saved operand was changed
+    z = _block(a, wn, w)
+    z.backward()
+    with pytest.raises(RuntimeError):
+        z.backward()                                 # the saved tensors are gone
