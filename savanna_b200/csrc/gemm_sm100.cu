@@ -23,12 +23,9 @@
 
 namespace sb {
 
-constexpr int BM = 128, BN = 256, BK = 64, STAGES = 4;
-constexpr int UMMA_K = 16;
+constexpr int BM = 128, BN = 256, BK = 64;
 constexpr int A_STAGE = BM * BK * 2;              // 16 KB
-constexpr int B_STAGE = BN * BK * 2;              // 32 KB
-constexpr int STAGE_BYTES = A_STAGE + B_STAGE;    // 48 KB
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+constexpr int SMEM_BYTES = 4 * 48 * 1024 + 1024 /*align*/ + 256 /*barriers*/;
 constexpr int TMEM_COLS = 512;
 constexpr int GROUP_M = 16;                       // raster: 16 m-tiles share the concurrently running n-tiles
 constexpr int NUM_THREADS = 192;
@@ -109,9 +106,12 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, int row, int co
 
 // EB = bytes per operand element: 2 = bf16 (kind::f16), 1 = fp8 e4m3 / e5m2 (kind::f8f6f4).  A shared-memory row is
 // always 128 bytes, so a k-block holds 64 bf16 or 128 fp8 values and every MMA consumes 32 bytes of K.
-template <int A_MN, int B_MN, int EB>
+// BN = tile width: 256, or 128 / 64 for outputs with too few 256-wide tiles to fill the chip (see pick_tile); the same
+// 192 KB of shared memory then hold 6 / 8 stages.
+template <int A_MN, int B_MN, int EB, int BN = 256>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmParams p) {
+  constexpr int B_STAGE = BN * 128, STAGE_BYTES = A_STAGE + B_STAGE, STAGES = 4 * 48 * 1024 / STAGE_BYTES;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -620,6 +620,46 @@ static int g_last_detail = 0;   // (which operand << 16) | CUresult of the last 
 
 static int g_pair_mode = 2;      // 1: CTA-pair kernel for one-byte operands, 2: for every GEMM, 0: never
 
+// Tile of a GEMM on `sms` SMs: 0 = the CTA-pair kernel's 256 x 256, or the width of a single-CTA tile 128 x {128, 64}, for
+// outputs with too few 256 x 256 tiles to fill the chip.  Compared are waves times cycles of a tile per 128-byte k-block: an SM
+// pair spends 512 on its 256 x 256 tile; a single-CTA tile is bound by shared memory, which takes both operands in and reads
+// them once (32 KB a k-block: 256 cycles and their share of latency, 320; 24 KB: 260).  A narrower tile has to win by an
+// eighth, because it reads its operands more often.  Kernel times, us, pair -> chosen: [999 x 1024] K = 5632 34 -> 18 and
+// K = 2816 27 -> 13 (64 wide), [512 x 4096] K = 8192 48 -> 37 (128 wide), weight gradients of a 256-wide model 18 -> 9;
+// [999 x 5632] K = 1024 keeps the pair (128 wide: 17 against 15 to 20).  `b_box128`: B comes in boxes of 128 columns (one-byte
+// MN-major operand), 64 is not possible.
+static int pick_tile(int M, int N, int sms, bool b_box128) {
+  const long long m1 = (M + 127) / 128, m2 = (M + 255) / 256;
+  auto waves = [](long long tiles, long long slots) { return (tiles + slots - 1) / slots; };
+  const long long pair = waves(m2 * ((N + 255) / 256), sms / 2) * 512;
+  const long long w128 = waves(m1 * ((N + 127) / 128), sms) * 320, w64 = waves(m1 * ((N + 63) / 64), sms) * 260;
+  if (8 * (w64 < w128 && !b_box128 ? w64 : w128) > 7 * pair) return 0;
+  return 8 * w64 <= 7 * w128 && !b_box128 ? 64 : 128;
+}
+
+// Launch the single-CTA kernel with tile width BNT.
+template <int EB, int BNT>
+static int launch_single(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, int a_mn, int b_mn, int max_ctas,
+                         cudaStream_t stream) {
+  const int tiles = ((p.M + BM - 1) / BM) * ((p.N + BNT - 1) / BNT);
+  int grid = tiles < g_num_sms ? tiles : g_num_sms;
+  if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
+  void (*kern)(const CUtensorMap, const CUtensorMap, GemmParams);
+  constexpr int BN_MN = EB == 1 && BNT < 128 ? 128 : BNT;          // never chosen (see pick_tile), but instantiated
+  if (!a_mn && !b_mn) kern = gemm_bf16_kernel<0, 0, EB, BNT>;
+  else if (!a_mn && b_mn) kern = gemm_bf16_kernel<0, 1, EB, BN_MN>;
+  else if (a_mn && b_mn) kern = gemm_bf16_kernel<1, 1, EB, BN_MN>;
+  else kern = gemm_bf16_kernel<1, 0, EB, BNT>;
+  static bool attr_set[4] = {false, false, false, false};
+  const int idx = a_mn * 2 + b_mn;
+  if (!attr_set[idx]) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess) return -5;
+    attr_set[idx] = true;
+  }
+  kern<<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(tmA, tmB, p);
+  return cudaGetLastError() == cudaSuccess ? 0 : -6;
+}
+
 // Launch the CTA-pair kernel (cluster of 2) on tensor maps whose boxes are 128 rows (K-major) / 128-byte MN boxes.
 template <int EB>
 static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, int a_mn, int b_mn,
@@ -672,42 +712,28 @@ extern "C" int sb_gemm_bf16(const void* A, const void* B, void* C, const void* b
   // K only has to be a multiple of 8 where it is the contiguous dim of an operand (a K-major one)
   if ((N % 8) || (lda % 8) || (ldb % 8) || (ldc % 8) || ((!a_mn || !b_mn) && (K % 8))) return -3;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 15) return -4;
-  CUtensorMap tmA, tmB;
-  int rc;
-  if (!a_mn) rc = make_tmap_2d_bf16(&tmA, A, K, M, lda, BK, BM);
-  else       rc = make_tmap_2d_bf16(&tmA, A, M, K, lda, 64, BK);
-  if (rc) { g_last_detail = (1 << 16) | (g_last_encode_result & 0xffff); return rc; }
-  if (!b_mn) rc = make_tmap_2d_bf16(&tmB, B, K, N, ldb, BK, BN);
-  else       rc = make_tmap_2d_bf16(&tmB, B, N, K, ldb, 64, BK);
-  if (rc) { g_last_detail = (2 << 16) | (g_last_encode_result & 0xffff); return rc; }
   if (!g_num_sms) {
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
   }
+  const bool paired = g_pair_mode >= 2 && max_ctas <= 0;
+  const int width = paired ? pick_tile(M, N, g_num_sms, false) : BN;
+  CUtensorMap tmA, tmB;
+  int rc;
+  if (!a_mn) rc = make_tmap_2d_bf16(&tmA, A, K, M, lda, BK, BM);
+  else       rc = make_tmap_2d_bf16(&tmA, A, M, K, lda, 64, BK);
+  if (rc) { g_last_detail = (1 << 16) | (g_last_encode_result & 0xffff); return rc; }
+  if (!b_mn) rc = make_tmap_2d_bf16(&tmB, B, K, N, ldb, BK, width ? width : 128);      // a pair: 128 B rows per CTA
+  else       rc = make_tmap_2d_bf16(&tmB, B, N, K, ldb, 64, BK);
+  if (rc) { g_last_detail = (2 << 16) | (g_last_encode_result & 0xffff); return rc; }
   if (residual && ((ldr % 8) || (reinterpret_cast<uintptr_t>(residual) & 15))) return -4;
   GemmParams p{reinterpret_cast<__nv_bfloat16*>(C), reinterpret_cast<const __nv_bfloat16*>(bias),
                reinterpret_cast<const __nv_bfloat16*>(residual), M, N, K, ldc, ldr, beta, status, nullptr, nullptr, 0, 0};
-  if (g_pair_mode >= 2 && max_ctas <= 0) {
-    if (!b_mn && (rc = make_tmap_2d_bf16(&tmB, B, K, N, ldb, BK, 128))) return rc;     // 128 B rows per CTA of the pair
-    return launch_pair<2>(tmA, tmB, p, a_mn, b_mn, stream);
-  }
-  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  int grid = tiles < g_num_sms ? tiles : g_num_sms;
-  if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
-  void (*kern)(const CUtensorMap, const CUtensorMap, GemmParams);
-  if (!a_mn && !b_mn) kern = gemm_bf16_kernel<0, 0, 2>;
-  else if (!a_mn && b_mn) kern = gemm_bf16_kernel<0, 1, 2>;
-  else if (a_mn && b_mn) kern = gemm_bf16_kernel<1, 1, 2>;
-  else kern = gemm_bf16_kernel<1, 0, 2>;
-  static bool attr_set[4] = {false, false, false, false};
-  const int idx = a_mn * 2 + b_mn;
-  if (!attr_set[idx]) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess) return -5;
-    attr_set[idx] = true;
-  }
-  kern<<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(tmA, tmB, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -6;
+  if (width == 0) return launch_pair<2>(tmA, tmB, p, a_mn, b_mn, stream);
+  if (width == 64) return launch_single<2, 64>(tmA, tmB, p, a_mn, b_mn, 0, stream);
+  if (width == 128) return launch_single<2, 128>(tmA, tmB, p, a_mn, b_mn, 0, stream);
+  return launch_single<2, 256>(tmA, tmB, p, a_mn, b_mn, max_ctas, stream);
 }
 
 // Gate projection of the gated MLP with the gate in the epilogue (CTA-pair kernel, GLU mode): AB [M, 2 F] bf16 =
@@ -807,35 +833,21 @@ extern "C" int sb_gemm_fp8(const void* A, const void* B, void* C, const void* bi
   if (!ctx_bound) { cudaFree(0); ctx_bound = true; }
   if ((N % 8) || (lda % 16) || (ldb % 16) || (ldc % 8) || ((!a_mn || !b_mn) && (K % 16))) return -3;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 15) return -4;
+  if (!g_num_sms) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev); }
+  const int width = g_pair_mode >= 1 ? pick_tile(M, N, g_num_sms, b_mn != 0) : BN;
   CUtensorMap tmA, tmB;
   int rc;
   if (!a_mn) rc = make_tmap_2d_u8(&tmA, A, K, M, lda, 128, BM);
   else       rc = make_tmap_2d_u8(&tmA, A, M, K, lda, 128, 128);
   if (rc) { g_last_detail = (1 << 16) | (g_last_encode_result & 0xffff); return rc; }
-  if (!b_mn) rc = make_tmap_2d_u8(&tmB, B, K, N, ldb, 128, BN);
+  if (!b_mn) rc = make_tmap_2d_u8(&tmB, B, K, N, ldb, 128, width ? width : 128);       // a pair: 128 B rows per CTA
   else       rc = make_tmap_2d_u8(&tmB, B, N, K, ldb, 128, 128);
   if (rc) { g_last_detail = (2 << 16) | (g_last_encode_result & 0xffff); return rc; }
-  if (!g_num_sms) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev); }
   if (residual && ((ldr % 8) || (reinterpret_cast<uintptr_t>(residual) & 15))) return -4;
   GemmParams p{reinterpret_cast<__nv_bfloat16*>(C), reinterpret_cast<const __nv_bfloat16*>(bias),
                reinterpret_cast<const __nv_bfloat16*>(residual), M, N, K, ldc, ldr, beta, status, alpha, alpha2, a_fmt, b_fmt};
-  if (g_pair_mode >= 1) {
-    if (!b_mn && (rc = make_tmap_2d_u8(&tmB, B, K, N, ldb, 128, 128))) return rc;      // 128 B rows per CTA of the pair
-    return launch_pair<1>(tmA, tmB, p, a_mn, b_mn, stream);
-  }
-  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  const int grid = tiles < g_num_sms ? tiles : g_num_sms;
-  void (*kern)(const CUtensorMap, const CUtensorMap, GemmParams);
-  if (!a_mn && !b_mn) kern = gemm_bf16_kernel<0, 0, 1>;
-  else if (!a_mn && b_mn) kern = gemm_bf16_kernel<0, 1, 1>;
-  else if (a_mn && b_mn) kern = gemm_bf16_kernel<1, 1, 1>;
-  else kern = gemm_bf16_kernel<1, 0, 1>;
-  static bool attr_set[4] = {false, false, false, false};
-  const int idx = a_mn * 2 + b_mn;
-  if (!attr_set[idx]) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess) return -5;
-    attr_set[idx] = true;
-  }
-  kern<<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(tmA, tmB, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -6;
+  if (width == 0) return launch_pair<1>(tmA, tmB, p, a_mn, b_mn, stream);
+  if (width == 64) return launch_single<1, 64>(tmA, tmB, p, a_mn, b_mn, 0, stream);
+  if (width == 128) return launch_single<1, 128>(tmA, tmB, p, a_mn, b_mn, 0, stream);
+  return launch_single<1, 256>(tmA, tmB, p, a_mn, b_mn, 0, stream);
 }

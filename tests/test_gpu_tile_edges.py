@@ -466,3 +466,21 @@ def test_rmsnorm_rows_in_pairs(T, D, form):
     # fp32 sums, one bf16 rounding of each result: 2^-9
     for got, want, n in ((y, yr, "y"), (a.grad, ar.grad, "dx"), (b.grad, br.grad, "dw")):
         _close(got, want, 4e-3, n)
+
+
+# outputs with few 256 x 256 tiles take 128 x 128 or 128 x 64 tiles: partial tiles in both directions, contractions shorter than the ring
+# of stages and with a ragged end, every operand order, bias, residual and accumulation
+@pytest.mark.parametrize("M,N,K", [(8, 8, 8), (999, 1024, 2816), (130, 72, 64), (512, 4096, 1000), (768, 256, 2048), (1, 200, 4096), (257, 136, 520)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
+def test_gemm_narrow_tiles(M, N, K, a_mn, b_mn):
+    from savanna_b200.ops import cuda_ops
+    torch.manual_seed(M + N)
+    if (a_mn and M % 8) or (b_mn and N % 8):
+        pytest.skip("rows of a transposed operand start on 16-byte boundaries")
+    a, b = torch.randn(M, K, device=DEV).to(BF), torch.randn(N, K, device=DEV).to(BF)
+    bias, res = torch.randn(N, device=DEV).to(BF), torch.randn(M, N, device=DEV).to(BF)
+    out = res.clone()
+    cuda_ops.gemm(a.t().contiguous() if a_mn else a, b.t().contiguous() if b_mn else b, out, a_mn, b_mn, bias=bias, accumulate=True, residual=res)
+    want = a.float() @ b.float().t() + bias.float() + 2 * res.float()
+    # fp32 accumulation, one bf16 rounding (two where the old value is added after the first): 2^-8
+    _close(out, want, 8e-3, "gemm")
