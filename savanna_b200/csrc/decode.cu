@@ -28,6 +28,8 @@
 
 #include <type_traits>
 
+#include "pdl.cuh"
+
 namespace sb {
 namespace dec {
 namespace cg = cooperative_groups;
@@ -37,6 +39,7 @@ constexpr int MAX_B = 8;
 constexpr int THREADS = 256;
 constexpr int ROWS_PER_WARP = 2;
 constexpr int ROWS_PER_BLOCK = THREADS / 32 * ROWS_PER_WARP;
+constexpr int AHEAD = 4;               // 16-byte weight loads per row and lane before the inputs are there: rows of up to 1024
 constexpr int HD = 128;                // head dimension of dec_attn
 constexpr int SPLIT = 8;               // blocks per head
 constexpr int ATT_THREADS = 128;
@@ -107,6 +110,8 @@ struct Taps {
   }
 };
 
+// The kernels of a step are a chain of programmatic dependents (pdl.cuh): weights, filters, caches and states, which earlier steps left,
+// are loaded ahead.
 struct LinArgs {
   const bf16* x;          // [B, K] (IN_GATE: [B, 2K] = [a | b])
   const bf16* norm_w;
@@ -124,6 +129,19 @@ dec_linear_kernel(LinArgs a) {
   extern __shared__ __align__(16) uint32_t xs[];          // [BT][K / 2] packed bf16
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, kv = a.K / 8;
   uint4* xv = reinterpret_cast<uint4*>(xs);
+  let_next_start();
+  const int n0 = (blockIdx.x * (THREADS / 32) + warp) * ROWS_PER_WARP;
+  const uint4* wr[ROWS_PER_WARP];
+#pragma unroll
+  for (int r = 0; r < ROWS_PER_WARP; ++r) wr[r] = reinterpret_cast<const uint4*>(a.W + (size_t)min(n0 + r, a.N - 1) * a.K);
+  // the first weights are on their way while the kernel before this one runs
+  uint4 ahead[AHEAD][ROWS_PER_WARP];
+#pragma unroll
+  for (int k = 0; k < AHEAD; ++k)
+#pragma unroll
+    for (int r = 0; r < ROWS_PER_WARP; ++r)
+      ahead[k][r] = lane + 32 * k < kv ? __ldg(wr[r] + lane + 32 * k) : make_uint4(0, 0, 0, 0);
+  wait_for_previous();
   if (a.mode == IN_NORM) {
     if (warp < BT) {
       const int b = warp;
@@ -175,21 +193,13 @@ dec_linear_kernel(LinArgs a) {
     }
   }
   __syncthreads();
-  const int n0 = (blockIdx.x * (THREADS / 32) + warp) * ROWS_PER_WARP;
   if (n0 >= a.N) return;
-  const uint4* wr[ROWS_PER_WARP];
-#pragma unroll
-  for (int r = 0; r < ROWS_PER_WARP; ++r) wr[r] = reinterpret_cast<const uint4*>(a.W + (size_t)min(n0 + r, a.N - 1) * a.K);
   float acc[ROWS_PER_WARP][BT];
 #pragma unroll
   for (int r = 0; r < ROWS_PER_WARP; ++r)
 #pragma unroll
     for (int b = 0; b < BT; ++b) acc[r][b] = 0.f;
-#pragma unroll 4
-  for (int i = lane; i < kv; i += 32) {
-    uint4 w[ROWS_PER_WARP];
-#pragma unroll
-    for (int r = 0; r < ROWS_PER_WARP; ++r) w[r] = __ldg(wr[r] + i);
+  auto use = [&](const uint4 (&w)[ROWS_PER_WARP], int i) {
 #pragma unroll
     for (int b = 0; b < BT; ++b) {
       const uint4 x = xv[b * kv + i];
@@ -205,6 +215,16 @@ dec_linear_kernel(LinArgs a) {
         }
       }
     }
+  };
+#pragma unroll
+  for (int k = 0; k < AHEAD; ++k)
+    if (lane + 32 * k < kv) use(ahead[k], lane + 32 * k);
+#pragma unroll 4
+  for (int i = lane + 32 * AHEAD; i < kv; i += 32) {
+    uint4 w[ROWS_PER_WARP];
+#pragma unroll
+    for (int r = 0; r < ROWS_PER_WARP; ++r) w[r] = __ldg(wr[r] + i);
+    use(w, i);
   }
 #pragma unroll
   for (int r = 0; r < ROWS_PER_WARP; ++r) {
@@ -228,31 +248,51 @@ dec_linear_kernel(LinArgs a) {
 // width 1024, two sequences, against 8.3 (average of all three) with a test of Layer::f32 at every load, which keeps the loads
 // from being issued together, and everything after the barrier.
 constexpr int HY_SLICES = 8;
+__device__ __forceinline__ float tap_at(const float (&t)[4], int j) { return j == 0 ? t[0] : j == 1 ? t[1] : j == 2 ? t[2] : t[3]; }
 template <int CONV, int FILT>
 __global__ void __launch_bounds__(32 * HY_SLICES)
-dec_hyena_kernel(Layer l, const bf16* __restrict__ proj, bf16* __restrict__ z, int pos) {
+dec_hyena_kernel(Layer l, const bf16* proj, bf16* z, int pos) {
   __shared__ float su[32], sx1[32], sb[32], part[HY_SLICES][32];
   const int cx = threadIdx.x & 31, sl = threadIdx.x >> 5, ch = blockIdx.x * 32 + cx, b = blockIdx.y;
   const bool live = ch < l.H;
+  let_next_start();
   if (sl == 0 && live) {
     float f[3];
     const int n = l.kf - 1;
+    constexpr int TAPS = 4;                                // featuriser taps loaded ahead, with the past rows they multiply
+    float past[3][TAPS], tap[3][TAPS];
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+      const int c = 3 * ch + p;
+      const size_t w = (size_t)(c / (3 * l.H / l.conv_g)) * l.kf;
+      const bf16* ring = l.proj_ring + (size_t)b * n * 3 * l.H + c;
+#pragma unroll
+      for (int j = 0; j < TAPS; ++j) {
+        tap[p][j] = j <= n ? param<CONV>(l.conv_w, w + j, l.f32 & F_CONV) : 0.f;
+        past[p][j] = j < n ? __bfloat162float(ring[(size_t)((pos + j) % n) * 3 * l.H]) : 0.f;
+      }
+    }
+    const float bias = l.kind == OP_SE ? 0.f : param<FILT>(l.bias, ch, l.f32 & F_BIAS);
+    wait_for_previous();
 #pragma unroll
     for (int p = 0; p < 3; ++p) {
       const int c = 3 * ch + p;
       const size_t w = (size_t)(c / (3 * l.H / l.conv_g)) * l.kf;
       const int wf = l.f32 & F_CONV;
       const bf16 cur = proj[(size_t)b * 3 * l.H + c];
-      float acc = param<CONV>(l.conv_w, w + n, wf) * __bfloat162float(cur);
       bf16* ring = l.proj_ring + (size_t)b * n * 3 * l.H + c;
-      for (int j = 0; j < n; ++j) acc += param<CONV>(l.conv_w, w + j, wf) * __bfloat162float(ring[(size_t)((pos + j) % n) * 3 * l.H]);
+      float acc = (n < TAPS ? tap_at(tap[p], n) : param<CONV>(l.conv_w, w + n, wf)) * __bfloat162float(cur);
+#pragma unroll
+      for (int j = 0; j < TAPS; ++j)
+        if (j < n) acc += tap[p][j] * past[p][j];
+      for (int j = TAPS; j < n; ++j) acc += param<CONV>(l.conv_w, w + j, wf) * __bfloat162float(ring[(size_t)((pos + j) % n) * 3 * l.H]);
       if (n > 0) ring[(size_t)(pos % n) * 3 * l.H] = cur;
       f[p] = rbf(acc);                                     // the parallel path rounds the featuriser output
     }
     const float u = f[1] * f[2];
     sx1[cx] = f[0];
     su[cx] = (l.kind == OP_SE && !l.pregate) ? f[2] : u;
-    sb[cx] = l.kind == OP_SE ? 0.f : param<FILT>(l.bias, ch, l.f32 & F_BIAS) * u;
+    sb[cx] = bias * u;
   }
   // what does not need the new u: the past of the FIR filters, the parameters and states of the first modes
   float y = 0.f;
@@ -317,7 +357,7 @@ dec_hyena_kernel(Layer l, const bf16* __restrict__ proj, bf16* __restrict__ z, i
 
 // ------------------------------------------------------------------------------------ attention
 __global__ void __cluster_dims__(SPLIT, 1, 1) __launch_bounds__(ATT_THREADS)
-dec_attn_kernel(Layer l, const bf16* __restrict__ proj, bf16* __restrict__ z, int pos) {
+dec_attn_kernel(Layer l, const bf16* proj, bf16* z, int pos) {
   __shared__ float raw[3][HD], sq[HD], sk[HD];
   __shared__ float wm[4], wl[4], wo[4][HD];
   __shared__ float cm, cl, co[HD];
@@ -325,6 +365,15 @@ dec_attn_kernel(Layer l, const bf16* __restrict__ proj, bf16* __restrict__ z, in
   const int rank = (int)cluster.block_rank();
   const int h = blockIdx.x / SPLIT, b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const bf16* row = proj + ((size_t)b * l.heads + h) * 3 * HD;
+  const size_t ld = (size_t)l.heads * HD, base = ((size_t)b * l.cap * l.heads + h) * HD;
+  const int chunk = (pos + SPLIT - 1) / SPLIT, j0 = rank * chunk, j1 = min(pos, j0 + chunk);
+  let_next_start();
+  for (int j = j0 + (tid >> 1); j < j1; j += ATT_THREADS / 2) {      // this block's keys and values: two 128-byte lines a row each
+    const size_t off = base + (size_t)j * ld + (tid & 1) * 64;
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(l.kc + off));
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(l.vc + off));
+  }
+  wait_for_previous();
 #pragma unroll
   for (int p = 0; p < 3; ++p) raw[p][tid] = __bfloat162float(row[p * HD + tid]);
   __syncthreads();
@@ -339,7 +388,6 @@ dec_attn_kernel(Layer l, const bf16* __restrict__ proj, bf16* __restrict__ z, in
     sq[tid] = rbf(q);
     sk[tid] = rbf(k);
   }
-  const size_t ld = (size_t)l.heads * HD, base = ((size_t)b * l.cap * l.heads + h) * HD;
   if (rank == 0) {                                         // append the new token
     l.kc[base + (size_t)pos * ld + tid] = __float2bfloat16_rn(sk[tid]);
     l.vc[base + (size_t)pos * ld + tid] = row[2 * HD + tid];
@@ -349,7 +397,6 @@ dec_attn_kernel(Layer l, const bf16* __restrict__ proj, bf16* __restrict__ z, in
   float qf[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) qf[i] = sq[4 * lane + i];
-  const int chunk = (pos + SPLIT - 1) / SPLIT, j0 = rank * chunk, j1 = min(pos, j0 + chunk);
   float m = -INFINITY, lsum = 0.f, o4[4] = {0.f, 0.f, 0.f, 0.f};
   constexpr int U = 4;
   for (int j = j0 + warp * U; j < j1; j += 4 * U) {
@@ -421,39 +468,31 @@ dec_attn_kernel(Layer l, const bf16* __restrict__ proj, bf16* __restrict__ z, in
   cluster.sync();                                          // peers' shared memory stays until it has been read
 }
 
-static void launch_hyena(const Layer& l, const bf16* proj, bf16* z, int B, int pos, cudaStream_t st) {
+static int launch_hyena(const Layer& l, const bf16* proj, bf16* z, int B, int pos, cudaStream_t st) {
   const int used = l.kind == OP_SE ? F_TAPS : l.kind == OP_MR ? F_TAPS | F_BIAS | (l.decay ? F_DECAY : 0) : F_BIAS | F_GAMMA | F_P | F_R;
   const dim3 grid((l.H + 31) / 32, B);
   const int threads = 32 * HY_SLICES;
-  if (l.f32 & F_CONV) dec_hyena_kernel<AS_F32, AS_STORED><<<grid, threads, 0, st>>>(l, proj, z, pos);
-  else if ((l.f32 & used) == used) dec_hyena_kernel<AS_BF16, AS_F32><<<grid, threads, 0, st>>>(l, proj, z, pos);
-  else if (!(l.f32 & used)) dec_hyena_kernel<AS_BF16, AS_BF16><<<grid, threads, 0, st>>>(l, proj, z, pos);
-  else dec_hyena_kernel<AS_BF16, AS_STORED><<<grid, threads, 0, st>>>(l, proj, z, pos);
+  auto* kernel = (l.f32 & F_CONV)            ? dec_hyena_kernel<AS_F32, AS_STORED>
+                 : (l.f32 & used) == used    ? dec_hyena_kernel<AS_BF16, AS_F32>
+                 : !(l.f32 & used)           ? dec_hyena_kernel<AS_BF16, AS_BF16>
+                                             : dec_hyena_kernel<AS_BF16, AS_STORED>;
+  return launch_chained(false, kernel, grid, threads, 0, st, l, proj, z, pos);
 }
 
-static int launch_linear(const LinArgs& a, cudaStream_t st) {
+static int launch_linear(const LinArgs& a, cudaStream_t st, bool first = false) {
   const int blocks = (a.N + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK;
   const int bt = a.B <= 1 ? 1 : a.B <= 2 ? 2 : a.B <= 4 ? 4 : 8;
   const size_t sm = (size_t)bt * a.K * 2;
-#define SB_DEC_LINEAR(BT)                                                                                                        \
-  do {                                                                                                                            \
-    if (sm > 48 * 1024 &&                                                                                                         \
-        cudaFuncSetAttribute(dec_linear_kernel<BT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess)         \
-      return -5;                                                                                                                  \
-    dec_linear_kernel<BT><<<blocks, THREADS, sm, st>>>(a);                                                                        \
-  } while (0)
-  if (bt == 1) SB_DEC_LINEAR(1);
-  else if (bt == 2) SB_DEC_LINEAR(2);
-  else if (bt == 4) SB_DEC_LINEAR(4);
-  else SB_DEC_LINEAR(8);
-#undef SB_DEC_LINEAR
-  return 0;
+  auto* kernel = bt == 1 ? dec_linear_kernel<1> : bt == 2 ? dec_linear_kernel<2> : bt == 4 ? dec_linear_kernel<4> : dec_linear_kernel<8>;
+  if (sm > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess) return -5;
+  return launch_chained(first, kernel, dim3(blocks), THREADS, sm, st, a);
 }
 
 }  // namespace dec
 }  // namespace sb
 
 using namespace sb::dec;
+using sb::launch_chained;
 
 // Largest input width of a projection at batch B (its inputs have to fit in shared memory).
 extern "C" int sb_decode_max_width(int B) { return B < 1 || B > MAX_B ? 0 : 200 * 1024 / 2 / (B <= 1 ? 1 : B <= 2 ? 2 : B <= 4 ? 4 : 8) / 8 * 8; }
@@ -471,10 +510,11 @@ extern "C" int sb_decode_step(const Layer* layers, int n_layers, void* x, void* 
   for (int i = 0; i < n_layers && !rc; ++i) {
     const Layer& l = layers[i];
     if ((l.H % 8) || (l.F % 8) || (l.kind == OP_ATTN && pos >= l.cap)) return -1;
-    rc = launch_linear(LinArgs{xb, l.norm1_w, l.w_in, nullptr, nullptr, pb, B, D, 3 * l.H, IN_NORM, 0, l.form1, 0, l.eps1}, st);
+    rc = launch_linear(LinArgs{xb, l.norm1_w, l.w_in, nullptr, nullptr, pb, B, D, 3 * l.H, IN_NORM, 0, l.form1, 0, l.eps1}, st, i == 0);
     if (rc) return rc;
-    if (l.kind == OP_ATTN) dec_attn_kernel<<<dim3(l.heads * SPLIT, B), ATT_THREADS, 0, st>>>(l, pb, zb, pos);
-    else launch_hyena(l, pb, zb, B, pos, st);
+    rc = l.kind == OP_ATTN ? launch_chained(false, dec_attn_kernel, dim3(l.heads * SPLIT, B), ATT_THREADS, 0, st, l, (const bf16*)pb, zb, pos)
+                           : launch_hyena(l, pb, zb, B, pos, st);
+    if (rc) return rc;
     rc = launch_linear(LinArgs{zb, nullptr, l.w_out, l.b_out, xb, abuf, B, l.H, D, IN_PLAIN, 0, 0, 0, 0.f}, st);
     if (rc) return rc;
     rc = launch_linear(LinArgs{abuf, l.norm2_w, l.w12, nullptr, nullptr, abb, B, D, 2 * l.F, l.norm2 ? IN_NORM : IN_PLAIN, 0, l.form2, 0,
