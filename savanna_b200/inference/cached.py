@@ -478,8 +478,10 @@ class CachedDecoder:
                     k, v = qkv[..., mod.hd: 2 * mod.hd], qkv[..., 2 * mod.hd:]
                     if mod._rotary:
                         cos, sin = mod._rotary[0](positions)
-                        k = ref.apply_rope(k.float(), cos, sin).to(qkv.dtype)
-                    st["k"], st["v"] = k.clone(), v.clone()
+                        k = ops.apply_rope(k, cos, sin) if k.dtype == torch.bfloat16 else ref.apply_rope(k.float(), cos, sin).to(qkv.dtype)
+                    else:
+                        k = k.clone()
+                    st["k"], st["v"] = k, v.clone()
                 hooks.append(inner.register_forward_pre_hook(grab_kv))
             else:
                 kf = mixer.short_conv_L
@@ -488,17 +490,17 @@ class CachedDecoder:
                     st["proj_tail"] = tail(args[0], kf - 1)
                 hooks.append(mixer.hyena_proj_conv.register_forward_pre_hook(grab_proj))
 
+                if isinstance(inner, HyenaOperator) and not inner.is_mr:
+                    # the layer's own scan leaves its state behind: no second pass over the prompt
+                    inner.state_sink = lambda s, st=st: st.__setitem__("s", s.float())
+                    continue
+
                 def grab_feat(mod, args, st=st):
-                    feat = args[0]
-                    u = feat[..., 1::3] * feat[..., 2::3]
-                    if isinstance(mod, ShortHyenaOperator):
-                        st["u_tail"] = tail(u if mod.pregate else feat[..., 2::3], mod.kernel_size - 1)
-                    elif mod.is_mr:
-                        st["u_tail"] = tail(u, min(mod.hyena_mr_len, 1 << 30) - 1)
-                    else:
-                        g, R, p = mod._modal()
-                        _, s = ops.hyena_li_modal(feat, g, R, p, mod.conv_bias, None, True)
-                        st["s"] = s.float()
+                    short = isinstance(mod, ShortHyenaOperator)
+                    n = (mod.kernel_size if short else min(mod.hyena_mr_len, 1 << 30)) - 1
+                    feat = args[0][:, -n:] if n > 0 else args[0][:, :0]          # only these rows are kept
+                    v = feat[..., 2::3]
+                    st["u_tail"] = tail(v if short and not mod.pregate else feat[..., 1::3] * v, n)
                 hooks.append(inner.register_forward_pre_hook(grab_feat))
         was_training = model.training
         switch = any(m.training for m in model.modules())          # a model in eval mode is left alone
@@ -509,6 +511,9 @@ class CachedDecoder:
         finally:
             for h in hooks:
                 h.remove()
+            for blk in self.blocks:
+                if isinstance(blk.mixer.mixer, HyenaOperator):
+                    blk.mixer.mixer.state_sink = None
             if switch:
                 model.train(was_training)
         self.pos = T

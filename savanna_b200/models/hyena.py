@@ -149,6 +149,7 @@ class HyenaOperator(nn.Module):
         self.conv_bias.model_parallel = True
         self.conv_bias.partition_dim = 0
         self.conv_bias.is_filter_param = True
+        self.state_sink = None             # prefill of cached generation: called with the modal state [B, D, O] behind the sequence
 
     # -- Hyena-MR ---------------------------------------------------------------
     def _forward_mr(self, feat, cp):
@@ -196,6 +197,10 @@ class HyenaOperator(nn.Module):
         modal = self._modal()
         if cp == 1:
             if modal is not None:
+                if self.state_sink is not None:
+                    z, s = ops.hyena_li_modal(feat, *modal, self.conv_bias, None, True)
+                    self.state_sink(s)
+                    return z
                 return ops.hyena_li_modal(feat, *modal, self.conv_bias)
             return ops.hyena_long_fft(feat, self.filter(L), self.conv_bias)
         r = state.get_context_parallel_rank()
