@@ -17,10 +17,10 @@
 //
 // Measured on a B200: four layers (one of each operator), width 1024, two sequences, a prompt of 517 tokens and 16 steps:
 // 50.2 ms operator by operator (3 ms a step, all of it launches; the key / value cache was copied and converted to fp32 on
-// every step), 4.4 ms with these kernels, half of it the prefill.  Two rows per warp keep 3072 outputs on 192 blocks while
-// every lane has eight 16-byte weight loads in flight (6 us a matrix-vector kernel, 5 to 6 us a Hyena step, 9 us attention
-// over 525 keys).  Launching the kernels as programmatic dependents with the weight loads ahead of the wait changed nothing
-// (4476 against 4482 us): the host issues them no faster.
+// every step), 3.6 ms with these kernels one after the other, 3.2 ms as programmatic dependents (with one scan less per Hyena-LI layer
+// in the prefill).  Two rows per warp keep 3072 outputs on 192 blocks while every lane has eight 16-byte weight loads in flight.  By
+// itself a matrix-vector kernel takes 6 us, a Hyena step 5 to 6, attention over 525 keys 9: launch gap, the first loads' latency and
+// the reductions, not bandwidth, which is why a kernel is under way before the one in front of it has finished.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
