@@ -21,6 +21,7 @@
 #include <stdint.h>
 
 #include "f32x2.cuh"
+#include "pdl.cuh"
 
 namespace sb {
 typedef __nv_bfloat16 bf16;
@@ -375,6 +376,7 @@ __device__ __forceinline__ float pole_corr(float ll, float lam) {
 __global__ void li_prep_kernel(const float* __restrict__ gamma, const float* __restrict__ p, const float* __restrict__ R,
                                float* __restrict__ out, int D, int O) {
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x, n = (size_t)D * LO;
+  let_next_start();
   if (i >= n) return;
   const int o = (int)(i % LO);
   const size_t j = i / LO * O + o;
@@ -449,8 +451,7 @@ __device__ __forceinline__ f2 li_pair(const uint32_t* row, int i) { return f2_bf
 // forward pass 3 (APPLY = true): rerun each chunk from its entering state S and emit z.
 template <bool APPLY>
 __global__ void __launch_bounds__(LV_PAIRS)
-li_fwd_tiled_kernel(const bf16* __restrict__ feat, const LiModal m, const float* __restrict__ bias, float* __restrict__ S,
-                    bf16* __restrict__ z, LiDims d) {
+li_fwd_tiled_kernel(const bf16* __restrict__ feat, const LiModal m, const float* __restrict__ bias, float* S, bf16* z, LiDims d) {
   __shared__ __align__(16) uint32_t ring[LV_STAGES][LV_ROWS][LV_FW];
   const int tid = threadIdx.x, c0 = blockIdx.x * LV_CH, ch = c0 + 2 * tid;
   const int n = blockIdx.y, b = blockIdx.z;
@@ -468,6 +469,8 @@ li_fwd_tiled_kernel(const bf16* __restrict__ feat, const LiModal m, const float*
       li_stage<LV_ROWS, 3 * LV_CH / 8, LV_PAIRS>(ring_a + k * TILE_B, src + (size_t)k * LV_ROWS * ld, ld, t1 - t0 - k * LV_ROWS, ncv, tid);
     li_cp_commit();
   }
+  let_next_start();
+  wait_for_previous();                   // the features are the call's own inputs; poles and entering states are not
   f2 lam[LO], s[LO], rr[APPLY ? LO : 1], be = 0;
   load_poles(m, (size_t)ch * LO, live, lam);
   float* Sp = S + (((size_t)b * d.NC + n) * d.D + ch) * LO;
@@ -530,7 +533,7 @@ li_fwd_tiled_kernel(const bf16* __restrict__ feat, const LiModal m, const float*
 // backward's 128 chunks 54 and 36 us, the forward's 64 chunks 10.2 and 11.6 us.
 constexpr int LP_AHEAD_FWD = 16, LP_AHEAD_BWD = 32;
 template <bool REVERSE, int AHEAD>
-__device__ __forceinline__ float li_carry(float* __restrict__ p, size_t per_b, float ll, float scale, float carry, float tail,
+__device__ __forceinline__ float li_carry(float* p, size_t per_b, float ll, float scale, float carry, float tail,
                                           const LiDims& d) {
   const float step = expf(ll * d.TC);
   for (int k0 = 0; k0 < d.NC; k0 += AHEAD) {
@@ -559,8 +562,9 @@ __device__ __forceinline__ float state_at(const float* s, int b, int ch, int o, 
 }
 
 __global__ void __launch_bounds__(128)
-li_prefix_tiled_kernel(float* __restrict__ S, const LiModal m, const float* __restrict__ state_in, float* __restrict__ state_out,
-                       LiDims d) {
+li_prefix_tiled_kernel(float* S, const LiModal m, const float* __restrict__ state_in, float* __restrict__ state_out, LiDims d) {
+  let_next_start();
+  wait_for_previous();
   const size_t per_b = (size_t)d.D * LO;
   const size_t r = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   const int b = blockIdx.y;
@@ -575,8 +579,10 @@ li_prefix_tiled_kernel(float* __restrict__ S, const LiModal m, const float* __re
 // Backward prefixes: blockIdx.z = 0 the states, 1 the adjoints (carrying R, `with_R`, when a state gradient has to ride along or
 // the caller wants finished partial sums).
 __global__ void __launch_bounds__(128)
-li_bwd_prefix_tiled_kernel(float* __restrict__ S, float* __restrict__ A, const LiModal m, const float* __restrict__ state_in,
-                           const float* __restrict__ dstate_out, float* __restrict__ dstate_in, int with_R, LiDims d) {
+li_bwd_prefix_tiled_kernel(float* S, float* A, const LiModal m, const float* __restrict__ state_in, const float* __restrict__ dstate_out,
+                           float* __restrict__ dstate_in, int with_R, LiDims d) {
+  let_next_start();
+  wait_for_previous();
   const size_t per_b = (size_t)d.D * LO;
   const size_t r = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   const int b = blockIdx.y;
@@ -615,6 +621,7 @@ li_bwd_local_tiled_kernel(const bf16* __restrict__ feat, const bf16* __restrict_
   li_stage<LB_TC, 3 * LV_CH / 8, 2 * LV_PAIRS>(f_a, feat + ((size_t)b * d.L + t0) * 3 * d.D + 3 * c0, (size_t)3 * d.D, rows, ncf, tid);
   li_stage<LB_TC, LV_CH / 8, 2 * LV_PAIRS>(g_a, dz + ((size_t)b * d.L + t0) * d.D + c0, d.D, rows, ncg, tid);
   li_cp_commit();
+  let_next_start();
   f2 lam[LO], s[LO];
   load_poles(m, (size_t)ch * LO, live, lam);
 #pragma unroll
@@ -665,6 +672,8 @@ li_bwd_apply_tiled_kernel(const bf16* __restrict__ feat, const bf16* __restrict_
   li_stage<LB_TC, 3 * LV_CH / 8, NT>(f_a, feat + ((size_t)b * d.L + t0) * 3 * d.D + 3 * c0, (size_t)3 * d.D, rows, ncf, tid);
   li_stage<LB_TC, LV_CH / 8, NT>(g_a, dz + ((size_t)b * d.L + t0) * d.D + c0, d.D, rows, ncg, tid);
   li_cp_commit();
+  let_next_start();
+  wait_for_previous();
   const size_t off = (((size_t)b * d.NC + n) * d.D + ch) * LO;
   f2 lam[LO], s[LO];                                     // s: state (roles 0, 1) or adjoint (role 2) entering the chunk
   load_poles(m, (size_t)ch * LO, live, lam);
@@ -787,8 +796,8 @@ li_bwd_apply_tiled_kernel(const bf16* __restrict__ feat, const bf16* __restrict_
 //   dR, dgamma = dp = dlam lam log(lam) ([D, O]) and dbias [D].  One thread per (channel, mode) column and row slice.
 constexpr int LR_COLS = 32, LR_SLICES = 8;
 __global__ void __launch_bounds__(LR_COLS * LR_SLICES)
-li_bwd_reduce_kernel(const float* __restrict__ dRp, const float* __restrict__ dLp, const float* __restrict__ dBp, const LiModal m,
-                     int scale_by_R, float* __restrict__ dR, float* __restrict__ dll, float* __restrict__ db, int n_rows, int D) {
+li_bwd_reduce_kernel(const float* dRp, const float* dLp, const float* dBp, const LiModal m, int scale_by_R, float* dR, float* dll, float* db,
+                     int n_rows, int D) {
   __shared__ float red[2][LR_SLICES][LR_COLS];
   const int cx = threadIdx.x % LR_COLS, sl = threadIdx.x / LR_COLS;
   const int n_modal = (D * LO + LR_COLS - 1) / LR_COLS;              // blocks [0, n_modal): dR / dlam; the rest: dbias
@@ -796,6 +805,7 @@ li_bwd_reduce_kernel(const float* __restrict__ dRp, const float* __restrict__ dL
   const size_t width = modal ? (size_t)D * LO : (size_t)D;
   const size_t col = (size_t)(modal ? blockIdx.x : blockIdx.x - n_modal) * LR_COLS + cx;
   float a0 = 0.f, a1 = 0.f;
+  wait_for_previous();
   if (col < width) {
     if (modal) {
 #pragma unroll 4
@@ -1094,6 +1104,37 @@ static inline bool aligned16(const void* a, const void* b, const void* c = nullp
   return (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) & 15) == 0;
 }
 
+// The forward's three passes, as a chain of programmatic dependents for chunks of up to 64 steps; `first`: nothing before them belongs to
+// the chain.  Blocks that wait for the pass before them take the slots that it leaves free, unevenly over the SMs, and a block of a longer
+// chunk is too much work for that.  Chained / one after the other, us: L = 300, D = 512 12.4 / 20.1, B = 2, L = 1237, D = 1024 30.6 / 33.0
+// (chunks of 32), but L = 2048, D = 4096 62 / 52, L = 8192, D = 1024 62 / 54 (128) and D = 4096 183 / 137 (512; 150 with the last pass
+// alone left out of the chain).
+static int li_fwd_chain(bool first, const bf16* feat, const LiModal& m, const float* bias, const float* state_in, float* state_out, float* S,
+                        bf16* z, dim3 grid, const LiDims& d, cudaStream_t st) {
+  const dim3 modes((unsigned)(((size_t)d.D * LO + 127) / 128), d.B);
+  const bool single = d.TC > 64;
+  int rc = launch_chained(first || single, li_fwd_tiled_kernel<false>, grid, LV_PAIRS, 0, st, feat, m, bias, S, (bf16*)nullptr, d);
+  if (!rc) rc = launch_chained(single, li_prefix_tiled_kernel, modes, 128, 0, st, S, m, state_in, state_out, d);
+  if (!rc) rc = launch_chained(single, li_fwd_tiled_kernel<true>, grid, LV_PAIRS, 0, st, feat, m, bias, S, z, d);
+  return rc;
+}
+
+// The backward's passes up to the chunks' partial sums, likewise (chunks of 64 steps).  Chained against one after the other, us, with the
+// reduction: L = 64, D = 256 26.6 / 30.8, L = 300, D = 512 34.8 / 31.8, B = 2, L = 1237, D = 1024 56.6 / 62, L = 2048, D = 4096 115 / 123,
+// L = 8192, D = 1024 118 / 125, D = 4096 396 / 408.
+template <bool GOUT>
+static int li_bwd_chain(const bf16* feat, const bf16* dz, const LiModal& m, const float* bias, const float* state_in, const float* dstate_out,
+                        float* dstate_in, int with_R, float* S, float* A, float* dRp, float* dLp, float* dBp, bf16* dfeat, const LiDims& d,
+                        cudaStream_t st) {
+  const dim3 grid((d.D + LV_CH - 1) / LV_CH, d.NC, d.B), modes((unsigned)(((size_t)d.D * LO + 127) / 128), d.B, 2);
+  int rc = launch_chained(true, li_bwd_local_tiled_kernel, grid, 2 * LV_PAIRS, LBL_SMEM, st, feat, dz, m, S, A, d);
+  if (!rc) rc = launch_chained(false, li_bwd_prefix_tiled_kernel, modes, 128, 0, st, S, A, m, state_in, dstate_out, dstate_in, with_R, d);
+  if (!rc)
+    rc = launch_chained(false, li_bwd_apply_tiled_kernel<GOUT>, grid, 3 * LV_PAIRS, LBA_SMEM, st, feat, dz, m, bias, (const float*)S,
+                        (const float*)A, dRp, dLp, dBp, dfeat, dstate_out, d);
+  return rc;
+}
+
 // The forward scan on prepared log-poles and residues ([D, 16]): the tiled kernels for D % 8 == 0 and 16-byte aligned features and
 // output, else the per-thread ones (L = 8192, D = 4096: 0.14 and 0.28 ms).
 static int li_forward(const void* feat, const float* loglam, const float* R, const float* bias, const float* state_in,
@@ -1102,9 +1143,7 @@ static int li_forward(const void* feat, const float* loglam, const float* R, con
   if (g_li_tiled && d.D % 8 == 0 && aligned16(feat, z)) {
     const LiModal m{loglam, nullptr, R, nullptr, LO};
     const dim3 grid((d.D + LV_CH - 1) / LV_CH, d.NC, d.B);
-    li_fwd_tiled_kernel<false><<<grid, LV_PAIRS, 0, st>>>((const bf16*)feat, m, bias, S, nullptr, d);
-    li_prefix_tiled_kernel<<<dim3((unsigned)((n + 127) / 128), d.B), 128, 0, st>>>(S, m, state_in, state_out, d);
-    li_fwd_tiled_kernel<true><<<grid, LV_PAIRS, 0, st>>>((const bf16*)feat, m, bias, S, (bf16*)z, d);
+    return li_fwd_chain(true, (const bf16*)feat, m, bias, state_in, state_out, S, (bf16*)z, grid, d, st);
   } else {
     const dim3 grid((d.D + LI_THREADS - 1) / LI_THREADS, d.NC, d.B);
     li_local_kernel<<<grid, LI_THREADS, 0, st>>>((const bf16*)feat, loglam, S, d);
@@ -1138,10 +1177,8 @@ extern "C" int sb_li_fwd_tiled(const void* feat, const float* gamma, const float
   const LiModal m{modal, modal + n, modal + 2 * n, modal + 3 * n, O};
   dim3 grid((D + LV_CH - 1) / LV_CH, d.NC, B);
   li_prep_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(gamma, p, R, modal, D, O);
-  li_fwd_tiled_kernel<false><<<grid, LV_PAIRS, 0, st>>>((const bf16*)feat, m, bias, S, nullptr, d);
-  li_prefix_tiled_kernel<<<dim3((unsigned)((n + 127) / 128), B), 128, 0, st>>>(S, m, state_in, state_out, d);
-  li_fwd_tiled_kernel<true><<<grid, LV_PAIRS, 0, st>>>((const bf16*)feat, m, bias, S, (bf16*)z, d);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  if (cudaGetLastError() != cudaSuccess) return -2;
+  return li_fwd_chain(false, (const bf16*)feat, m, bias, state_in, state_out, S, (bf16*)z, grid, d, st);
 }
 
 extern "C" int sb_li_bwd_tiled_chunk() { return LB_TC; }
@@ -1164,19 +1201,14 @@ extern "C" int sb_li_bwd_tiled(const void* feat, const void* dz, const float* mo
   LiDims d = li_dims(B, L, D, LB_TC);
   const size_t n = (size_t)D * LO;
   const LiModal m{modal, modal + n, modal + 2 * n, modal + 3 * n, O};
-  const dim3 grid((D + LV_CH - 1) / LV_CH, d.NC, B);
-  li_bwd_local_tiled_kernel<<<grid, 2 * LV_PAIRS, LBL_SMEM, st>>>((const bf16*)feat, (const bf16*)dz, m, S, A, d);
-  li_bwd_prefix_tiled_kernel<<<dim3((unsigned)((n + 127) / 128), B, 2), 128, 0, st>>>(S, A, m, state_in, dstate_out, dstate_in,
-                                                                                              dstate_out != nullptr, d);
-  if (dstate_out)
-    li_bwd_apply_tiled_kernel<true><<<grid, 3 * LV_PAIRS, LBA_SMEM, st>>>((const bf16*)feat, (const bf16*)dz, m, bias, S, A, dRp, A, dBp,
-                                                                         (bf16*)dfeat, dstate_out, d);
-  else
-    li_bwd_apply_tiled_kernel<false><<<grid, 3 * LV_PAIRS, LBA_SMEM, st>>>((const bf16*)feat, (const bf16*)dz, m, bias, S, A, dRp, A, dBp,
-                                                                          (bf16*)dfeat, nullptr, d);
+  const int rc = dstate_out ? li_bwd_chain<true>((const bf16*)feat, (const bf16*)dz, m, bias, state_in, dstate_out, dstate_in, 1, S, A, dRp, A,
+                                                dBp, (bf16*)dfeat, d, st)
+                            : li_bwd_chain<false>((const bf16*)feat, (const bf16*)dz, m, bias, state_in, nullptr, dstate_in, 0, S, A, dRp, A,
+                                                 dBp, (bf16*)dfeat, d, st);
+  if (rc) return rc;
   const unsigned blocks = (unsigned)((n + LR_COLS - 1) / LR_COLS + (D + LR_COLS - 1) / LR_COLS);
-  li_bwd_reduce_kernel<<<blocks, LR_COLS * LR_SLICES, 0, st>>>(dRp, A, dBp, m, dstate_out ? 0 : 1, dR, dll, db, B * d.NC, D);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return launch_chained(false, li_bwd_reduce_kernel, dim3(blocks), LR_COLS * LR_SLICES, 0, st, (const float*)dRp, (const float*)A,
+                        (const float*)dBp, m, dstate_out ? 0 : 1, dR, dll, db, B * d.NC, D);
 }
 
 // Scratch: S, W, A, dRp, dLp each B*NC*D*16 floats; dBp B*NC*D floats; dx1_tmp B*L*D bf16.
@@ -1192,13 +1224,8 @@ extern "C" int sb_li_bwd(const void* feat, const void* dz, const float* loglam, 
   if (g_li_tiled && D % 8 == 0 && TC == LB_TC && !dstate_out && !w_end && aligned16(feat, dz, dfeat)) {
     if (!li_bwd_tiled_ready()) return -5;
     const LiModal m{loglam, nullptr, R, nullptr, LO};
-    const dim3 tiles((D + LV_CH - 1) / LV_CH, d.NC, B);
-    li_bwd_local_tiled_kernel<<<tiles, 2 * LV_PAIRS, LBL_SMEM, st>>>((const bf16*)feat, (const bf16*)dz, m, S, A, d);
-    li_bwd_prefix_tiled_kernel<<<dim3((unsigned)(((size_t)D * LO + 127) / 128), B, 2), 128, 0, st>>>(S, A, m, state_in, nullptr,
-                                                                                                     dstate_in, 1, d);
-    li_bwd_apply_tiled_kernel<true><<<tiles, 3 * LV_PAIRS, LBA_SMEM, st>>>((const bf16*)feat, (const bf16*)dz, m, bias, S, A, dRp, dLp,
-                                                                          dBp, (bf16*)dfeat, nullptr, d);
-    return cudaGetLastError() == cudaSuccess ? 0 : -2;
+    return li_bwd_chain<true>((const bf16*)feat, (const bf16*)dz, m, bias, state_in, nullptr, dstate_in, 1, S, A, dRp, dLp, dBp, (bf16*)dfeat, d,
+                              st);
   }
   if (!dx1_tmp || !W) return -1;
   dim3 grid((D + LI_THREADS - 1) / LI_THREADS, d.NC, B);
