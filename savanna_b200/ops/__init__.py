@@ -1,9 +1,9 @@
 """Operator front-end.
 
 Every hot operator of the model goes through a function of this module.  A CUDA tensor runs the
-hand-written sm_100a kernel (ops/cuda_ops.py over the in-tree extension `savanna_b200._C`); a CPU
-tensor runs the fp32-capable PyTorch statement in ops/reference.py, which is also the oracle of the
-kernel tests.  `set_backend("torch")` (or SAVANNA_B200_BACKEND=torch) forces the PyTorch statement
+hand-written sm_100a kernel (ops/cuda_ops.py over the in-tree kernel library, differentiated by the
+C++ functions of csrc/autograd_native.cpp); a CPU tensor runs the fp32-capable PyTorch statement in
+ops/reference.py, which is also the oracle of the kernel tests.  `set_backend("torch")` (or SAVANNA_B200_BACKEND=torch) forces the PyTorch statement
 for CUDA tensors too: the comparison arm of tests and benchmarks, never the default.  There is no
 silent fallback: a CUDA tensor without the built extension raises.
 """
