@@ -764,9 +764,10 @@ attn_stats_kernel(const __nv_bfloat16* __restrict__ go, const __nv_bfloat16* __r
 // accumulator and the key gradient, inverse).  A block takes one token of one tensor; a thread keeps 8 channels and their
 // partners half a rotation away of ROPE_HEADS heads, so both halves are loaded once, the fp32 table row is read once for all of
 // them (it is as large as the data of four heads) and a bf16 destination may be its own source.  Channels beyond the rotary
-// dimension are copied.  Bound by loads in flight: at L = 8192 with 32 heads 77 us for queries and keys (one launch each way;
-// 89 with both tensors in one block, two heads at a time), where the general kernel took 59 us a tensor and a cast of dq
-// another 31.
+// dimension are copied.  Bound by loads in flight, so a thread issues those of all its heads before it computes the first, and
+// whether the source is fp32 is settled outside of the loops: at L = 8192 with 32 heads forward and backward launch together
+// take 109 us (154 with a head's loads after the previous head's stores; 92 at the copy rate), two sequences of 1333 with 16 heads
+// 7.4 (10.2).
 struct RopeSide {
   const void* src;
   __nv_bfloat16* dst;
@@ -775,31 +776,42 @@ struct RopeSide {
 };
 struct RopeArgs { RopeSide side[2]; const float* cs; const float* sn; int H, rd; float sign; };
 
-__device__ __forceinline__ void rope_ld8(const void* p, long long off, int f32, float (&f)[8]) {
-  if (f32) {
-    const float4* q = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p) + off);
-    const float4 x = q[0], y = q[1];
-    f[0] = x.x; f[1] = x.y; f[2] = x.z; f[3] = x.w; f[4] = y.x; f[5] = y.y; f[6] = y.z; f[7] = y.w;
-  } else {
-    const uint4 q = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p) + off);
-    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 t = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[j]));
-      f[2 * j] = t.x; f[2 * j + 1] = t.y;
-    }
-  }
+__device__ __forceinline__ void rope_ld8(const float* p, float (&f)[8]) {
+  const float4 x = reinterpret_cast<const float4*>(p)[0], y = reinterpret_cast<const float4*>(p)[1];
+  f[0] = x.x; f[1] = x.y; f[2] = x.z; f[3] = x.w; f[4] = y.x; f[5] = y.y; f[6] = y.z; f[7] = y.w;
 }
 __device__ __forceinline__ void rope_st8(__nv_bfloat16* p, const float (&f)[8]) {
   *reinterpret_cast<uint4*>(p) = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
 }
 
 constexpr int ROPE_HEADS = 4;
-__global__ void __launch_bounds__(256)
-attn_rope_kernel(const RopeArgs a) {
-  const int l = blockIdx.x, b = blockIdx.y;
-  const RopeSide& d = a.side[blockIdx.z];
-  const int half = a.rd / 2, nrot = half / 8, units = nrot + (HD - a.rd) / 8;
+template <bool F32> struct RopeRaw { uint4 v[F32 ? 2 : 1]; };
+template <bool F32> __device__ __forceinline__ RopeRaw<F32> rope_raw(const void* p, long long off) {
+  RopeRaw<F32> r;
+  const uint4* q = reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(p) + off * (F32 ? 4 : 2));
+#pragma unroll
+  for (int i = 0; i < (F32 ? 2 : 1); ++i) r.v[i] = q[i];
+  return r;
+}
+template <bool F32> __device__ __forceinline__ void rope_f(const RopeRaw<F32>& r, float (&f)[8]) {
+#pragma unroll
+  for (int i = 0; i < (F32 ? 2 : 1); ++i) {
+    const uint32_t w[4] = {r.v[i].x, r.v[i].y, r.v[i].z, r.v[i].w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (F32) f[4 * i + j] = __uint_as_float(w[j]);
+      else { f[2 * j] = __uint_as_float(w[j] << 16); f[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u); }
+    }
+  }
+}
+
+// One row of one side: eight lanes share a head, a thread takes ROPE_HEADS heads at a time, all of whose loads are issued before
+// the first is used (a destination may be its own source, so the compiler may not move the next head's loads over a store).
+template <bool F32>
+__device__ __forceinline__ void rope_row(const RopeArgs& a, const RopeSide& d, int l, int b) {
+  const int half = a.rd / 2, nrot = half / 8, units = nrot + (HD - a.rd) / 8, cols = blockDim.x >> 3;
+  const long long s0 = b * d.s_sb + l * d.s_sl;
+  __nv_bfloat16* dst0 = d.dst + b * d.d_sb + l * d.d_sl;
   for (int u = threadIdx.x & 7; u < units; u += 8) {
     const bool rot = u < nrot;
     const int c0 = rot ? u * 8 : a.rd + (u - nrot) * 8;
@@ -807,30 +819,46 @@ attn_rope_kernel(const RopeArgs a) {
     if (rot) {
       const float* cr = a.cs + (long long)l * a.rd + c0;
       const float* sr = a.sn + (long long)l * a.rd + c0;
-      rope_ld8(cr, 0, 1, c1); rope_ld8(cr, half, 1, c2);
-      rope_ld8(sr, 0, 1, s1); rope_ld8(sr, half, 1, s2);
+      rope_ld8(cr, c1); rope_ld8(cr + half, c2);
+      rope_ld8(sr, s1); rope_ld8(sr + half, s2);
     }
-#pragma unroll 4
-    for (int h = threadIdx.x >> 3; h < a.H; h += blockDim.x >> 3) {
-      const long long so = b * d.s_sb + l * d.s_sl + h * d.s_sh + c0;
-      __nv_bfloat16* dst = d.dst + b * d.d_sb + l * d.d_sl + h * d.d_sh + c0;
-      float lo[8];
-      rope_ld8(d.src, so, d.f32, lo);
-      if (rot) {
-        float hi[8], o1[8], o2[8];
-        rope_ld8(d.src, so + half, d.f32, hi);
+    for (int h0 = threadIdx.x >> 3; h0 < a.H; h0 += cols * ROPE_HEADS) {
+      RopeRaw<F32> lo[ROPE_HEADS], hi[ROPE_HEADS];
+#pragma unroll
+      for (int i = 0; i < ROPE_HEADS; ++i) {
+        const int h = h0 + i * cols;
+        if (h < a.H) {
+          lo[i] = rope_raw<F32>(d.src, s0 + h * d.s_sh + c0);
+          if (rot) hi[i] = rope_raw<F32>(d.src, s0 + h * d.s_sh + c0 + half);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < ROPE_HEADS; ++i) {
+        const int h = h0 + i * cols;
+        if (h >= a.H) break;
+        __nv_bfloat16* dst = dst0 + h * d.d_sh + c0;
+        float x[8];
+        rope_f<F32>(lo[i], x);
+        if (!rot) { rope_st8(dst, x); continue; }
+        float y[8], o1[8], o2[8];
+        rope_f<F32>(hi[i], y);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          o1[j] = lo[j] * c1[j] - hi[j] * (a.sign * s1[j]);
-          o2[j] = hi[j] * c2[j] + lo[j] * (a.sign * s2[j]);
+          o1[j] = x[j] * c1[j] - y[j] * (a.sign * s1[j]);
+          o2[j] = y[j] * c2[j] + x[j] * (a.sign * s2[j]);
         }
         rope_st8(dst, o1);
         rope_st8(dst + half, o2);
-      } else {
-        rope_st8(dst, lo);
       }
     }
   }
+}
+
+__global__ void __launch_bounds__(256)
+attn_rope_kernel(const RopeArgs a) {
+  const RopeSide& d = a.side[blockIdx.z];
+  if (d.f32) rope_row<true>(a, d, blockIdx.x, blockIdx.y);
+  else rope_row<false>(a, d, blockIdx.x, blockIdx.y);
 }
 
 // dq[b, i, h, :] (bf16, strided) = dq_acc (fp32, contiguous [B, L, H, 128])
