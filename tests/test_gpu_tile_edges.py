@@ -361,6 +361,31 @@ def test_packed_attention_rotary():
         _close(qkv.grad, qr.grad, 4e-2, "dqkv")          # as in test_attention_tiles, and the rounded q, k enter the scores
 
 
+@pytest.mark.parametrize("H,rd", [(4, 128), (5, 32), (130, 64)])
+def test_rotary_heads(H, rd):
+    """Head counts that leave a thread of the packed rotary kernel short of its four heads (5) or send it round again (130): the
+    rotated queries and keys are written in place, the rest of the packed tensor stays as it was."""
+    import ctypes
+    from savanna_b200.ops import cuda_ops
+    cuda_ops.require()
+    entry = ctypes.CDLL(cuda_ops._LIB_PATH).sb_attn_rope
+    L = 3
+    torch.manual_seed(H)
+    qkv = torch.randn(2, L, H, 384, device=DEV).to(BF)
+    cos, sin = ref.rope_tables(torch.arange(L, device=DEV), rd)
+    out = qkv.clone()
+    views = [out[..., :128], out[..., 128:256]]
+    ptrs = (ctypes.c_void_p * 2)(*[v.data_ptr() for v in views])
+    strides = (ctypes.c_longlong * 6)(*[s for v in views for s in v.stride()[:3]])
+    cos, sin = cos.float().contiguous(), sin.float().contiguous()
+    assert entry(ptrs, ptrs, strides, strides, (ctypes.c_int * 2)(0, 0), 2, ctypes.c_void_p(cos.data_ptr()),
+                 ctypes.c_void_p(sin.data_ptr()), 2, L, H, rd, 0, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    for i, v in enumerate(views):
+        want = ref.apply_rope(qkv[..., 128 * i:128 * i + 128].float(), cos, sin)
+        _close(v, want, 2.0 ** -8, "qk"[i])              # one rounding to bf16
+    assert torch.equal(out[..., 256:], qkv[..., 256:])
+
+
 def _conv_grads(B, L, D, G, K, halo, pre=True, post=True, bf16_taps=False):
     torch.manual_seed(L + K)
     feat, w = torch.randn(B, L, 3 * D, device=DEV).to(BF), torch.randn(G, K, device=DEV) * 0.4
