@@ -478,7 +478,9 @@ class CachedDecoder:
                     k, v = qkv[..., mod.hd: 2 * mod.hd], qkv[..., 2 * mod.hd:]
                     if mod._rotary:
                         cos, sin = mod._rotary[0](positions)
-                        k = ops.apply_rope(k, cos, sin) if k.dtype == torch.bfloat16 else ref.apply_rope(k.float(), cos, sin).to(qkv.dtype)
+                        # three fp32 operations and one rounding, as the operator-by-operator step rotates: the rotary kernel contracts
+                        # product and sum, and keys near a rounding boundary would land on its other side
+                        k = ref.apply_rope(k.float(), cos, sin).to(qkv.dtype)
                     else:
                         k = k.clone()
                     st["k"], st["v"] = k, v.clone()

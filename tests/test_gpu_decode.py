@@ -10,6 +10,8 @@ from savanna_b200.config import GlobalConfig
 from savanna_b200.inference import cached
 from savanna_b200.inference.cached import CachedDecoder
 from savanna_b200.models import build_model
+from savanna_b200.models.mixer import SelfAttention
+from savanna_b200.ops import reference as ref
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -72,6 +74,26 @@ def test_forms(form, B, T, monkeypatch):
     fast.prefill(toks[:, :T])
     assert fast._fused is not None and (fast._fused.head is None) == (form in ("untied_head", "scaled_head"))
     _agree(fast, slow, toks[:, T:])
+
+
+@pytest.mark.parametrize("form", ["", "partial_rotary", "linear_rotary", "no_rotary"])
+@pytest.mark.parametrize("B,T", [(1, 1), (2, 517)])
+def test_prefilled_keys(form, B, T):
+    """The keys that a prefill leaves are those of the fp32 statement, rounded once, bit for bit."""
+    model = _model(**_FORMS.get(form, {}))
+    dec, seen = CachedDecoder(model), {}
+    mods = {i: b.mixer.mixer for i, b in enumerate(dec.blocks) if isinstance(b.mixer.mixer, SelfAttention)}
+    hooks = [m.register_forward_pre_hook(lambda m, a, i=i: seen.update({i: (a[0].clone(), a[1].clone())})) for i, m in mods.items()]
+    dec.prefill(_toks(model, B, T))
+    for h in hooks:
+        h.remove()
+    assert mods and seen.keys() == mods.keys()
+    for i, m in mods.items():
+        q = seen[i][0].view(B, T, m.heads, 3 * m.hd)
+        k = q[..., m.hd:2 * m.hd].float()
+        if m._rotary:
+            k = ref.apply_rope(k, *m._rotary[0](seen[i][1]))
+        assert torch.equal(dec.states[i]["k"][:, :T], k.to(q.dtype)) and torch.equal(dec.states[i]["v"][:, :T], q[..., 2 * m.hd:])
 
 
 @pytest.mark.parametrize("B,ffn,native", [(8, 12800, True), (8, 12816, False), (4, 12816, True), (9, 512, False)])
