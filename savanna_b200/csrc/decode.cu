@@ -292,7 +292,7 @@ dec_hyena_kernel(Layer l, const bf16* proj, bf16* z, int pos) {
     const float u = f[1] * f[2];
     sx1[cx] = f[0];
     su[cx] = (l.kind == OP_SE && !l.pregate) ? f[2] : u;
-    sb[cx] = bias * u;
+    sb[cx] = l.kind == OP_SE ? 0.f : bias * u;             // no bias, and without its pre-gate u may be what it likes
   }
   // what does not need the new u: the past of the FIR filters, the parameters and states of the first modes
   float y = 0.f;

@@ -10,6 +10,7 @@ from savanna_b200.config import GlobalConfig
 from savanna_b200.inference import cached
 from savanna_b200.inference.cached import CachedDecoder
 from savanna_b200.models import build_model
+from savanna_b200.models.hyena import ShortHyenaOperator
 from savanna_b200.models.mixer import SelfAttention
 from savanna_b200.ops import reference as ref
 
@@ -105,6 +106,21 @@ def test_limits(B, ffn, native, monkeypatch):
     fast.prefill(toks[:, :9])
     assert (fast._fused is not None) == native
     _agree(fast, slow, toks[:, 9:])
+
+
+@pytest.mark.parametrize("x2", [float("inf"), float("nan")])
+def test_unused_stream_stays_out(x2, monkeypatch):
+    """Without its pre-gate the short filter does not read the second stream: what is not finite there reaches nothing."""
+    model = _model(hyena_se_pregate=False)
+    toks = _toks(model, 2, 30)
+    conv = next(b.mixer.hyena_proj_conv for b in model.blocks() if isinstance(b.mixer.mixer, ShortHyenaOperator))
+    assert conv.group_dim == 1
+    with torch.no_grad():
+        conv.short_conv_weight[1::3] = x2
+    fast, slow = CachedDecoder(model), _slow(model, toks[:, :20], monkeypatch)
+    assert fast.prefill(toks[:, :20]).isfinite().all() and fast._fused is not None
+    _agree(fast, slow, toks[:, 20:])
+    assert fast._fused is not None
 
 
 def _is_filter(n):
