@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "device_info.h"
 #include "f32x2.cuh"
 #include "pdl.cuh"
 
@@ -1119,18 +1120,26 @@ static int li_fwd_chain(bool first, const bf16* feat, const LiModal& m, const fl
   return rc;
 }
 
-// The backward's passes up to the chunks' partial sums, likewise (chunks of 64 steps).  Chained against one after the other, us, with the
-// reduction: L = 64, D = 256 26.6 / 30.8, L = 300, D = 512 34.8 / 31.8, B = 2, L = 1237, D = 1024 56.6 / 62, L = 2048, D = 4096 115 / 123,
-// L = 8192, D = 1024 118 / 125, D = 4096 396 / 408.
+// The backward's passes up to the chunks' partial sums (chunks of 64 steps); the reduction behind them is chained as well.  The apply pass
+// has one block of 112 KB per chunk and 128 channels: launched while the prefix pass still runs, two of them share an SM beside idle ones,
+// unless there is a block for every SM anyway, or the blocks of all three passes find an SM each.  In between it waits for the prefix pass
+// to end.  us with the reduction, one after the other / all chained / all but the apply pass (* the one chosen here):
+//   L = 64, D = 256 30.8 / *26.6 / 27.8        L = 1237, D = 1024 46.2 / *40.6 / 43.0        L = 200, D = 512 32.6 / 34.9 / *28.7
+//   L = 300, D = 256 31.8 / *26.7 / 28.7       L = 1024, D = 2048 49.2 / *43.1 / 45.2        L = 300, D = 1024 32.9 / 36.8 / *30.0
+//   L = 2048, D = 4096 121 / *115 / 118        L = 8192, D = 4096 401 / *396 / 401           L = 64, D = 3072 34.9 / 36.7 / *33.6
+// The rule gives away 2 us at L <= 128 where the prefix pass's own blocks (512, 1024) happen to occupy the SMs evenly: L = 64,
+// D = 4096 39.0 / 32.9 / *34.9.
 template <bool GOUT>
 static int li_bwd_chain(const bf16* feat, const bf16* dz, const LiModal& m, const float* bias, const float* state_in, const float* dstate_out,
                         float* dstate_in, int with_R, float* S, float* A, float* dRp, float* dLp, float* dBp, bf16* dfeat, const LiDims& d,
                         cudaStream_t st) {
   const dim3 grid((d.D + LV_CH - 1) / LV_CH, d.NC, d.B), modes((unsigned)(((size_t)d.D * LO + 127) / 128), d.B, 2);
+  const long long blocks = (long long)grid.x * grid.y * grid.z, sms = sb::num_sms();
+  const bool own_sms = 2 * blocks + (long long)modes.x * modes.y * modes.z <= sms;
   int rc = launch_chained(true, li_bwd_local_tiled_kernel, grid, 2 * LV_PAIRS, LBL_SMEM, st, feat, dz, m, S, A, d);
   if (!rc) rc = launch_chained(false, li_bwd_prefix_tiled_kernel, modes, 128, 0, st, S, A, m, state_in, dstate_out, dstate_in, with_R, d);
   if (!rc)
-    rc = launch_chained(false, li_bwd_apply_tiled_kernel<GOUT>, grid, 3 * LV_PAIRS, LBA_SMEM, st, feat, dz, m, bias, (const float*)S,
+    rc = launch_chained(blocks < sms && !own_sms, li_bwd_apply_tiled_kernel<GOUT>, grid, 3 * LV_PAIRS, LBA_SMEM, st, feat, dz, m, bias, (const float*)S,
                         (const float*)A, dRp, dLp, dBp, dfeat, dstate_out, d);
   return rc;
 }

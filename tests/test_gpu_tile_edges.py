@@ -509,3 +509,28 @@ def test_gemm_narrow_tiles(M, N, K, a_mn, b_mn):
     want = a.float() @ b.float().t() + bias.float() + 2 * res.float()
     # fp32 accumulation, one bf16 rounding (two where the old value is added after the first): 2^-8
     _close(out, want, 8e-3, "gemm")
+
+
+# blocks of the backward's passes against the SMs: each with an SM of its own, more prefix blocks than SMs, one row of blocks short of a full
+# chip and a full one (148 SMs: D = 1024 has 8 blocks for a chunk of 64 steps)
+@pytest.mark.parametrize("B,L,D", [(1, 300, 256), (2, 300, 256), (1, 1152, 1024), (1, 1217, 1024)])
+@pytest.mark.parametrize("state", [False, True])
+def test_li_backward_launch_forms(B, L, D, state):
+    torch.manual_seed(L + D)
+    O = 16
+    args = [(torch.randn(B, L, 3 * D, device=DEV) * 0.7).to(BF), (torch.rand(D, O, device=DEV) * 0.09 + 0.01).log(),
+            torch.randn(D, O, device=DEV) / math.sqrt(O), -torch.ones(D, O, device=DEV), torch.randn(D, device=DEV)]
+    args += [torch.randn(B, D, O, device=DEV)] if state else []
+    g, gs = torch.randn(B, L, D, device=DEV).to(BF), torch.randn(B, D, O, device=DEV)
+
+    def grads(fn, f32):
+        leaves = [(t.float() if f32 else t).clone().requires_grad_() for t in args]
+        out = fn(*leaves, *([True] if state else []))
+        torch.autograd.backward(out, (g.float() if f32 else g, gs) if state else g.float() if f32 else g)
+        return [t.grad for t in leaves]
+    want = grads(ref.hyena_li_modal, True)
+    first = grads(ops.hyena_li_modal, False)
+    for _ in range(3):                                   # every sum has a fixed order
+        assert all(torch.equal(a, b) for a, b in zip(first, grads(ops.hyena_li_modal, False)))
+    for a, b, n in zip(first, want, ("dfeat", "dgamma", "dR", "dp", "dbias", "dstate")):
+        _close(a, b, 8e-3 if n == "dfeat" else 2e-3, n)  # as in test_li_scan
