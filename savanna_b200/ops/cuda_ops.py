@@ -1202,12 +1202,15 @@ def _li_tiled_chunk(B: int, L: int, D: int) -> int:
         1, 2048, 4096  +69     58    *58     56     87    153
         1, 8192, 1024  +77     62    *58     58     87    153
         1, 8192, 4096  222    165   +148    152   *142    163
-        1, 32768, 4096 849    601    484    443  *+427    472"""
+        1, 32768, 4096 849    601    484    443  *+427    472
+    A sequence of more than 512 * 65535 steps takes longer chunks: a grid has 65535 rows of blocks."""
     if LI_CHUNK_OVERRIDE:
         return int(LI_CHUNK_OVERRIDE)
     tc = 512
     while tc > 32 and B * ((D + 127) // 128) * ((L + tc - 1) // tc) < 512:
         tc //= 2
+    while (L + tc - 1) // tc > 65535:
+        tc *= 2
     return tc
 
 

@@ -279,3 +279,13 @@ def test_li_scan_refuses_shapes_that_do_not_broadcast(shapes, monkeypatch):
     with pytest.raises((RuntimeError, IndexError)):
         cuda_ops.hyena_li_modal(torch.randn(2, 5, 24).bfloat16(), *args)
     assert not lib.calls
+
+
+@pytest.mark.parametrize("L", [1, 512 * 65535, 512 * 65535 + 1, 1024 * 65535])
+@pytest.mark.parametrize("B,D", [(1, 8), (3, 4096)])
+def test_li_chunks_fit_a_grid(B, D, L):
+    """One block row per chunk of the scan: 65535 at most."""
+    from savanna_b200.ops import cuda_ops
+    tc = cuda_ops._li_tiled_chunk(B, L, D)
+    assert (L + tc - 1) // tc <= 65535 and tc >= 32
+    assert tc <= 512 or L > 512 * 65535
