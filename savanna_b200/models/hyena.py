@@ -125,6 +125,9 @@ class HyenaOperator(nn.Module):
     """Hyena-MR (`hyena_mr`, explicit decaying filter of `hyena_mr_len` taps) and Hyena-LI (`hyena`,
     implicit filter as long as the sequence):  z = x1 * ( h * (x2 v) + conv_bias * (x2 v) )."""
 
+    # prefill of cached generation: called with the modal state [B, D, O] behind the sequence (of the class: pickled models have none)
+    state_sink = None
+
     def __init__(self, hidden_size: int, cfg, layer_number: int, operator_type: str, dtype=None, device=None):
         super().__init__()
         self.cfg, self.operator_type = cfg, operator_type
@@ -149,7 +152,6 @@ class HyenaOperator(nn.Module):
         self.conv_bias.model_parallel = True
         self.conv_bias.partition_dim = 0
         self.conv_bias.is_filter_param = True
-        self.state_sink = None             # prefill of cached generation: called with the modal state [B, D, O] behind the sequence
 
     # -- Hyena-MR ---------------------------------------------------------------
     def _forward_mr(self, feat, cp):

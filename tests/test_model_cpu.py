@@ -521,3 +521,29 @@ def test_block_norm_placements_follow_the_reference_order(over):
     assert torch.allclose(got, want, atol=1e-5), (got - want).abs().max()
     losses = [float(tr.train_step(_iter(cfg))) for _ in range(3)]
     assert losses[-1] < losses[0]
+
+
+def test_operator_pickled_before_the_state_sink():
+    """Long operators that were pickled when they had no `state_sink` run and prefill."""
+    import io
+    from savanna_b200.inference.cached import CachedDecoder
+    from savanna_b200.models import build_model
+    from savanna_b200.models.hyena import HyenaOperator
+    cfg = _cfg()
+    cfg.build_tokenizer()
+    torch.manual_seed(0)
+    model = build_model(cfg, device="cpu").eval()
+    toks = torch.randint(0, 256, (1, 20), generator=torch.Generator().manual_seed(1))
+    with torch.no_grad():
+        want = model(toks)
+    for blk in model.blocks():
+        if isinstance(blk.mixer.mixer, HyenaOperator):
+            blk.mixer.mixer.__dict__.pop("state_sink", None)
+            buf = io.BytesIO()
+            torch.save(blk.mixer.mixer, buf)
+            buf.seek(0)
+            blk.mixer.mixer = torch.load(buf, weights_only=False)
+    with torch.no_grad():
+        assert torch.equal(model(toks), want)
+    dec = CachedDecoder(model)
+    assert torch.equal(dec.prefill(toks), want[:, -1].float()) and any("s" in s for s in dec.states)
