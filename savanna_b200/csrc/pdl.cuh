@@ -26,7 +26,9 @@ static int launch_chained(bool first, void (*kernel)(P...), dim3 grid, int threa
   cfg.stream = st;
   cfg.attrs = &attr;
   cfg.numAttrs = first ? 0 : 1;
-  return cudaLaunchKernelEx(&cfg, kernel, P(args)...) == cudaSuccess ? 0 : -2;
+  if (cudaLaunchKernelEx(&cfg, kernel, P(args)...) == cudaSuccess) return 0;
+  (void)cudaGetLastError();              // reported here: the next entry point of this thread would take it for its own
+  return -2;
 }
 
 }  // namespace sb

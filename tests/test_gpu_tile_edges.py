@@ -534,3 +534,16 @@ def test_li_backward_launch_forms(B, L, D, state):
         assert all(torch.equal(a, b) for a, b in zip(first, grads(ops.hyena_li_modal, False)))
     for a, b, n in zip(first, want, ("dfeat", "dgamma", "dR", "dp", "dbias", "dstate")):
         _close(a, b, 8e-3 if n == "dfeat" else 2e-3, n)  # as in test_li_scan
+
+
+def test_refused_launch_is_reported_once():
+    """More sequences than a grid has layers: the scan's launch is refused, and the next operator on this thread is none the wiser."""
+    B, D, O = 65536, 8, 16
+    x, w = torch.randn(4, 128, device=DEV).to(BF), torch.ones(128, device=DEV, dtype=BF)
+    want = ops.rmsnorm(x, w, 1e-6)
+    feat, g = torch.randn(B, 1, 3 * D, device=DEV).to(BF), torch.zeros(D, O, device=DEV)
+    with torch.no_grad():
+        with pytest.raises(RuntimeError, match="code -2"):
+            ops.hyena_li_modal(feat, g, g, g, torch.zeros(D, device=DEV))
+        assert torch.equal(ops.rmsnorm(x, w, 1e-6), want)
+        assert ops.hyena_li_modal(feat[:4], g, g, g, torch.zeros(D, device=DEV)).shape == (4, 1, D)
