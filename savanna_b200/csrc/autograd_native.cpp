@@ -16,6 +16,8 @@
 
 #include <c10/cuda/CUDAStream.h>
 #include <nvtx3/nvToolsExt.h>
+#include <torch/csrc/autograd/graph_task.h>
+#include <torch/csrc/autograd/saved_variable.h>
 #include <torch/extension.h>
 
 namespace {
@@ -208,6 +210,35 @@ Tensor sink(AutogradContext* ctx, const char* key) {
   return it == ctx->saved_data.end() ? Tensor() : it->second.toTensor();
 }
 
+// Intermediate results of a node that joins several operators.  What save_for_backward keeps lives until the whole node has run; these
+// are let go one by one, at their last use in the backward, as they would be between nodes of their own (unless the graph is kept).
+// Hooks and version checks are those of any saved tensor.  Only made when there will be a backward (`train`).
+struct Kept : torch::CustomClassHolder { std::vector<torch::autograd::SavedVariable> v; };
+void keep(AutogradContext* ctx, bool train, std::initializer_list<Tensor> ts) {
+  if (!train) return;
+  auto k = c10::make_intrusive<Kept>();
+  for (const Tensor& t : ts) k->v.emplace_back(t, /*is_output=*/false);
+  ctx->saved_data["kept"] = c10::IValue::make_capsule(std::move(k));
+}
+struct Taker {
+  Kept* k;
+  bool hold = torch::autograd::get_current_graph_task_keep_graph();
+  explicit Taker(AutogradContext* ctx) : k(static_cast<Kept*>(ctx->saved_data["kept"].toCapsule().get())) {}
+  ~Taker() { for (size_t i = 0; !hold && i < k->v.size(); ++i) k->v[i].reset_data(); }
+  Tensor operator()(int i) {
+    Tensor t = k->v[i].unpack();
+    if (!hold) k->v[i].reset_data();
+    return t;
+  }
+};
+bool wants_grad(std::initializer_list<const Tensor*> ts) {
+  if (!at::GradMode::is_enabled()) return false;
+  for (const Tensor* t : ts)
+    if (t && t->requires_grad()) return true;
+  return false;
+}
+const Tensor* given(const OptTensor& t) { return t.has_value() ? &*t : nullptr; }
+
 struct Linear : Function<Linear> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const OptTensor& bias, const OptTensor& residual, bool fuse) {
     Tensor x2 = rows(x), o = alloc({x2.size(0), w.size(0)}, BF16, x.device());
@@ -299,11 +330,12 @@ struct RmsNormResidual : Function<RmsNormResidual> {
 // (linear(norm(x)), x) as one node
 struct NormLinear : Function<NormLinear> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& wn, double eps, int64_t form, const Tensor& w,
-                               const OptTensor& bias, bool fuse) {
+                               const OptTensor& bias, bool fuse, bool train) {
     Norm n = norm_fwd(x, wn, eps, form);
     Tensor y2 = rows(n.y), o = alloc({y2.size(0), w.size(0)}, BF16, x.device());
     gemm(y2, w, o, false, false, opt(bias));
-    ctx->save_for_backward({n.x2, n.w, n.a, y2, w});
+    ctx->save_for_backward({n.x2, n.w, n.a, w});
+    keep(ctx, train, {y2});
     save_norm(ctx, x, eps, form);
     ctx->saved_data["bias"] = bias.has_value();
     if (fuse) ctx->saved_data["sink"] = w;
@@ -311,14 +343,16 @@ struct NormLinear : Function<NormLinear> {
     return {o.view(with_last(x.sizes(), w.size(0))), x.view_as(x)};
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
-    if (!g[0].defined()) return {g[1], Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+    Taker kept(ctx);
+    if (!g[0].defined()) return {g[1], Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
     const variable_list s = ctx->get_saved_variables();
-    const Tensor &x2 = s[0], &wn = s[1], &a = s[2], &y2 = s[3], &w = s[4];
-    Tensor g2 = rows(g[0]), gx, gwn, gw, gb;
-    if (ctx->needs_input_grad(0) || ctx->needs_input_grad(1)) std::tie(gx, gwn) = saved_norm_bwd(ctx, x2, wn, a, input_grad(g2, w), g[1]);
+    const Tensor &x2 = s[0], &wn = s[1], &a = s[2], &w = s[3];
+    Tensor y2 = kept(0), g2 = rows(g[0]), gx, gwn, gw, gb;
     if (ctx->needs_input_grad(2)) gw = weight_grad(g2, y2, w, sink(ctx, "sink"));
+    y2.reset();
+    if (ctx->needs_input_grad(0) || ctx->needs_input_grad(1)) std::tie(gx, gwn) = saved_norm_bwd(ctx, x2, wn, a, input_grad(g2, w), g[1]);
     if (ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(3)) gb = colsum(g2, g[0].scalar_type());
-    return {gx, gwn, Tensor(), Tensor(), gw, gb, Tensor()};
+    return {gx, gwn, Tensor(), Tensor(), gw, gb, Tensor(), Tensor()};
   }
 };
 
@@ -348,7 +382,7 @@ struct Glu : Function<Glu> {
 // one; the residual's gradient is added in the norm's backward kernel.
 struct MlpGated : Function<MlpGated> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& wn, double eps, int64_t form, const Tensor& w12, const Tensor& w3,
-                        const OptTensor& b3, int64_t act, bool fuse12, bool fuse3) {
+                        const OptTensor& b3, int64_t act, bool fuse12, bool fuse3, bool train) {
     Norm n = norm_fwd(x, wn, eps, form);
     const int64_t T = n.x2.size(0), F = w12.size(0) / 2;
     Tensor y2 = rows(n.y), ab = alloc({T, 2 * F}, BF16, x.device()), h = alloc({T, F}, BF16, x.device());
@@ -356,7 +390,8 @@ struct MlpGated : Function<MlpGated> {
     SB_CALL(sb_glu_fwd, 1, ptr(ab), out(h), (long long)T, (int)F, (int)act, stream());
     Tensor h2 = rows(h), o = alloc({T, w3.size(0)}, BF16, x.device());
     gemm(h2, w3, o, false, false, opt(b3), false, rows(n.x2));
-    ctx->save_for_backward({n.x2, n.w, n.a, y2, w12, ab, h2, w3});
+    ctx->save_for_backward({n.x2, n.w, n.a, w12, w3});
+    keep(ctx, train, {y2, ab, h2});
     save_norm(ctx, x, eps, form);
     ctx->saved_data["act"] = act;
     ctx->saved_data["b3"] = b3.has_value();
@@ -366,21 +401,27 @@ struct MlpGated : Function<MlpGated> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     const variable_list s = ctx->get_saved_variables();
-    const Tensor &x2 = s[0], &wn = s[1], &a = s[2], &y2 = s[3], &w12 = s[4], &ab = s[5], &h2 = s[6], &w3 = s[7];
+    const Tensor &x2 = s[0], &wn = s[1], &a = s[2], &w12 = s[3], &w3 = s[4];
+    Taker kept(ctx);
     Tensor g2 = rows(g[0]), gx, gwn, gw12, gw3, gb3;
-    // edges: x, norm weight, w12, w3, b3
+    // edges: x, norm weight, w12, w3, b3.  Alive at most: the gate's inputs, their gradients and the gradient of its output.
     const bool stem = ctx->needs_input_grad(0) || ctx->needs_input_grad(1), need12 = ctx->needs_input_grad(2);
-    Tensor gh = stem || need12 ? input_grad(g2, w3) : Tensor();
+    Tensor h2 = kept(2);
     if (ctx->needs_input_grad(3)) gw3 = weight_grad(g2, h2, w3, sink(ctx, "sink3"));
-    if (gh.defined()) {
-      Tensor dab = alloc_like(ab);
+    h2.reset();
+    if (stem || need12) {
+      Tensor gh = input_grad(g2, w3), ab = kept(1), dab = alloc_like(ab);
       SB_CALL(sb_glu_bwd, 1, ptr(ab), ptr(gh), out(dab), (long long)ab.size(0), (int)(ab.size(1) / 2), (int)ctx->saved_data["act"].toInt(), stream());
-      Tensor gy = stem ? input_grad(dab, w12) : Tensor();
+      gh.reset(); ab.reset();
+      Tensor y2 = kept(0), gy;
       if (need12) gw12 = weight_grad(dab, y2, w12, sink(ctx, "sink12"));
+      y2.reset();
+      if (stem) gy = input_grad(dab, w12);
+      dab.reset();
       if (stem) std::tie(gx, gwn) = saved_norm_bwd(ctx, x2, wn, a, gy, g[0]);
     }
     if (ctx->saved_data["b3"].toBool() && ctx->needs_input_grad(4)) gb3 = colsum(g2, g[0].scalar_type());
-    return {gx, gwn, Tensor(), Tensor(), gw12, gw3, gb3, Tensor(), Tensor(), Tensor()};
+    return {gx, gwn, Tensor(), Tensor(), gw12, gw3, gb3, Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };
 
@@ -639,14 +680,16 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   });
   m.def("norm_linear", [](const Tensor& x, const Tensor& wn, double eps, int64_t form, const py::object& w, const OptTensor& bias) {
     no_transforms();
-    variable_list r = NormLinear::apply(x, wn, eps, form, w.cast<Tensor>(), bias, fused(w));
+    const Tensor wt = w.cast<Tensor>();
+    variable_list r = NormLinear::apply(x, wn, eps, form, wt, bias, fused(w), wants_grad({&x, &wn, &wt, given(bias)}));
     return std::make_tuple(r[0], r[1]);
   });
   m.def("glu", [](const Tensor& ab, int64_t act) { no_transforms(); return Glu::apply(ab, act); });
   m.def("mlp_gated", [](const Tensor& x, const Tensor& wn, double eps, int64_t form, const py::object& w12, const py::object& w3, const OptTensor& b3,
                         int64_t act) {
     no_transforms();
-    return MlpGated::apply(x, wn, eps, form, w12.cast<Tensor>(), w3.cast<Tensor>(), b3, act, fused(w12), fused(w3));
+    const Tensor a = w12.cast<Tensor>(), b = w3.cast<Tensor>();
+    return MlpGated::apply(x, wn, eps, form, a, b, b3, act, fused(w12), fused(w3), wants_grad({&x, &wn, &a, &b, given(b3)}));
   });
   m.def("cross_entropy", [](const Tensor& logits, const Tensor& labels) { no_transforms(); return CrossEntropy::apply(logits, labels); });
   m.def("dwconv", [](const Tensor& x, const Tensor& w, const OptTensor& halo, bool fast) { no_transforms(); return DwConv::apply(x, w, halo, fast); });
@@ -656,9 +699,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   });
   m.def("hyena_mr", [](const Tensor& feat, const Tensor& h, const Tensor& bias, const OptTensor& halo) {
     no_transforms();
-    const bool train = at::GradMode::is_enabled() &&
-                       (feat.requires_grad() || h.requires_grad() || bias.requires_grad() || (halo.has_value() && halo->requires_grad()));
-    return HyenaMR::apply(feat, h, bias, halo, train);
+    return HyenaMR::apply(feat, h, bias, halo, wants_grad({&feat, &h, &bias, given(halo)}));
   });
   m.def("hyena_li", [](const Tensor& feat, const Tensor& gamma, const Tensor& R, const Tensor& p, const Tensor& bias, const OptTensor& state_in,
                        bool want_state, int64_t tc) {

@@ -66,6 +66,68 @@ def test_norm_and_projection_are_their_parts(bias):
             assert a is None or torch.equal(a, b) or (a.float() - b.float()).norm() <= 2 ** -9 * b.float().norm()
 
 
+def _joined(kind):
+    T, D, F = 4096, 512, 4096
+    x, wn = _rand(1, T, D), _rand(D)
+    if kind == "mlp":
+        ws = [_rand(2 * F, D, std=D ** -0.5), _rand(D, F, std=F ** -0.5)]
+
+        def whole(x, wn, w12, w3):
+            return ops.mlp_gated(x, wn, 1e-6, "te", w12, w3, None, "silu")
+
+        def parts(x, wn, w12, w3):
+            y, res = ops.rmsnorm_residual(x, wn, 1e-6)
+            return ops.linear(ops.glu_act_packed(ops.linear(y, w12), "silu"), w3, None, residual=res)
+    else:
+        ws = [_rand(3 * D, D, std=D ** -0.5)]
+
+        def whole(x, wn, w):
+            y, res = ops.norm_linear(x, wn, 1e-6, "te", w, None)
+            return torch.cat([y, res], -1)
+
+        def parts(x, wn, w):
+            y, res = ops.rmsnorm_residual(x, wn, 1e-6)
+            return torch.cat([ops.linear(y, w), res], -1)
+    return [x, wn] + ws, whole, parts
+
+
+def _leaves(ts, frozen=()):
+    return [t.clone().requires_grad_(i not in frozen) for i, t in enumerate(ts)]
+
+
+@pytest.mark.parametrize("kind", ["mlp", "norm_linear"])
+@pytest.mark.parametrize("frozen", [(), (2,), (3,), (0, 1)])
+def test_joined_nodes_need_no_more_memory_than_their_parts(kind, frozen):
+    ts, whole, parts = _joined(kind)
+    peak = []
+    for fn in (whole, parts, whole, parts):
+        leaves = _leaves(ts, frozen)
+        out = fn(*leaves)
+        g = torch.randn_like(out)
+        del fn
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        out.backward(g)
+        torch.cuda.synchronize()
+        peak.append(torch.cuda.max_memory_allocated() - before)
+        del out, g, leaves
+    # the parts allocate the same tensors; a megabyte for the norm's partial sums, of which both have one set
+    assert min(peak[0], peak[2]) <= max(peak[1], peak[3]) + 2 ** 20, [p / 2 ** 20 for p in peak]
+
+
+@pytest.mark.parametrize("kind", ["mlp", "norm_linear"])
+def test_joined_nodes_keep_their_graph_when_asked(kind):
+    ts, whole, _ = _joined(kind)
+    leaves = _leaves([t[:, :64] if i == 0 else t for i, t in enumerate(ts)])
+    out = whole(*leaves)
+    g = torch.randn_like(out)
+    a, b, c = (torch.autograd.grad(out, leaves, g, retain_graph=r) for r in (True, True, False))
+    assert all(torch.equal(x, y) and torch.equal(x, z) for x, y, z in zip(a, b, c))
+    with pytest.raises(RuntimeError, match="second time"):
+        torch.autograd.grad(out, leaves, g)
+
+
 def test_only_the_residual_branch_is_used():
     x = _rand(2, 8, 128).requires_grad_()
     _, res = ops.norm_linear(x, _rand(128), 1e-6, "te", _rand(64, 128))
