@@ -13,6 +13,7 @@
 
 #include <atomic>
 #include <mutex>
+#include <sstream>
 
 #include <c10/cuda/CUDAStream.h>
 #include <nvtx3/nvToolsExt.h>
@@ -36,6 +37,8 @@ constexpr auto F32 = at::kFloat;
 // ------------------------------------------------------------------------------------ the library's entry points
 #define SB_ENTRIES(X)                                                                                                                  \
   X(sb_gemm_bf16, const void*, const void*, void*, const void*, const void*, int, int, int, int, int, int, int, int, int, int, void*, int, Stream) \
+  X(sb_gemm_last_error_detail)                                                                                                         \
+  X(sb_attn_last_encode_result)                                                                                                        \
   X(sb_colsum, const void*, float*, int, int, Stream)                                                                                  \
   X(sb_rmsnorm_fwd, const void*, const void*, void*, float*, int, int, float, int, Stream)                                             \
   X(sb_rmsnorm_bwd_blocks, int, int)                                                                                                   \
@@ -82,17 +85,32 @@ void load(const std::string& path, py::object ops) {
   g_ops = ops.release().ptr();             // lives as long as the process
 }
 
-// One call of an entry point: NVTX range while the profiler wants one, launch count, error code.
+// What was handed to an entry point that refused it: name, shape, strides, address.
+std::string layouts(std::initializer_list<std::pair<const char*, const Tensor*>> ts) {
+  std::ostringstream s;
+  for (const auto& [name, t] : ts) {
+    s << (s.tellp() > 0 ? ", " : "") << name;
+    if (t->defined()) s << t->sizes() << '/' << t->strides() << " at " << t->const_data_ptr();
+    else s << " none";
+  }
+  return s.str();
+}
+// One call of an entry point: NVTX range while the profiler wants one, launch count; its error code.
 template <class... A, class... B>
-void call(const char* name, int launches, int (*fn)(A...), B... args) {
+int run(const char* name, int launches, int (*fn)(A...), B... args) {
   const bool mark = g_nvtx.load(std::memory_order_relaxed);
   if (mark) nvtxRangePushA(name);
   const int rc = fn(args...);
   if (mark) nvtxRangePop();
-  TORCH_CHECK(rc == 0, "savanna_b200 kernel `", name + 3, "` rejected its arguments or failed to launch (code ", rc, ")");
-  g_launches.fetch_add(launches, std::memory_order_relaxed);
+  if (rc == 0) g_launches.fetch_add(launches, std::memory_order_relaxed);
+  return rc;
 }
-#define SB_CALL(name, launches, ...) call(#name, launches, L.name, __VA_ARGS__)
+#define SB_RUN(name, launches, ...) run(#name, launches, L.name, __VA_ARGS__)
+#define SB_CALL(name, launches, ...)                                                                                     \
+  do {                                                                                                                   \
+    const int rc_ = SB_RUN(name, launches, __VA_ARGS__);                                                                 \
+    TORCH_CHECK(rc_ == 0, "savanna_b200 kernel `", #name + 3, "` rejected its arguments or failed to launch (code ", rc_, ")"); \
+  } while (0)
 
 Stream stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 
@@ -175,8 +193,14 @@ void gemm(const Tensor& a, const Tensor& b, const Tensor& o, bool a_mn, bool b_m
   TORCH_CHECK_VALUE(!residual.defined() || (residual.dim() == 2 && residual.stride(1) == 1 && residual.scalar_type() == BF16 &&
                                             residual.size(0) == M && residual.size(1) == N),
                     "gemm residual must be a [M, N] bf16 matrix with unit inner stride");
-  SB_CALL(sb_gemm_bf16, 1, ptr(a), ptr(b), out(o), ptr(bias), ptr(residual), M, N, K, (int)a.stride(0), (int)b.stride(0), (int)o.stride(0),
-          residual.defined() ? (int)residual.stride(0) : 0, (int)a_mn, (int)b_mn, (int)accumulate, status_word(o.device()), 0, stream());
+  const int rc = SB_RUN(sb_gemm_bf16, 1, ptr(a), ptr(b), out(o), ptr(bias), ptr(residual), M, N, K, (int)a.stride(0), (int)b.stride(0),
+                        (int)o.stride(0), residual.defined() ? (int)residual.stride(0) : 0, (int)a_mn, (int)b_mn, (int)accumulate,
+                        status_word(o.device()), 0, stream());
+  if (rc) {
+    const int detail = L.sb_gemm_last_error_detail();
+    TORCH_CHECK(false, "gemm_bf16 failed (code ", rc, ", operand ", detail >> 16, ", driver result ", detail & 0xffff, "): M=", M, " N=", N, " K=", K,
+                " a_mn=", a_mn, " b_mn=", b_mn, " ", layouts({{"a", &a}, {"b", &b}, {"out", &o}, {"residual", &residual}}));
+  }
 }
 
 Tensor colsum(const Tensor& g2, at::ScalarType dtype) {
@@ -602,8 +626,9 @@ void rope2(const Tensor& s0, const Tensor& d0, const Tensor& s1, const Tensor& d
   const Strides a(s0), b(s1), c(d0), d(d1);
   const long long ss[6] = {a.s[0], a.s[1], a.s[2], b.s[0], b.s[1], b.s[2]}, ds[6] = {c.s[0], c.s[1], c.s[2], d.s[0], d.s[1], d.s[2]};
   const int wide[2] = {s0.scalar_type() == F32, s1.scalar_type() == F32};
-  SB_CALL(sb_attn_rope, 1, src, dst, ss, ds, wide, 2, f32(cos), f32(sin), (int)s0.size(0), (int)s0.size(1), (int)s0.size(2), (int)cos.size(-1),
-          (int)inverse, stream());
+  const int rc = SB_RUN(sb_attn_rope, 1, src, dst, ss, ds, wide, 2, f32(cos), f32(sin), (int)s0.size(0), (int)s0.size(1), (int)s0.size(2),
+                        (int)cos.size(-1), (int)inverse, stream());
+  TORCH_CHECK(rc == 0, "rotary embedding failed (code ", rc, "): ", layouts({{"cos", &cos}, {"from", &s0}, {"to", &d0}, {"from", &s1}, {"to", &d1}}));
 }
 bool packed_rows(const Tensor& t) {        // what the kernels read in place: unit inner stride, the others on 16-byte boundaries
   return t.dim() == 4 && t.scalar_type() == BF16 && t.size(3) == 128 && t.stride(3) == 1 && t.stride(0) % 8 == 0 && t.stride(1) % 8 == 0 &&
@@ -626,8 +651,9 @@ struct FlashPacked : Function<FlashPacked> {
     }
     Tensor o = alloc({B, Ln, H, 128}, BF16, dev), lse = alloc({B, H, Ln}, F32, dev);
     const Strides qs(q), ks(k), vs(v), os(o);
-    SB_CALL(sb_attn_fwd, 1, ptr(q), ptr(k), ptr(v), out(o), f32o(lse), (int)B, (int)H, (int)Ln, (int)Ln, qs.s, ks.s, vs.s, os.s, (int)causal,
-            0.08838834764831845f, status_word(dev), stream());
+    const int rc = SB_RUN(sb_attn_fwd, 1, ptr(q), ptr(k), ptr(v), out(o), f32o(lse), (int)B, (int)H, (int)Ln, (int)Ln, qs.s, ks.s, vs.s, os.s,
+                          (int)causal, 0.08838834764831845f, status_word(dev), stream());
+    TORCH_CHECK(rc == 0, "attention forward failed (code ", rc, ", encode ", L.sb_attn_last_encode_result(), "): ", layouts({{"q", &q}, {"k", &k}, {"v", &v}}));
     ctx->save_for_backward({qkv, qr, kr, o, lse, cos, sin});
     ctx->saved_data["causal"] = causal;
     return o;
@@ -643,9 +669,11 @@ struct FlashPacked : Function<FlashPacked> {
     Tensor dqkv = alloc(qkv.sizes(), BF16, dev), dq = dqkv.slice(3, 0, 128), dk = dqkv.slice(3, 128, 256), dv = dqkv.slice(3, 256, 384);
     Tensor acc = zeros({B, Ln, H, 128}, F32, dev), stats = alloc({2 * B * H * ((Ln + 63) / 64 * 64)}, F32, dev);
     const Strides gs(go), qs(q), ks(k), vs(v), os(o), dqs(rot ? o : dq), dks(dk), dvs(dv);
-    SB_CALL(sb_attn_bwd, 3, ptr(go), ptr(q), ptr(k), ptr(v), ptr(o), f32(lse), (const float*)nullptr, f32o(stats), f32o(acc),
-            rot ? (void*)nullptr : out(dq), out(dk), (int)B, (int)H, (int)Ln, (int)Ln, out(dv), gs.s, qs.s, ks.s, vs.s, os.s, dqs.s, dks.s, dvs.s,
-            (int)ctx->saved_data["causal"].toBool(), 0.08838834764831845f, status_word(dev), stream());
+    const int rc = SB_RUN(sb_attn_bwd, 3, ptr(go), ptr(q), ptr(k), ptr(v), ptr(o), f32(lse), (const float*)nullptr, f32o(stats), f32o(acc),
+                          rot ? (void*)nullptr : out(dq), out(dk), (int)B, (int)H, (int)Ln, (int)Ln, out(dv), gs.s, qs.s, ks.s, vs.s, os.s, dqs.s,
+                          dks.s, dvs.s, (int)ctx->saved_data["causal"].toBool(), 0.08838834764831845f, status_word(dev), stream());
+    TORCH_CHECK(rc == 0, "attention backward failed (code ", rc, ", encode ", L.sb_attn_last_encode_result(), "): ",
+                layouts({{"dout", &go}, {"q", &q}, {"k", &k}, {"v", &v}}));
     if (rot) rope2(acc, dq, dk, dk, cos, sin, true);
     return {dqkv, Tensor(), Tensor(), Tensor()};
   }

@@ -185,3 +185,15 @@ def test_refusals():
     z.backward()
     with pytest.raises(RuntimeError):
         z.backward()                                 # the saved tensors are gone
+
+
+def test_refusals_name_what_was_handed_over():
+    """A weight two bytes off a 16-byte boundary and a rotary width that the kernels do not have: refused on the host, with the operands."""
+    from savanna_b200.ops import flash_sm100
+    x, w = _rand(4, 128), _rand(64 * 128 + 1)[1:].view(64, 128)
+    with pytest.raises(RuntimeError, match=r"gemm_bf16 failed \(code -4.*M=4 N=64 K=128 .*a\[4, 128\]/\[128, 1\] at 0x\w+, b\[64, 128\]/\[128, 1\] at 0x\w+2, out\[4, 64\]"):
+        ops.linear(x, w)
+    qkv, t = _rand(1, 8, 2, 384), torch.zeros(8, 24, device=DEV)
+    with pytest.raises(RuntimeError, match=r"rotary embedding failed \(code -3\): cos\[8, 24\].*from\[1, 8, 2, 128\]/\[6144, 768, 384, 1\]"):
+        flash_sm100.attention_packed(qkv, t, t, True)
+    assert torch.equal(ops.linear(x, w.clone()), ops.linear(x, w.clone()))
