@@ -116,6 +116,7 @@ def bench_gemm(T, iters):
         report(f"gemm.{name}.fwd.ours_fp8_pair", timeit(lambda: cuda_ops.gemm_fp8(xq, wq, out, al), iters), fl)
         report(f"gemm.{name}.dgrad.ours_fp8_pair", timeit(lambda: cuda_ops.gemm_fp8(gq, wq, gx, al, b_mn=True, a_fmt=1), iters), fl)
         report(f"gemm.{name}.wgrad.ours_fp8_pair", timeit(lambda: cuda_ops.gemm_fp8(gq, xq, gw, al, a_mn=True, b_mn=True, a_fmt=1), iters), fl)
+        cuda_ops.set_gemm_pair_mode(3)
         if N % 32 == 0 and K % 32 == 0 and M % 32 == 0:
             # block-scaled fp8: the three products of a projection on operands quantised along their own contraction
             xm, sxm = cuda_ops.mx_quantize(x); wm, swm = cuda_ops.mx_quantize(w); gm, sgm = cuda_ops.mx_quantize(gy)

@@ -618,7 +618,7 @@ int make_tmap_2d_u8(CUtensorMap* out, const void* base, uint64_t inner, uint64_t
 static int g_num_sms = 0;
 static int g_last_detail = 0;   // (which operand << 16) | CUresult of the last failed tensor-map encode
 
-static int g_pair_mode = 2;      // 1: CTA-pair kernel for one-byte operands, 2: for every GEMM, 0: never
+static int g_pair_mode = 3;      // CTA-pair kernel 0: never, 1: for one-byte operands, 2: for every GEMM, 3: where pick_tile chooses it
 
 // Tile of a GEMM on `sms` SMs: 0 = the CTA-pair kernel's 256 x 256, or the width of a single-CTA tile 128 x {128, 64}, for
 // outputs with too few 256 x 256 tiles to fill the chip.  Compared are waves times cycles of a tile per 128-byte k-block: an SM
@@ -635,6 +635,12 @@ static int pick_tile(int M, int N, int sms, bool b_box128) {
   const long long w128 = waves(m1 * ((N + 127) / 128), sms) * 320, w64 = waves(m1 * ((N + 63) / 64), sms) * 260;
   if (8 * (w64 < w128 && !b_box128 ? w64 : w128) > 7 * pair) return 0;
   return 8 * w64 <= 7 * w128 && !b_box128 ? 64 : 128;
+}
+
+// The kernel that a GEMM takes in the present mode: 0 = the CTA pair, else the width of a single-CTA tile.
+static int chosen_tile(int M, int N, int sms, bool one_byte, bool b_mn, int max_ctas) {
+  if (g_pair_mode < (one_byte ? 1 : 2) || max_ctas > 0) return BN;
+  return g_pair_mode == 3 ? pick_tile(M, N, sms, one_byte && b_mn) : 0;
 }
 
 // Launch the single-CTA kernel with tile width BNT.
@@ -694,8 +700,12 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const Gem
 }  // namespace sb
 
 extern "C" int sb_gemm_last_error_detail() { return sb::g_last_detail; }
-// 0: single-CTA tiles only; 1: CTA pairs (cta_group::2) for fp8 operands; 2: CTA pairs for bf16 operands too
+// 0: single-CTA tiles only; 1: CTA pairs (cta_group::2) for fp8 operands; 2: CTA pairs for bf16 operands too; 3 (default): by size
 extern "C" int sb_gemm_set_pair_mode(int mode) { sb::g_pair_mode = mode; return 0; }
+// What a GEMM of this size runs on a chip of `sms` SMs in the present mode: 0 = CTA pairs, else the width of a 128-row tile.
+extern "C" int sb_gemm_tile(int M, int N, int one_byte, int b_mn, int max_ctas, int sms) {
+  return sb::chosen_tile(M, N, sms, one_byte != 0, b_mn != 0, max_ctas);
+}
 
 // C = A * B^T (+bias) (+residual) (+C).  a_mn = 0: A is [M, K] row-major with leading dim lda; a_mn = 1: A is stored
 // transposed as [K, M] with leading dim lda.  b_mn likewise for B ([N, K] or [K, N]).  All leading dims and
@@ -717,8 +727,7 @@ extern "C" int sb_gemm_bf16(const void* A, const void* B, void* C, const void* b
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
   }
-  const bool paired = g_pair_mode >= 2 && max_ctas <= 0;
-  const int width = paired ? pick_tile(M, N, g_num_sms, false) : BN;
+  const int width = chosen_tile(M, N, g_num_sms, false, b_mn != 0, max_ctas);
   CUtensorMap tmA, tmB;
   int rc;
   if (!a_mn) rc = make_tmap_2d_bf16(&tmA, A, K, M, lda, BK, BM);
@@ -834,7 +843,7 @@ extern "C" int sb_gemm_fp8(const void* A, const void* B, void* C, const void* bi
   if ((N % 8) || (lda % 16) || (ldb % 16) || (ldc % 8) || ((!a_mn || !b_mn) && (K % 16))) return -3;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 15) return -4;
   if (!g_num_sms) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev); }
-  const int width = g_pair_mode >= 1 ? pick_tile(M, N, g_num_sms, b_mn != 0) : BN;
+  const int width = chosen_tile(M, N, g_num_sms, true, b_mn != 0, 0);
   CUtensorMap tmA, tmB;
   int rc;
   if (!a_mn) rc = make_tmap_2d_u8(&tmA, A, K, M, lda, 128, BM);

@@ -140,6 +140,7 @@ class _Sig:
     sb_gemm_bf16 = [P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, P, I, P]
     sb_colsum = [P, P, I, I, P]
     sb_gemm_set_pair_mode = [I]
+    sb_gemm_tile = [I, I, I, I, I, I]
     sb_gemm_fp8 = [P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, I, P, P]
     sb_quantize_fp8 = [P, P, P, P, LL, I, P]
     sb_quantize_fp8_delayed = [P, P, P, I, I, P, LL, I, P]
@@ -360,14 +361,21 @@ def set_conv_forward_variant(tiled: bool) -> None:
     require().sb_conv_set_fwd_variant(int(CONV_FWD_FAST))
 
 
-_PAIR_MODE = 2
+_PAIR_MODE = 3
 
 
 def set_gemm_pair_mode(mode: int) -> None:
-    """0: one CTA per 128 x 256 tile; 1: CTA pairs (cta_group::2, 256 x 256 tiles) for fp8 operands; 2: for bf16 too."""
+    """0: one CTA per 128 x 256 tile; 1: CTA pairs (cta_group::2, 256 x 256 tiles) for fp8 operands; 2: for bf16 too; 3 (default): CTA
+    pairs, or single-CTA tiles 128 x 128 or 128 x 64 for outputs that leave the chip idle in 256 x 256 ones."""
     global _PAIR_MODE
     require().sb_gemm_set_pair_mode(int(mode))
     _PAIR_MODE = int(mode)
+
+
+def gemm_tile(M: int, N: int, fp8: bool = False, b_mn: bool = False, max_ctas: int = 0, sms: Optional[int] = None) -> int:
+    """The kernel of an [M, N] product in the present mode: 0 for CTA pairs, else the width of its 128-row tiles."""
+    sms = sms or torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+    return require().sb_gemm_tile(M, N, int(fp8), int(b_mn), max_ctas, sms)
 
 
 def colsum(x2: torch.Tensor) -> torch.Tensor:

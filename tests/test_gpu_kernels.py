@@ -45,8 +45,10 @@ def pair_mode(request):
     """Runs a GEMM test with the single-CTA kernel and with the cta_group::2 kernel."""
     from savanna_b200.ops import cuda_ops
     cuda_ops.set_gemm_pair_mode(request.param)
+    # whatever the size, with fp8 operands too
+    assert {cuda_ops.gemm_tile(M, N, fp8) for M in (128, 8192) for N in (264, 4096) for fp8 in (False, True)} == {0 if request.param else 256}
     yield request.param
-    cuda_ops.set_gemm_pair_mode(2)
+    cuda_ops.set_gemm_pair_mode(3)
 
 
 @pytest.mark.parametrize("M,N,K", [(128, 256, 64), (256, 512, 256), (300, 264, 136), (1024, 768, 512), (8192, 512, 1024)])
@@ -434,6 +436,7 @@ def test_gemm_cta_pair_bf16(M, N, K):
     from savanna_b200.ops import cuda_ops
     torch.manual_seed(40)
     cuda_ops.set_gemm_pair_mode(2)
+    assert cuda_ops.gemm_tile(M, N) == 0
     try:
         a = torch.randn(M, K, device=DEV, dtype=BF); b = torch.randn(N, K, device=DEV, dtype=BF)
         at, bt = a.t().contiguous(), b.t().contiguous()
@@ -452,7 +455,7 @@ def test_gemm_cta_pair_bf16(M, N, K):
         cuda_ops.gemm(a, b, out, bias=bias, residual=res, accumulate=True)
         _status_ok(); _rel(out, want + bias.float() + res.float() + c0.float(), 1e-2, "pair epilogue")
     finally:
-        cuda_ops.set_gemm_pair_mode(2)
+        cuda_ops.set_gemm_pair_mode(3)
 
 
 @pytest.mark.parametrize("M,N,K", [(256, 256, 128), (384, 512, 640), (1008, 528, 1040)])
@@ -463,6 +466,7 @@ def test_gemm_cta_pair_fp8(M, N, K):
     def deq(q, sinv, fmt):
         return q.view(torch.float8_e4m3fn if fmt == 0 else torch.float8_e5m2).float() * sinv
     cuda_ops.set_gemm_pair_mode(1)
+    assert cuda_ops.gemm_tile(M, N, fp8=True) == cuda_ops.gemm_tile(M, N, fp8=True, b_mn=True) == 0 and cuda_ops.gemm_tile(M, N) == 256
     try:
         a = torch.randn(M, K, device=DEV, dtype=BF); b = torch.randn(N, K, device=DEV, dtype=BF)
         aq, sa = cuda_ops.quantize_fp8(a, 1); bq, sb_ = cuda_ops.quantize_fp8(b, 0)
@@ -475,7 +479,7 @@ def test_gemm_cta_pair_fp8(M, N, K):
         out.fill_(float("nan")); cuda_ops.gemm_fp8(atq, btq, out, sat, alpha2=sbt, a_mn=True, b_mn=True, a_fmt=1, b_fmt=0)
         _status_ok(); _rel(out, deq(atq, sat, 1).t() @ deq(btq, sbt, 0), 1e-2, "pair fp8 wgrad layout")
     finally:
-        cuda_ops.set_gemm_pair_mode(2)
+        cuda_ops.set_gemm_pair_mode(3)
 
 
 def test_quantize_fp8_matches_torch():

@@ -502,6 +502,7 @@ def test_gemm_narrow_tiles(M, N, K, a_mn, b_mn):
     torch.manual_seed(M + N)
     if (a_mn and M % 8) or (b_mn and N % 8):
         pytest.skip("rows of a transposed operand start on 16-byte boundaries")
+    assert cuda_ops.gemm_tile(M, N) in (64, 128)
     a, b = torch.randn(M, K, device=DEV).to(BF), torch.randn(N, K, device=DEV).to(BF)
     bias, res = torch.randn(N, device=DEV).to(BF), torch.randn(M, N, device=DEV).to(BF)
     out = res.clone()
