@@ -548,3 +548,33 @@ def test_refused_launch_is_reported_once():
             ops.hyena_li_modal(feat, g, g, g, torch.zeros(D, device=DEV))
         assert torch.equal(ops.rmsnorm(x, w, 1e-6), want)
         assert ops.hyena_li_modal(feat[:4], g, g, g, torch.zeros(D, device=DEV)).shape == (4, 1, D)
+
+
+# narrow tiles of which a CTA takes two or more (148 SMs): both accumulators, their barriers' phases, a ring of stages that goes on into the
+# next tile; partial tiles at both edges, contractions shorter and longer than the ring
+@pytest.mark.parametrize("M,N,K,width", [(384, 10240, 520, 128), (333, 22528, 200, 128), (19001, 56, 200, 64), (38301, 64, 1032, 64)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_gemm_narrow_tiles_in_turn(M, N, K, width, a_mn, b_mn, fp8):
+    from savanna_b200.ops import cuda_ops
+    torch.manual_seed(M + N)
+    unit = 16 if fp8 else 8
+    if fp8:
+        K += -K % 16                                     # rows of an fp8 operand start on 16-byte boundaries
+    if a_mn:
+        M += -M % unit
+    if b_mn:
+        N += -N % unit
+    want_width = 128 if fp8 and b_mn else width          # an MN-major fp8 operand comes in boxes of 128 columns
+    assert cuda_ops.gemm_tile(M, N, fp8, b_mn) == want_width and -(-M // 128) * -(-N // want_width) > 148
+    a, b = torch.randn(M, K, device=DEV).to(BF), torch.randn(N, K, device=DEV).to(BF)
+    out = torch.full((M, N), float("nan"), device=DEV, dtype=BF)
+    if fp8:
+        (aq, sa), (bq, sb_) = (cuda_ops.quantize_fp8(t.t().contiguous() if mn else t, 0) for t, mn in ((a, a_mn), (b, b_mn)))
+        cuda_ops.gemm_fp8(aq, bq, out, sa, alpha2=sb_, a_mn=a_mn, b_mn=b_mn)
+        a, b = (q.view(torch.float8_e4m3fn).float() * s for q, s in ((aq, sa), (bq, sb_)))
+        a, b = a.t() if a_mn else a, b.t() if b_mn else b
+    else:
+        cuda_ops.gemm(a.t().contiguous() if a_mn else a, b.t().contiguous() if b_mn else b, out, a_mn, b_mn)
+    cuda_ops.check_status()
+    _close(out, a.float() @ b.float().t(), 4e-3, "gemm")  # fp32 accumulation, one bf16 rounding: 2^-9
