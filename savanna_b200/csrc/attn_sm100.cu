@@ -17,6 +17,7 @@
 //               memory, rescale of O in TMEM only when the running maximum grew by more than 2^8
 //
 // Every wait is bounded (sm100.cuh); on a timeout the CTA records a status code, frees TMEM and returns.
+#include "entries.h"
 #include "sm100.cuh"
 
 namespace sb {

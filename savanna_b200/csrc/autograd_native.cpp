@@ -8,7 +8,7 @@
 // gated MLP [999 x 1024] 329 -> 168, a step of a four-operator model, 2 x 1024 tokens of 256 channels, 4181 -> 2201.
 // Python keeps what decides (ops/cuda_ops.py: shapes, types, which operator), and the oracle.
 //
-// Nothing is cached between calls but the entry points and the address of the per-device status word.
+// Nothing is cached between calls but the entry points (entries.h) and the address of the per-device status word.
 #include <dlfcn.h>
 
 #include <atomic>
@@ -21,6 +21,8 @@
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/extension.h>
 
+#include "entries.h"
+
 namespace {
 
 namespace py = pybind11;
@@ -29,43 +31,19 @@ using torch::autograd::AutogradContext;
 using torch::autograd::Function;
 using torch::autograd::variable_list;
 typedef std::optional<Tensor> OptTensor;
-typedef void* Stream;
 
 constexpr auto BF16 = at::kBFloat16;
 constexpr auto F32 = at::kFloat;
 
 // ------------------------------------------------------------------------------------ the library's entry points
-#define SB_ENTRIES(X)                                                                                                                  \
-  X(sb_gemm_bf16, const void*, const void*, void*, const void*, const void*, int, int, int, int, int, int, int, int, int, int, void*, int, Stream) \
-  X(sb_gemm_last_error_detail)                                                                                                         \
-  X(sb_attn_last_encode_result)                                                                                                        \
-  X(sb_colsum, const void*, float*, int, int, Stream)                                                                                  \
-  X(sb_rmsnorm_fwd, const void*, const void*, void*, float*, int, int, float, int, Stream)                                             \
-  X(sb_rmsnorm_bwd_blocks, int, int)                                                                                                   \
-  X(sb_rmsnorm_bwd, const void*, const void*, const void*, const float*, const void*, void*, void*, float*, int, int, float, int, Stream) \
-  X(sb_glu_fwd, const void*, void*, long long, int, int, Stream)                                                                       \
-  X(sb_glu_bwd, const void*, const void*, void*, long long, int, int, Stream)                                                          \
-  X(sb_ce_fwd, const void*, const void*, float*, float*, long long, int, Stream)                                                       \
-  X(sb_ce_bwd, const void*, const void*, const float*, const float*, void*, long long, int, Stream)                                    \
-  X(sb_dwconv_fwd, const void*, const void*, const float*, void*, int, int, int, int, Stream)                                          \
-  X(sb_dwconv_fwd_taps, const void*, const void*, const void*, int, float*, void*, int, int, int, int, Stream)                         \
-  X(sb_dwconv_bwd, const void*, const void*, const float*, const void*, void*, void*, float*, int, int, int, int, Stream)              \
-  X(sb_se_fwd, const void*, const void*, const float*, void*, int, int, int, int, int, int, int, Stream)                               \
-  X(sb_se_fwd_taps, const void*, const void*, const void*, int, float*, void*, int, int, int, int, int, int, int, Stream)              \
-  X(sb_se_bwd, const void*, const void*, const float*, const void*, void*, void*, float*, int, int, int, int, int, int, int, Stream)   \
-  X(sb_mr_fwd, const void*, const void*, const float*, const float*, void*, void*, int, int, int, int, int, Stream)                    \
-  X(sb_mr_bwd, const void*, const void*, const float*, const float*, const void*, const void*, void*, void*, float*, float*, int, int, int, int, int, Stream) \
-  X(sb_mr_tc_fwd, const void*, const void*, const float*, const float*, void*, int, int, int, int, int, Stream)                        \
-  X(sb_mr_tc_bwd, const void*, const void*, const float*, const float*, const void*, void*, void*, float*, float*, int, int, int, int, int, Stream) \
-  X(sb_li_fwd_tiled, const void*, const float*, const float*, const float*, const float*, const float*, float*, float*, float*, void*, int, int, int, int, int, Stream) \
-  X(sb_li_bwd_tiled_chunk)                                                                                                             \
-  X(sb_li_bwd_tiled, const void*, const void*, const float*, const float*, const float*, const float*, float*, float*, float*, float*, void*, float*, float*, float*, float*, int, int, int, int, Stream) \
-  X(sb_attn_fwd, const void*, const void*, const void*, void*, float*, int, int, int, int, const long long*, const long long*, const long long*, const long long*, int, float, void*, Stream) \
-  X(sb_attn_bwd, const void*, const void*, const void*, const void*, const void*, const float*, const float*, float*, float*, void*, void*, int, int, int, int, void*, const long long*, const long long*, const long long*, const long long*, const long long*, const long long*, const long long*, const long long*, int, float, void*, Stream) \
-  X(sb_attn_rope, const void* const*, void* const*, const long long*, const long long*, const int*, int, const float*, const float*, int, int, int, int, int, Stream)
+#define SB_ENTRIES(X) \
+  X(sb_gemm_bf16) X(sb_gemm_last_error_detail) X(sb_attn_last_encode_result) X(sb_colsum) X(sb_rmsnorm_fwd) X(sb_rmsnorm_bwd_blocks) \
+  X(sb_rmsnorm_bwd) X(sb_glu_fwd) X(sb_glu_bwd) X(sb_ce_fwd) X(sb_ce_bwd) X(sb_dwconv_fwd) X(sb_dwconv_fwd_taps) X(sb_dwconv_bwd) \
+  X(sb_se_fwd) X(sb_se_fwd_taps) X(sb_se_bwd) X(sb_mr_fwd) X(sb_mr_bwd) X(sb_mr_tc_fwd) X(sb_mr_tc_bwd) X(sb_li_fwd_tiled) \
+  X(sb_li_bwd_tiled_chunk) X(sb_li_bwd_tiled) X(sb_attn_fwd) X(sb_attn_bwd) X(sb_attn_rope)
 
 struct {
-#define SB_DECLARE(name, ...) int (*name)(__VA_ARGS__) = nullptr;
+#define SB_DECLARE(name) decltype(&::name) name = nullptr;
   SB_ENTRIES(SB_DECLARE)
 #undef SB_DECLARE
 } L;
@@ -77,7 +55,7 @@ std::atomic<bool> g_guarded{false}, g_nvtx{false};
 void load(const std::string& path, py::object ops) {
   void* h = dlopen(path.c_str(), RTLD_NOW | RTLD_LOCAL);
   if (!h) throw std::runtime_error(std::string("cannot load ") + path + ": " + dlerror());
-#define SB_RESOLVE(name, ...)                                     \
+#define SB_RESOLVE(name)                                          \
   *reinterpret_cast<void**>(&L.name) = dlsym(h, #name);           \
   if (!L.name) throw std::runtime_error("no entry point " #name " in " + path);
   SB_ENTRIES(SB_RESOLVE)
@@ -112,7 +90,7 @@ int run(const char* name, int launches, int (*fn)(A...), B... args) {
     TORCH_CHECK(rc_ == 0, "savanna_b200 kernel `", #name + 3, "` rejected its arguments or failed to launch (code ", rc_, ")"); \
   } while (0)
 
-Stream stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+cudaStream_t stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 
 // ------------------------------------------------------------------------------------ tensors
 Tensor alloc(at::IntArrayRef shape, at::ScalarType dtype, at::Device device) {
@@ -130,6 +108,7 @@ Tensor zeros(at::IntArrayRef shape, at::ScalarType dtype, at::Device device) { r
 
 const void* ptr(const Tensor& t) { return t.defined() ? t.const_data_ptr() : nullptr; }
 void* out(const Tensor& t) { return t.defined() ? t.mutable_data_ptr() : nullptr; }
+const long long* i64(const Tensor& t) { return static_cast<const long long*>(ptr(t)); }
 const float* f32(const Tensor& t) { return static_cast<const float*>(ptr(t)); }
 float* f32o(const Tensor& t) { return static_cast<float*>(out(t)); }
 // Operands that may be absent reach Function::apply as empty optionals (it refuses undefined tensors) and have no edge then: the edges
@@ -162,9 +141,9 @@ std::vector<int64_t> with_last(at::IntArrayRef shape, int64_t n) {
   return s;
 }
 
-void* status_word(at::Device device) {
+unsigned int* status_word(at::Device device) {
   static std::mutex m;
-  static void* word[64] = {nullptr};
+  static unsigned int* word[64] = {nullptr};
   const int i = device.index() < 0 ? 0 : device.index();
   TORCH_CHECK(i < 64, "device index ", i);
   {
@@ -172,7 +151,8 @@ void* status_word(at::Device device) {
     if (word[i]) return word[i];
   }
   py::gil_scoped_acquire gil;
-  void* p = py::handle(g_ops).attr("status_word")(py::cast(device)).cast<Tensor>().mutable_data_ptr();    // kept by cuda_ops
+  void* t = py::handle(g_ops).attr("status_word")(py::cast(device)).cast<Tensor>().mutable_data_ptr();    // kept by cuda_ops
+  unsigned int* p = static_cast<unsigned int*>(t);
   std::lock_guard<std::mutex> lock(m);
   return word[i] = p;
 }
@@ -456,7 +436,7 @@ struct CrossEntropy : Function<CrossEntropy> {
     Tensor l2 = contiguous(logits.reshape({-1, V})), lab = contiguous(labels.reshape({-1}));
     const int64_t T = l2.size(0);
     Tensor loss = alloc({T}, F32, logits.device()), lse = alloc({T}, F32, logits.device());
-    SB_CALL(sb_ce_fwd, 1, ptr(l2), ptr(lab), f32o(loss), f32o(lse), (long long)T, (int)V, stream());
+    SB_CALL(sb_ce_fwd, 1, ptr(l2), i64(lab), f32o(loss), f32o(lse), (long long)T, (int)V, stream());
     ctx->save_for_backward({l2, lab, lse});
     ctx->saved_data["shape"] = logits.sizes().vec();
     return loss.view(labels.sizes());
@@ -468,7 +448,7 @@ struct CrossEntropy : Function<CrossEntropy> {
     if (gc.scalar_type() != F32) gc = gc.to(F32);
     gc = contiguous(gc);
     Tensor dl = alloc_like(l2);
-    SB_CALL(sb_ce_bwd, 1, ptr(l2), ptr(lab), f32(lse), f32(gc), out(dl), (long long)l2.size(0), (int)l2.size(1), stream());
+    SB_CALL(sb_ce_bwd, 1, ptr(l2), i64(lab), f32(lse), f32(gc), out(dl), (long long)l2.size(0), (int)l2.size(1), stream());
     return {dl.view(ctx->saved_data["shape"].toIntVector()), Tensor()};
   }
 };

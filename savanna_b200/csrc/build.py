@@ -27,6 +27,7 @@ CUDA_LIB = os.path.join(PKG, "libsavanna_b200.so")
 DATA_LIB = os.path.join(PKG, "libsavanna_data.so")
 NATIVE_MODULE = os.path.join(PKG, "_native.so")
 NATIVE_SOURCES = ("autograd_native.cpp",)
+NATIVE_HEADERS = ("entries.h",)
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-Xptxas", "-v"]
@@ -112,7 +113,7 @@ def build_native(force=False):
     import torch
     from torch.utils import cpp_extension
     cpps = [os.path.join(HERE, c) for c in NATIVE_SOURCES]
-    digest = _digest(cpps, f"{torch.__version__} {sys.version}")
+    digest = _digest(cpps + [os.path.join(HERE, h) for h in NATIVE_HEADERS], f"{torch.__version__} {sys.version}")
     if not force and _fresh(NATIVE_MODULE, digest):
         return NATIVE_MODULE
     cxx = shutil.which("g++") or "g++"

@@ -12,6 +12,7 @@
 
 #include "conv_stream.cuh"
 #include "device_info.h"
+#include "entries.h"
 #include "halo_src.cuh"
 
 namespace sb {

@@ -19,6 +19,7 @@
 // TMEM is freed and the kernel returns.
 #include <cuda_fp8.h>
 
+#include "entries.h"
 #include "sm100.cuh"
 
 namespace sb {

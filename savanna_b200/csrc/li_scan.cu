@@ -21,6 +21,7 @@
 #include <stdint.h>
 
 #include "device_info.h"
+#include "entries.h"
 #include "f32x2.cuh"
 #include "pdl.cuh"
 

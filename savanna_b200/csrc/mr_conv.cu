@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "entries.h"
+
 namespace sb {
 typedef __nv_bfloat16 bf16;
 

@@ -26,6 +26,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "entries.h"
 #include "halo_src.cuh"
 
 #include "device_info.h"

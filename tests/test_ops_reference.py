@@ -1,5 +1,6 @@
 """Algebraic checks of the oracle operators themselves (the kernels are tested against these)."""
 import math
+import os
 
 import pytest
 
@@ -289,3 +290,24 @@ def test_li_chunks_fit_a_grid(B, D, L):
     tc = cuda_ops._li_tiled_chunk(B, L, D)
     assert (L + tc - 1) // tc <= 65535 and tc >= 32
     assert tc <= 512 or L > 512 * 65535
+
+
+def test_entry_points_are_declared_once():
+    """The entry points that the C++ autograd functions call: every source that defines or looks one up compiles against the same
+    declaration, both builds depend on it, and the ctypes signatures have its arguments."""
+    import re
+    from savanna_b200.csrc import build
+    from savanna_b200.ops import cuda_ops
+    text = {f: open(os.path.join(build.HERE, f)).read() for f in os.listdir(build.HERE) if f.endswith((".cu", ".cpp", ".h"))}
+    decl = dict(re.findall(r"^int (sb_\w+)\(([^;]*)\);", text["entries.h"], re.M))
+    assert len(decl) > 20 and set(re.findall(r"X\((sb_\w+)\)", text["autograd_native.cpp"])) == decl.keys()
+    assert '#include "entries.h"' in text["autograd_native.cpp"] and "entries.h" in build.NATIVE_HEADERS
+    for name, args in decl.items():
+        where = [f for f, t in text.items() if f.endswith(".cu") and re.search(rf'extern "C" int {name}\(', t)]
+        assert len(where) == 1 and '#include "entries.h"' in text[where[0]], name
+        kinds = ["P" if "*" in a or "cudaStream_t" in a else "LL" if "long long" in a else "F" if "float" in a else "I"
+                 for a in args.split(",") if a.strip()]
+        sig = getattr(cuda_ops._Sig, name, None)
+        if sig is not None:
+            names = {cuda_ops.c_void_p: "P", cuda_ops.c_ll: "LL", cuda_ops.c_float: "F", cuda_ops.c_int: "I"}
+            assert [names[s] for s in sig] == kinds, name
