@@ -1231,61 +1231,6 @@ def _pad_order(t, fill):
     return out
 
 
-class _HyenaLITiled(torch.autograd.Function):
-    """The shared-memory tiled scan (csrc/li_scan.cu): D % 8 == 0.  The filter is prepared by the forward's first kernel and
-    handed to the backward; the filter gradients come finished out of the backward's last one.  CUDA tensors take the same
-    steps in C++ (HyenaLI in csrc/autograd_native.cpp); this form calls whatever library `require` returns, which lets a stand-in
-    for it see without a GPU what the kernels are handed."""
-
-    @staticmethod
-    def forward(ctx, feat, gamma, R, p, bias, state_in, want_state):
-        lib = require()
-        B, L, C3 = feat.shape
-        D, O = C3 // 3, gamma.shape[1]
-        dev = feat.device
-        fc, bf = _aligned(feat), _f32c(bias)
-        sin = _f32c(state_in) if state_in is not None else None
-        if sin is not None and sin.data_ptr() == state_in.data_ptr():
-            sin = sin.clone()                    # the backward reads it: the caller may go on with its own buffer
-        tc = _li_tiled_chunk(B, L, D)
-        modal = _alloc((4 * D, LI_ORDER), dtype=torch.float32, device=dev)
-        S = _alloc((B, (L + tc - 1) // tc, D, LI_ORDER), dtype=torch.float32, device=dev)
-        sout = _alloc((B, D, O), dtype=torch.float32, device=dev) if want_state else None
-        z = _alloc((B, L, D), dtype=bf16, device=dev)
-        gf, pf, Rf = _f32c(gamma), _f32c(p), _f32c(R)
-        _check(lib.sb_li_fwd_tiled(fc.data_ptr(), gf.data_ptr(), pf.data_ptr(), Rf.data_ptr(), bf.data_ptr(), _ptr(sin), _ptr(sout),
-                                   modal.data_ptr(), S.data_ptr(), z.data_ptr(), B, L, D, O, tc, _stream()), "li_fwd_tiled")
-        _count(4)
-        ctx.save_for_backward(fc, modal, bf, sin)
-        ctx.meta = (O, gamma.dtype, R.dtype, p.dtype, bias.dtype, want_state)
-        return z, sout
-
-    @staticmethod
-    def backward(ctx, gz, gstate):
-        lib = require()
-        fc, modal, bf, sin = ctx.saved_tensors
-        O, gdt, rdt, pdt, bdt, want_state = ctx.meta
-        B, L, C3 = fc.shape
-        D = C3 // 3
-        dev = fc.device
-        tc = int(lib.sb_li_bwd_tiled_chunk())
-        NC = (L + tc - 1) // tc
-        g = _aligned(gz)
-        S, A, dRp = (_alloc((B, NC, D, LI_ORDER), dtype=torch.float32, device=dev) for _ in range(3))
-        dBp = _alloc((B, NC, D), dtype=torch.float32, device=dev)
-        df = _alloc_like(fc)
-        dso = _f32c(gstate) if (want_state and gstate is not None) else None
-        dR, dll = (_alloc((D, O), dtype=torch.float32, device=dev) for _ in range(2))
-        db = _alloc(D, dtype=torch.float32, device=dev)
-        dsi = _alloc((B, D, O), dtype=torch.float32, device=dev) if sin is not None else None
-        _check(lib.sb_li_bwd_tiled(fc.data_ptr(), g.data_ptr(), modal.data_ptr(), bf.data_ptr(), _ptr(sin), _ptr(dso), S.data_ptr(),
-                                   A.data_ptr(), dRp.data_ptr(), dBp.data_ptr(), df.data_ptr(), dR.data_ptr(), dll.data_ptr(), db.data_ptr(),
-                                   _ptr(dsi), B, L, D, O, _stream()), "li_bwd_tiled")
-        _count(4)
-        dp = dll.to(pdt) if pdt != torch.float32 else dll.clone()          # gamma and p get gradients of their own storage
-        return df, dll.to(gdt), dR.to(rdt), dp, db.to(bdt), dsi, None
-
-
 class _HyenaLI(torch.autograd.Function):
     """The per-thread streaming scan: any D."""
 
@@ -1382,10 +1327,7 @@ def hyena_li_modal(feat, gamma, R, p, bias, state_in=None, return_state=False):
     if feat.dtype != bf16 or O > LI_ORDER:
         return ref.hyena_li_modal(feat, gamma, R, p, bias, state_in, return_state)
     if LI_TILED and C3 % 24 == 0 and B * L > 0:
-        if feat.is_cuda:
-            z, s = _native("hyena_li", feat, gamma, R, p, bias, state_in, bool(return_state), _li_tiled_chunk(B, L, D))
-        else:
-            z, s = _HyenaLITiled.apply(feat, gamma, R, p, bias, state_in, return_state)
+        z, s = _native("hyena_li", feat, gamma, R, p, bias, state_in, bool(return_state), _li_tiled_chunk(B, L, D))
     else:
         z, s = _HyenaLI.apply(feat, gamma, R, p, bias, state_in, return_state)
     return (z, s) if return_state else z

@@ -229,45 +229,28 @@ _LI_SHAPES = [  # gamma, R, p, bias, state_in for D = 8, O = 4, B = 2
     ((1, 4), (1, 4), (1, 4), (8,), (1, 1, 8, 4))]
 
 
-class _LiLibrary:
-    """Stands in for the native library: notes how many elements lie behind each address that the scan is handed."""
-
-    def __init__(self, sizes):
-        self.sizes, self.calls = sizes, []
-
-    def sb_li_fwd_tiled(self, feat, gamma, p, R, bias, sin, sout, modal, S, z, B, L, D, O, tc, stream):
-        self.calls.append([self.sizes[a] if a else None for a in (gamma, p, R, bias, sin)])
-        assert (B, D, O) == (2, 8, 4)
-        return 0
-
-    def sb_li_fwd(self, feat, ll, R, bias, sin, sout, S, z, B, L, D, tc, stream):
-        return 0
-
-
 def _li_fake(monkeypatch):
+    """Stands in for the C++ functions: notes the shapes that the scan is handed."""
     from savanna_b200.ops import cuda_ops
-    sizes = {}
-    real = cuda_ops._f32c
+    calls = []
 
-    def f32c(t):
-        t = real(t)
-        sizes[t.data_ptr()] = t.numel()
-        return t
-    lib = _LiLibrary(sizes)
-    for name, fn in (("require", lambda: lib), ("_f32c", f32c), ("_stream", lambda: 0)):
-        monkeypatch.setattr(cuda_ops, name, fn)
-    return cuda_ops, lib
+    def native(name, feat, *args):
+        assert name == "hyena_li"
+        calls.append([None if t is None else tuple(t.shape) for t in args[:5]])
+        return torch.zeros(2, 5, 8, dtype=torch.bfloat16), None
+    monkeypatch.setattr(cuda_ops, "_native", native)
+    return cuda_ops, calls
 
 
 @pytest.mark.parametrize("shapes", _LI_SHAPES, ids=str)
 def test_li_scan_is_handed_whole_tensors(shapes, monkeypatch):
     """The scan kernels index gamma, R, p as [D, O], bias as [D] and the state as [B, D, O]: operands that broadcast to those
-    shapes are accepted, as by the fp32 statement, and reach them in full."""
-    cuda_ops, lib = _li_fake(monkeypatch)
+    shapes are accepted, as by the fp32 statement, and reach the function in full (what it makes of them is tested on the GPU)."""
+    cuda_ops, calls = _li_fake(monkeypatch)
     feat = torch.randn(2, 5, 24).bfloat16()
     args = [torch.randn(s) * 0.1 if s is not None else None for s in shapes]
     cuda_ops.hyena_li_modal(feat, *args)
-    assert lib.calls == [[32, 32, 32, 8, 64 if shapes[4] else None]]
+    assert calls == [[(8, 4), (8, 4), (8, 4), (8,), (2, 8, 4) if shapes[4] else None]]
 
 
 @pytest.mark.parametrize("shapes", [((8, 4), (8, 4), (8, 3), (8,), None), ((8, 4), (8, 4), (4, 4), (8,), None),
@@ -275,11 +258,11 @@ def test_li_scan_is_handed_whole_tensors(shapes, monkeypatch):
                                     ((8, 4), (8, 4), (8, 4), (8,), (2, 8, 3)), ((8, 4), (8, 4), (8, 4), (8,), (3, 8, 4)),
                                     ((4,), (8, 4), (8, 4), (8,), None)], ids=str)
 def test_li_scan_refuses_shapes_that_do_not_broadcast(shapes, monkeypatch):
-    cuda_ops, lib = _li_fake(monkeypatch)
+    cuda_ops, calls = _li_fake(monkeypatch)
     args = [torch.randn(s) * 0.1 if s is not None else None for s in shapes]
     with pytest.raises((RuntimeError, IndexError)):
         cuda_ops.hyena_li_modal(torch.randn(2, 5, 24).bfloat16(), *args)
-    assert not lib.calls
+    assert not calls
 
 
 @pytest.mark.parametrize("L", [1, 512 * 65535, 512 * 65535 + 1, 1024 * 65535])
