@@ -197,3 +197,25 @@ def test_refusals_name_what_was_handed_over():
     with pytest.raises(RuntimeError, match=r"rotary embedding failed \(code -3\): cos\[8, 24\].*from\[1, 8, 2, 128\]/\[6144, 768, 384, 1\]"):
         flash_sm100.attention_packed(qkv, t, t, True)
     assert torch.equal(ops.linear(x, w.clone()), ops.linear(x, w.clone()))
+
+
+@pytest.mark.parametrize("kind,marked", [("mlp", (2,)), ("mlp", (3,)), ("mlp", (2, 3)), ("norm_linear", (2,))])
+def test_joined_nodes_add_into_marked_gradients(kind, marked):
+    """Weights whose gradient lives in a persistent buffer get theirs added into it, each into its own; the others get one of their own."""
+    ts, whole, parts = _joined(kind)
+    ts[0] = ts[0][:, :100]
+    g = [_rand(*whole(*ts).shape) for _ in range(2)]
+    leaves, plain = _leaves(ts), _leaves(ts)
+    buffers = {}
+    for i in marked:
+        leaves[i].grad = buffers[i] = torch.zeros_like(leaves[i])
+        leaves[i]._fuse_grad_accum = True                # what the optimizers with flat buffers set
+    for dy in g:
+        whole(*leaves).backward(dy)
+    want = [torch.autograd.grad(parts(*plain), plain, dy) for dy in g]
+    for i, (a, w) in enumerate(zip(leaves, zip(*want))):
+        # the buffer's second addition and the sum of the two bf16 gradients round once more than fp32: 2^-8
+        total = w[0].float() + w[1].float()
+        assert (a.grad.float() - total).norm() <= 2 ** -8 * total.norm(), i
+        assert i not in buffers or a.grad is buffers[i]
+    assert all(leaves[i].grad.abs().sum() > 0 for i in range(len(ts)))
