@@ -652,10 +652,11 @@ se_bwd_tiled_kernel(const bf16* __restrict__ feat, const HaloSrc halo, const int
 }
 
 // Which kernels run (16-byte aligned tensors; the switches below pick the run-per-thread ones for A/B measurements):
-//   streaming   channels % 8 == 0 and at least CS_FULL rows of 128 channels per SM: one wave of runs keeps every SM busy
-//   tiled       fewer rows and whole tiles of channels: a block's 128 steps in parallel beat a warp's run (its edge rows and the
-//               latency of its first copies are the run's whole time)
-//   per thread  the rest
+//   tiled       fewer than CS_FULL rows of 128 channels per SM and whole tiles of channels (64 for the featuriser, 32 for Hyena-SE): a
+//               block's 128 steps in parallel beat a warp's run (its edge rows and the latency of its first copies are the run's whole time)
+//   streaming   everything else with channels % 8 == 0: one wave of runs keeps every SM busy, and off the channel tiles it is the faster
+//               one at any number of rows but one
+//   per thread  channels % 8 == 4 in the backward's C entries, and behind the switches
 // us, streaming / tiled, taps 3 (featuriser forward, backward) and 7 (Hyena-SE forward, backward):
 //   B, L, D             rows of 128 channels per SM (featuriser, Hyena-SE)
 //   1, 8192, 4096       5314, 1771     69 /  75     97 / 128     49 /  62     88 / 129
@@ -663,6 +664,13 @@ se_bwd_tiled_kernel(const bf16* __restrict__ feat, const HaloSrc halo, const int
 //   2, 1237, 1024        401,  134    8.4 / 10.4    15 /  19   10.4 / 8.4     22 /  17
 //   3,  777,  512        189,   63    6.4 /  6.8    11 /  11    8.3 / 6.4     13 /  11     (4 taps)
 //   1,   64,  256          3,    1    6.3 /  5.3   6.5 / 6.3    8.4 / 4.7     13 / 8.4
+// us, streaming / per thread off the channel tiles (cold L2, event ticks of 2 us), the same taps:
+//   1,    1, 1000          0,    0    8.2 /  6.1   8.2 /  8.2   8.2 / 8.2     10 / 9.7
+//   1,   16, 1000          3,    1    8.2 /   14    10 /  18     12 / 12      16 / 27
+//   1,   64, 1016         10,    3    8.2 /   16    10 /  18     12 / 16      16 / 33
+//   1,  200,   72          3,    1    8.2 /   16    10 /  18     12 / 14      14 / 29
+//   2,  333, 1000        108,   36     10 /   16    12 /  25     12 / 16      16 / 49
+//   2, 1237, 1016        401,  134     14 /   21    18 /  35     14 / 16      27 / 115
 static int g_bwd_fast = 1;
 static int g_fwd_fast = 1;
 constexpr int CS_FULL = 200;

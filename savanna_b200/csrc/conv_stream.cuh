@@ -3,12 +3,14 @@
 // A warp owns a strip of neighbouring channels and walks down the rows of a run on its own: asynchronous 16-byte copies put the
 // next rows into a ring of shared memory that belongs to this warp alone, the filter windows are registers, every fp32 quantity is
 // a pair of channels in one 64-bit register.  No block barrier anywhere: a warp waits for its own copies and for nothing else, so
-// the memory system always has about a hundred kilobytes per SM in flight, which is what the tiled kernels these replace lacked
-// (stage a tile, wait, barrier, compute; 55 to 85 % of the copy rate).  The interleaved (x1, x2, v) triples of four channels are 24 bytes,
+// copies are in flight all the time, which is what the tiled kernels these replace lacked (stage a tile, wait, barrier, compute; 55 to
+// 85 % of the copy rate).  KB of copies in flight per SM (blocks of four warps x rows of the ring ahead x bytes of a row): featuriser
+// forward 4 x 11 x 512 B, 90 with 3 taps; its backward 2 x 11 x 512 B, 45; Hyena-SE forward 3 x 13 x 768 B, 120 with 7 taps; its
+// backward 2 x 6 x 1024 B, 49 with 7 taps, where issue (52 % of the slots) and the serial body bound it more than copies.  The interleaved (x1, x2, v) triples of four channels are 24 bytes,
 // read as three 8-byte words at a stride of 24 bytes (no bank conflict); gradients of triples go back into the ring slot their
 // row came from and leave with full 16-byte stores.
-// Two or three blocks of four warps per SM (one wave; the featuriser's forward, whose runs have two edge rows only, goes in three
-// waves): the registers of a fourth are worth more to the scheduling of the unrolled bodies - Hyena-SE backward, L = 8192, D = 4096:
+// Two or three blocks of four warps per SM (one wave; the featuriser's forward, whose runs have two edge rows only, is cut for nine
+// blocks per SM, of which four run at a time): the registers of a fourth are worth more to the scheduling of the unrolled bodies - Hyena-SE backward, L = 8192, D = 4096:
 // 88 us with two blocks, 97 with three (168 registers), 123 with four (128).  Whole blocks per strip: four blocks too many for the
 // wave cost a second one.
 #pragma once

@@ -124,8 +124,8 @@ rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16*
 // partial[block, col] = sum over the block's rows of dy * x * a; rmsnorm_dw_reduce_kernel adds the blocks up.
 // Each thread owns VPT fixed column-vectors (8 columns each) so its weight-gradient sums stay in registers over the
 // row loop; the next row's x and dy are in flight (packed, 8 registers per vector) while this row is reduced and stored.
-template <int VPT>
-__global__ void __launch_bounds__(512, VPT == 1 ? 2 : 1)
+template <int VPT>                                      // 2 or 4: rows of one vector per thread go in pairs (below)
+__global__ void __launch_bounds__(512, 1)
 rmsnorm_bwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const bf16* __restrict__ dy,
                    const float* __restrict__ a_in, const bf16* __restrict__ gres, bf16* __restrict__ dx,
                    float* __restrict__ partial,

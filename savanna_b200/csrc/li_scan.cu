@@ -532,7 +532,8 @@ li_fwd_tiled_kernel(const bf16* __restrict__ feat, const LiModal m, const float*
 // loads of AHEAD chunks in flight ahead of the serial carry.  REVERSE: exclusive suffix (the adjoint).  `scale`: factor on the
 // local terms; `carry`: what enters at the first chunk; `tail`: gradient of the returned state (REVERSE).
 // Bound by the latency of one batch of loads after another.  At L = 8192, D = 4096 with 16 and with 32 loads in flight: the
-// backward's 128 chunks 54 and 36 us, the forward's 64 chunks 10.2 and 11.6 us.
+// backward's 128 chunks 54 and 36 us.  The whole forward with 8, 16 and 32: L = 8192, D = 4096 (16 chunks) 137.1, 137.5 and 139.6 us,
+// L = 32768 (64 chunks) 424, 414 and 416, L = 1237, D = 1024 (39 chunks, chained launches) 22.6, 20.7 and 25.8.
 constexpr int LP_AHEAD_FWD = 16, LP_AHEAD_BWD = 32;
 template <bool REVERSE, int AHEAD>
 __device__ __forceinline__ float li_carry(float* p, size_t per_b, float ll, float scale, float carry, float tail,

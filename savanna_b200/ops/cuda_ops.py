@@ -350,12 +350,12 @@ CONV_FWD_FAST = True
 
 
 def set_se_backward_variant(tiled: bool) -> None:
-    """Hyena-SE and featuriser backward: streaming or tiled kernels by size (default), or one run per thread reading global memory."""
+    """Hyena-SE and featuriser backward: streaming or tiled kernels by size and channels (default), or one run per thread reading global memory."""
     require().sb_se_set_bwd_variant(int(bool(tiled)))
 
 
 def set_conv_forward_variant(tiled: bool) -> None:
-    """Hyena-SE and featuriser forward: streaming or tiled kernels by size (default), or one run per thread."""
+    """Hyena-SE and featuriser forward: streaming or tiled kernels by size and channels (default), or one run per thread."""
     global CONV_FWD_FAST
     CONV_FWD_FAST = bool(tiled)
     require().sb_conv_set_fwd_variant(int(CONV_FWD_FAST))

@@ -227,7 +227,7 @@ def test_sqnorm_adam():
     assert torch.equal(p, master.to(BF))
 
 
-@pytest.fixture(params=[(True, True), (False, False)], ids=["tiled", "per_thread_run"])
+@pytest.fixture(params=[(True, True), (False, False)], ids=["by_size", "per_thread_run"])
 def conv_variant(request):
     from savanna_b200.ops import cuda_ops
     cuda_ops.set_conv_forward_variant(request.param[0])
@@ -260,7 +260,7 @@ def test_dwconv(K, halo, C, L, conv_variant):
         _close(h.grad, hr.grad, what="dwconv dhalo")
 
 
-@pytest.fixture(params=[True, False], ids=["tiled", "per_thread_run"])
+@pytest.fixture(params=[True, False], ids=["by_size", "per_thread_run"])
 def se_bwd_variant(request):
     from savanna_b200.ops import cuda_ops
     cuda_ops.set_se_backward_variant(request.param)
