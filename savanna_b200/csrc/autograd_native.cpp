@@ -39,7 +39,8 @@ constexpr auto F32 = at::kFloat;
 #define SB_ENTRIES(X) \
   X(sb_gemm_bf16) X(sb_gemm_last_error_detail) X(sb_attn_last_encode_result) X(sb_colsum) X(sb_rmsnorm_fwd) X(sb_rmsnorm_bwd_blocks) \
   X(sb_rmsnorm_bwd) X(sb_glu_fwd) X(sb_glu_bwd) X(sb_ce_fwd) X(sb_ce_bwd) X(sb_dwconv_fwd) X(sb_dwconv_fwd_taps) X(sb_dwconv_bwd) \
-  X(sb_se_fwd) X(sb_se_fwd_taps) X(sb_se_bwd) X(sb_mr_fwd) X(sb_mr_bwd) X(sb_mr_tc_fwd) X(sb_mr_tc_bwd) X(sb_li_fwd_tiled) \
+  X(sb_se_fwd) X(sb_se_fwd_taps) X(sb_se_bwd) X(sb_mr_fwd) X(sb_mr_bwd) X(sb_mr_tc_fwd) X(sb_mr_tc_bwd) X(sb_mr_umma_fwd) X(sb_mr_umma_bwd) \
+  X(sb_li_fwd_tiled) \
   X(sb_li_bwd_tiled_chunk) X(sb_li_bwd_tiled) X(sb_attn_fwd) X(sb_attn_bwd) X(sb_attn_rope)
 
 struct {
@@ -518,14 +519,16 @@ struct HyenaSE : Function<HyenaSE> {
   }
 };
 
-// Tensor-core kernels (mr_conv_tc.cu) when a 16-channel slab shares one filter, else the CUDA-core kernels (mr_conv.cu), whose backward
-// wants the convolution itself (kept when `train`).
+// Tensor-core kernels when a 16-channel slab shares one filter (mr_conv_umma.cu, with halo rows mr_conv_tc.cu), else the CUDA-core
+// kernels (mr_conv.cu), whose backward wants the convolution itself (kept when `train`).
 struct HyenaMR : Function<HyenaMR> {
   static Tensor forward(AutogradContext* ctx, const Tensor& feat, const Tensor& h, const Tensor& bias, const OptTensor& halo, bool train) {
     const int B = feat.size(0), Ln = feat.size(1), D = feat.size(2) / 3, G = h.size(0), K = h.size(1);
     Tensor fc = aligned(feat), hc = aligned(halo), hf = f32c(h), bf = f32c(bias), z = alloc({B, Ln, D}, BF16, feat.device()), y;
     const bool tc = (D / G) % 16 == 0 && D % 8 == 0;
-    if (tc) {
+    if (tc && !hc.defined()) {
+      SB_CALL(sb_mr_umma_fwd, 1, ptr(fc), f32(hf), f32(bf), out(z), B, Ln, D, G, K, status_word(feat.device()), stream());
+    } else if (tc) {
       SB_CALL(sb_mr_tc_fwd, 1, ptr(fc), ptr(hc), f32(hf), f32(bf), out(z), B, Ln, D, G, K, stream());
     } else {
       if (train) y = alloc_like(z);
@@ -543,7 +546,10 @@ struct HyenaMR : Function<HyenaMR> {
     const int B = fc.size(0), Ln = fc.size(1), D = fc.size(2) / 3, G = hf.size(0), K = hf.size(1);
     Tensor gc = aligned(g[0]), df = alloc_like(fc), dhalo = hc.defined() ? alloc_like(hc).zero_() : Tensor(),
            dh = zeros(hf.sizes(), F32, hf.device()), db = zeros(bf.sizes(), F32, bf.device());
-    if (ctx->saved_data["tc"].toBool()) {
+    const bool tc = ctx->saved_data["tc"].toBool();
+    if (tc && !hc.defined()) {
+      SB_CALL(sb_mr_umma_bwd, 1, ptr(fc), f32(hf), f32(bf), ptr(gc), out(df), f32o(dh), f32o(db), B, Ln, D, G, K, status_word(fc.device()), stream());
+    } else if (tc) {
       SB_CALL(sb_mr_tc_bwd, 1, ptr(fc), ptr(hc), f32(hf), f32(bf), ptr(gc), out(df), out(dhalo), f32o(dh), f32o(db), B, Ln, D, G, K, stream());
     } else {
       SB_CALL(sb_mr_bwd, 2, ptr(fc), ptr(hc), f32(hf), f32(bf), ptr(gc), ptr(y), out(df), out(dhalo), f32o(dh), f32o(db), B, Ln, D, G, K, stream());

@@ -208,6 +208,54 @@ def test_mr_fir_non_finite_values_stay_in_their_column():
     assert z[0, t0:t0 + K, c].isnan().all()
 
 
+def _mr_grads(halo, *args):
+    leaves = [t.clone().requires_grad_() for t in args[:3]]
+    z = ops.hyena_mr_inner(*leaves, halo)
+    z.backward(args[3])
+    return [z.detach()] + [t.grad for t in leaves]
+
+
+# one row; a tile less one, whole, and one more; an odd and an even number of tiles; several runs per block; a filter for 64 channels
+@pytest.mark.parametrize("B,L,D,G,K", [(1, 1, 16, 1, 128), (2, 127, 32, 2, 128), (1, 128, 16, 1, 1), (1, 129, 48, 3, 31), (1, 1025, 64, 1, 128),
+                                       (2, 2304, 128, 2, 113), (3, 777, 2048, 128, 128), (5, 300, 1024, 16, 7)])
+def test_mr_fir_tiles_of_128_rows_match_the_16_row_blocks(B, L, D, G, K):
+    """Without halo rows the products come from whole tiles, with (zero) halo rows from 16-row blocks: the same roundings of the
+    operands, fp32 sums in another order, one rounding of the result, which may fall on either side."""
+    torch.manual_seed(L + D)
+    a = [torch.randn(B, L, 3 * D, device=DEV).to(BF), torch.randn(G, K, device=DEV) / math.sqrt(K), torch.randn(D, device=DEV),
+         torch.randn(B, L, D, device=DEV).to(BF)]
+    new = _mr_grads(None, *a)
+    for got, want, tol, what in zip(new, _mr_grads(torch.zeros(B, K - 1, 3 * D, device=DEV, dtype=BF), *a), (2 ** -7, 2 ** -7, 1e-5, 1e-5),
+                                    ("z", "dfeat", "dh", "dbias")):
+        _close(got, want, tol, what)
+    assert torch.equal(new[0], _mr_grads(None, *a)[0])
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("t0", [130, 511])
+def test_mr_fir_non_finite_values_reach_only_what_their_taps_touch(bad, t0):
+    torch.manual_seed(13)
+    B, L, D, G, K, c = 1, 900, 64, 4, 100, 21
+    a = [torch.randn(B, L, 3 * D, device=DEV).to(BF), torch.randn(G, K, device=DEV) / 11, torch.randn(D, device=DEV),
+         torch.randn(B, L, D, device=DEV).to(BF)]
+    clean = _mr_grads(None, *a)
+    a[0][0, t0, 3 * c + 2] = bad
+    z, df = _mr_grads(None, *a)[:2]
+    others = [i for i in range(D) if i != c]
+    _same(z[..., others], clean[0][..., others], "other channels")
+    assert not z[0, t0:t0 + K, c].isfinite().any()
+    for part in (slice(0, t0), slice(t0 + K, L)):      # formed again tap by tap next to the bad value: fp32 sums in another order
+        _close(z[:, part, c], clean[0][:, part, c], 2 ** -7, "beyond the taps")
+    a[0][0, t0, 3 * c + 2] = 1.0
+    a[3][0, t0, c] = bad
+    df = _mr_grads(None, *a)[1].view(B, L, D, 3)
+    want = clean[1].view(B, L, D, 3)
+    _same(df[:, :, others], want[:, :, others], "dfeat, other channels")
+    assert not df[0, t0 - K + 1:t0 + 1, c, 1:].isfinite().any()
+    for part in (slice(0, t0 - K + 1), slice(t0 + K, L)):
+        _close(df[:, part, c], want[:, part, c], 2 ** -7, "dfeat beyond the taps")
+
+
 @pytest.mark.parametrize("D,offset,tiled", [(24, 0, True), (136, 0, True), (20, 0, False), (24, 1, False)])
 @pytest.mark.parametrize("state", [False, True])
 def test_li_c_entries(D, offset, tiled, state):
