@@ -44,7 +44,6 @@ int sb_mr_tc_fwd(const void* feat, const void* halo, const float* h, const float
 int sb_mr_tc_bwd(const void* feat, const void* halo, const float* h, const float* bias, const void* dz, void* dfeat, void* dhalo, float* dh,
                  float* dbias, int B, int L, int D, int G, int K, cudaStream_t st);
 // mr_conv_umma.cu
-int sb_mr_umma_supported(int D, int G, int K);
 int sb_mr_umma_fwd(const void* feat, const float* h, const float* bias, void* z, int B, int L, int D, int G, int K, unsigned int* status,
                    cudaStream_t st);
 int sb_mr_umma_bwd(const void* feat, const float* h, const float* bias, const void* dz, void* dfeat, float* dh, float* dbias, int B, int L,

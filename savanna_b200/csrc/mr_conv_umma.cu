@@ -692,12 +692,12 @@ static int tiles_per_run(int tiles, int columns, int slots, float once) {
 using namespace sb;
 using namespace sb::mru;
 
-extern "C" int sb_mr_umma_supported(int D, int G, int K) { return G > 0 && D % G == 0 && (D / G) % CH == 0 && K >= 1 && K <= TILE; }
+static bool supported(int D, int G, int K) { return G > 0 && D % G == 0 && (D / G) % CH == 0 && K >= 1 && K <= TILE; }
 
 // feat [B, L, 3D], z [B, L, D]: bf16, 16-byte aligned.  h [G, K], bias [D] fp32.
 extern "C" int sb_mr_umma_fwd(const void* feat, const float* h, const float* bias, void* z, int B, int L, int D, int G, int K,
                               unsigned int* status, cudaStream_t st) {
-  if (!sb_mr_umma_supported(D, G, K) || ((reinterpret_cast<uintptr_t>(feat) | reinterpret_cast<uintptr_t>(z)) & 15)) return -1;
+  if (!supported(D, G, K) || ((reinterpret_cast<uintptr_t>(feat) | reinterpret_cast<uintptr_t>(z)) & 15)) return -1;
   if (B <= 0 || L <= 0 || D <= 0) return 0;
   if (cudaFuncSetAttribute(mr_umma_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F_SMEM) != cudaSuccess) return -5;
   CUtensorMap tf, tz;
@@ -714,7 +714,7 @@ extern "C" int sb_mr_umma_fwd(const void* feat, const float* h, const float* bia
 // dz like z, dfeat like feat; adds into dh [G, K] and dbias [D], fp32.
 extern "C" int sb_mr_umma_bwd(const void* feat, const float* h, const float* bias, const void* dz, void* dfeat, float* dh, float* dbias,
                               int B, int L, int D, int G, int K, unsigned int* status, cudaStream_t st) {
-  if (!sb_mr_umma_supported(D, G, K) ||
+  if (!supported(D, G, K) ||
       ((reinterpret_cast<uintptr_t>(feat) | reinterpret_cast<uintptr_t>(dz) | reinterpret_cast<uintptr_t>(dfeat)) & 15)) return -1;
   if (B <= 0 || L <= 0 || D <= 0) return 0;
   if (cudaFuncSetAttribute(mr_umma_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, B_SMEM) != cudaSuccess) return -5;
