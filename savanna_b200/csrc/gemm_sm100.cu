@@ -3,7 +3,7 @@
 // One persistent CTA per SM, warp-specialised:
 //   warp 0   : TMA producer  (one elected lane issues cp.async.bulk.tensor loads, 128-byte swizzle, no multicast)
 //   warp 1   : MMA issuer    (one elected lane issues tcgen05.mma; owns the TMEM allocation)
-//   warps 2-5: epilogue      (tcgen05.ld TMEM -> registers -> bf16 -> global), one TMEM lane quarter each
+//   warps 2-9: epilogue      (tcgen05.ld TMEM -> registers -> bf16 -> shared memory -> global), two per TMEM lane quarter
 // Tile 128 x 256 x 64, 4-stage shared-memory ring (48 KB per stage), two 256-column TMEM accumulators so
 // the epilogue of tile i overlaps the main loop of tile i+1.
 //
@@ -25,11 +25,13 @@
 namespace sb {
 
 constexpr int BM = 128, BN = 256, BK = 64;
+constexpr int EPI_WARPS = 8;                      // two per TMEM lane quarter, each takes half of a tile's columns
 constexpr int A_STAGE = BM * BK * 2;              // 16 KB
-constexpr int SMEM_BYTES = 4 * 48 * 1024 + 1024 /*align*/ + 256 /*barriers*/;
+constexpr int EPI_OFF = 4 * 48 * 1024 + 256;      // behind the stages and the barriers
+constexpr int SMEM_BYTES = EPI_OFF + EPI_WARPS * 32 * 64 /*EPI_BYTES*/ + 1024 /*align*/;
 constexpr int TMEM_COLS = 512;
 constexpr int GROUP_M = 16;                       // raster: 16 m-tiles share the concurrently running n-tiles
-constexpr int NUM_THREADS = 192;
+constexpr int NUM_THREADS = 64 + 32 * EPI_WARPS;
 
 struct GemmParams {
   __nv_bfloat16* C;
@@ -66,42 +68,89 @@ __device__ __forceinline__ void tile_coords(int tile, int m_tiles, int n_tiles, 
   nt = r / gsz;
 }
 
-// Epilogue of 32 accumulator columns of one row: scale, + bias, + residual, (+ C), bf16, 16-byte stores.
-__device__ __forceinline__ void store_chunk(const GemmParams& p, int row, int col0, const uint32_t (&r)[32], float alpha,
-                                            __nv_bfloat16* crow) {
-  if (row < p.M && col0 < p.N) {
+// A warp's 32 rows x 32 columns on their way to memory.  A lane holds a row (that is how tensor memory is read); stored from there, a
+// 16-byte store touches 32 lines and half a sector of each, and a 256 x 256 tile took 8 us to leave: more than the products of a tile need
+// at K = 512.  Through 2 KB of shared memory four lanes store 64 consecutive bytes of a row, eight rows at a time.  The 16-byte chunks of a row
+// are permuted so that neither side meets a bank twice.
+constexpr int EPI_WARP_BYTES = 32 * 64, EPI_BYTES = EPI_WARPS * EPI_WARP_BYTES;
+__device__ __forceinline__ void epi_put(uint32_t at, const uint4 v) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ uint4 epi_get(uint32_t at) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at) : "memory");
+  return v;
+}
+// bf16: out = the lane's row, 4 x 8 columns from col0 on; rows row0 .. row0 + 31 of dst (leading dimension ld)
+__device__ __forceinline__ void store_rows(uint32_t stage, const uint4 (&out)[4], __nv_bfloat16* dst, int ld, int row0, int rows, int col0,
+                                           int cols, int lane) {
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int col = col0 + v * 8;
-      if (col + 8 <= p.N) {
-        float f[8];
+  for (int v = 0; v < 4; ++v) epi_put(stage + lane * 64 + ((v ^ (lane >> 1 & 3)) << 4), out[v]);
+  __syncwarp();
+  const int c = lane & 3, col = col0 + 8 * c;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(r[v * 8 + j]) * alpha;
-        if (p.bias) {
-          const uint4 bv = *reinterpret_cast<const uint4*>(p.bias + col);
-          const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&bv);
+  for (int i = 0; i < 4; ++i) {
+    const int r = 8 * i + (lane >> 2);
+    const uint4 v = epi_get(stage + r * 64 + ((c ^ (r >> 1 & 3)) << 4));
+    if (row0 + r < rows && col + 8 <= cols) *reinterpret_cast<uint4*>(dst + size_t(row0 + r) * ld + col) = v;
+  }
+  __syncwarp();
+}
+// one byte a value: 2 x 16 columns
+__device__ __forceinline__ void store_rows_u8(uint32_t stage, const uint4 a, const uint4 b, uint8_t* dst, int ld, int row0, int rows, int col0,
+                                              int lane) {
+  epi_put(stage + lane * 32 + ((lane >> 2 & 1) << 4), a);
+  epi_put(stage + lane * 32 + ((lane >> 2 & 1 ^ 1) << 4), b);
+  __syncwarp();
+  const int c = lane & 1;
 #pragma unroll
-          for (int j = 0; j < 4; ++j) { float2 t = __bfloat1622float2(b2[j]); f[2 * j] += t.x; f[2 * j + 1] += t.y; }
-        }
-        if (p.residual) {
-          const uint4 rv = *reinterpret_cast<const uint4*>(p.residual + size_t(row) * p.ldr + col);
-          const __nv_bfloat162* r2 = reinterpret_cast<const __nv_bfloat162*>(&rv);
+  for (int i = 0; i < 2; ++i) {
+    const int r = 16 * i + (lane >> 1);
+    const uint4 v = epi_get(stage + r * 32 + ((c ^ (r >> 2 & 1)) << 4));
+    if (row0 + r < rows) *reinterpret_cast<uint4*>(dst + size_t(row0 + r) * ld + col0 + 16 * c) = v;
+  }
+  __syncwarp();
+}
+
+// Epilogue of 32 accumulator columns of one row: scale, + bias, + residual, (+ C), bf16.  Most products have none of the additions: without
+// the tests for them between its columns a chunk takes 400 cycles less (a tile of 128 x 256 per warp has four).
+__device__ __forceinline__ void finish_chunk(const GemmParams& p, bool plain, int row, int col0, const uint32_t (&r)[32], float alpha,
+                                             uint4 (&out)[4]) {
+  if (plain) {
+    __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&out[0]);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) { float2 t = __bfloat1622float2(r2[j]); f[2 * j] += t.x; f[2 * j + 1] += t.y; }
-        }
-        if (p.beta) {
-          const uint4 ov = *reinterpret_cast<const uint4*>(crow + col);
-          const __nv_bfloat162* o2 = reinterpret_cast<const __nv_bfloat162*>(&ov);
+    for (int j = 0; j < 16; ++j) o2[j] = __floats2bfloat162_rn(__uint_as_float(r[2 * j]) * alpha, __uint_as_float(r[2 * j + 1]) * alpha);
+    return;
+  }
+  const __nv_bfloat16* crow = p.C + size_t(row) * p.ldc;
 #pragma unroll
-          for (int j = 0; j < 4; ++j) { float2 t = __bfloat1622float2(o2[j]); f[2 * j] += t.x; f[2 * j + 1] += t.y; }
-        }
-        uint4 out;
-        __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&out);
+  for (int v = 0; v < 4; ++v) {
+    const int col = col0 + v * 8;
+    const bool live = row < p.M && col + 8 <= p.N;
+    float f[8];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) o2[j] = __floats2bfloat162_rn(f[2 * j], f[2 * j + 1]);
-        *reinterpret_cast<uint4*>(crow + col) = out;
-      }
+    for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(r[v * 8 + j]) * alpha;
+    if (p.bias && live) {
+      const uint4 bv = *reinterpret_cast<const uint4*>(p.bias + col);
+      const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&bv);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) { float2 t = __bfloat1622float2(b2[j]); f[2 * j] += t.x; f[2 * j + 1] += t.y; }
     }
+    if (p.residual && live) {
+      const uint4 rv = *reinterpret_cast<const uint4*>(p.residual + size_t(row) * p.ldr + col);
+      const __nv_bfloat162* r2 = reinterpret_cast<const __nv_bfloat162*>(&rv);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) { float2 t = __bfloat1622float2(r2[j]); f[2 * j] += t.x; f[2 * j + 1] += t.y; }
+    }
+    if (p.beta && live) {
+      const uint4 ov = *reinterpret_cast<const uint4*>(crow + col);
+      const __nv_bfloat162* o2 = reinterpret_cast<const __nv_bfloat162*>(&ov);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) { float2 t = __bfloat1622float2(o2[j]); f[2 * j] += t.x; f[2 * j + 1] += t.y; }
+    }
+    __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&out[v]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o2[j] = __floats2bfloat162_rn(f[2 * j], f[2 * j + 1]);
   }
 }
 
@@ -136,7 +185,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(tfull_bar(a), 1); mbar_init(tempty_bar(a), 4); }
+    for (int a = 0; a < 2; ++a) { mbar_init(tfull_bar(a), 1); mbar_init(tempty_bar(a), EPI_WARPS); }
     *abort_flag = 0;
     fence_barrier_init();
     prefetch_tmap(&tmA);
@@ -222,28 +271,32 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
     }
   } else {
-    // ------------------------------------------------------------------ epilogue (warps 2..5)
+    // ------------------------------------------------------------------ epilogue (warps 2..9)
     const int q = warp & 3;                         // TMEM lane quarter this warp may access
+    const int half = (warp - 2) >> 2;               // its half of the columns
+    const uint32_t stage_w = smem_base + EPI_OFF + (warp - 2) * EPI_WARP_BYTES;
     uint32_t acc_phase[2] = {0u, 0u};
     int local = 0;
     bool ok = true;
     const float alpha = (p.alpha ? p.alpha[0] : 1.f) * (p.alpha2 ? p.alpha2[0] : 1.f);
+    const bool plain = !p.bias && !p.residual && !p.beta;
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local) {
       const int acc = local & 1;
       int mt, nt; tile_coords(tile, m_tiles, n_tiles, mt, nt);
       if (!mbar_wait(tfull_bar(acc), acc_phase[acc], abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       acc_phase[acc] ^= 1u;
       tc_fence_after();
-      const int row = mt * BM + q * 32 + lane;
+      const int row0 = mt * BM + q * 32;
       const int n0 = nt * BN;
       const uint32_t t_row = tmem_base + (uint32_t(q * 32) << 16) + acc * BN;
-      __nv_bfloat16* crow = p.C + size_t(row) * p.ldc;
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
+      for (int c = half * (BN / 64); c < (half + 1) * (BN / 64); ++c) {
         uint32_t r[32];
         tmem_ld_32x32(t_row + c * 32, r);
         tmem_wait_ld();
-        store_chunk(p, row, n0 + c * 32, r, alpha, crow);
+        uint4 out[4];
+        finish_chunk(p, plain, row0 + lane, n0 + c * 32, r, alpha, out);
+        store_rows(stage_w, out, p.C, p.ldc, row0, p.M, n0 + c * 32, p.N, lane);
       }
       tc_fence_before();
       __syncwarp();
@@ -269,7 +322,8 @@ constexpr int P_STAGES = 6;
 constexpr int P_A_STAGE = 128 * 128;                 // 16 KB: this CTA's 128 rows of A (128-byte rows)
 constexpr int P_B_STAGE = 128 * 128;                 // 16 KB: this CTA's 128 rows of B
 constexpr int P_STAGE_BYTES = P_A_STAGE + P_B_STAGE;
-constexpr int P_SMEM_BYTES = P_STAGES * P_STAGE_BYTES + 1024 + 256;
+constexpr int P_EPI_OFF = P_STAGES * P_STAGE_BYTES + 256;
+constexpr int P_SMEM_BYTES = P_EPI_OFF + EPI_BYTES + 1024;
 constexpr int P_GROUP_M = 8;
 
 __device__ __forceinline__ void pair_tile_coords(int tile, int m_tiles, int n_tiles, int& mt, int& nt) {
@@ -314,7 +368,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < P_STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(tfull_bar(a), 1); mbar_init(tempty_bar(a), 8); }   // 4 warps of each CTA
+    for (int a = 0; a < 2; ++a) { mbar_init(tfull_bar(a), 1); mbar_init(tempty_bar(a), 2 * EPI_WARPS); }   // of both CTAs
     *abort_flag = 0;
     fence_barrier_init();
     prefetch_tmap(&tmA);
@@ -404,12 +458,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
     }
   } else {
-    // ------------------------------------------------------------------ epilogue (warps 2..5 of both CTAs)
+    // ------------------------------------------------------------------ epilogue (warps 2..9 of both CTAs)
     const int q = warp & 3;
+    const int half = (warp - 2) >> 2;
+    const uint32_t stage_w = smem_base + P_EPI_OFF + (warp - 2) * EPI_WARP_BYTES;
     uint32_t acc_phase[2] = {0u, 0u};
     int local = 0;
     bool ok = true;
     const float alpha = (p.alpha ? p.alpha[0] : 1.f) * (p.alpha2 ? p.alpha2[0] : 1.f);
+    const bool plain = !p.bias && !p.residual && !p.beta;
     float q_scale = 1.f, q_amax = 0.f;
     if (GLU) {
       // delayed scaling of the gated output: scale from the amax ring (all slots but this call's and the next one's)
@@ -431,14 +488,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       if (!mbar_wait(tfull_bar(acc), acc_phase[acc], abort_flag, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       acc_phase[acc] ^= 1u;
       tc_fence_after();
-      const int row = mt * 256 + int(rank) * 128 + q * 32 + lane;
+      const int row0 = mt * 256 + int(rank) * 128 + q * 32, row = row0 + lane;
       const int n0 = nt * BN;
       const uint32_t t_row = tmem_base + (uint32_t(q * 32) << 16) + acc * BN;
-      __nv_bfloat16* crow = p.C + size_t(row) * p.ldc;
       if (GLU == 2) {
         const int F = p.glu_F;
 #pragma unroll 1
-        for (int c = 0; c < BN / 32; ++c) {
+        for (int c = half * (BN / 64); c < (half + 1) * (BN / 64); ++c) {
           uint32_t r[32];
           tmem_ld_32x32(t_row + c * 32, r);
           const int f = n0 + c * 32;
@@ -451,8 +507,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             for (int v = 0; v < 4; ++v) { av[v] = pa[v]; bv[v] = pb[v]; }
           }
           tmem_wait_ld();
+          uint32_t qa[8], qb[8];
           if (live) {
-            uint32_t qa[8], qb[8];
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
               const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&av[v]);
@@ -483,28 +539,28 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 qb[2 * v + h] = uint32_t(y0) | (uint32_t(y1) << 16);
               }
             }
-            uint4* da_dst = reinterpret_cast<uint4*>(p.glu_q + size_t(row) * 2 * F + f);
-            uint4* db_dst = reinterpret_cast<uint4*>(p.glu_q + size_t(row) * 2 * F + F + f);
-            da_dst[0] = make_uint4(qa[0], qa[1], qa[2], qa[3]); da_dst[1] = make_uint4(qa[4], qa[5], qa[6], qa[7]);
-            db_dst[0] = make_uint4(qb[0], qb[1], qb[2], qb[3]); db_dst[1] = make_uint4(qb[4], qb[5], qb[6], qb[7]);
+          }
+          if (f < F) {
+            store_rows_u8(stage_w, make_uint4(qa[0], qa[1], qa[2], qa[3]), make_uint4(qa[4], qa[5], qa[6], qa[7]), p.glu_q, 2 * F, row0, p.M, f, lane);
+            store_rows_u8(stage_w, make_uint4(qb[0], qb[1], qb[2], qb[3]), make_uint4(qb[4], qb[5], qb[6], qb[7]), p.glu_q, 2 * F, row0, p.M, F + f, lane);
           }
         }
       } else if (GLU) {
         const int f0 = nt * 128;
 #pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 2 * half; c < 2 * half + 2; ++c) {
           uint32_t ra[32], rb[32];
           tmem_ld_32x32(t_row + c * 32, ra);
           tmem_ld_32x32(t_row + 128 + c * 32, rb);
           tmem_wait_ld();
-          if (row < p.M) {
+          {
             const int f = f0 + c * 32;
             uint32_t qw[8];
+            uint4 oa[4], ob[4];
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
-              uint4 oa, ob;
-              __nv_bfloat162* a2 = reinterpret_cast<__nv_bfloat162*>(&oa);
-              __nv_bfloat162* b2 = reinterpret_cast<__nv_bfloat162*>(&ob);
+              __nv_bfloat162* a2 = reinterpret_cast<__nv_bfloat162*>(&oa[v]);
+              __nv_bfloat162* b2 = reinterpret_cast<__nv_bfloat162*>(&ob[v]);
               float o[8];
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
@@ -515,10 +571,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 const float2 af = __bfloat1622float2(a2[j]), bf = __bfloat1622float2(b2[j]);
                 o[2 * j] = __bfloat162float(__float2bfloat16_rn(af.x * __fdividef(1.f, 1.f + __expf(-af.x)) * bf.x));
                 o[2 * j + 1] = __bfloat162float(__float2bfloat16_rn(af.y * __fdividef(1.f, 1.f + __expf(-af.y)) * bf.y));
-                q_amax = fmaxf(q_amax, fmaxf(fabsf(o[2 * j]), fabsf(o[2 * j + 1])));
+                if (row < p.M) q_amax = fmaxf(q_amax, fmaxf(fabsf(o[2 * j]), fabsf(o[2 * j + 1])));
               }
-              *reinterpret_cast<uint4*>(crow + f + v * 8) = oa;
-              *reinterpret_cast<uint4*>(crow + p.glu_F + f + v * 8) = ob;
               const unsigned short h0 = __nv_cvt_float2_to_fp8x2(make_float2(o[0] * q_scale, o[1] * q_scale), __NV_SATFINITE, __NV_E4M3);
               const unsigned short h1 = __nv_cvt_float2_to_fp8x2(make_float2(o[2] * q_scale, o[3] * q_scale), __NV_SATFINITE, __NV_E4M3);
               const unsigned short h2 = __nv_cvt_float2_to_fp8x2(make_float2(o[4] * q_scale, o[5] * q_scale), __NV_SATFINITE, __NV_E4M3);
@@ -526,23 +580,25 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               qw[2 * v] = uint32_t(h0) | (uint32_t(h1) << 16);
               qw[2 * v + 1] = uint32_t(h2) | (uint32_t(h3) << 16);
             }
-            uint4* qd = reinterpret_cast<uint4*>(p.glu_q + size_t(row) * p.glu_F + f);
-            qd[0] = make_uint4(qw[0], qw[1], qw[2], qw[3]);
-            qd[1] = make_uint4(qw[4], qw[5], qw[6], qw[7]);
+            store_rows(stage_w, oa, p.C, p.ldc, row0, p.M, f, p.N, lane);
+            store_rows(stage_w, ob, p.C, p.ldc, row0, p.M, p.glu_F + f, p.N, lane);
+            store_rows_u8(stage_w, make_uint4(qw[0], qw[1], qw[2], qw[3]), make_uint4(qw[4], qw[5], qw[6], qw[7]), p.glu_q, p.glu_F, row0, p.M, f, lane);
           }
         }
       } else {
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
+      for (int c = half * (BN / 64); c < (half + 1) * (BN / 64); ++c) {
         uint32_t r[32];
         tmem_ld_32x32(t_row + c * 32, r);
         tmem_wait_ld();
-        store_chunk(p, row, n0 + c * 32, r, alpha, crow);
+        uint4 out[4];
+        finish_chunk(p, plain, row, n0 + c * 32, r, alpha, out);
+        store_rows(stage_w, out, p.C, p.ldc, row0, p.M, n0 + c * 32, p.N, lane);
       }
       }
       tc_fence_before();
       __syncwarp();
-      // the MMA thread of the even CTA waits for the four epilogue warps of both CTAs
+      // the MMA thread of the even CTA waits for the epilogue warps of both CTAs
       if (lane == 0) mbar_arrive_cluster(map_to_cta(tempty_bar(acc), 0));
     }
     if (GLU) {
