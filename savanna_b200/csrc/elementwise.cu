@@ -53,70 +53,59 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 // ------------------------------------------------------------------------------------ RMSNorm
 // form 0 ("te"):      y = w * x * rsqrt(mean(x^2) + eps);       saved a = rsqrt(mean + eps)
 // form 1 ("classic"): y = w * x / (sqrt(mean(x^2)) + eps);      saved a = 1 / (rms + eps)
-// Persistent blocks walk over the rows; a row stays in registers (packed) between the sum of squares and the scaling,
-// and the next row is in flight meanwhile.
-template <int VPT>
-__global__ void __launch_bounds__(512, VPT == 1 ? 4 : 2)
-rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __restrict__ y,
-                   float* __restrict__ a_out, int T, int D, float eps, int form) {
-  __shared__ float red[2][32];
-  const int nv = D >> 3;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  uint4 wv[VPT], xn[VPT];
+// W warps take a row, all of whose loads (V 16-byte vectors a lane) are under way before the first sum; a row of up to 2048 is one warp's and
+// needs no barrier.  A persistent block of 512 threads per row had one vector per thread in flight and two barriers a row.  T = 8192, back to
+// back, us: D = 4096 29.0 -> 22.9 (copying 20.5), 2048 16.5 -> 10.5, 1024 10.4 -> 6.7, 256 6.3 -> 4.3, 8192 47.2 -> 45.9; one byte out 33.9 ->
+// 22.8, 18.6 -> 12.4, 15.4 -> 8.8, 8.3 -> 8.3, 49.3 -> 45.2.  One warp for a row of 4096 took 33: its arithmetic is serial.  OUT takes vector i
+// of the row as eight scaled values.
+template <int V, int W, class OUT>
+__device__ __forceinline__ void norm_row(const bf16* __restrict__ x, const bf16* __restrict__ w, float* __restrict__ a_out, size_t row, int D,
+                                         float eps, int form, float* red, OUT out) {
+  const int lane = threadIdx.x & 31, warp = W > 1 ? (threadIdx.x >> 5) % W : 0, i0 = warp * 32 + lane, nv = D >> 3;
+  const uint4* src = reinterpret_cast<const uint4*>(x + row * D);
+  uint4 xv[V];
 #pragma unroll
-  for (int v = 0; v < VPT; ++v) {
-    const int i = threadIdx.x + v * blockDim.x;
-    wv[v] = i < nv ? reinterpret_cast<const uint4*>(w)[i] : make_uint4(0, 0, 0, 0);
-    xn[v] = make_uint4(0, 0, 0, 0);
+  for (int v = 0; v < V; ++v) xv[v] = i0 + 32 * W * v < nv ? src[i0 + 32 * W * v] : make_uint4(0, 0, 0, 0);
+  float ss = 0.f;
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    float f[8]; unpack8(xv[v], f);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
   }
-  size_t row = blockIdx.x;
-  if (row < (size_t)T) {
-#pragma unroll
-    for (int v = 0; v < VPT; ++v) {
-      const int i = threadIdx.x + v * blockDim.x;
-      if (i < nv) xn[v] = reinterpret_cast<const uint4*>(x + row * D)[i];
-    }
-  }
-  int it = 0;
-  for (; row < (size_t)T; row += gridDim.x, ++it) {
-    uint4 xc[VPT];
-#pragma unroll
-    for (int v = 0; v < VPT; ++v) xc[v] = xn[v];
-    const size_t nxt = row + gridDim.x;
-    if (nxt < (size_t)T) {
-#pragma unroll
-      for (int v = 0; v < VPT; ++v) {
-        const int i = threadIdx.x + v * blockDim.x;
-        if (i < nv) xn[v] = reinterpret_cast<const uint4*>(x + nxt * D)[i];
-      }
-    }
-    float ss = 0.f;
-#pragma unroll
-    for (int v = 0; v < VPT; ++v) {
-      float f[8]; unpack8(xc[v], f);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
-    }
-    ss = warp_sum(ss);
-    float* rr = red[it & 1];
-    if (lane == 0) rr[wid] = ss;
+  ss = warp_sum(ss);
+  if (W > 1) {
+    if (lane == 0) red[warp] = ss;
     __syncthreads();
-    float tot = lane < nw ? rr[lane] : 0.f;
-    tot = warp_sum(tot);
-    const float mean = tot / D;
-    const float a = form == 0 ? rsqrtf(mean + eps) : 1.f / (sqrtf(mean) + eps);
-    if (threadIdx.x == 0) a_out[row] = a;
+    ss = 0.f;
 #pragma unroll
-    for (int v = 0; v < VPT; ++v) {
-      const int i = threadIdx.x + v * blockDim.x;
-      if (i < nv) {
-        float f[8], g[8]; unpack8(xc[v], f); unpack8(wv[v], g);
+    for (int k = 0; k < W; ++k) ss += red[k];
+  }
+  const float mean = ss / D;
+  const float a = form == 0 ? rsqrtf(mean + eps) : 1.f / (sqrtf(mean) + eps);
+  if (i0 == 0) a_out[row] = a;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) f[j] = f[j] * a * g[j];
-        reinterpret_cast<uint4*>(y + row * D)[i] = pack8(f);
-      }
+  for (int v = 0; v < V; ++v) {
+    const int i = i0 + 32 * W * v;
+    if (i < nv) {
+      float f[8], g[8]; unpack8(xv[v], f); unpack8(__ldg(reinterpret_cast<const uint4*>(w) + i), g);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = f[j] * a * g[j];
+      out(i, f);
     }
   }
+}
+// rows of a block, threads of a block: four rows of one warp, else one row
+__host__ __device__ constexpr int norm_rows(int W) { return W == 1 ? 4 : 1; }
+__host__ __device__ constexpr int norm_block(int W) { return 32 * W * norm_rows(W); }
+template <int V, int W>
+__global__ void __launch_bounds__(norm_block(W))
+rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __restrict__ y, float* __restrict__ a_out, int T, int D,
+                   float eps, int form) {
+  __shared__ float red[W];
+  const size_t row = (size_t)blockIdx.x * norm_rows(W) + threadIdx.x / (32 * W);
+  if (row >= (size_t)T) return;
+  norm_row<V, W>(x, w, a_out, row, D, eps, form, red, [&](int i, float (&f)[8]) { reinterpret_cast<uint4*>(y + row * D)[i] = pack8(f); });
 }
 
 // dx = a * g - x * c * mean(g * x) (+ gres), g = w * dy;  c = a^3 (form 0) or a^2 / rms (form 1); gres is the gradient
@@ -807,78 +796,27 @@ __device__ __forceinline__ float delayed_scale(float* hist, int slots, int cur, 
   return fmax / a;
 }
 
-// RMSNorm whose output goes out as e4m3 (no bf16 copy): q = sat(w * x * a * scale)
-template <int VPT>
-__global__ void __launch_bounds__(512, VPT == 1 ? 4 : 2)
-rmsnorm_fwd_fp8_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, uint8_t* __restrict__ q,
-                       float* __restrict__ a_out, int T, int D, float eps, int form, float* __restrict__ hist, int slots,
-                       int cur, float* __restrict__ scale_inv) {
-  __shared__ float red[2][32];
+// RMSNorm whose output goes out as e4m3 (no bf16 copy): q = sat(w * x * a * scale).  Blocks walk over rows, so that each hands in its largest
+// value once.
+template <int V, int W>
+__global__ void __launch_bounds__(norm_block(W))
+rmsnorm_fwd_fp8_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, uint8_t* __restrict__ q, float* __restrict__ a_out, int T, int D,
+                       float eps, int form, float* __restrict__ hist, int slots, int cur, float* __restrict__ scale_inv) {
+  __shared__ float red[2][W];
   const float scale = delayed_scale(hist, slots, cur, scale_inv, 448.f);
-  const int nv = D >> 3;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  uint4 wv[VPT], xn[VPT];
-#pragma unroll
-  for (int v = 0; v < VPT; ++v) {
-    const int i = threadIdx.x + v * blockDim.x;
-    wv[v] = i < nv ? reinterpret_cast<const uint4*>(w)[i] : make_uint4(0, 0, 0, 0);
-    xn[v] = make_uint4(0, 0, 0, 0);
-  }
-  size_t row = blockIdx.x;
-  if (row < (size_t)T) {
-#pragma unroll
-    for (int v = 0; v < VPT; ++v) {
-      const int i = threadIdx.x + v * blockDim.x;
-      if (i < nv) xn[v] = reinterpret_cast<const uint4*>(x + row * D)[i];
-    }
-  }
   float m = 0.f;
   int it = 0;
-  for (; row < (size_t)T; row += gridDim.x, ++it) {
-    uint4 xc[VPT];
+  for (size_t row = (size_t)blockIdx.x * norm_rows(W) + threadIdx.x / (32 * W); row < (size_t)T; row += (size_t)gridDim.x * norm_rows(W), ++it)
+    norm_row<V, W>(x, w, a_out, row, D, eps, form, red[it & 1], [&](int i, float (&f)[8]) {
 #pragma unroll
-    for (int v = 0; v < VPT; ++v) xc[v] = xn[v];
-    const size_t nxt = row + gridDim.x;
-    if (nxt < (size_t)T) {
-#pragma unroll
-      for (int v = 0; v < VPT; ++v) {
-        const int i = threadIdx.x + v * blockDim.x;
-        if (i < nv) xn[v] = reinterpret_cast<const uint4*>(x + nxt * D)[i];
+      for (int j = 0; j < 8; ++j) {
+        f[j] = __bfloat162float(__float2bfloat16_rn(f[j]));          // the value the un-fused path would have stored as bf16
+        m = fmaxf(m, fabsf(f[j]));
       }
-    }
-    float ss = 0.f;
-#pragma unroll
-    for (int v = 0; v < VPT; ++v) {
-      float f[8]; unpack8(xc[v], f);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
-    }
-    ss = warp_sum(ss);
-    float* rr = red[it & 1];
-    if (lane == 0) rr[wid] = ss;
-    __syncthreads();
-    float tot = lane < nw ? rr[lane] : 0.f;
-    tot = warp_sum(tot);
-    const float mean = tot / D;
-    const float a = form == 0 ? rsqrtf(mean + eps) : 1.f / (sqrtf(mean) + eps);
-    if (threadIdx.x == 0) a_out[row] = a;
-#pragma unroll
-    for (int v = 0; v < VPT; ++v) {
-      const int i = threadIdx.x + v * blockDim.x;
-      if (i < nv) {
-        float f[8], g[8]; unpack8(xc[v], f); unpack8(wv[v], g);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          // the value the un-fused path would have stored as bf16
-          f[j] = __bfloat162float(__float2bfloat16_rn(f[j] * a * g[j]));
-          m = fmaxf(m, fabsf(f[j]));
-        }
-        reinterpret_cast<uint2*>(q + row * D)[i] = quant8(f, scale, 0);
-      }
-    }
-  }
+      reinterpret_cast<uint2*>(q + row * D)[i] = quant8(f, scale, 0);
+    });
   m = warp_max(m);
-  if (lane == 0 && m > 0.f) atomicMax(reinterpret_cast<unsigned int*>(hist + cur), __float_as_uint(m));
+  if ((threadIdx.x & 31) == 0 && m > 0.f) atomicMax(reinterpret_cast<unsigned int*>(hist + cur), __float_as_uint(m));
 }
 
 // gated activation with e4m3 output: q [T, F] = sat(act(a) * b * scale) for ab [T, 2F] = [a | b]; F % 16 == 0, each
@@ -963,8 +901,8 @@ static inline int grid_for(size_t work, int threads, int cap = sb::num_sms() * 1
 
 using namespace sb;
 
-// Threads of a norm block for rows of nv 16-byte vectors, and blocks for T rows: `warps` of them per SM at most, at most 16 blocks.
-// (Forward, T = 8192, us: D = 1024 12.4 -> 10.3, D = 256 10.3 -> 6.2 against four blocks per SM whatever their size.)
+// Threads of a block of the norm's backward for rows of nv 16-byte vectors, and blocks for T rows: `warps` of them per SM at most, at most 16
+// blocks.
 static int norm_threads(int nv) { return nv >= 512 ? 512 : nv <= 64 ? 64 : (nv + 31) / 32 * 32; }
 static int norm_grid(int T, int threads, int warps) {
   const int per_sm = warps * 32 / threads < 16 ? warps * 32 / threads : 16, cap = sb::num_sms() * per_sm;
@@ -975,16 +913,16 @@ extern "C" int sb_rmsnorm_fwd(const void* x, const void* w, void* y, float* a_ou
                               cudaStream_t st) {
   if (D % 8) return -1;
   if (T == 0) return 0;
-  const int nv = D / 8;
-  const int threads = norm_threads(nv);
-  const int vpt = (nv + threads - 1) / threads;
-  const int grid = norm_grid(T, threads, vpt == 1 ? 64 : 4 * threads / 32);
-#define LAUNCH(V) rmsnorm_fwd_kernel<V><<<grid, threads, 0, st>>>((const bf16*)x, (const bf16*)w, (bf16*)y, a_out, T, D, eps, form)
-  if (vpt <= 1) LAUNCH(1);
-  else if (vpt <= 2) LAUNCH(2);
-  else if (vpt <= 4) LAUNCH(4);
-  else return -3;
-#undef LAUNCH
+  if (D > 16384) return -3;
+  auto go = [&](auto* kern, int W) {
+    kern<<<(T + norm_rows(W) - 1) / norm_rows(W), norm_block(W), 0, st>>>((const bf16*)x, (const bf16*)w, (bf16*)y, a_out, T, D, eps, form);
+  };
+  if (D <= 512) go(rmsnorm_fwd_kernel<2, 1>, 1);
+  else if (D <= 1024) go(rmsnorm_fwd_kernel<4, 1>, 1);
+  else if (D <= 2048) go(rmsnorm_fwd_kernel<8, 1>, 1);
+  else if (D <= 4096) go(rmsnorm_fwd_kernel<4, 4>, 4);
+  else if (D <= 8192) go(rmsnorm_fwd_kernel<8, 4>, 4);
+  else go(rmsnorm_fwd_kernel<8, 8>, 8);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -1168,16 +1106,18 @@ extern "C" int sb_rmsnorm_fwd_fp8(const void* x, const void* w, void* q, float* 
                                   float* hist, int slots, int cur, float* scale_inv, cudaStream_t st) {
   if ((D % 8) || slots < 3 || cur < 0 || cur >= slots) return -1;
   if (T == 0) return 0;
-  const int nv = D / 8;
-  const int threads = norm_threads(nv);
-  const int vpt = (nv + threads - 1) / threads;
-  const int grid = norm_grid(T, threads, vpt == 1 ? 64 : 4 * threads / 32);
-#define LAUNCH(V) rmsnorm_fwd_fp8_kernel<V><<<grid, threads, 0, st>>>((const bf16*)x, (const bf16*)w, (uint8_t*)q, a_out, T, D, eps, form, hist, slots, cur, scale_inv)
-  if (vpt <= 1) LAUNCH(1);
-  else if (vpt <= 2) LAUNCH(2);
-  else if (vpt <= 4) LAUNCH(4);
-  else return -3;
-#undef LAUNCH
+  if (D > 16384) return -3;
+  auto go = [&](auto* kern, int W, int per_sm) {
+    const int need = (T + norm_rows(W) - 1) / norm_rows(W), cap = sb::num_sms() * per_sm;
+    kern<<<need < cap ? need : cap, norm_block(W), 0, st>>>((const bf16*)x, (const bf16*)w, (uint8_t*)q, a_out, T, D, eps, form, hist, slots, cur,
+                                                              scale_inv);
+  };
+  if (D <= 512) go(rmsnorm_fwd_fp8_kernel<2, 1>, 1, 8);      // more blocks wait for each other's atomic maximum: 12.2 us
+  else if (D <= 1024) go(rmsnorm_fwd_fp8_kernel<4, 1>, 1, 8);
+  else if (D <= 2048) go(rmsnorm_fwd_fp8_kernel<8, 1>, 1, 5);
+  else if (D <= 4096) go(rmsnorm_fwd_fp8_kernel<4, 4>, 4, 8);
+  else if (D <= 8192) go(rmsnorm_fwd_fp8_kernel<8, 4>, 4, 5);
+  else go(rmsnorm_fwd_fp8_kernel<8, 8>, 8, 2);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
