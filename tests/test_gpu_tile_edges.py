@@ -626,3 +626,31 @@ def test_gemm_narrow_tiles_in_turn(M, N, K, width, a_mn, b_mn, fp8):
         cuda_ops.gemm(a.t().contiguous() if a_mn else a, b.t().contiguous() if b_mn else b, out, a_mn, b_mn)
     cuda_ops.check_status()
     _close(out, a.float() @ b.float().t(), 4e-3, "gemm")  # fp32 accumulation, one bf16 rounding: 2^-9
+
+
+# the forward norm takes four rows of one warp to a block, or a row to a block of four or eight warps: the widths at which that changes and the
+# next one up, rows that fill the last block of four and rows that do not
+@pytest.mark.parametrize("form", ["te", "classic"])
+@pytest.mark.parametrize("D", [8, 264, 512, 520, 1024, 1032, 2048, 2056, 4096, 4104, 8192, 8200, 16384])
+@pytest.mark.parametrize("T", [1, 3, 4, 5, 3001])
+def test_norm_rows_and_widths(T, D, form):
+    from savanna_b200.ops import cuda_ops
+    torch.manual_seed(T + D)
+    x, w = torch.randn(T + 1, D, device=DEV).to(BF), (1 + 0.1 * torch.randn(D, device=DEV)).to(BF)
+    x[T] = float("nan")                                   # the row behind the last one
+    _, _, a, y = cuda_ops._rmsnorm_fwd(x[:T], w, 1e-6, 0 if form == "te" else 1)
+    ms = x[:T].double().pow(2).mean(-1)
+    want_a = (ms + 1e-6).rsqrt() if form == "te" else 1 / (ms.sqrt() + 1e-6)
+    # a lane adds up to 64 squares, then 8 more sums: 72 * 2^-24, halved by the root, and two ulp of the root itself
+    assert ((a.double() - want_a).abs() / want_a).max() < 2.5e-6
+    _close(y, x[:T].double() * want_a[:, None] * w.double(), 2.0 ** -8, "y")   # one bf16 rounding, 2^-9
+
+    # one byte out: the bf16 result under the scale that the history gives (its maximum, 3, outside this call's two slots)
+    hist, si = torch.tensor([3.0, 0.5, 0.0, 9.0], device=DEV), torch.empty(1, device=DEV)
+    q, a8 = torch.full((T + 1, D), 0x55, device=DEV, dtype=torch.uint8), torch.empty(T, device=DEV)
+    rc = cuda_ops.require().sb_rmsnorm_fwd_fp8(x.data_ptr(), w.data_ptr(), q.data_ptr(), a8.data_ptr(), T, D, 1e-6, 0 if form == "te" else 1,
+                                               hist.data_ptr(), 4, 2, si.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    assert rc == 0 and torch.equal(a8, a) and (q[T] == 0x55).all()
+    got, want = q[:T].view(torch.float8_e4m3fn).float() * (3.0 / 448), y.float().clamp(-3, 3)
+    assert ((got - want).abs() <= 2.0 ** -4 * 1.00001 * want.abs() + 2.0 ** -10 * 3 / 448).all()     # half a step of e4m3; below 2^-6 2^-10
+    assert hist.tolist() == [3.0, 0.5, y.float().abs().max().item(), 0.0]
