@@ -15,11 +15,19 @@
 // MN-major tiles are fetched as 64x64 boxes so that the shared-memory image is the canonical
 // MN-major 128B-swizzle layout (64-element blocks LBO apart, 8-row groups SBO apart).
 //
+// Every launch is a programmatic dependent of the kernel before it: the launch, the barriers, the tensor memory and the descriptors of a
+// GEMM are ready when the last block of that kernel leaves, and all its warps wait there for the kernel's results before they touch memory.
+// Back to back, us: [2048 x 512] K = 256 6.2 -> 3.9, [768 x 256] K = 2048 9.3 -> 7.3, [1024 x 2048] K = 2048 12.4 -> 9.8,
+// [8192 x 4096] K = 512 35.1 -> 32.9, [512 x 4096] K = 8192 31 -> 28.4.  A GEMM does not let its successor start before its own last CTA
+// ends (let_next_start): the CTAs of a successor of one wave then took whatever SMs were idle, and the last of these sizes 31.4, probably
+// because neighbouring tiles no longer met in one half of the L2 cache (CTA pairs would gain 0.5 of 33).
+//
 // All waits are bounded (sm100.cuh); on a timeout the kernel records a status word, every role unwinds,
 // TMEM is freed and the kernel returns.
 #include <cuda_fp8.h>
 
 #include "entries.h"
+#include "pdl.cuh"
 #include "sm100.cuh"
 
 namespace sb {
@@ -199,6 +207,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  wait_for_previous();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -385,6 +394,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   cluster_wait();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  wait_for_previous();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (both CTAs)
@@ -700,6 +710,26 @@ static int chosen_tile(int M, int N, int sms, bool one_byte, bool b_mn, int max_
   return g_pair_mode == 3 ? pick_tile(M, N, sms, one_byte && b_mn) : 0;
 }
 
+// A launch in clusters of `cluster` CTAs, as a programmatic dependent of the kernel before it (see the kernels' wait_for_previous).
+static int launch_behind(void (*kern)(const CUtensorMap, const CUtensorMap, GemmParams), int grid, int cluster, int smem, cudaStream_t stream,
+                         const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p) {
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(NUM_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  if (cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p) == cudaSuccess) return 0;
+  (void)cudaGetLastError();              // reported here, as in launch_chained
+  return -6;
+}
+
 // Launch the single-CTA kernel with tile width BNT.
 template <int EB, int BNT>
 static int launch_single(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, int a_mn, int b_mn, int max_ctas,
@@ -719,8 +749,7 @@ static int launch_single(const CUtensorMap& tmA, const CUtensorMap& tmB, const G
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess) return -5;
     attr_set[idx] = true;
   }
-  kern<<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(tmA, tmB, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -6;
+  return launch_behind(kern, grid, 1, SMEM_BYTES, stream, tmA, tmB, p);
 }
 
 // Launch the CTA-pair kernel (cluster of 2) on tensor maps whose boxes are 128 rows (K-major) / 128-byte MN boxes.
@@ -741,17 +770,7 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const Gem
   const int tiles = ((p.M + 255) / 256) * ((p.N + BN - 1) / BN);
   int pairs = g_num_sms / 2;
   if (tiles < pairs) pairs = tiles;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2 * pairs);
-  cfg.blockDim = dim3(NUM_THREADS);
-  cfg.dynamicSmemBytes = P_SMEM_BYTES;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p) == cudaSuccess ? 0 : -6;
+  return launch_behind(kern, 2 * pairs, 2, P_SMEM_BYTES, stream, tmA, tmB, p);
 }
 
 }  // namespace sb
@@ -832,17 +851,7 @@ extern "C" int sb_gemm_fp8_glu(const void* A, const void* W12, void* AB, void* Q
   const int tiles = ((M + 255) / 256) * (F / 128);
   int pairs = g_num_sms / 2;
   if (tiles < pairs) pairs = tiles;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2 * pairs);
-  cfg.blockDim = dim3(NUM_THREADS);
-  cfg.dynamicSmemBytes = P_SMEM_BYTES;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p) == cudaSuccess ? 0 : -6;
+  return launch_behind(kern, 2 * pairs, 2, P_SMEM_BYTES, stream, tmA, tmB, p);
 }
 
 // Input-gradient product of the gated MLP's output projection with the gate backward in the epilogue (GLU = 2):
@@ -874,17 +883,7 @@ extern "C" int sb_gemm_fp8_glu_bwd(const void* G, const void* W3, const void* AB
   const int tiles = ((M + 255) / 256) * ((F + BN - 1) / BN);
   int pairs = g_num_sms / 2;
   if (tiles < pairs) pairs = tiles;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2 * pairs);
-  cfg.blockDim = dim3(NUM_THREADS);
-  cfg.dynamicSmemBytes = P_SMEM_BYTES;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p) == cudaSuccess ? 0 : -6;
+  return launch_behind(kern, 2 * pairs, 2, P_SMEM_BYTES, stream, tmA, tmB, p);
 }
 
 // fp8 GEMM: C[M,N] (bf16) = alpha * A * B^T (+bias) (+residual) (+C) with one-byte operands (e4m3 = 0 / e5m2 = 1) and

@@ -654,3 +654,39 @@ def test_norm_rows_and_widths(T, D, form):
     got, want = q[:T].view(torch.float8_e4m3fn).float() * (3.0 / 448), y.float().clamp(-3, 3)
     assert ((got - want).abs() <= 2.0 ** -4 * 1.00001 * want.abs() + 2.0 ** -10 * 3 / 448).all()     # half a step of e4m3; below 2^-6 2^-10
     assert hist.tolist() == [3.0, 0.5, y.float().abs().max().item(), 0.0]
+
+
+@pytest.mark.parametrize("M,N,K", [(64, 64, 64), (999, 1024, 264), (512, 4096, 4096), (8192, 512, 512), (8192, 2048, 256)])
+@pytest.mark.parametrize("captured", [False, True])
+def test_gemm_behind_the_kernel_that_feeds_it(M, N, K, captured):
+    """A GEMM is launched while the kernel before it still runs: what it reads (operands, residual, C) and writes over is what it would be
+    with the device idle between the launches, behind other kernels, another GEMM and a memset, eagerly and in a graph."""
+    from savanna_b200.ops import cuda_ops
+    torch.manual_seed(M + K)
+    x, w, v = (torch.randn(*s, device=DEV).to(BF) for s in ((M, K), (N, K), (K, N)))
+    a, y, z, c = torch.empty_like(x), torch.empty(M, N, device=DEV, dtype=BF), torch.empty(M, K, device=DEV, dtype=BF), torch.empty(M, N, device=DEV, dtype=BF)
+
+    def steps(between=lambda: None):
+        for i in range(4):
+            torch.mul(x, 1.0 + 0.5 * i, out=a); between()
+            cuda_ops.gemm(a, w, y); between()
+            cuda_ops.gemm(y, v, z); between()                        # [M, N] x [K, N]^T
+            torch.add(z, a, out=a); between()
+            c.zero_(); between()
+            cuda_ops.gemm(a, w, c, residual=y); between()            # the residual is two kernels old
+            cuda_ops.gemm(x, w, c, accumulate=True); between()
+            torch.mul(c, 0.01, out=y); between()
+    for t in (a, y, z, c):
+        t.zero_()
+    steps(torch.cuda.synchronize)
+    want = [t.clone() for t in (a, y, z, c)]
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            steps()
+    for _ in range(3):
+        for t in (a, y, z, c):
+            t.fill_(float("nan"))
+        graph.replay() if captured else steps()
+        assert all(torch.equal(p, q) for p, q in zip((a, y, z, c), want))
+    cuda_ops.check_status()
