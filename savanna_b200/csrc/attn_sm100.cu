@@ -16,8 +16,13 @@
 //   warps 2-5   softmax of tile 0, warps 6-9 of tile 1: row max, exp2, row sum, P as bf16 into swizzled shared
 //               memory, rescale of O in TMEM only when the running maximum grew by more than 2^8
 //
+// Forward, backward and the rotary kernel are programmatic dependents of the kernels before them: launch, barriers and tensor memory are
+// ready when the last block of those leaves.  Rotary embedding and forward of two sequences of 1333, 16 heads: 41.9 -> 38.0 us a call; letting
+// the attention start earlier still, as soon as the last rotary blocks run, gains nothing more (38.1).
+//
 // Every wait is bounded (sm100.cuh); on a timeout the CTA records a status code, frees TMEM and returns.
 #include "entries.h"
+#include "pdl.cuh"
 #include "sm100.cuh"
 
 namespace sb {
@@ -151,6 +156,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  wait_for_previous();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -509,6 +515,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  wait_for_previous();
   constexpr uint32_t T_S = 0, T_DP = 128, T_DQ = 192, T_DV = 256, T_DK = 384;
 
   if (warp == 0) {
@@ -857,6 +864,7 @@ __device__ __forceinline__ void rope_row(const RopeArgs& a, const RopeSide& d, i
 
 __global__ void __launch_bounds__(256)
 attn_rope_kernel(const RopeArgs a) {
+  wait_for_previous();
   const RopeSide& d = a.side[blockIdx.z];
   if (d.f32) rope_row<true>(a, d, blockIdx.x, blockIdx.y);
   else rope_row<false>(a, d, blockIdx.x, blockIdx.y);
@@ -960,9 +968,7 @@ extern "C" int sb_attn_fwd(const void* q, const void* k, const void* v, void* ou
   // measured gain at 128 MB, and nothing to gain at 256 MB.
   p.heads_fast = causal && (long long)B * H * Lk * HD * 4 <= (128LL << 20) && qblocks <= 65535 && B <= 65535;
   const dim3 grid = p.heads_fast ? dim3(H, B, qblocks) : dim3(qblocks, H, B);
-  if (g_fwd_p_tmem) attn_fwd_kernel<true><<<grid, FWD_THREADS, FWD_SMEM, stream>>>(tq, tk, tv, p);
-  else attn_fwd_kernel<false><<<grid, FWD_THREADS, FWD_SMEM, stream>>>(tq, tk, tv, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -6;
+  return launch_chained(false, g_fwd_p_tmem ? attn_fwd_kernel<true> : attn_fwd_kernel<false>, grid, FWD_THREADS, FWD_SMEM, stream, tq, tk, tv, p) ? -6 : 0;
 }
 
 // Attention backward.  go/q/out [B, Lq, H, 128], k/v [B, Lk, H, 128] (bf16, strided as in the forward); lse and the
@@ -1017,8 +1023,7 @@ extern "C" int sb_attn_bwd(const void* go, const void* q, const void* k, const v
               {dk_str[0], dk_str[1], dk_str[2]}, {dv_str[0], dv_str[1], dv_str[2]}, B, H, Lq, Lk,
               causal, scale * 1.4426950408889634f, scale, status};
   dim3 grid((Lk + BK - 1) / BK, H, B);
-  if (g_p_tmem) attn_bwd_kernel<true><<<grid, BWD_THREADS, BWD_SMEM, stream>>>(tq, tk, tv, tg, tdq, p);
-  else attn_bwd_kernel<false><<<grid, BWD_THREADS, BWD_SMEM, stream>>>(tq, tk, tv, tg, tdq, p);
+  if (launch_chained(false, g_p_tmem ? attn_bwd_kernel<true> : attn_bwd_kernel<false>, grid, BWD_THREADS, BWD_SMEM, stream, tq, tk, tv, tg, tdq, p)) return -6;
   const long long orows = (long long)B * Lq * H;
   // dq == null: the caller keeps accumulating into dq_acc over several calls (ring attention) and casts at the end
   if (dq)
@@ -1047,8 +1052,7 @@ extern "C" int sb_attn_rope(const void* const* src, void* const* dst, const long
   }
   a.cs = cs; a.sn = sn; a.H = H; a.rd = rd; a.sign = inverse ? -1.f : 1.f;
   const int cols = (H + ROPE_HEADS - 1) / ROPE_HEADS;          // head columns of a block
-  attn_rope_kernel<<<dim3(L, B, n), cols < 4 ? 32 : (cols > 32 ? 256 : cols * 8), 0, stream>>>(a);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return sb::launch_chained(false, attn_rope_kernel, dim3(L, B, n), cols < 4 ? 32 : (cols > 32 ? 256 : cols * 8), 0, stream, a);
 }
 
 // ------------------------------------------------------------------------------------ merging partial attention results

@@ -690,3 +690,33 @@ def test_gemm_behind_the_kernel_that_feeds_it(M, N, K, captured):
         graph.replay() if captured else steps()
         assert all(torch.equal(p, q) for p, q in zip((a, y, z, c), want))
     cuda_ops.check_status()
+
+
+@pytest.mark.parametrize("B,L,H", [(1, 1, 1), (2, 333, 3), (1, 1024, 8), (1, 2600, 16)])
+@pytest.mark.parametrize("captured", [False, True])
+def test_attention_behind_the_kernel_that_feeds_it(B, L, H, captured):
+    """As above for the rotary embedding of what a kernel has just written and the attention behind it."""
+    torch.manual_seed(B * L + H)
+    x = (torch.randn(B, L, 3 * H * 128, device=DEV) * 0.5).to(BF)
+    cos, sin = (f(torch.rand(L, 128, device=DEV) * 6) for f in (torch.cos, torch.sin))
+    qkv = torch.empty_like(x)
+
+    def steps(between=lambda: None):
+        out = []
+        for i in range(4):
+            torch.mul(x, 1.0 - 0.2 * i, out=qkv); between()
+            out.append(ops.attention_packed(qkv.view(B, L, H, 384), cos, sin)); between()
+        return out
+    with torch.no_grad():
+        want = [t.clone() for t in steps(torch.cuda.synchronize)]
+        if captured:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                got = steps()
+        for _ in range(3):
+            qkv.fill_(float("nan"))
+            if captured:
+                graph.replay()
+            else:
+                got = steps()
+            assert all(torch.equal(a, b) for a, b in zip(got, want))
