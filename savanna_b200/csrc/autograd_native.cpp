@@ -4,8 +4,8 @@
 // ctypes calls, an autograd.Function forward and backward per operator) the host needed 80 to 150 us for a forward and backward whose
 // kernels take 50.  Here the same allocations and the same entry points are called from one C++ frame, the backward runs in the engine
 // without the interpreter lock, and a gated MLP or a norm with its projection is one node instead of four or two.
-// Forward and backward, us, Python -> here: gated Hyena-MR [3 x 777 x 512] 120 -> 80 (an operator that does nothing costs 53 through the engine),
-// gated MLP [999 x 1024] 329 -> 168, a step of a four-operator model, 2 x 1024 tokens of 256 channels, 4181 -> 2201.
+// Forward and backward, us, Python -> here: gated Hyena-MR [3 x 777 x 512] 120 -> 77 (an operator that does nothing costs 53 through the engine),
+// gated MLP [999 x 1024] 329 -> 130, a step of a four-operator model, 2 x 1024 tokens of 256 channels, 4181 -> 2200.
 // Python keeps what decides (ops/cuda_ops.py: shapes, types, which operator), and the oracle.
 //
 // Nothing is cached between calls but the entry points (entries.h) and the address of the per-device status word.

@@ -691,9 +691,9 @@ static int g_pair_mode = 3;      // CTA-pair kernel 0: never, 1: for one-byte op
 // outputs with too few 256 x 256 tiles to fill the chip.  Compared are waves times cycles of a tile per 128-byte k-block: an SM
 // pair spends 512 on its 256 x 256 tile; a single-CTA tile is bound by shared memory, which takes both operands in and reads
 // them once (32 KB a k-block: 256 cycles and their share of latency, 320; 24 KB: 260).  A narrower tile has to win by an
-// eighth, because it reads its operands more often.  Kernel times, us, pair -> chosen: [999 x 1024] K = 5632 34 -> 18 and
-// K = 2816 27 -> 13 (64 wide), [512 x 4096] K = 8192 48 -> 37 (128 wide), weight gradients of a 256-wide model 18 -> 9;
-// [999 x 5632] K = 1024 keeps the pair (128 wide: 17 against 15 to 20).  `b_box128`: B comes in boxes of 128 columns (one-byte
+// eighth, because it reads its operands more often.  Back to back, us, pair -> chosen: [999 x 1024] K = 5632 32 -> 16 and
+// K = 2816 20 -> 11 (64 wide), [512 x 4096] K = 8192 48 -> 28 (128 wide), weight gradients of a 256-wide model 18 -> 7;
+// [999 x 5632] K = 1024 keeps the pair (17 with either).  `b_box128`: B comes in boxes of 128 columns (one-byte
 // MN-major operand), 64 is not possible.
 static int pick_tile(int M, int N, int sms, bool b_box128) {
   const long long m1 = (M + 127) / 128, m2 = (M + 255) / 256;
