@@ -656,6 +656,34 @@ def test_norm_rows_and_widths(T, D, form):
     assert hist.tolist() == [3.0, 0.5, y.float().abs().max().item(), 0.0]
 
 
+def _sum_of_squares(x):
+    """fp32 sum of a row's squares (exact products of bf16 values) in the order of a block with a thread for each of 512 vectors of eight."""
+    T, D = x.shape
+    p = torch.nn.functional.pad(x.float().square(), (0, -D % 4096)).view(T, -1, 512, 8)
+    s = torch.zeros(T, 512, device=x.device)
+    for g in range(p.shape[1]):
+        for j in range(8):
+            s = s + p[:, g, :, j]
+    s = s.view(T, 16, 32)
+    for o in (16, 8, 4, 2, 1):
+        s = s[..., :o] + s[..., o:2 * o]
+    s = s[..., 0]
+    for o in (8, 4, 2, 1):
+        s = s[..., :o] + s[..., o:2 * o]
+    return s[:, 0]
+
+
+@pytest.mark.parametrize("D", [8, 256, 264, 512, 520, 768, 1024, 1032, 2040, 2048, 2056, 4096, 4104, 8192, 8200, 12296, 16384])
+@pytest.mark.parametrize("T", [1, 5, 149, 1500])
+def test_norm_sums_have_one_order_at_all_widths(T, D):
+    from savanna_b200.ops import cuda_ops
+    torch.manual_seed(T + D)
+    x, w = torch.randn(T, D, device=DEV).to(BF), torch.ones(D, device=DEV, dtype=BF)
+    _, _, a, _ = cuda_ops._rmsnorm_fwd(x, w, 1e-6, 1)
+    mean = _sum_of_squares(x) / torch.full((T,), float(D), device=DEV)
+    assert torch.equal(a, torch.ones_like(mean) / (mean.sqrt() + torch.full_like(mean, 1e-6)))
+
+
 @pytest.mark.parametrize("M,N,K", [(64, 64, 64), (999, 1024, 264), (512, 4096, 4096), (8192, 512, 512), (8192, 2048, 256)])
 @pytest.mark.parametrize("captured", [False, True])
 def test_gemm_behind_the_kernel_that_feeds_it(M, N, K, captured):
