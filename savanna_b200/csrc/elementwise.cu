@@ -72,19 +72,21 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 // ------------------------------------------------------------------------------------ RMSNorm
 // form 0 ("te"):      y = w * x * rsqrt(mean(x^2) + eps);       saved a = rsqrt(mean + eps)
 // form 1 ("classic"): y = w * x / (sqrt(mean(x^2)) + eps);      saved a = 1 / (rms + eps)
-// W warps take a row, all of whose loads (V 16-byte vectors a lane) are under way before the first sum; a row of up to 2048 is one warp's and
-// needs no barrier.  A persistent block of 512 threads per row had one vector per thread in flight and two barriers a row.  T = 8192, back to
-// back, us: D = 4096 29.0 -> 22.9 (copying 20.5), 2048 16.5 -> 10.5, 1024 10.4 -> 6.7, 256 6.3 -> 4.3, 8192 47.2 -> 45.9; one byte out 33.9 ->
-// 22.8, 18.6 -> 12.4, 15.4 -> 8.8, 8.3 -> 8.3, 49.3 -> 45.2.  One warp for a row of 4096 took 33: its arithmetic is serial.  OUT takes vector i
-// of the row as eight scaled values.
+// W warps take a row, all of whose loads (V 16-byte vectors a lane) are under way before the first sum.  A persistent block of up to 512 threads
+// per row had one vector per thread in flight and two barriers a row.  T = 8192, in a graph, us, that block -> here: D = 4096 27.1 -> 22.1, 2048
+// 13.7 -> 8.5, 1024 7.7 -> 5.4, 256 4.7 -> 2.5, 8192 45.0 -> 44.4; one byte out 31.6 -> 21.7, 17.1 -> 11.1, 13.1 -> 7.8, 6.1 -> 5.8, 46.9 -> 43.6.
+// What bounds many rows is memory (copying 8192 x 4096 takes 20.5), a few rows the chain of one row: load, sum, barrier, store.  OUT takes
+// vector i of the row as eight scaled values.
 template <int V, int W, class OUT>
 __device__ __forceinline__ void norm_row(const bf16* __restrict__ x, const bf16* __restrict__ w, float* __restrict__ a_out, size_t row, int D,
                                          float eps, int form, float (&red)[16], OUT out) {
   const int lane = threadIdx.x & 31, warp = W > 1 ? (threadIdx.x >> 5) % W : 0, i0 = warp * 32 + lane, nv = D >> 3;
   const uint4* src = reinterpret_cast<const uint4*>(x + row * D);
-  uint4 xv[V];
+  uint4 xv[V], wv[V];                                  // the weights as well where a lane has few: a row alone on its SM waits once
 #pragma unroll
   for (int v = 0; v < V; ++v) xv[v] = i0 + 32 * W * v < nv ? src[i0 + 32 * W * v] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+  for (int v = 0; v < V; ++v) wv[v] = V <= 2 && i0 + 32 * W * v < nv ? __ldg(reinterpret_cast<const uint4*>(w) + i0 + 32 * W * v) : make_uint4(0, 0, 0, 0);
   // The additions come in the order of a block of up to 512 threads with a vector each, whatever V and W: vectors 512 apart add up in one sum,
   // 32 neighbouring sums as in warp_sum, the (up to 16) results the same way.  One long sum per lane has 1.4 times the error at D = 2048
   // (6.2e-8), and a row's bits would change with the rule that picks V and W.  A lane has P sums, a block N results: the last two steps are
@@ -124,7 +126,7 @@ __device__ __forceinline__ void norm_row(const bf16* __restrict__ x, const bf16*
   for (int v = 0; v < V; ++v) {
     const int i = i0 + 32 * W * v;
     if (i < nv) {
-      float f[8], g[8]; unpack8(xv[v], f); unpack8(__ldg(reinterpret_cast<const uint4*>(w) + i), g);
+      float f[8], g[8]; unpack8(xv[v], f); unpack8(V <= 2 ? wv[v] : __ldg(reinterpret_cast<const uint4*>(w) + i), g);
 #pragma unroll
       for (int j = 0; j < 8; ++j) f[j] = f[j] * a * g[j];
       out(i, f);
@@ -953,11 +955,18 @@ extern "C" int sb_rmsnorm_fwd(const void* x, const void* w, void* y, float* a_ou
   auto go = [&](auto* kern, int W) {
     kern<<<(T + norm_rows(W) - 1) / norm_rows(W), norm_block(W), 0, st>>>((const bf16*)x, (const bf16*)w, (bf16*)y, a_out, T, D, eps, form);
   };
-  if (D <= 512) go(rmsnorm_fwd_kernel<2, 1>, 1);
-  else if (D <= 1024) go(rmsnorm_fwd_kernel<4, 1>, 1);
-  else if (D <= 2048) go(rmsnorm_fwd_kernel<8, 1>, 1);
-  else if (D <= 4096) go(rmsnorm_fwd_kernel<4, 4>, 4);
-  else if (D <= 8192) go(rmsnorm_fwd_kernel<8, 4>, 4);
+  // A row is spread over so many warps that a lane has two vectors for as long as all its blocks run at once (five of 2 x 8, three of 2 x 16 per
+  // SM); with more rows than that fewer warps, and so fewer barriers and results to add, do better.  us, other form -> chosen: D = 1024 200 rows
+  // 2.6 -> 1.7, 4096 rows 3.7 -> 3.4; D = 2048 (8 x 1 -> 2 x 4 at any number) 200 rows 3.6 -> 1.9, 8192 rows 9.0 -> 8.5, 32768 rows 43.4 -> 41.7;
+  // D = 4096 200 rows 2.8 -> 2.1, 888 rows 3.6 -> 3.4; D = 8192 200 rows 3.8 -> 2.7, 888 rows 5.3 -> 5.0, 1184 rows (two waves of either)
+  // 7.5 -> 6.6.
+  const int per_sm = (T + sb::num_sms() - 1) / sb::num_sms();
+  if (D <= 256) go(rmsnorm_fwd_kernel<1, 1>, 1);
+  else if (D <= 512) go(rmsnorm_fwd_kernel<2, 1>, 1);
+  else if (D <= 1024) per_sm <= 20 ? go(rmsnorm_fwd_kernel<2, 2>, 2) : go(rmsnorm_fwd_kernel<4, 1>, 1);
+  else if (D <= 2048) go(rmsnorm_fwd_kernel<2, 4>, 4);
+  else if (D <= 4096) per_sm <= 5 ? go(rmsnorm_fwd_kernel<2, 8>, 8) : go(rmsnorm_fwd_kernel<4, 4>, 4);
+  else if (D <= 8192) per_sm <= 3 || per_sm == 7 || per_sm == 8 ? go(rmsnorm_fwd_kernel<2, 16>, 16) : go(rmsnorm_fwd_kernel<8, 4>, 4);
   else go(rmsnorm_fwd_kernel<8, 8>, 8);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -1143,16 +1152,21 @@ extern "C" int sb_rmsnorm_fwd_fp8(const void* x, const void* w, void* q, float* 
   if ((D % 8) || slots < 3 || cur < 0 || cur >= slots) return -1;
   if (T == 0) return 0;
   if (D > 16384) return -3;
-  auto go = [&](auto* kern, int W, int per_sm) {
-    const int need = (T + norm_rows(W) - 1) / norm_rows(W), cap = sb::num_sms() * per_sm;
+  auto go = [&](auto* kern, int W, int blocks) {                // at most so many per SM
+    const int need = (T + norm_rows(W) - 1) / norm_rows(W), cap = sb::num_sms() * blocks;
     kern<<<need < cap ? need : cap, norm_block(W), 0, st>>>((const bf16*)x, (const bf16*)w, (uint8_t*)q, a_out, T, D, eps, form, hist, slots, cur,
                                                               scale_inv);
   };
-  if (D <= 512) go(rmsnorm_fwd_fp8_kernel<2, 1>, 1, 8);      // more blocks wait for each other's atomic maximum: 12.2 us
-  else if (D <= 1024) go(rmsnorm_fwd_fp8_kernel<4, 1>, 1, 8);
-  else if (D <= 2048) go(rmsnorm_fwd_fp8_kernel<8, 1>, 1, 5);
-  else if (D <= 4096) go(rmsnorm_fwd_fp8_kernel<4, 4>, 4, 8);
-  else if (D <= 8192) go(rmsnorm_fwd_fp8_kernel<8, 4>, 4, 5);
+  // As above; the blocks stay and take row after row, so few of them pay for their atomic maximum and the lines lie lower.  us, other form ->
+  // chosen: D = 1024 200 rows 3.3 -> 2.4, 8192 rows 8.1 -> 7.8; D = 2048 592 rows 4.5 -> 3.8, 1024 rows 5.0 -> 5.0, 8192 rows 12.2 -> 11.1;
+  // D = 4096 148 rows 3.5 -> 3.0, 400 rows 4.5 -> 4.1; D = 8192 148 rows 4.5 -> 4.1, 400 rows 9.1 -> 5.2.
+  const int per_sm = (T + sb::num_sms() - 1) / sb::num_sms();
+  if (D <= 256) go(rmsnorm_fwd_fp8_kernel<1, 1>, 1, 8);      // more blocks wait for each other's atomic maximum: 12.2 us
+  else if (D <= 512) go(rmsnorm_fwd_fp8_kernel<2, 1>, 1, 8);
+  else if (D <= 1024) per_sm <= 20 ? go(rmsnorm_fwd_fp8_kernel<2, 2>, 2, 8) : go(rmsnorm_fwd_fp8_kernel<4, 1>, 1, 8);
+  else if (D <= 2048) per_sm <= 4 ? go(rmsnorm_fwd_fp8_kernel<2, 4>, 4, 8) : go(rmsnorm_fwd_fp8_kernel<8, 1>, 1, 5);
+  else if (D <= 4096) per_sm <= 1 ? go(rmsnorm_fwd_fp8_kernel<2, 8>, 8, 4) : go(rmsnorm_fwd_fp8_kernel<4, 4>, 4, 8);
+  else if (D <= 8192) per_sm <= 1 ? go(rmsnorm_fwd_fp8_kernel<2, 16>, 16, 2) : go(rmsnorm_fwd_fp8_kernel<8, 4>, 4, 5);
   else go(rmsnorm_fwd_fp8_kernel<8, 8>, 8, 2);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }

@@ -628,8 +628,8 @@ def test_gemm_narrow_tiles_in_turn(M, N, K, width, a_mn, b_mn, fp8):
     _close(out, a.float() @ b.float().t(), 4e-3, "gemm")  # fp32 accumulation, one bf16 rounding: 2^-9
 
 
-# the forward norm takes four rows of one warp to a block, or a row to a block of four or eight warps: the widths at which that changes and the
-# next one up, rows that fill the last block of four and rows that do not
+# the forward norm takes four rows of one warp to a block, or a row to a block of 2 to 16 warps, by its width and the rows per SM: the widths at
+# which that changes and the next one up, rows that fill the last block of four and rows that do not, few and many
 @pytest.mark.parametrize("form", ["te", "classic"])
 @pytest.mark.parametrize("D", [8, 264, 512, 520, 1024, 1032, 2048, 2056, 4096, 4104, 8192, 8200, 16384])
 @pytest.mark.parametrize("T", [1, 3, 4, 5, 3001])
@@ -674,7 +674,7 @@ def _sum_of_squares(x):
 
 
 @pytest.mark.parametrize("D", [8, 256, 264, 512, 520, 768, 1024, 1032, 2040, 2048, 2056, 4096, 4104, 8192, 8200, 12296, 16384])
-@pytest.mark.parametrize("T", [1, 5, 149, 1500])
+@pytest.mark.parametrize("T", [1, 5, 149, 741, 1037, 1500, 15000])
 def test_norm_sums_have_one_order_at_all_widths(T, D):
     from savanna_b200.ops import cuda_ops
     torch.manual_seed(T + D)
