@@ -556,7 +556,8 @@ struct HyenaMR : Function<HyenaMR> {
            dh = zeros(hf.sizes(), F32, hf.device()), db = zeros(bf.sizes(), F32, bf.device());
     const bool tc = ctx->saved_data["tc"].toBool();
     if (tc && !hc.defined()) {
-      SB_CALL(sb_mr_umma_bwd, 1, ptr(fc), f32(hf), f32(bf), ptr(gc), out(df), f32o(dh), f32o(db), B, Ln, D, G, K, status_word(fc.device()), stream());
+      const Tensor ba = aligned(bf);       // read in 16-byte vectors; a parameter may lie anywhere in a flat buffer
+      SB_CALL(sb_mr_umma_bwd, 1, ptr(fc), f32(hf), f32(ba), ptr(gc), out(df), f32o(dh), f32o(db), B, Ln, D, G, K, status_word(fc.device()), stream());
     } else if (tc) {
       SB_CALL(sb_mr_tc_bwd, 1, ptr(fc), ptr(hc), f32(hf), f32(bf), ptr(gc), out(df), out(dhalo), f32o(dh), f32o(db), B, Ln, D, G, K, stream());
     } else {

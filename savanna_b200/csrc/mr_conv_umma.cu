@@ -711,11 +711,11 @@ extern "C" int sb_mr_umma_fwd(const void* feat, const float* h, const float* bia
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-// dz like z, dfeat like feat; adds into dh [G, K] and dbias [D], fp32.
+// dz like z, dfeat like feat, bias 16-byte aligned; adds into dh [G, K] and dbias [D], fp32.
 extern "C" int sb_mr_umma_bwd(const void* feat, const float* h, const float* bias, const void* dz, void* dfeat, float* dh, float* dbias,
                               int B, int L, int D, int G, int K, unsigned int* status, cudaStream_t st) {
-  if (!supported(D, G, K) ||
-      ((reinterpret_cast<uintptr_t>(feat) | reinterpret_cast<uintptr_t>(dz) | reinterpret_cast<uintptr_t>(dfeat)) & 15)) return -1;
+  if (!supported(D, G, K) || ((reinterpret_cast<uintptr_t>(feat) | reinterpret_cast<uintptr_t>(dz) | reinterpret_cast<uintptr_t>(dfeat) |
+                               reinterpret_cast<uintptr_t>(bias)) & 15)) return -1;
   if (B <= 0 || L <= 0 || D <= 0) return 0;
   if (cudaFuncSetAttribute(mr_umma_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, B_SMEM) != cudaSuccess) return -5;
   CUtensorMap tf, tz, td;

@@ -169,6 +169,8 @@ class _Sig:
     sb_se_set_bwd_variant = [I]
     sb_conv_set_fwd_variant = [I]
     sb_mr_tc_bwd = [P, P, P, P, P, P, P, P, P, I, I, I, I, I, P]
+    sb_mr_umma_fwd = [P, P, P, P, I, I, I, I, I, P, P]
+    sb_mr_umma_bwd = [P, P, P, P, P, P, P, I, I, I, I, I, P, P]
     sb_li_fwd = [P, P, P, P, P, P, P, P, I, I, I, I, P]
     sb_li_set_variant = [I]
     sb_li_bwd_chunk = [I, I]

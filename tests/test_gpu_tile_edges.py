@@ -231,6 +231,35 @@ def test_mr_fir_tiles_of_128_rows_match_the_16_row_blocks(B, L, D, G, K):
     assert torch.equal(new[0], _mr_grads(None, *a)[0])
 
 
+@pytest.mark.parametrize("off", [1, 2, 3])
+def test_mr_fir_parameters_off_16_byte_boundaries(off):
+    """Taps and bias as views into the middle of a flat buffer, as an optimizer lays them out: the results of aligned copies."""
+    from savanna_b200.ops import cuda_ops
+    torch.manual_seed(off)
+    B, L, D, G, K = 2, 300, 64, 4, 31
+    feat, dz = torch.randn(B, L, 3 * D, device=DEV).to(BF), torch.randn(B, L, D, device=DEV).to(BF)
+    flat = torch.randn(off + D + off + G * K, device=DEV)
+    h, bias = flat[off + D + off:].view(G, K), flat[off:off + D]
+    assert bias.data_ptr() % 16 and h.is_contiguous()
+    got, want = [], []
+    for out, hh, bb in ((got, h, bias), (want, h.clone(), bias.clone())):
+        leaves = [feat.clone().requires_grad_(), hh.detach().requires_grad_(), bb.detach().requires_grad_()]
+        z = ops.hyena_mr_inner(*leaves)
+        z.backward(dz)
+        out += [z.detach()] + [t.grad for t in leaves]
+    _same(got[0], want[0], "z")
+    _same(got[1], want[1], "dfeat")
+    for a, b, what in zip(got[2:], want[2:], ("dh", "dbias")):          # atomic sums: any order
+        _close(a, b, 1e-5, what)
+    # the entry itself takes no such bias (refused on the host, nothing is launched)
+    dfeat, dh, db = torch.empty_like(feat), torch.zeros(G, K, device=DEV), torch.zeros(D, device=DEV)
+    rc = cuda_ops.require().sb_mr_umma_bwd(feat.data_ptr(), h.data_ptr(), bias.data_ptr(), dz.data_ptr(), dfeat.data_ptr(), dh.data_ptr(),
+                                           db.data_ptr(), B, L, D, G, K, cuda_ops.status_word(feat.device).data_ptr(),
+                                           torch.cuda.current_stream().cuda_stream)
+    assert rc == -1
+    cuda_ops.check_status()
+
+
 @pytest.mark.parametrize("bad", [float("nan"), float("inf")])
 @pytest.mark.parametrize("t0", [130, 511])
 def test_mr_fir_non_finite_values_reach_only_what_their_taps_touch(bad, t0):
