@@ -19,8 +19,9 @@
 // operands again (16 tiles: 131).  The backward as one chain of steps per block, with rows kept in registers and T' in shared memory, took
 // 170; with two groups of warps forming u and g, so that registers spill, 123.
 //
-// A Toeplitz product multiplies whole tiles, zero taps included, so an Inf or NaN would spread over its tile and the next: once one has
-// been seen, results that are not finite are formed again tap by tap.
+// A Toeplitz product multiplies whole tiles, zero taps included, so an Inf or NaN would spread over its tile and the next, and into taps whose
+// lag reaches beyond the sequence, where the tap gradient multiplies zero rows: once one has been seen, results that are not finite are
+// formed again, tap by tap or row by row.
 //
 // Halo rows and the context-parallel forms stay with mr_conv_tc.cu, group widths that are not a multiple of 16 with mr_conv.cu.
 #include <cuda.h>
@@ -144,6 +145,32 @@ __device__ __noinline__ float fir_element(const bf16* feat, const bf16* dz, cons
     y += __bfloat162float(__float2bfloat16_rn(h[s])) * __bfloat162float(u);
   }
   return y;
+}
+// The gradient of tap s over rows t0 .. t1 - 1 and the 16 channels from c0 on, by the products that exist: a zero row beyond the sequence times
+// an Inf or NaN has spoilt the sum of the tensor cores.
+__device__ __noinline__ float tap_gradient(const bf16* feat, const bf16* dz, int t0, int t1, int D, int c0, int s) {
+  float sum = 0.f;
+  for (int t = max(t0, s); t < t1 && sum == sum; ++t) {
+    const uint4* f = reinterpret_cast<const uint4*>(feat + (size_t)t * 3 * D + 3 * c0);
+    const uint4* q = reinterpret_cast<const uint4*>(feat + (size_t)(t - s) * 3 * D + 3 * c0);
+    const uint4* z = reinterpret_cast<const uint4*>(dz + (size_t)t * D + c0);
+    float row = 0.f;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      uint4 fv[3], qv[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) { fv[k] = f[3 * half + k]; qv[k] = q[3 * half + k]; }
+      const uint4 zv = z[half];
+      const uint32_t *fw = reinterpret_cast<const uint32_t*>(fv), *qw = reinterpret_cast<const uint32_t*>(qv), *zw = reinterpret_cast<const uint32_t*>(&zv);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint32_t g = gate_g(fw[3 * k], fw[3 * k + 1], zw[k]), u = gate_u(qw[3 * k], qw[3 * k + 1], qw[3 * k + 2]);
+        row += lo(g) * lo(u) + hi(g) * hi(u);
+      }
+    }
+    sum += row;
+  }
+  return sum;
 }
 
 __device__ __forceinline__ void linger() {            // copies of this block may still be in flight: not before they have landed
@@ -641,6 +668,11 @@ mr_umma_bwd_kernel(const __grid_constant__ CUtensorMap tmF, const __grid_constan
         for (int k = 0; k < 24; ++k) {
           const int d = r - 16 * (k / 6) - 128 + 32 * (k % 6);
           if (d >= -31 && d <= 15) sum += sDiag[k * 48 + d + 31];
+        }
+        if (*bad && !finite(sum)) {
+          const int D = p.slabs * CH;
+          sum = tap_gradient(p.feat + (size_t)un.b * p.L * 3 * D, p.dz + (size_t)un.b * p.L * D, un.j0 * TILE, min((un.j0 + un.n) * TILE, p.L), D,
+                             un.slab * CH, r);
         }
         atomicAdd(p.dh + (size_t)(un.slab * CH / p.dg) * p.K + r, sum);
       }

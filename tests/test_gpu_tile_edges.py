@@ -285,6 +285,29 @@ def test_mr_fir_non_finite_values_reach_only_what_their_taps_touch(bad, t0):
         _close(df[:, part, c], want[:, part, c], 2 ** -7, "dfeat beyond the taps")
 
 
+# near both ends of the sequence and of its tiles and of the runs of tiles that a block takes
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("L,t0", [(900, 0), (900, 50), (900, 127), (900, 128), (900, 768), (900, 801), (900, 850), (900, 899), (130, 125), (128, 127),
+                                  (20, 3), (4096, 4090)])
+def test_mr_fir_non_finite_values_reach_only_the_taps_they_meet(bad, L, t0):
+    """A non-finite u[t0] meets g[t0 + s] in the gradient of tap s, a non-finite g[t0] meets u[t0 - s]: taps without such a row stay as they are."""
+    torch.manual_seed(17)
+    B, D, G, K, c = 2, 64, 4, 100, 21
+    a = [torch.randn(B, L, 3 * D, device=DEV).to(BF), torch.randn(G, K, device=DEV) / 11, torch.randn(D, device=DEV),
+         torch.randn(B, L, D, device=DEV).to(BF)]
+    g, others, taps = c // (D // G), [i for i in range(D) if i != c], torch.arange(K, device=DEV)
+    v0, clean = a[0][1, t0, 3 * c + 2].item(), _mr_grads(None, *a)
+    for what, met in (("u", taps <= L - 1 - t0), ("g", taps <= t0)):
+        a[0][1, t0, 3 * c + 2] = bad if what == "u" else v0
+        a[3][1, t0, c] = a[3][1, t0, c] if what == "u" else bad
+        dh, db = _mr_grads(None, *a)[2:]
+        _close(dh[[i for i in range(G) if i != g]], clean[2][[i for i in range(G) if i != g]], 1e-5, what + ": dh, other groups")
+        _close(db[others], clean[3][others], 1e-5, what + ": dbias, other channels")
+        assert not dh[g, met].isfinite().any() and not db[c].isfinite()
+        if (~met).any():        # formed again row by row: at most 128 x 2 rows x 16 products in another order
+            _close(dh[g, ~met], clean[2][g, ~met], 1e-5, what + ": dh, taps that meet no such value")
+
+
 @pytest.mark.parametrize("D,offset,tiled", [(24, 0, True), (136, 0, True), (20, 0, False), (24, 1, False)])
 @pytest.mark.parametrize("state", [False, True])
 def test_li_c_entries(D, offset, tiled, state):
