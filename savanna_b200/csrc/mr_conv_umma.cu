@@ -137,7 +137,7 @@ __device__ __forceinline__ bool finite(float v) { return (__float_as_uint(v) & 0
 template <int DIR>
 __device__ __noinline__ float fir_element(const bf16* feat, const bf16* dz, const float* h, int K, int L, int D, int t, int c) {
   float y = 0.f;
-  for (int s = 0; s < K; ++s) {
+  for (int s = 0; s < K && y == y; ++s) {              // a NaN stays one: a row of them takes one step an element, not K
     const int q = t + DIR * s;
     if (q < 0 || q >= L) break;
     const bf16* f = feat + (size_t)q * 3 * D + 3 * c;
