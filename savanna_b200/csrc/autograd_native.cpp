@@ -529,12 +529,20 @@ struct HyenaSE : Function<HyenaSE> {
 
 // Tensor-core kernels when a 16-channel slab shares one filter (mr_conv_umma.cu, with halo rows mr_conv_tc.cu), else the CUDA-core
 // kernels (mr_conv.cu), whose backward wants the convolution itself (kept when `train`).
+//
+// A forward without halo rows stays with mr_conv_tc.cu where that is faster: its products grow with the filter in steps of 16 taps, those of
+// mr_conv_umma.cu are 256 taps whatever K is.  us, mr_conv_tc.cu / mr_conv_umma.cu: K = 16 8192 x 1024 16.9 / 19.5, 2 x 1237 x 1024 8.9 / 10.0,
+// 300 x 4096 7.6 / 8.1, 600 x 1024 6.9 / 6.4; K = 31 17.5 / 19.4, 9.3 / 10.1, 7.9 / 8.1, 7.3 / 6.5, 1237 x 1024 8.0 / 7.4; K = 40 18.6 / 19.4, 10.4 /
+// 10.1, 9.0 / 8.1; one row of 256 3.9 / 4.7 (K = 3).  The backward is faster on mr_conv_umma.cu at every size measured (K = 3, one row 12.7 -> 10.4).
+bool short_filter(int64_t B, int64_t Ln, int64_t D, int64_t K) {
+  return K <= 32 && B <= 65535 && (Ln <= 32 || B * Ln * D >= 65536 * std::max<int64_t>(K, 16));
+}
 struct HyenaMR : Function<HyenaMR> {
   static Tensor forward(AutogradContext* ctx, const Tensor& feat, const Tensor& h, const Tensor& bias, const OptTensor& halo, bool train) {
     const int B = feat.size(0), Ln = feat.size(1), D = feat.size(2) / 3, G = h.size(0), K = h.size(1);
     Tensor fc = aligned(feat), hc = aligned(halo), hf = f32c(h), bf = f32c(bias), z = alloc({B, Ln, D}, BF16, feat.device()), y;
     const bool tc = (D / G) % 16 == 0 && D % 8 == 0;
-    if (tc && !hc.defined()) {
+    if (tc && !hc.defined() && !short_filter(B, Ln, D, K)) {
       SB_CALL(sb_mr_umma_fwd, 1, ptr(fc), f32(hf), f32(bf), out(z), B, Ln, D, G, K, status_word(feat.device()), stream());
     } else if (tc) {
       SB_CALL(sb_mr_tc_fwd, 1, ptr(fc), ptr(hc), f32(hf), f32(bf), out(z), B, Ln, D, G, K, stream());

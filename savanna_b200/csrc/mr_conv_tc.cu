@@ -14,7 +14,7 @@
 //               y recomputed instead of saved
 // Both walk a segment of 32-row tiles of 64 channels.
 //
-// Calls without halo rows take mr_conv_umma.cu, which is faster at every size.
+// Calls without halo rows take mr_conv_umma.cu, but for forwards with short filters (autograd_native.cpp: short_filter).
 // Measured at B = 1, L = 8192, D = 4096, K = 128 on a B200 (us; in brackets the kernels these replace, which staged 128-row
 // tiles with their halo, or rebuilt 72 fragment registers from global memory for every 64-row tile): forward 73 (108),
 // backward 260 (475), forward and backward with their host side 589 -> 333.  Copying the data takes 40 and 71 us.  What bounds

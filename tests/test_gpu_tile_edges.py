@@ -231,6 +231,23 @@ def test_mr_fir_tiles_of_128_rows_match_the_16_row_blocks(B, L, D, G, K):
     assert torch.equal(new[0], _mr_grads(None, *a)[0])
 
 
+# one row and one more than 32; filters of 32 and 33 taps; sizes on both sides of where a short filter keeps the 16-row blocks
+@pytest.mark.parametrize("B,L,D,G,K,blocks", [(1, 1, 32, 2, 3, True), (2, 32, 48, 3, 32, True), (1, 33, 48, 3, 32, False), (1, 32, 48, 3, 33, False),
+                                              (1, 1023, 1024, 64, 7, False), (1, 1024, 1024, 64, 16, True), (1, 1024, 1024, 64, 17, False),
+                                              (4, 2048, 256, 4, 32, True), (4, 2047, 256, 4, 32, False), (4, 2048, 256, 4, 33, False)])
+def test_mr_fir_short_filters(B, L, D, G, K, blocks):
+    torch.manual_seed(L + K)
+    feat, h, bias = torch.randn(B, L, 3 * D, device=DEV).to(BF), torch.randn(G, K, device=DEV) / math.sqrt(K), torch.randn(D, device=DEV)
+    with torch.no_grad():
+        z, tiled = ops.hyena_mr_inner(feat, h, bias), ops.hyena_mr_inner(feat, h, bias, torch.zeros(B, K - 1, 3 * D, device=DEV, dtype=BF))
+    if blocks:
+        assert torch.equal(z, tiled)
+    _close(z, tiled, 2 ** -7, "z")                        # fp32 sums in another order, one rounding of the result either way
+    want = ref.hyena_mr_inner(feat.double(), h.to(BF).double(), bias.double())
+    # u rounded to bf16: y is off by 2^-9 / sqrt(3) of its rms (one sigma); that and x1 at most 4.5 sigma; one rounding of the result, 2^-9
+    _close(z, want, 4.5 * 4.5 * 2 ** -9 / 3 ** 0.5, "z")
+
+
 @pytest.mark.parametrize("off", [1, 2, 3])
 def test_mr_fir_parameters_off_16_byte_boundaries(off):
     """Taps and bias as views into the middle of a flat buffer, as an optimizer lays them out: the results of aligned copies."""
