@@ -35,7 +35,6 @@ constexpr int TILE_BYTES = 128 * HD * 2;   // 32 KB: two boxes of 16 KB
 constexpr int BOX_BYTES = 128 * 128;       // 16 KB: 128 rows of 128 bytes
 constexpr int FWD_THREADS = 320;
 constexpr int FWD_SMEM = 7 * TILE_BYTES + 256 + 1024;
-constexpr uint32_t ST_ATTN = 0x20;      // status codes 0x20.. identify attention waits
 
 struct FwdParams {
   __nv_bfloat16* out;        // [B, Lq, H, 128]

@@ -44,7 +44,6 @@ constexpr int TMEM_COLS = 512;
 constexpr int T_SFA = 256, T_SFB = 260;            // TMEM columns of the scale words (A: 4, B: 8)
 constexpr int NUM_THREADS = 192;
 constexpr int GROUP_M = 16;
-constexpr uint32_t ST_MX = 0x60;
 
 struct Params {
   __nv_bfloat16* C;

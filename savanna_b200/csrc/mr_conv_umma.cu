@@ -41,7 +41,6 @@ constexpr int THREADS = 320, ROWS_T = 256;        // forward: 8 warps of rows, l
 constexpr uint32_t IMG = TILE * CH * 2;           // a tile of u or g: 4 KB
 constexpr uint32_t RING = 5 * IMG;                // slots 0..3 and a second copy of slot 0 behind slot 3, so that pairs are contiguous
 constexpr uint32_t FEAT_B = TILE * 3 * CH * 2, DZ_B = TILE * CH * 2;
-constexpr uint32_t ST_MR = 0x60;
 
 // barriers (offsets in the barrier block)
 enum { RAW_FULL = 0, RAW_FREE = 32, UG_READY = 64, ACC_FULL = 72, ABORT = 80, TMEM_SLOT = 84, BAD = 88, BAR_BYTES = 128 };
@@ -220,7 +219,7 @@ mr_umma_fwd_kernel(const __grid_constant__ CUtensorMap tmF, const __grid_constan
         for (int i = -1; i < un.n && ok; ++i) {
           const int w = i & 1;
           const uint32_t c = cnt[w]++, slot = 2 * w + (c & 1);
-          if (c >= 2) ok = mbar_wait(bar + RAW_FREE + 8 * slot, ((c >> 1) & 1) ^ 1u, abort_flag, p.status, ST_MR);
+          if (c >= 2) ok = mbar_wait(bar + RAW_FREE + 8 * slot, ((c >> 1) & 1) ^ 1u, abort_flag, p.status, ST_MR_FWD);
           if (!ok) break;
           mbar_expect_tx(bar + RAW_FULL + 8 * slot, FEAT_B);
           tma_load_3d(base + F_RAW + slot * FEAT_B, &tmF, 3 * CH * un.slab, (un.j0 + i) * TILE, un.b, bar + RAW_FULL + 8 * slot);
@@ -236,7 +235,7 @@ mr_umma_fwd_kernel(const __grid_constant__ CUtensorMap tmF, const __grid_constan
       for (int u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
         const Unit un = unit_of(p, u);
         for (int k = 1; k <= (un.n + 1) / 2; ++k, ++gs) {
-          ok = mbar_wait(bar + UG_READY, gs & 1u, abort_flag, p.status, ST_MR + 1);
+          ok = mbar_wait(bar + UG_READY, gs & 1u, abort_flag, p.status, ST_MR_FWD + 1);
           if (!ok) break;
           tc_fence_after();
           const uint32_t prev = base + ((2 * k - 3) & 3) * IMG, cur = base + ((2 * k - 2) & 3) * IMG;
@@ -274,7 +273,7 @@ mr_umma_fwd_kernel(const __grid_constant__ CUtensorMap tmF, const __grid_constan
         uint4 x[6];
         if (live) {
           const uint32_t slot = 2 * w + (cnt & 1);
-          if (ok) ok = mbar_wait(bar + RAW_FULL + 8 * slot, (cnt >> 1) & 1u, abort_flag, p.status, ST_MR + 2);
+          if (ok) ok = mbar_wait(bar + RAW_FULL + 8 * slot, (cnt >> 1) & 1u, abort_flag, p.status, ST_MR_FWD + 2);
           ++cnt;
           const uint32_t src = base + F_RAW + slot * FEAT_B + r * 96u;
 #pragma unroll
@@ -301,7 +300,7 @@ mr_umma_fwd_kernel(const __grid_constant__ CUtensorMap tmF, const __grid_constan
         tc_fence_before();
         if (k > 0) {
           mbar_arrive(bar + UG_READY);
-          if (ok) ok = mbar_wait(bar + ACC_FULL, ga & 1u, abort_flag, p.status, ST_MR + 3);
+          if (ok) ok = mbar_wait(bar + ACC_FULL, ga & 1u, abort_flag, p.status, ST_MR_FWD + 3);
           ++ga;
         }
         if (k == 0 || !live) continue;
@@ -391,7 +390,7 @@ mr_umma_bwd_kernel(const __grid_constant__ CUtensorMap tmF, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  auto wait = [&](uint32_t b, uint32_t phase, uint32_t code) { return mbar_wait(bar + b, phase & 1u, abort_flag, p.status, ST_MR + code); };
+  auto wait = [&](uint32_t b, uint32_t phase, uint32_t code) { return mbar_wait(bar + b, phase & 1u, abort_flag, p.status, ST_MR_BWD + code); };
 
   // Tiles of a run by index i: 0 is the one before it, 1 .. n its own, n + 1 the one behind it.  q counts the tiles of all runs, o the
   // runs' own tiles, v the runs.

@@ -18,6 +18,8 @@ constexpr unsigned long long WAIT_BUDGET_NS = 1500ull * 1000ull * 1000ull;  // 1
 // status word layout: 0 = ok; otherwise (code << 24) | detail
 enum : uint32_t { ST_OK = 0, ST_TIMEOUT_FULL = 1, ST_TIMEOUT_EMPTY = 2, ST_TIMEOUT_TMEM_FULL = 3,
                   ST_TIMEOUT_TMEM_EMPTY = 4, ST_TIMEOUT_PEER = 5, ST_BAD_ARG = 6 };
+// First codes of kernels that number their own waits, all of them here: the word names one kernel.
+enum : uint32_t { ST_ATTN = 0x20, ST_MX = 0x60, ST_MR_FWD = 0x70, ST_MR_BWD = 0x80 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
