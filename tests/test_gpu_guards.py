@@ -77,6 +77,14 @@ def test_hyena_mr(K, L):
     _run(lambda a, c, d, e: ops.hyena_mr_inner(a, c, d, e), feat, h, bias, halo)
 
 
+@pytest.mark.parametrize("B,L,D,G,K", [(2, 333, 256, 16, 128), (1, 70, 48, 3, 37), (3, 1, 16, 1, 33), (1, 2049, 64, 1, 128), (2, 40, 1024, 64, 7)])
+def test_hyena_mr_without_halo(B, L, D, G, K):
+    feat = torch.randn(B, L, 3 * D, device=DEV, dtype=BF, requires_grad=True)
+    h = (torch.randn(G, K, device=DEV) / math.sqrt(K)).requires_grad_()
+    bias = torch.randn(D, device=DEV, requires_grad=True)
+    _run(lambda a, c, d: ops.hyena_mr_inner(a, c, d), feat, h, bias)
+
+
 @pytest.mark.parametrize("L,D", [(300, 128), (1300, 160)])
 def test_hyena_li(L, D):
     O = 16

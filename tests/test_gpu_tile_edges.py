@@ -278,7 +278,7 @@ def test_mr_fir_parameters_off_16_byte_boundaries(off):
 
 
 @pytest.mark.parametrize("bad", [float("nan"), float("inf")])
-@pytest.mark.parametrize("t0", [130, 511])
+@pytest.mark.parametrize("t0", [130, 200, 511])
 def test_mr_fir_non_finite_values_reach_only_what_their_taps_touch(bad, t0):
     torch.manual_seed(13)
     B, L, D, G, K, c = 1, 900, 64, 4, 100, 21
@@ -300,6 +300,7 @@ def test_mr_fir_non_finite_values_reach_only_what_their_taps_touch(bad, t0):
     assert not df[0, t0 - K + 1:t0 + 1, c, 1:].isfinite().any()
     for part in (slice(0, t0 - K + 1), slice(t0 + K, L)):
         _close(df[:, part, c], want[:, part, c], 2 ** -7, "dfeat beyond the taps")
+    _close(df[:, t0 + 1:, c, 1:], want[:, t0 + 1:, c, 1:], 2 ** -7, "gradients of x2 and v behind the value")     # anticausal: not reached
 
 
 # near both ends of the sequence and of its tiles and of the runs of tiles that a block takes
@@ -321,7 +322,7 @@ def test_mr_fir_non_finite_values_reach_only_the_taps_they_meet(bad, L, t0):
         _close(dh[[i for i in range(G) if i != g]], clean[2][[i for i in range(G) if i != g]], 1e-5, what + ": dh, other groups")
         _close(db[others], clean[3][others], 1e-5, what + ": dbias, other channels")
         assert not dh[g, met].isfinite().any() and not db[c].isfinite()
-        if (~met).any():        # formed again row by row: at most 128 x 2 rows x 16 products in another order
+        if (~met).any():                                  # formed again row by row: fp32 sums in another order
             _close(dh[g, ~met], clean[2][g, ~met], 1e-5, what + ": dh, taps that meet no such value")
 
 
@@ -756,8 +757,9 @@ def test_norm_sums_have_one_order_at_all_widths(T, D):
 @pytest.mark.parametrize("M,N,K", [(64, 64, 64), (999, 1024, 264), (512, 4096, 4096), (8192, 512, 512), (8192, 2048, 256)])
 @pytest.mark.parametrize("captured", [False, True])
 def test_gemm_behind_the_kernel_that_feeds_it(M, N, K, captured):
-    """A GEMM is launched while the kernel before it still runs: what it reads (operands, residual, C) and writes over is what it would be
-    with the device idle between the launches, behind other kernels, another GEMM and a memset, eagerly and in a graph."""
+    """A GEMM's launch does not wait for the kernel before it to be done: what it reads (operands, residual, C) and writes over is what it
+    would be with the device idle between the launches, behind other kernels and another GEMM, eagerly and in a graph.  None of these lets
+    its successor start before its own last block ends; the kernels of the next test do."""
     from savanna_b200.ops import cuda_ops
     torch.manual_seed(M + K)
     x, w, v = (torch.randn(*s, device=DEV).to(BF) for s in ((M, K), (N, K), (K, N)))
@@ -817,3 +819,99 @@ def test_attention_behind_the_kernel_that_feeds_it(B, L, H, captured):
             else:
                 got = steps()
             assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_dependents_of_a_kernel_that_lets_them_start(captured):
+    """The scan on short chunks lets the next kernel start as soon as all its own blocks run, so the dependent is there long before its
+    operand is: GEMMs that read the scan's output as A, in either layout, as residual and as C, the rotary kernel with the attention behind
+    it, and a GEMM behind a memset.  Buffers hold NaN before each pass, so a value read too early shows."""
+    import ctypes
+    from savanna_b200.ops import cuda_ops
+    torch.manual_seed(23)
+    lib, memset = cuda_ops.require(), ctypes.CDLL("libcudart.so.12").cudaMemsetAsync
+    memset.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_size_t, ctypes.c_void_p]
+    L, H, N, TC = 2048, 3, 512, 64
+    D = 3 * H * 128
+    feat = (torch.randn(L, 3 * D, device=DEV) * 0.7).to(BF)
+    gamma, p = (torch.rand(D, 16, device=DEV) * 0.09 + 0.01).log(), -torch.ones(D, 16, device=DEV)
+    R, bias = torch.randn(D, 16, device=DEV) / 4, torch.randn(D, device=DEV)
+    modal, S = torch.empty(4 * D * 16, device=DEV), torch.empty(L // TC * D * 16, device=DEV)
+    w, x, v = (torch.randn(*s, device=DEV).to(BF) for s in ((N, D), (L, N), (D, N)))
+    cos, sin = (f(torch.rand(L, 128, device=DEV) * 6) for f in (torch.cos, torch.sin))
+    scans = [torch.empty(L, D, device=DEV, dtype=BF) for _ in range(5)]
+    outs = [torch.empty(*s, device=DEV, dtype=BF) for s in ((L, N), (D, N), (L, D), (L, D))]
+
+    def scan(z):
+        rc = lib.sb_li_fwd_tiled(feat.data_ptr(), gamma.data_ptr(), p.data_ptr(), R.data_ptr(), bias.data_ptr(), None, None, modal.data_ptr(),
+                                 S.data_ptr(), z.data_ptr(), 1, L, D, 16, TC, torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+
+    def steps(between=lambda: None):
+        scan(scans[0]); between()
+        cuda_ops.gemm(scans[0], w, outs[0]); between()
+        scan(scans[1]); between()
+        cuda_ops.gemm(scans[1], x, outs[1], a_mn=True, b_mn=True); between()        # as a weight gradient
+        scan(scans[2]); between()
+        cuda_ops.gemm(x, v, outs[2], residual=scans[2]); between()
+        scan(scans[3]); between()
+        cuda_ops.gemm(x, v, scans[3], accumulate=True); between()
+        scan(scans[4]); between()
+        att = ops.attention_packed(scans[4].view(1, L, H, 384), cos, sin); between()
+        assert memset(outs[3].data_ptr(), 0, outs[3].nbytes, torch.cuda.current_stream().cuda_stream) == 0; between()
+        cuda_ops.gemm(x, v, outs[3], accumulate=True); between()
+        return att
+
+    with torch.no_grad():
+        att = steps(torch.cuda.synchronize)
+        want = [t.clone() for t in (*scans, *outs, att)]
+        assert all(t.isfinite().all() for t in want)
+        if captured:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                att = steps()
+        for _ in range(5):
+            for t in (*scans, *outs):
+                t.fill_(float("nan"))
+            if captured:
+                graph.replay()
+            else:
+                att = steps()
+            assert all(torch.equal(a, b) for a, b in zip((*scans, *outs, att), want))
+    cuda_ops.check_status()
+
+
+@pytest.mark.parametrize("B,L,H", [(1, 1, 1), (2, 333, 3), (1, 1024, 8)])
+@pytest.mark.parametrize("captured", [False, True])
+def test_attention_backward_behind_the_kernels_that_feed_it(B, L, H, captured):
+    """The backward's main kernel, a dependent of the one that forms its row statistics, behind a kernel that writes the output's gradient."""
+    torch.manual_seed(B * L + H)
+    qkv = (torch.randn(B, L, H, 384, device=DEV) * 0.5).to(BF).requires_grad_()
+    cos, sin = (f(torch.rand(L, 128, device=DEV) * 6) for f in (torch.cos, torch.sin))
+    g0, go = torch.randn(B, L, H, 128, device=DEV).to(BF), torch.empty(B, L, H, 128, device=DEV, dtype=BF)
+
+    def steps(between=lambda: None):
+        grads = []
+        for i in range(3):
+            out = ops.attention_packed(qkv, cos, sin); between()
+            torch.mul(g0, 1.0 - 0.3 * i, out=go); between()
+            grads += torch.autograd.grad(out, qkv, go); between()
+        return grads
+    stream = torch.cuda.Stream()                          # captures want a stream of their own, warmed up
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        want = [t.clone() for t in steps(torch.cuda.synchronize)]
+    torch.cuda.synchronize()
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            got = steps()
+    for _ in range(3):
+        go.fill_(float("nan"))
+        if captured:
+            graph.replay()
+        else:
+            got = steps()
+        torch.cuda.synchronize()
+        for a, b in zip(got, want):                       # dq adds up over key blocks in any order, in fp32: one rounding, either side
+            _close(a, b, 2 ** -8, "dqkv")
