@@ -15,8 +15,9 @@
 // MN-major tiles are fetched as 64x64 boxes so that the shared-memory image is the canonical
 // MN-major 128B-swizzle layout (64-element blocks LBO apart, 8-row groups SBO apart).
 //
-// Every launch is a programmatic dependent of the kernel before it: the launch, the barriers, the tensor memory and the descriptors of a
-// GEMM are ready when the last block of that kernel leaves, and all its warps wait there for the kernel's results before they touch memory.
+// Every launch is a programmatic dependent of the kernel before it (pdl.cuh, the second kind): the launch, the barriers, the tensor memory and
+// the descriptors of a GEMM are ready when the last block of that kernel leaves, or long before where that kernel lets its successor start
+// early, and all its warps wait for the kernel's results before they touch memory.
 // Back to back, us: [2048 x 512] K = 256 6.2 -> 3.9, [768 x 256] K = 2048 9.3 -> 7.3, [1024 x 2048] K = 2048 12.4 -> 9.8,
 // [8192 x 4096] K = 512 35.1 -> 32.9, [512 x 4096] K = 8192 31 -> 28.4.  A GEMM does not let its successor start before its own last CTA
 // ends (let_next_start): the CTAs of a successor of one wave then took whatever SMs were idle, and the last of these sizes 31.4, probably
@@ -77,7 +78,7 @@ __device__ __forceinline__ void tile_coords(int tile, int m_tiles, int n_tiles, 
 }
 
 // A warp's 32 rows x 32 columns on their way to memory.  A lane holds a row (that is how tensor memory is read); stored from there, a
-// 16-byte store touches 32 lines and half a sector of each, and a 256 x 256 tile took 8 us to leave: more than the products of a tile need
+// 16-byte store touches 32 lines and half a sector of each, and a 256 x 256 tile took 5.6 us to leave: more than the products of a tile need
 // at K = 512.  Through 2 KB of shared memory four lanes store 64 consecutive bytes of a row, eight rows at a time.  The 16-byte chunks of a row
 // are permuted so that neither side meets a bank twice.
 constexpr int EPI_WARP_BYTES = 32 * 64, EPI_BYTES = EPI_WARPS * EPI_WARP_BYTES;

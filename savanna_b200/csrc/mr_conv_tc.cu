@@ -16,8 +16,8 @@
 //
 // Calls without halo rows take mr_conv_umma.cu, but for forwards with short filters (autograd_native.cpp: short_filter).
 // Measured at B = 1, L = 8192, D = 4096, K = 128 on a B200 (us; in brackets the kernels these replace, which staged 128-row
-// tiles with their halo, or rebuilt 72 fragment registers from global memory for every 64-row tile): forward 73 (108),
-// backward 260 (475), forward and backward with their host side 589 -> 333.  Copying the data takes 40 and 71 us.  What bounds
+// tiles with their halo, or rebuilt 72 fragment registers from global memory for every 64-row tile): forward 71 (108),
+// backward 256 (475), forward and backward with their host side 589 -> 333.  Copying the data takes 40 and 71 us.  What bounds
 // them now is issue slots and latency at four (two) blocks per SM: of the first streaming version (106 and 411 us) most of
 // the difference was address arithmetic of the copies, unpacking to fp32 for the gates, and spilled fragments.
 // Rows before the sequence start come from `halo` [B, K-1, 3D] (context-parallel shards) or are zero; the

@@ -11,13 +11,16 @@
 //
 // The Toeplitz product takes twice the multiplications of the 16-row blocks of mr_conv_tc.cu, whose mma.sync fragments were bound by issue
 // slots and their latency (a thousand warp instructions for 16 x 16 outputs of the backward; here 350).  Measured on a B200, B = 1, L = 8192, D = 4096,
-// K = 128, us: forward 71 -> 65 (copying the data 41), backward 256 -> 107 (72); [3 x 777 x 512] 12 -> 10 and 36 -> 17, [2 x 1024 x 256]
-// 11 -> 7 and 29 -> 15, [2048 x 2048] of 64 taps 14.5 -> 14.5 and 45 -> 23.  What bounds them now is memory: DRAM moves the case's own bytes
-// and nothing else (ncu: 269 MB read, 163 written in the backward; 45 % of the issue slots), at 5.2 TB/s while all blocks run, and the second
-// wave of runs is three quarters full.  Runs of equal length keep neighbouring blocks, which share 128-byte lines, at the same rows: dealing
-// the tiles out evenly instead (132 -> 116 tiles a block) took 207 for the backward.  Shorter runs pay for their first tiles and for the
-// operands again (16 tiles: 131).  The backward as one chain of steps per block, with rows kept in registers and T' in shared memory, took
-// 170; with two groups of warps forming u and g, so that registers spill, 123.
+// K = 128, us, L2 flushed: forward 71 -> 65 (copying the data 41), backward 256 -> 107 (72); [3 x 777 x 512] 12 -> 10 and 36 -> 17, [2 x 1024 x 256]
+// 11 -> 7 and 29 -> 15, [2048 x 2048] of 64 taps 14.5 -> 14.5 and 45 -> 23.  Forwards of up to 32 taps are mostly faster there (autograd_native.cpp:
+// short_filter).  What bounds these is memory: DRAM moves the case's own bytes and nothing else (ncu: backward 269 MB read, 163 written, 48 % of
+// the issue slots, forward 202, 45 and 35 %).  The backward has one block per SM, moves 5.2 TB/s while all of them run, and its 256 runs are
+// 1.7 waves; the forward has two, and its 256 runs are one wave that leaves 40 SMs with one block.  Runs of equal length keep neighbouring blocks, which
+// share 128-byte lines, at the same rows: dealing the tiles out evenly instead (132 -> 116 tiles a block) took 207 for the backward.  Shorter runs
+// pay for their first tiles and for the operands again (16 tiles: 131).  The backward as one chain of steps per block, with rows kept in
+// registers and T' in shared memory, took 170; with two groups of warps forming u and g, so that registers spill, 123.
+// A run's tap gradient adds up in one accumulator, so the rounding of its fp32 sum grows with the run (32 tiles 1.2e-6, 64 2.4e-6; u and g
+// rounded to bf16 2.3e-3).
 //
 // A Toeplitz product multiplies whole tiles, zero taps included, so an Inf or NaN would spread over its tile and the next, and into taps whose
 // lag reaches beyond the sequence, where the tap gradient multiplies zero rows: once one has been seen, results that are not finite are
@@ -85,8 +88,10 @@ __device__ __forceinline__ void tmem_ld_16(uint32_t taddr, uint32_t (&r)[16]) {
                  "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                : "r"(taddr) : "memory");
 }
-// Volatile, so that it stays in front of the arrival that hands the buffer back to the loader.  That alone is not enough: the arrival does
-// not wait for loads in flight (tiles were overwritten under them), so it comes after a branch on the values.
+// Volatile, so that it stays in front of the arrival that hands the buffer back to the loader.  That alone is not enough: the refill is a write
+// of the async proxy, which the arrival's release does not order behind reads of the generic proxy (tiles were overwritten under loads in
+// flight).  A load is over once its value has been used: the test for Inf and NaN takes in every word that was loaded, and has to stay
+// in front of the arrival.
 __device__ __forceinline__ uint4 lds128(uint32_t a) {
   uint4 v;
   asm volatile("ld.volatile.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
