@@ -140,6 +140,7 @@ class _Sig:
     sb_gemm_bf16 = [P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, P, I, P]
     sb_colsum = [P, P, I, I, P]
     sb_gemm_set_pair_mode = [I]
+    sb_status_word = [P]
     sb_gemm_tile = [I, I, I, I, I, I]
     sb_gemm_fp8 = [P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, I, P, P]
     sb_quantize_fp8 = [P, P, P, P, LL, I, P]
@@ -289,12 +290,25 @@ def _check(rc: int, what: str) -> None:
         raise RuntimeError(f"savanna_b200 kernel `{what}` rejected its arguments or failed to launch (code {rc})")
 
 
+class _Word:
+    """One int32 at a device address, as `torch.as_tensor` takes it."""
+
+    def __init__(self, address):
+        self.__cuda_array_interface__ = {"data": (address, False), "shape": (1,), "typestr": "<i4", "version": 3}
+
+
 def status_word(device) -> torch.Tensor:
-    """Per-device uint32 word the bounded waits of the kernels write when they give up."""
-    key = (device if isinstance(device, torch.device) else torch.device(device)).index or 0
+    """Per-device uint32 word the bounded waits of the kernels write when they give up (csrc/status_word.cu)."""
+    device = device if isinstance(device, torch.device) else torch.device(device)
+    key = device.index or 0
     word = _STATUS.get(key)
+    if word is None and _LIB is None and not os.path.exists(_LIB_PATH):
+        word = _STATUS[key] = torch.zeros(1, dtype=torch.int32, device=device)      # PyTorch backend: nothing writes it
     if word is None:
-        word = _STATUS[key] = _zeros(1, dtype=torch.int32, device=device)
+        address = c_void_p()
+        with torch.cuda.device(key):
+            _check(require().sb_status_word(ctypes.byref(address)), "status_word")
+            word = _STATUS[key] = torch.as_tensor(_Word(address.value), device=torch.device("cuda", key))
     return word
 
 

@@ -1,6 +1,9 @@
 """The C++ autograd functions (csrc/autograd_native.cpp): the nodes that join several operators against the operators one by one, which
 inputs get gradients, tracing, saved-tensor hooks, and what autograd refuses."""
 import itertools
+import os
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -219,3 +222,33 @@ def test_joined_nodes_add_into_marked_gradients(kind, marked):
         assert (a.grad.float() - total).norm() <= 2 ** -8 * total.norm(), i
         assert i not in buffers or a.grad is buffers[i]
     assert all(leaves[i].grad.abs().sum() > 0 for i in range(len(ts)))
+
+
+FIRST_CALL_CAPTURED = """
+import torch
+from savanna_b200 import ops
+from savanna_b200.ops import cuda_ops
+torch.manual_seed(0)
+args = [torch.randn(2, 300, 192, device="cuda").bfloat16(), torch.randn(4, 64, device="cuda") / 8, torch.randn(64, device="cuda")]
+graph = torch.cuda.CUDAGraph()
+with torch.no_grad():
+    with torch.cuda.graph(graph):
+        z = ops.hyena_mr_inner(*args)
+    want = ops.hyena_mr_inner(*args)
+graph.replay()
+assert torch.equal(z, want) and cuda_ops.check_status() == 0
+cuda_ops.status_word(z.device).fill_(7 << 24)
+graph.replay()
+try:
+    cuda_ops.check_status()
+except RuntimeError as e:
+    assert "code 7" in str(e)
+    print("kept")
+"""
+
+
+def test_first_call_of_a_process_under_capture():
+    """The word for timed-out waits is made at the first call that wants it.  Made on the capturing stream, every replay would clear it."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", FIRST_CALL_CAPTURED], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "kept", r.stdout + r.stderr[-2000:]
