@@ -994,8 +994,8 @@ extern "C" int sb_rmsnorm_bwd(const void* x, const void* w, const void* dy, cons
 #define PAIR(R) rmsnorm_bwd_pair_kernel<R><<<grid, threads, ring, st>>>((const bf16*)x, (const bf16*)w, (const bf16*)dy, a_in, (const bf16*)gres, (bf16*)dx, partial, T, D, eps, form)
   if (vpt <= 1) {
     const int ring = 4 * threads * 16 * (gres ? 3 : 2);
-    if (ring > 49152 && (cudaFuncSetAttribute(rmsnorm_bwd_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 512 * 16 * 3) != cudaSuccess ||
-                         cudaFuncSetAttribute(rmsnorm_bwd_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 512 * 16 * 2) != cudaSuccess))
+    if (ring + 512 /*red*/ > 49152 && (cudaFuncSetAttribute(rmsnorm_bwd_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 512 * 16 * 3) != cudaSuccess ||
+                                      cudaFuncSetAttribute(rmsnorm_bwd_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 512 * 16 * 2) != cudaSuccess))
       return -2;
     if (gres) PAIR(true);
     else PAIR(false);

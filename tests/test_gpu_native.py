@@ -252,3 +252,31 @@ def test_first_call_of_a_process_under_capture():
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", FIRST_CALL_CAPTURED], cwd=root, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip() == "kept", r.stdout + r.stderr[-2000:]
+
+
+FIRST_NORM = """
+import sys, torch
+from savanna_b200 import ops
+D, residual = int(sys.argv[1]), sys.argv[2] == "True"
+torch.manual_seed(0)
+x, w = (torch.randn(*s, device="cuda").bfloat16() for s in ((37, D), (D,)))
+x.requires_grad_(), w.requires_grad_()
+y, res = ops.rmsnorm_residual(x, w, 1e-6) if residual else (ops.rmsnorm(x, w, 1e-6), None)
+loss = y.float().pow(2).sum() + (res.float().sum() if residual else 0)
+loss.backward()
+xd, wd = (t.detach().double().requires_grad_() for t in (x, w))
+yd = xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-6) * wd
+(yd.pow(2).sum() + (xd.sum() if residual else 0)).backward()
+for a, b in ((x.grad, xd.grad), (w.grad, wd.grad)):
+    assert (a - b).norm() < 1e-2 * b.norm()
+print("ok")
+"""
+
+
+@pytest.mark.parametrize("D,residual", [(3072, False), (2048, True), (2040, True), (2056, True), (3064, False), (3080, False)])
+def test_norm_backward_as_the_first_of_a_process(D, residual):
+    """A ring of exactly 48 KB, and widths next to it: beside the kernel's own shared memory that is more than a launch gets unasked, and
+    asking lasts for the process, so only a process of its own shows it.  bf16 gradients: 2^-9 each of dy, y and the result."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", FIRST_NORM, str(D), str(residual)], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr[-2000:]
