@@ -1,6 +1,6 @@
 // Memory-bound row / elementwise kernels (bf16 activations, fp32 math): RMSNorm fwd/bwd, gated-MLP
 // activation fwd/bwd, rotate-half RoPE, cross-entropy fwd/bwd, squared-norm reduction, fused Adam.
-// All use 16-byte vector accesses; grids are sized from the problem, row kernels use one CTA per row
+// All use 16-byte vector accesses; grids are sized from the problem, row kernels use one to sixteen warps per row
 // (forward) or a grid-stride over rows with per-thread column ownership (weight-gradient reductions).
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
